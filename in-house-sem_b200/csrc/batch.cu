@@ -475,11 +475,11 @@ void Batch::enqueue(cudaEvent_t tiles_begin, cudaEvent_t tiles_end) {
     CUDA_LAUNCH_CHECK();
   }
   if (n_pv_items > 0) {
-    particle_velocity_batch_kernel<<<n_pv_items, kRecChunk, 0, stream>>>(drec_segs.get(), dpv_items.get());
+    particle_velocity_batch_kernel<<<n_pv_items, kRecThreads, 0, stream>>>(drec_segs.get(), dpv_items.get());
     CUDA_LAUNCH_CHECK();
   }
   if (n_rec_items > 0) {
-    record_batch_kernel<<<n_rec_items, kRecChunk, 0, stream>>>(drec_segs.get(), drec_items.get());
+    record_batch_kernel<<<n_rec_items, kRecThreads, 0, stream>>>(drec_segs.get(), drec_items.get());
     CUDA_LAUNCH_CHECK();
   }
   if (n_energy > 0) {

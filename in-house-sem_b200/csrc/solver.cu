@@ -288,8 +288,10 @@ void Solver::build_receivers(const insem_cuda_problem& p) {
     offsets.push_back(static_cast<int32_t>(points.size()));
     dom.push_back(rc.domain);
     rho.push_back(rc.rho);
-    if (d.medium == INSEM_ACOUSTIC) acoustic.push_back(r);
     const auto qs = host_vec(rc.quantities, rc.n_quantities);
+    // only receivers that record it integrate the particle velocity
+    if (d.medium == INSEM_ACOUSTIC && std::count(qs.begin(), qs.end(), INSEM_Q_PARTICLE_VELOCITY) > 0)
+      acoustic.push_back(r);
     for (int32_t q : qs) {
       TraceInfo ti;
       ti.first_col = static_cast<int32_t>(cols.size());
@@ -594,12 +596,12 @@ void Solver::compute_acceleration(int force_energy, double h, int step_override)
 
 void Solver::observers(int force_energy, int init) {
   if (n_acoustic_rec > 0) {
-    particle_velocity_kernel<<<ceil_div(n_acoustic_rec, 64), 64, 0, stream>>>(
+    particle_velocity_kernel<<<ceil_div(n_acoustic_rec, kRecChunk), kRecThreads, 0, stream>>>(
         receivers_view(), fields_view(), rec_acoustic.get(), n_acoustic_rec, dt, init);
     CUDA_LAUNCH_CHECK();
   }
   if (n_cols > 0) {
-    record_kernel<<<ceil_div(n_cols, 64), 64, 0, stream>>>(receivers_view(), fields_view(), rec_cols.get(), n_cols,
+    record_kernel<<<ceil_div(n_cols, kRecChunk), kRecThreads, 0, stream>>>(receivers_view(), fields_view(), rec_cols.get(), n_cols,
                                                             st, record_every, trace_buf.get(), max_samples);
     CUDA_LAUNCH_CHECK();
   }
@@ -1042,13 +1044,13 @@ void Solver::enqueue_tiled(int par, bool init) {
   ReceiversDev rv = receivers_view();
   rv.points = trec_points.get();
   if (n_acoustic_rec > 0) {
-    particle_velocity_kernel<<<ceil_div(n_acoustic_rec, 64), 64, 0, stream>>>(rv, tiled_fields(par),
+    particle_velocity_kernel<<<ceil_div(n_acoustic_rec, kRecChunk), kRecThreads, 0, stream>>>(rv, tiled_fields(par),
                                                                               rec_acoustic.get(), n_acoustic_rec, dt,
                                                                               init ? 1 : 0);
     CUDA_LAUNCH_CHECK();
   }
   if (n_cols > 0) {
-    record_kernel<<<ceil_div(n_cols, 64), 64, 0, stream>>>(rv, tiled_fields(par), rec_cols.get(), n_cols, st,
+    record_kernel<<<ceil_div(n_cols, kRecChunk), kRecThreads, 0, stream>>>(rv, tiled_fields(par), rec_cols.get(), n_cols, st,
                                                             record_every, trace_buf.get(), max_samples);
     CUDA_LAUNCH_CHECK();
   }

@@ -170,7 +170,10 @@ static __global__ void zero_kernel(int32_t n, const int64_t* __restrict__ idx, f
   if (i < n) x[idx[i]] = 0.0f;
 }
 
-// Receivers (solver.cpp:780-811, 945-958).  One record column per thread.
+// Receivers (solver.cpp:780-811, 945-958).  One record column per warp,
+// kRecChunk columns per CTA.
+constexpr int kRecChunk = 4;
+constexpr int kRecThreads = 32 * kRecChunk;
 struct ReceiversDev {
   int32_t n = 0;
   const int32_t* offsets = nullptr;  // [n+1] into points/value/d_dx/d_dz
@@ -203,35 +206,43 @@ struct AllFields {
   DomainFields d[2];
 };
 
-// sum over q = beg .. end-1 of (double)coef[q] * (double)field[pts[q]], added
-// in ascending q (the reference's order); the loads of four terms are issued
-// before their four additions, so their latencies overlap.
-__device__ __forceinline__ double ordered_dot(const float* __restrict__ coef, const int32_t* __restrict__ pts,
-                                              int32_t beg, int32_t end, const float* __restrict__ field) {
-  double s = 0.0;
-  int32_t q = beg;
-  for (; q + 4 <= end; q += 4) {
-    int32_t p[4];
-    float c[4], f[4];
+// N ordered sums over a receiver's interpolation points by one warp:
+// out[k] = sum over q = beg .. end-1 of (double)coef[k][q] * (double)field[k][pts[q]],
+// added in ascending q from +0 (the reference's order).  Each lane loads and
+// multiplies one term of a group of 32, so the loads of a sum overlap; the
+// products then reach every lane by shuffles and are added in order.  Lanes
+// past the end hold +0, which leaves a sum that started at +0 unchanged.
+// Bound by the chain of dependent FP64 additions.  A thread per sum that also
+// walked the loads took 7-20 us a launch (25-81 terms): 287 steps of 32 x 32
+// order-4 acoustic elements went from 6.45 to 4.54 ms with a warp per sum and
+// without the particle velocities that no trace records.
+template <int N>
+__device__ __forceinline__ void warp_ordered_dots(const float* const (&coef)[N], const int32_t* __restrict__ pts,
+                                                  int32_t beg, int32_t end, const float* const (&field)[N],
+                                                  double (&out)[N]) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) p[k] = pts[q + k];
+  for (int k = 0; k < N; ++k) out[k] = 0.0;
+  for (int32_t q0 = beg; q0 < end; q0 += 32) {
+    const int32_t m = min(32, end - q0);
+    double term[N] = {};
+    if (lane < m) {
+      const int32_t p = pts[q0 + lane];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      c[k] = coef[q + k];
-      f[k] = field[p[k]];
+      for (int k = 0; k < N; ++k)
+        term[k] = dmul(static_cast<double>(coef[k][q0 + lane]), static_cast<double>(field[k][p]));
     }
+    for (int32_t q = 0; q < m; q += 8) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) s = dadd(s, dmul(static_cast<double>(c[k]), static_cast<double>(f[k])));
+      for (int w = 0; w < 8; ++w)
+#pragma unroll
+        for (int k = 0; k < N; ++k) out[k] = dadd(out[k], __shfl_sync(0xffffffffu, term[k], q + w));
+    }
   }
-  for (; q < end; ++q) s = dadd(s, dmul(static_cast<double>(coef[q]), static_cast<double>(field[pts[q]])));
-  return s;
 }
 
-__device__ __forceinline__ double interp(const ReceiversDev& r, int32_t rec, const float* field, int32_t ng, int c) {
-  return ordered_dot(r.value, r.points, r.offsets[rec], r.offsets[rec + 1], field + static_cast<size_t>(c) * ng);
-}
-
-// Particle velocity of acoustic receivers: trapezoid of -grad(p)/rho.  With
+// Particle velocity of acoustic receivers that record it: trapezoid of
+// -grad(p)/rho, one warp per receiver (entry t of acoustic_recv).  With
 // init != 0 only prev_a is set (Solver::initialize, solver.cpp:883-893).
 __device__ __forceinline__ void particle_velocity_body(const ReceiversDev& r, const AllFields& fl,
                                                        const int32_t* __restrict__ acoustic_recv, int32_t n_acoustic,
@@ -239,10 +250,12 @@ __device__ __forceinline__ void particle_velocity_body(const ReceiversDev& r, co
   if (t >= n_acoustic) return;
   const int32_t rec = acoustic_recv[t];
   const DomainFields& d = fl.d[r.domain[rec]];
-  // two independent sums, each in ascending point order
-  const double gx = ordered_dot(r.d_dx, r.points, r.offsets[rec], r.offsets[rec + 1], d.u);
-  const double gz = ordered_dot(r.d_dz, r.points, r.offsets[rec], r.offsets[rec + 1], d.u);
-  const double ax = __ddiv_rn(-gx, r.rho[rec]), az = __ddiv_rn(-gz, r.rho[rec]);
+  const float* const coef[2] = {r.d_dx, r.d_dz};
+  const float* const field[2] = {d.u, d.u};
+  double g[2];
+  warp_ordered_dots<2>(coef, r.points, r.offsets[rec], r.offsets[rec + 1], field, g);
+  if (threadIdx.x & 31) return;
+  const double ax = __ddiv_rn(-g[0], r.rho[rec]), az = __ddiv_rn(-g[1], r.rho[rec]);
   double* pv = r.pv + static_cast<size_t>(rec) * 4;
   if (!init) {
     const double hdt = dmul(0.5, dt);
@@ -255,9 +268,10 @@ __device__ __forceinline__ void particle_velocity_body(const ReceiversDev& r, co
 
 static __global__ void particle_velocity_kernel(ReceiversDev r, AllFields fl, const int32_t* __restrict__ acoustic_recv,
                                          int32_t n_acoustic, double dt, int init) {
-  particle_velocity_body(r, fl, acoustic_recv, n_acoustic, dt, init, blockIdx.x * blockDim.x + threadIdx.x);
+  particle_velocity_body(r, fl, acoustic_recv, n_acoustic, dt, init, blockIdx.x * kRecChunk + (threadIdx.x >> 5));
 }
 
+// One recorded column (entry t of cols) by one warp.
 __device__ __forceinline__ void record_body(const ReceiversDev& r, const AllFields& fl,
                                             const RecordColumn* __restrict__ cols, int32_t n_cols, int32_t step,
                                             int32_t record_every, double* __restrict__ traces, int32_t max_samples,
@@ -272,20 +286,29 @@ __device__ __forceinline__ void record_body(const ReceiversDev& r, const AllFiel
   } else {
     const DomainFields& d = fl.d[r.domain[col.receiver]];
     const float* field = col.field == 0 ? d.u : col.field == 1 ? d.v : d.a;
+    const int32_t beg = r.offsets[col.receiver], end = r.offsets[col.receiver + 1];
     if (col.mode == 0) {
-      out = interp(r, col.receiver, field, d.ng, col.comp);
+      const float* const coef[1] = {r.value};
+      const float* const f[1] = {field + static_cast<size_t>(col.comp) * d.ng};
+      double x[1];
+      warp_ordered_dots<1>(coef, r.points, beg, end, f, x);
+      out = x[0];
     } else {
-      const double up = interp(r, col.receiver, field, d.ng, 0), um = interp(r, col.receiver, field, d.ng, 1);
-      out = dmul(kSqrtHalf, col.mode == 1 ? dadd(up, um) : dsub(up, um));
+      const float* const coef[2] = {r.value, r.value};
+      const float* const f[2] = {field, field + d.ng};
+      double x[2];
+      warp_ordered_dots<2>(coef, r.points, beg, end, f, x);
+      out = dmul(kSqrtHalf, col.mode == 1 ? dadd(x[0], x[1]) : dsub(x[0], x[1]));
     }
   }
-  traces[static_cast<size_t>(sample) * n_cols + t] = out;
+  if ((threadIdx.x & 31) == 0) traces[static_cast<size_t>(sample) * n_cols + t] = out;
 }
 
 static __global__ void record_kernel(ReceiversDev r, AllFields fl, const RecordColumn* __restrict__ cols, int32_t n_cols,
                               const StepState* st, int32_t record_every, double* __restrict__ traces,
                               int32_t max_samples) {
-  record_body(r, fl, cols, n_cols, st->step, record_every, traces, max_samples, blockIdx.x * blockDim.x + threadIdx.x);
+  record_body(r, fl, cols, n_cols, st->step, record_every, traces, max_samples,
+              blockIdx.x * kRecChunk + (threadIdx.x >> 5));
 }
 
 // ---------------------------------------------------------------- energy

@@ -1156,7 +1156,6 @@ static __global__ void tiled_energy_kernel(const double* __restrict__ epartial, 
 // scalars, the solve's StepState its step, mode and buffer parity.
 constexpr int kHaloChunk = 256;
 constexpr int kConsChunk = 128;
-constexpr int kRecChunk = 64;
 
 struct HaloSeg {
   TiledDev td;          // parity-0 view
@@ -1227,22 +1226,22 @@ struct RecSeg {
   int32_t max_samples;
 };
 
-static __global__ void __launch_bounds__(kRecChunk) particle_velocity_batch_kernel(const RecSeg* __restrict__ segs,
+static __global__ void __launch_bounds__(kRecThreads) particle_velocity_batch_kernel(const RecSeg* __restrict__ segs,
                                                                                    const int2* __restrict__ items) {
   const int2 it = items[blockIdx.x];
   const RecSeg& sg = segs[it.x];
   if (sg.st->mode == kModeIdle) return;
   particle_velocity_body(sg.rv, sg.st->parity ? sg.f1 : sg.f0, sg.acoustic_recv, sg.n_acoustic, sg.dt, 0,
-                         it.y * kRecChunk + static_cast<int32_t>(threadIdx.x));
+                         it.y * kRecChunk + static_cast<int32_t>(threadIdx.x >> 5));
 }
 
-static __global__ void __launch_bounds__(kRecChunk) record_batch_kernel(const RecSeg* __restrict__ segs,
+static __global__ void __launch_bounds__(kRecThreads) record_batch_kernel(const RecSeg* __restrict__ segs,
                                                                         const int2* __restrict__ items) {
   const int2 it = items[blockIdx.x];
   const RecSeg& sg = segs[it.x];
   if (sg.st->mode == kModeIdle) return;
   record_body(sg.rv, sg.st->parity ? sg.f1 : sg.f0, sg.cols, sg.n_cols, sg.st->step, sg.record_every, sg.traces,
-              sg.max_samples, it.y * kRecChunk + static_cast<int32_t>(threadIdx.x));
+              sg.max_samples, it.y * kRecChunk + static_cast<int32_t>(threadIdx.x >> 5));
 }
 
 struct EnergySeg {
