@@ -36,21 +36,9 @@ void Solver::batch_prepare() {
   INSEM_REQUIRE(tiled, INSEM_CUDA_ERR_STATE, "batched solves run on the tiled path");
   INSEM_REQUIRE(snap_every <= 0, INSEM_CUDA_ERR_STATE, "a solve that records snapshots is stepped on its own");
   if (in_batch) return;  // prepared already
-  if (!initialized) {
-    set_mode(kModeInit);
-    enqueue_tiled(parity, true);
-    parity ^= 1;
-    complete = true;
-    initialized = true;
-  }
-  tiled_begin_steps();
-  // the begin kernel flips the parity before each step; the first batched
-  // step must use the host's current parity
-  const int32_t vals[2] = {parity ^ 1, n_steps};
-  static_assert(offsetof(StepState, last_step) == offsetof(StepState, parity) + sizeof(int32_t), "StepState layout");
-  CUDA_CHECK(cudaMemcpyAsync(&st->parity, vals, sizeof(vals), cudaMemcpyHostToDevice, stream));
+  tiled_initialize();
+  tiled_begin_steps(n_steps);
   CUDA_CHECK(cudaStreamSynchronize(stream));
-  cur_mode = -1;
   in_batch = true;
 }
 
@@ -62,13 +50,6 @@ void Solver::batch_collect(BatchTables& T) {
   T.row_cols += n_cols;
   const StepScalars sc{static_cast<float>(dt), static_cast<float>(0.5 * dt), static_cast<float>(0.5 * dt * dt),
                        energy_every};
-  for (auto& t : tdom) {
-    if (t.n_cslots <= 0) continue;
-    const int32_t seg = static_cast<int32_t>(T.cons_segs.size());
-    T.cons_segs.push_back(ConsSeg{t.n_cslots, t.cs_row.get(), t.rows(), t.u0.get(), t.u1.get(), t.ng, t.ncomp,
-                                  t.cval.get(), st});
-    for (int k = 0; k < ceil_div(t.n_cslots, kConsChunk); ++k) T.cons_items.push_back(int2{seg, k});
-  }
   for (int di : {solid, fluid}) {
     if (di < 0) continue;
     TiledDomain& t = tdom[di];
@@ -182,16 +163,11 @@ void Solver::batch_advanced(int32_t k) {
   step += k;
   if (k & 1) parity ^= 1;
   complete = step == n_steps;  // the last step ran in final mode
-  cur_mode = -1;
 }
 
 void Solver::check_fields() {
   DeviceGuard dg(device);
-  for (auto& t : tdom) {
-    const int64_t nn = static_cast<int64_t>(t.ncomp) * t.ng;
-    finite_check_kernel<<<grid_for(nn), 256, 0, stream>>>(t.u_cur(parity), nn, st);
-    CUDA_LAUNCH_CHECK();
-  }
+  enqueue_finite_check();
   StepState hs;
   CUDA_CHECK(cudaMemcpyAsync(&hs, st, sizeof(hs), cudaMemcpyDeviceToHost, stream));
   CUDA_CHECK(cudaStreamSynchronize(stream));
@@ -212,35 +188,20 @@ Batch::Batch(const insem_cuda_options* opt) {
   CUDA_CHECK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   CUDA_CHECK(cudaEventCreate(&ev0));
   CUDA_CHECK(cudaEventCreate(&ev1));
-  INSEM_REQUIRE(opts.tile_streams >= 0 && opts.tile_streams <= kMaxLanes, INSEM_CUDA_ERR_INVALID,
-                "tile_streams must be 0..8");
-  n_lanes = opts.tile_streams > 0 ? opts.tile_streams : 2;
-  CUDA_CHECK(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming));
-  for (int k = 0; k + 1 < n_lanes; ++k) {
-    CUDA_CHECK(cudaStreamCreateWithFlags(&lanes[k], cudaStreamNonBlocking));
-    CUDA_CHECK(cudaEventCreateWithFlags(&join_ev[k], cudaEventDisableTiming));
-  }
-  CUDA_CHECK(cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, opts.device));
+  INSEM_REQUIRE(opts.tile_streams >= 0 && opts.tile_streams <= 8, INSEM_CUDA_ERR_INVALID, "tile_streams must be 0..8");
   CUDA_CHECK(cudaMallocHost(&herr, sizeof(int32_t)));
   derr.resize(1);
 }
 
 Batch::~Batch() {
   DeviceGuard dg(opts.device);
-  // members' buffers are released below: both streams must be done with them
+  // members' buffers are released below: the stream must be done with them
   if (stream) cudaStreamSynchronize(stream);
-  for (cudaStream_t l : lanes)
-    if (l) cudaStreamSynchronize(l);
   if (graph) cudaGraphExecDestroy(graph);
   members.clear();
   if (herr) cudaFreeHost(herr);
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
-  if (fork_ev) cudaEventDestroy(fork_ev);
-  for (cudaEvent_t e : join_ev)
-    if (e) cudaEventDestroy(e);
-  for (cudaStream_t l : lanes)
-    if (l) cudaStreamDestroy(l);
   if (stream) cudaStreamDestroy(stream);
 }
 
@@ -317,7 +278,6 @@ void Batch::rebuild() {
     s.batch_collect(T);
   }
   dclasses.clear();
-  std::vector<std::pair<double, std::size_t>> work;  // (elements x points per element x components, class)
   for (auto& kv : T.tiles) {
     TileClass& c = kv.second;
     DevClass d;
@@ -342,37 +302,16 @@ void Batch::rebuild() {
     // one CTA per item (the call above also sets the kernel's shared memory size)
     (void)per_sm;
     d.grid = d.n_items;  // CTA b reads item b: no launch without items
-    double w = 0.0;
-    for (const TileItem& it : c.items) w += static_cast<double>(it.th.ne);
-    work.emplace_back(w * c.ngll * c.ngll * c.ncomp, dclasses.size());
+    for (const TileItem& it : c.items) d.work += static_cast<double>(it.th.ne) * c.ngll * c.ngll * c.ncomp;
     dclasses.push_back(std::move(d));
   }
-  {
-    // lanes: elastic classes by component count, then the acoustic classes
-    // by work, largest first, each to the least loaded lane
-    std::sort(work.begin(), work.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
-    std::vector<double> load(n_lanes, 0.0);
-    for (const auto& w : work) {
-      DevClass& d = dclasses[w.second];
-      if (!d.elastic) continue;
-      d.lane = d.ncomp == 3 ? lane3() : 0;
-      load[d.lane] += w.first;
-    }
-    for (const auto& w : work) {
-      DevClass& d = dclasses[w.second];
-      if (d.elastic) continue;
-      d.lane = static_cast<int>(std::min_element(load.begin(), load.end()) - load.begin());
-      load[d.lane] += w.first;
-    }
-  }
+  // largest class first: the small ones fill the chip as its last tiles run out
+  std::stable_sort(dclasses.begin(), dclasses.end(), [](const DevClass& x, const DevClass& y) { return x.work > y.work; });
   for (int c = 0; c < 3; ++c) {
     dhalo_segs[c].upload_async(T.halo_segs[c], stream);
     dhalo_items[c].upload_async(T.halo_items[c], stream);
     n_halo_items[c] = static_cast<int32_t>(T.halo_items[c].size());
   }
-  dcons_segs.upload_async(T.cons_segs, stream);
-  dcons_items.upload_async(T.cons_items, stream);
-  n_cons_items = static_cast<int32_t>(T.cons_items.size());
   drec_segs.upload_async(T.rec_segs, stream);
   dpv_items.upload_async(T.pv_items, stream);
   drec_items.upload_async(T.rec_items, stream);
@@ -402,38 +341,19 @@ void Batch::rebuild() {
     CUDA_CHECK(cudaStreamEndCapture(stream, &g));
     std::size_t nn = 0;
     CUDA_CHECK(cudaGraphGetNodes(g, nullptr, &nn));
-    std::vector<cudaGraphNode_t> nodes(nn);
-    if (nn) CUDA_CHECK(cudaGraphGetNodes(g, nodes.data(), &nn));
-    kernels_per_step = 0;
-    for (auto nd : nodes) {
-      cudaGraphNodeType ty;
-      CUDA_CHECK(cudaGraphNodeGetType(nd, &ty));
-      if (ty == cudaGraphNodeTypeKernel) ++kernels_per_step;
-    }
+    kernels_per_step = static_cast<int32_t>(nn);  // kernel nodes only
     CUDA_CHECK(cudaGraphInstantiate(&graph, g, 0));
     CUDA_CHECK(cudaGraphDestroy(g));
   }
   dirty = false;
 }
 
+// One batched step as one chain of launches (see DepMode): tile classes side by
+// side, then the halo points, receivers and energy of every solve.
 void Batch::enqueue(cudaEvent_t tiles_begin, cudaEvent_t tiles_end) {
-  const int32_t nq = static_cast<int32_t>(dclasses.size());
-  batch_begin_kernel<<<ceil_div(std::max(n_states, 1), 256), 256, 0, stream>>>(dstates.get(), n_states);
-  CUDA_LAUNCH_CHECK();
-  if (n_cons_items > 0) {
-    constrained_batch_kernel<<<n_cons_items, kConsChunk, 0, stream>>>(dcons_segs.get(), dcons_items.get());
-    CUDA_LAUNCH_CHECK();
-  }
   if (tiles_begin) CUDA_CHECK(cudaEventRecord(tiles_begin, stream));
-  int used = 1;  // lanes in use: 0 .. used-1
-  for (const DevClass& d : dclasses) used = std::max(used, d.lane + 1);
-  if (n_halo_items[2] > 0) used = std::max(used, lane3() + 1);
-  if (used > 1) {
-    CUDA_CHECK(cudaEventRecord(fork_ev, stream));
-    for (int k = 1; k < used; ++k) CUDA_CHECK(cudaStreamWaitEvent(lanes[k - 1], fork_ev, 0));
-  }
-  for (int32_t q = 0; q < nq; ++q) {
-    const DevClass& d = dclasses[q];
+  bool first = true;
+  for (const DevClass& d : dclasses) {
     if (d.n_items == 0) continue;
     TileBatchLaunch a;
     a.kind = d.kind;
@@ -445,47 +365,36 @@ void Batch::enqueue(cudaEvent_t tiles_begin, cudaEvent_t tiles_end) {
     a.L = d.L;
     a.smem = d.L.total;
     a.grid = d.grid;
-    a.stream = d.lane == 0 ? stream : lanes[d.lane - 1];
+    a.ix = StepIdx{0, 0, first ? kDepFirst : kDepLate};
+    a.overlap = !first;
+    a.stream = stream;
     tile_batch(d.ngll, a, true);
+    first = false;
   }
-  auto join = [&]() {
-    for (int k = 1; k < used; ++k) {
-      CUDA_CHECK(cudaEventRecord(join_ev[k - 1], lanes[k - 1]));
-      CUDA_CHECK(cudaStreamWaitEvent(stream, join_ev[k - 1], 0));
-    }
-  };
+  if (tiles_end) CUDA_CHECK(cudaEventRecord(tiles_end, stream));
   // solid halos first: the fluid's coupling term reads the solid's new
-  // acceleration.  Timed runs (tiles_end) keep every tile ahead of the halos.
-  if (tiles_end) {
-    join();
-    CUDA_CHECK(cudaEventRecord(tiles_end, stream));
-  }
-  if (n_halo_items[1] > 0) {
-    halo_batch_kernel<2, true><<<n_halo_items[1], kHaloChunk, 0, stream>>>(dhalo_segs[1].get(), dhalo_items[1].get());
-    CUDA_LAUNCH_CHECK();
-  }
-  if (n_halo_items[2] > 0) {
-    cudaStream_t s3 = tiles_end || lane3() == 0 ? stream : lanes[lane3() - 1];
-    halo_batch_kernel<3, true><<<n_halo_items[2], kHaloChunk, 0, s3>>>(dhalo_segs[2].get(), dhalo_items[2].get());
-    CUDA_LAUNCH_CHECK();
-  }
-  if (!tiles_end) join();
-  if (n_halo_items[0] > 0) {
-    halo_batch_kernel<1, false><<<n_halo_items[0], kHaloChunk, 0, stream>>>(dhalo_segs[0].get(), dhalo_items[0].get());
-    CUDA_LAUNCH_CHECK();
-  }
-  if (n_pv_items > 0) {
-    particle_velocity_batch_kernel<<<n_pv_items, kRecThreads, 0, stream>>>(drec_segs.get(), dpv_items.get());
-    CUDA_LAUNCH_CHECK();
-  }
-  if (n_rec_items > 0) {
-    record_batch_kernel<<<n_rec_items, kRecThreads, 0, stream>>>(drec_segs.get(), drec_items.get());
-    CUDA_LAUNCH_CHECK();
-  }
-  if (n_energy > 0) {
-    energy_batch_kernel<<<n_energy, kReduceThreads, 0, stream>>>(denergy.get());
-    CUDA_LAUNCH_CHECK();
-  }
+  // acceleration.  The two solid kernels run side by side.
+  bool overlap = tiles_end == nullptr;
+  const bool both = n_halo_items[1] > 0 && n_halo_items[2] > 0;
+  auto halo = [&](auto kernel, int cls, DepMode dep) {
+    if (n_halo_items[cls] == 0) return;
+    CUDA_CHECK(launch_chained(kernel, n_halo_items[cls], kHaloChunk, 0, stream, overlap, dhalo_segs[cls].get(),
+                              dhalo_items[cls].get(), StepIdx{0, 0, dep}));
+    overlap = true;
+  };
+  halo(halo_batch_kernel<2, true>, 1, both ? kDepFirst : kDepAll);
+  halo(halo_batch_kernel<3, true>, 2, both ? kDepLate : kDepAll);
+  halo(halo_batch_kernel<1, false>, 0, kDepAll);
+  if (n_pv_items > 0)
+    CUDA_CHECK(launch_chained(particle_velocity_batch_kernel, n_pv_items, kRecThreads, 0, stream, true, drec_segs.get(),
+                              dpv_items.get(), StepIdx{}));
+  if (n_rec_items > 0)
+    CUDA_CHECK(launch_chained(record_batch_kernel, n_rec_items, kRecThreads, 0, stream, true, drec_segs.get(),
+                              drec_items.get(), StepIdx{}));
+  if (n_energy > 0)
+    CUDA_CHECK(launch_chained(energy_batch_kernel, n_energy, kReduceThreads, 0, stream, true, denergy.get(), StepIdx{}));
+  CUDA_CHECK(launch_chained(batch_end_kernel, ceil_div(std::max(n_states, 1), 256), 256, 0, stream, true, dstates.get(),
+                            n_states, 1));
 }
 
 int32_t Batch::max_remaining() const {

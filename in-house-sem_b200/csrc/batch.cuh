@@ -4,13 +4,15 @@
 //
 // A batched step is one CUDA graph of a fixed number of launches whatever
 // the number of solves:
-//   begin (step counters, buffer parities, modes; tile queues reset)
-//   constrained-slot gathers of every solve
 //   one tile launch per tile class (ngll, kind, medium, order): one CTA
 //     per (segment, tile) item
 //   halo points of every solve (elastic classes, then acoustic: the fluid's
 //     coupling term reads the solid's new acceleration)
 //   receivers (particle velocity, then recording) and energy of every solve
+//   step counters and buffer parities
+// The launches form one chain in which a launch may start before the one
+// ahead of it has ended (DepMode in step_kernels.cuh): the tile classes fill
+// the chip one behind the other without waiting for each other's last tiles.
 // Each solve keeps its own device data, time step, parity and step count,
 // so its results are the ones it gets alone, bit for bit.  Solves that
 // reach their last step run it in final mode and idle (every batched kernel
@@ -49,8 +51,6 @@ struct BatchTables {
   std::map<int, TileClass> tiles;  // key: ((ngll * 4 + kind) * 2 + elastic) * 2 + m
   std::vector<HaloSeg> halo_segs[3];  // 1 component (acoustic), 2 and 3 components (elastic)
   std::vector<int2> halo_items[3];
-  std::vector<ConsSeg> cons_segs;
-  std::vector<int2> cons_items;
   std::vector<RecSeg> rec_segs;
   std::vector<int2> pv_items, rec_items;
   std::vector<EnergySeg> energy_segs;
@@ -109,7 +109,7 @@ class Batch {
     DeviceBuffer<TileSeg> segs;
     DeviceBuffer<TileItem> items;
     int32_t n_items = 0;
-    int lane = 0;
+    double work = 0.0;  // elements x points per element x components
     int te = 0;
     TileLayout L{};
     int grid = 0;
@@ -117,23 +117,6 @@ class Batch {
 
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  // The tile classes of a step run side by side on `n_lanes` streams (lane 0
-  // is `stream`, lane k > 0 is lanes[k - 1]): no tile writes what another
-  // tile reads (complete points belong to one tile, halo contributions have
-  // their own places), so classes need no order among them.  The lanes fork
-  // after the constrained gathers.  Elastic classes of two components go to
-  // lane 0 and those of three to lane 1, and each lane then runs the halo
-  // kernel of its component count, which reads only those tiles' output;
-  // acoustic classes go to the least loaded lane.  The lanes join before the
-  // acoustic halo kernel, whose coupling term reads the solid's new
-  // acceleration.
-  static constexpr int kMaxLanes = 8;
-  int n_lanes = 1;
-  int lane3() const { return n_lanes > 1 ? 1 : 0; }  // the lane of three-component elastic classes
-  cudaStream_t lanes[kMaxLanes - 1] = {};
-  cudaEvent_t fork_ev = nullptr;
-  cudaEvent_t join_ev[kMaxLanes - 1] = {};
-  int n_sms = 0;
   std::vector<std::unique_ptr<insem_cuda_solver>> members;  // null after remove()
   std::vector<char> prepared;
   bool dirty = true;
@@ -143,9 +126,6 @@ class Batch {
   DeviceBuffer<HaloSeg> dhalo_segs[3];
   DeviceBuffer<int2> dhalo_items[3];
   int32_t n_halo_items[3] = {0, 0, 0};
-  DeviceBuffer<ConsSeg> dcons_segs;
-  DeviceBuffer<int2> dcons_items;
-  int32_t n_cons_items = 0;
   DeviceBuffer<RecSeg> drec_segs;
   DeviceBuffer<int2> dpv_items, drec_items;
   int32_t n_pv_items = 0, n_rec_items = 0;

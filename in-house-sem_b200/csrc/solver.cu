@@ -20,8 +20,6 @@
 
 namespace insem_b200 {
 
-int32_t* pinned_modes();
-
 void DeviceDomainData::upload(const insem_cuda_domain& d, const insem_cuda_basis& basis) {
   medium = d.medium;
   INSEM_REQUIRE(medium == INSEM_ACOUSTIC || medium == INSEM_ELASTIC, INSEM_CUDA_ERR_INVALID, "unknown medium");
@@ -110,9 +108,6 @@ Solver::Solver(const insem_cuda_problem& p, const insem_cuda_options* opt, bool 
   CUDA_CHECK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   CUDA_CHECK(cudaEventCreate(&ev0));
   CUDA_CHECK(cudaEventCreate(&ev1));
-  CUDA_CHECK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-  CUDA_CHECK(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming));
-  CUDA_CHECK(cudaEventCreateWithFlags(&join_ev, cudaEventDisableTiming));
   check_ngll(p.basis.ngll);
   ngll = p.basis.ngll;
   INSEM_REQUIRE(p.n_domains >= 1 && p.n_domains <= 2, INSEM_CUDA_ERR_INVALID, "a problem has 1 or 2 domains");
@@ -184,18 +179,13 @@ Solver::Solver(const insem_cuda_problem& p, const insem_cuda_options* opt, bool 
 
 Solver::~Solver() {
   DeviceGuard dg(device);
-  // buffers go back to the pool below: both streams must be done with them
+  // buffers go back to the pool below: the stream must be done with them
   if (stream) cudaStreamSynchronize(stream);
-  if (side) cudaStreamSynchronize(side);
   if (graph_exec) cudaGraphExecDestroy(graph_exec);
-  for (auto& g : tgraph)
-    if (g) cudaGraphExecDestroy(g);
+  for (auto& kv : tgraph) cudaGraphExecDestroy(kv.second);
   device_free(st);
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
-  if (fork_ev) cudaEventDestroy(fork_ev);
-  if (join_ev) cudaEventDestroy(join_ev);
-  if (side) cudaStreamDestroy(side);
   if (stream) cudaStreamDestroy(stream);
 }
 
@@ -597,12 +587,13 @@ void Solver::compute_acceleration(int force_energy, double h, int step_override)
 void Solver::observers(int force_energy, int init) {
   if (n_acoustic_rec > 0) {
     particle_velocity_kernel<<<ceil_div(n_acoustic_rec, kRecChunk), kRecThreads, 0, stream>>>(
-        receivers_view(), fields_view(), rec_acoustic.get(), n_acoustic_rec, dt, init);
+        receivers_view(), fields_view(), rec_acoustic.get(), n_acoustic_rec, dt, init, StepIdx{-1});
     CUDA_LAUNCH_CHECK();
   }
   if (n_cols > 0) {
     record_kernel<<<ceil_div(n_cols, kRecChunk), kRecThreads, 0, stream>>>(receivers_view(), fields_view(), rec_cols.get(), n_cols,
-                                                            st, record_every, trace_buf.get(), max_samples);
+                                                            st, record_every, trace_buf.get(), max_samples,
+                                                            StepIdx{-1});
     CUDA_LAUNCH_CHECK();
   }
   if (energy_every > 0 || force_energy) {
@@ -630,7 +621,7 @@ void Solver::enqueue_step() {
     predictor_kernel<<<grid_for(n), 256, 0, stream>>>(d.u.get(), d.v.get(), d.a.get(), n, rdt, half_dt, half_dt2);
     CUDA_LAUNCH_CHECK();
   }
-  advance_step_kernel<<<1, 1, 0, stream>>>(st);
+  advance_step_kernel<<<1, 1, 0, stream>>>(st, 1);
   CUDA_LAUNCH_CHECK();
   compute_acceleration(0, 0.5 * dt, -1);
   for (auto& d : domains) {
@@ -730,7 +721,7 @@ void Solver::advance_span(int32_t n) {
   if (opts.check_finite) {
     for (auto& d : domains) {
       const int64_t nn = static_cast<int64_t>(d.ncomp) * d.ng;
-      finite_check_kernel<<<grid_for(nn), 256, 0, stream>>>(d.u.get(), nn, st);
+      finite_check_kernel<<<grid_for(nn), 256, 0, stream>>>(d.u.get(), nn, nullptr, 0, st);
       CUDA_LAUNCH_CHECK();
     }
   }
@@ -927,7 +918,6 @@ void Solver::build_tiled(const insem_cuda_problem& p) {
   }
   epart.resize(2 * static_cast<std::size_t>(std::max(base, 1)));
   epart.zero();
-  mode_host = pinned_modes();
   tiled = true;
 }
 
@@ -938,146 +928,152 @@ AllFields Solver::tiled_fields(int par) {
   return f;
 }
 
-// Pinned {normal, final, init} shared by every solver for the whole process
-// (a per-solver pinned buffer would cost a device-wide wait when freed).
-int32_t* pinned_modes() {
-  static std::once_flag once;
-  static int32_t* modes = nullptr;
-  std::call_once(once, [] {
-    CUDA_CHECK(cudaMallocHost(&modes, 4 * sizeof(int32_t)));
-    modes[0] = kModeNormal;
-    modes[1] = kModeFinal;
-    modes[2] = kModeInit;
-    modes[3] = kModeIdle;
-  });
-  return modes;
-}
-
-void Solver::set_mode(int mode) {
-  if (mode == cur_mode) return;
-  CUDA_CHECK(cudaMemcpyAsync(&st->mode, mode_host + mode, sizeof(int32_t), cudaMemcpyHostToDevice, stream));
-  cur_mode = mode;
-}
-
-// One step of the tiled path on the field buffers of `par` (init: step 0,
-// explicit damping, no step increment).
-void Solver::enqueue_tiled(int par, bool init) {
-  if (!init) {
-    advance_step_kernel<<<1, 1, 0, stream>>>(st);
-    CUDA_LAUNCH_CHECK();
-  }
-  StepScalars sc{static_cast<float>(dt), static_cast<float>(0.5 * dt), static_cast<float>(0.5 * dt * dt),
-                 energy_every};
-  for (std::size_t di = 0; di < tdom.size(); ++di) {
-    TiledDomain& t = tdom[di];
-    if (t.n_cslots > 0) {
-      constrained_gather_kernel<<<ceil_div(t.n_cslots, 128), 128, 0, stream>>>(
-          t.n_cslots, t.cs_row.get(), t.rows(), t.u_cur(par), t.ng, t.ncomp, t.cval.get());
-      CUDA_LAUNCH_CHECK();
-    }
-  }
-  // the fluid's tiles beside the solid's: neither reads what the other
-  // writes (the solid's halo kernel reads the fluid's current field only)
-  const bool split = solid >= 0 && fluid >= 0;
-  if (split) {
-    CUDA_CHECK(cudaEventRecord(fork_ev, stream));
-    CUDA_CHECK(cudaStreamWaitEvent(side, fork_ev, 0));
-  }
-  for (int di : {solid, fluid}) {
-    if (di < 0) continue;
-    TiledDomain& t = tdom[di];
-    for (std::size_t b = 0; b < t.blocks.size(); ++b) {
-      TileLaunch a;
-      a.dom = &t;
-      a.block = static_cast<int>(b);
-      a.parity = par;
-      a.sc = sc;
-      a.st = st;
-      a.epartial = epart.get() + 2 * static_cast<std::size_t>(ep_tile[di]);
-      a.elastic = t.medium == INSEM_ELASTIC;
-      a.stream = split && di == fluid ? side : stream;
-      launch_tiles(ngll, a);
-    }
-  }
-  if (split) {
-    CUDA_CHECK(cudaEventRecord(join_ev, side));
-    CUDA_CHECK(cudaStreamWaitEvent(stream, join_ev, 0));
-  }
+// n steps of the tiled path from the field buffers of `par` on (init: step 0,
+// explicit damping, no step count), as one chain of launches on the stream
+// (see DepMode).  A step's critical path is tiles -> halo points (solid, then
+// fluid).  The fluid's tiles run beside the solid's, and a step's receivers
+// beside the next step's tiles: they read halo points only, which the next
+// step's halo kernels overwrite, not its tiles.   The first
+// kernel of a sequence keeps a full boundary to what is ahead of it.
+void Solver::enqueue_tiled(int par0, bool init, int n) {
+  const StepScalars sc{static_cast<float>(dt), static_cast<float>(0.5 * dt), static_cast<float>(0.5 * dt * dt),
+                       energy_every};
   const double h_damp = init ? 0.0 : 0.5 * dt;
-  CouplingDev cp{tcpl_fluid.get(), tcpl_solid.get(), cpl_cx.get(), cpl_cz.get()};
-  for (int di : {solid, fluid}) {
-    if (di < 0) continue;
-    TiledDomain& t = tdom[di];
-    if (t.n_halo == 0) continue;
-    const bool el = t.medium == INSEM_ELASTIC;
-    const float* other = nullptr;
-    int32_t other_ng = 0;
-    bool pm = false;
-    if (n_cpl > 0) {
-      if (el) {
-        other = tdom[fluid].u_cur(par);
-        other_ng = tdom[fluid].ng;
-        pm = t.m == 1;
-      } else {
-        other = tdom[solid].a.get();
-        other_ng = tdom[solid].ng;
-        pm = tdom[solid].m == 1;
-      }
-    }
-    const int grid = ceil_div(t.n_halo, 256);
-    double* ep = epart.get();
-    const int e0 = ep_halo[di];
-    const TiledDev tv = t.view(par);
-    const HaloDev hv = t.halo_view();
-    if (!el) {
-      halo_step_kernel<1, false><<<grid, 256, 0, stream>>>(tv, hv, cp, other, other_ng, pm, src_amp.get(), n_amp, sc,
-                                                           h_damp, st, ep, e0);
-    } else if (t.ncomp == 2) {
-      halo_step_kernel<2, true><<<grid, 256, 0, stream>>>(tv, hv, cp, other, other_ng, pm, src_amp.get(), n_amp, sc,
-                                                          h_damp, st, ep, e0);
-    } else {
-      halo_step_kernel<3, true><<<grid, 256, 0, stream>>>(tv, hv, cp, other, other_ng, pm, src_amp.get(), n_amp, sc,
-                                                          h_damp, st, ep, e0);
-    }
-    CUDA_LAUNCH_CHECK();
-  }
+  const CouplingDev cp{tcpl_fluid.get(), tcpl_solid.get(), cpl_cx.get(), cpl_cz.get()};
   ReceiversDev rv = receivers_view();
   rv.points = trec_points.get();
-  if (n_acoustic_rec > 0) {
-    particle_velocity_kernel<<<ceil_div(n_acoustic_rec, kRecChunk), kRecThreads, 0, stream>>>(rv, tiled_fields(par),
-                                                                              rec_acoustic.get(), n_acoustic_rec, dt,
-                                                                              init ? 1 : 0);
-    CUDA_LAUNCH_CHECK();
+  auto observe = [&](int k, bool beside) {
+    // particle velocity, then the recorded columns (which read it)
+    StepIdx ix{k, init ? 1 : 0, beside ? kDepLate : kDepAll};
+    const AllFields f = tiled_fields(par0 ^ (k & 1));
+    if (n_acoustic_rec > 0) {
+      CUDA_CHECK(launch_chained(particle_velocity_kernel, ceil_div(n_acoustic_rec, kRecChunk), kRecThreads, 0, stream,
+                                true, rv, f, rec_acoustic.get(), n_acoustic_rec, dt, init ? 1 : 0, ix));
+      ix.dep = kDepAll;
+    }
+    if (n_cols > 0)
+      CUDA_CHECK(launch_chained(record_kernel, ceil_div(n_cols, kRecChunk), kRecThreads, 0, stream, true, rv, f,
+                                rec_cols.get(), n_cols, st, record_every, trace_buf.get(), max_samples, ix));
+  };
+  for (int k = 0; k < n; ++k) {
+    const int par = par0 ^ (k & 1);
+    bool first = true;
+    for (int di : {solid, fluid}) {
+      if (di < 0) continue;
+      TiledDomain& t = tdom[di];
+      for (std::size_t b = 0; b < t.blocks.size(); ++b) {
+        if (t.blocks[b].ntiles == 0) continue;
+        TileLaunch a;
+        a.dom = &t;
+        a.block = static_cast<int>(b);
+        a.parity = par;
+        a.sc = sc;
+        a.st = st;
+        a.epartial = epart.get() + 2 * static_cast<std::size_t>(ep_tile[di]);
+        a.elastic = t.medium == INSEM_ELASTIC;
+        a.ix = StepIdx{k, init ? 1 : 0, first ? kDepFirst : kDepLate};
+        a.overlap = !first || k > 0;
+        a.stream = stream;
+        launch_tiles(ngll, a);
+        first = false;
+      }
+    }
+    if (k > 0) observe(k - 1, true);
+    for (int di : {solid, fluid}) {
+      if (di < 0) continue;
+      TiledDomain& t = tdom[di];
+      if (t.n_halo == 0) continue;
+      const bool el = t.medium == INSEM_ELASTIC;
+      const float* other = nullptr;
+      int32_t other_ng = 0;
+      bool pm = false;
+      if (n_cpl > 0) {
+        if (el) {
+          other = tdom[fluid].u_cur(par);
+          other_ng = tdom[fluid].ng;
+          pm = t.m == 1;
+        } else {
+          other = tdom[solid].a.get();
+          other_ng = tdom[solid].ng;
+          pm = tdom[solid].m == 1;
+        }
+      }
+      const StepIdx ix{k, init ? 1 : 0, kDepAll};
+      auto go = [&](auto kernel) {
+        CUDA_CHECK(launch_chained(kernel, ceil_div(t.n_halo, 256), 256, 0, stream, true, t.view(par), t.halo_view(), cp,
+                                  other, other_ng, pm, src_amp.get(), n_amp, sc, h_damp, st, epart.get(),
+                                  static_cast<int32_t>(ep_halo[di]), ix));
+      };
+      if (!el) go(halo_step_kernel<1, false>);
+      else if (t.ncomp == 2) go(halo_step_kernel<2, true>);
+      else go(halo_step_kernel<3, true>);
+    }
+    if (energy_every > 0) {
+      // potential order: elastic first
+      const int d0 = solid >= 0 ? solid : fluid;
+      const int d1 = solid >= 0 ? fluid : -1;
+      const int n_dom = d1 >= 0 ? 2 : 1;
+      int4 s0{ep_tile[d0], ep_ntile[d0], ep_halo[d0], tdom[d0].n_halo > 0 ? ep_nhalo[d0] : 0};
+      int4 s1{0, 0, 0, 0};
+      if (d1 >= 0) s1 = int4{ep_tile[d1], ep_ntile[d1], ep_halo[d1], tdom[d1].n_halo > 0 ? ep_nhalo[d1] : 0};
+      CUDA_CHECK(launch_chained(tiled_energy_kernel, 1, kReduceThreads, 0, stream, true, epart.get(), n_dom, s0, s1, st,
+                                energy_every, dt, energy.get(), static_cast<int32_t>(energy.size() / 3),
+                                StepIdx{k, init ? 1 : 0, kDepAll}));
+    }
   }
-  if (n_cols > 0) {
-    record_kernel<<<ceil_div(n_cols, kRecChunk), kRecThreads, 0, stream>>>(rv, tiled_fields(par), rec_cols.get(), n_cols, st,
-                                                            record_every, trace_buf.get(), max_samples);
-    CUDA_LAUNCH_CHECK();
-  }
-  if (energy_every > 0) {
-    // potential order: elastic first
-    const int d0 = solid >= 0 ? solid : fluid;
-    const int d1 = solid >= 0 ? fluid : -1;
-    const int n_dom = d1 >= 0 ? 2 : 1;
-    int4 s0{ep_tile[d0], ep_ntile[d0], ep_halo[d0], tdom[d0].n_halo > 0 ? ep_nhalo[d0] : 0};
-    int4 s1{0, 0, 0, 0};
-    if (d1 >= 0) s1 = int4{ep_tile[d1], ep_ntile[d1], ep_halo[d1], tdom[d1].n_halo > 0 ? ep_nhalo[d1] : 0};
-    tiled_energy_kernel<<<1, kReduceThreads, 0, stream>>>(epart.get(), n_dom, s0, s1, st, energy_every, dt,
-                                                          energy.get(), static_cast<int32_t>(energy.size() / 3));
-    CUDA_LAUNCH_CHECK();
-  }
+  observe(n - 1, false);
+  if (!init) CUDA_CHECK(launch_chained(advance_step_kernel, 1, 1, 0, stream, true, st, n));
 }
 
-void Solver::tiled_begin_steps() {
-  if (!complete) return;
-  for (auto& t : tdom) {
-    const int64_t n = static_cast<int64_t>(t.ncomp) * t.ng;
-    predictor_inplace_kernel<<<grid_for(n), 256, 0, stream>>>(t.u_cur(parity), t.v.get(), t.a.get(), n,
-                                                             static_cast<float>(dt), static_cast<float>(0.5 * dt),
-                                                             static_cast<float>(0.5 * dt * dt));
-    CUDA_LAUNCH_CHECK();
+// The state becomes that of a span of steps up to last_step.
+void Solver::tiled_begin_steps(int32_t last_step) {
+  SpanField f[2] = {};
+  int64_t total = 0;
+  for (std::size_t i = 0; complete && i < tdom.size() && i < 2; ++i) {
+    TiledDomain& t = tdom[i];
+    f[i] = SpanField{t.u_cur(parity), t.v.get(), t.a.get(), static_cast<int64_t>(t.ncomp) * t.ng};
+    total += f[i].n;
   }
+  begin_span_kernel<<<grid_for(total), 256, 0, stream>>>(f[0], f[1], static_cast<float>(dt), static_cast<float>(0.5 * dt),
+                                                         static_cast<float>(0.5 * dt * dt), st, last_step, parity);
+  CUDA_LAUNCH_CHECK();
   complete = false;
+}
+
+// The graph of n steps from the buffers of `par` on, captured at first use.
+cudaGraphExec_t Solver::tiled_graph(int par, int n) {
+  const auto it = tgraph.find({par, n});
+  if (it != tgraph.end()) return it->second;
+  cudaGraph_t g = nullptr;
+  CUDA_CHECK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+  try {
+    enqueue_tiled(par, false, n);
+  } catch (...) {
+    cudaStreamEndCapture(stream, &g);
+    if (g) cudaGraphDestroy(g);
+    throw;
+  }
+  CUDA_CHECK(cudaStreamEndCapture(stream, &g));
+  if (kernels_per_step == 0) {
+    std::size_t nn = 0;
+    CUDA_CHECK(cudaGraphGetNodes(g, nullptr, &nn));
+    kernels_per_step = static_cast<int32_t>(nn) / n;  // kernel nodes only
+  }
+  cudaGraphExec_t ge = nullptr;
+  const cudaError_t e = cudaGraphInstantiate(&ge, g, 0);
+  cudaGraphDestroy(g);
+  CUDA_CHECK(e);
+  tgraph[{par, n}] = ge;
+  return ge;
+}
+
+// The initial step (accelerations and observers at t = 0).
+void Solver::tiled_initialize() {
+  if (initialized) return;
+  enqueue_tiled(parity, true, 1);
+  parity ^= 1;
+  complete = true;
+  initialized = true;
 }
 
 // advance(n) on the tiled path; with rows_out, the streamed variant (amplitudes
@@ -1085,55 +1081,27 @@ void Solver::tiled_begin_steps() {
 void Solver::advance_tiled(int32_t n, const float* amp_in, double* rows_out, int32_t* n_rows) {
   const bool streamed = rows_out != nullptr || amp_in != nullptr;
   CUDA_CHECK(cudaEventRecord(ev0, stream));
-  if (!initialized) {
-    set_mode(kModeInit);
-    enqueue_tiled(parity, true);
-    parity ^= 1;
-    complete = true;
-    initialized = true;
-  }
+  tiled_initialize();
   const int32_t todo = std::min<int32_t>(n, n_steps - step);
-  if (todo > 0 && opts.use_graphs && !tgraph[0]) {
-    for (int par = 0; par < 2; ++par) {
-      cudaGraph_t g = nullptr;
-      CUDA_CHECK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-      try {
-        enqueue_tiled(par, false);
-      } catch (...) {
-        cudaStreamEndCapture(stream, &g);
-        if (g) cudaGraphDestroy(g);
-        throw;
-      }
-      CUDA_CHECK(cudaStreamEndCapture(stream, &g));
-      if (par == 0) {
-        std::size_t nn = 0;
-        CUDA_CHECK(cudaGraphGetNodes(g, nullptr, &nn));
-        std::vector<cudaGraphNode_t> nodes(nn);
-        if (nn) CUDA_CHECK(cudaGraphGetNodes(g, nodes.data(), &nn));
-        kernels_per_step = 0;
-        for (auto nd : nodes) {
-          cudaGraphNodeType ty;
-          CUDA_CHECK(cudaGraphNodeGetType(nd, &ty));
-          if (ty == cudaGraphNodeTypeKernel) ++kernels_per_step;
-        }
-      }
-      CUDA_CHECK(cudaGraphInstantiate(&tgraph[par], g, 0));
-      CUDA_CHECK(cudaGraphDestroy(g));
-    }
-  }
   int32_t rows = 0;
-  for (int32_t k = 0; k < todo; ++k) {
-    tiled_begin_steps();
-    set_mode(k == todo - 1 ? kModeFinal : kModeNormal);
+  if (todo > 0) tiled_begin_steps(step + todo);
+  for (int32_t k = 0; k < todo;) {
     const int32_t s = step + 1 + k;
     if (amp_in)
       for (int q = 0; q < n_sources; ++q)
         CUDA_CHECK(cudaMemcpyAsync(src_amp.get() + static_cast<std::size_t>(q) * n_amp + s,
                                    amp_in + static_cast<std::size_t>(k) * n_sources + q, sizeof(float),
                                    cudaMemcpyHostToDevice, stream));
-    if (opts.use_graphs) CUDA_CHECK(cudaGraphLaunch(tgraph[parity], stream));
-    else enqueue_tiled(parity, false);
-    parity ^= 1;
+    // Sequences of 16 steps for long spans, of 4, then single steps: every
+    // boundary between graphs costs the overlap of one step with the next and
+    // a launch, and every further sequence length a capture on its first use
+    // (so the longest only where it is replayed several times).
+    const int32_t left = todo - k;
+    const int32_t c = streamed ? 1 : (left >= 16 && todo >= 64) ? 16 : left >= 4 ? 4 : 1;
+    if (opts.use_graphs) CUDA_CHECK(cudaGraphLaunch(tiled_graph(parity, c), stream));
+    else enqueue_tiled(parity, false, c);
+    if (c & 1) parity ^= 1;
+    k += c;
     if (rows_out && s % record_every == 0 && n_cols > 0) {
       CUDA_CHECK(cudaMemcpyAsync(rows_out + static_cast<std::size_t>(rows) * n_cols,
                                  trace_buf.get() + static_cast<std::size_t>(s / record_every) * n_cols,
@@ -1144,24 +1112,29 @@ void Solver::advance_tiled(int32_t n, const float* amp_in, double* rows_out, int
   if (todo > 0) complete = true;
   step += todo;
   CUDA_CHECK(cudaEventRecord(ev1, stream));
-  if (opts.check_finite && !streamed) {
-    for (auto& t : tdom) {
-      const int64_t nn = static_cast<int64_t>(t.ncomp) * t.ng;
-      finite_check_kernel<<<grid_for(nn), 256, 0, stream>>>(t.u_cur(parity), nn, st);
-      CUDA_LAUNCH_CHECK();
-    }
-  }
+  if (opts.check_finite && !streamed) enqueue_finite_check();
+  StepState hs;
+  CUDA_CHECK(cudaMemcpyAsync(&hs, st, sizeof(hs), cudaMemcpyDeviceToHost, stream));
   CUDA_CHECK(cudaStreamSynchronize(stream));
   float ms = 0.0f;
   CUDA_CHECK(cudaEventElapsedTime(&ms, ev0, ev1));
   last_ms = ms;
   *n_rows = rows;
-  StepState hs;
-  CUDA_CHECK(cudaMemcpy(&hs, st, sizeof(hs), cudaMemcpyDeviceToHost));
   INSEM_REQUIRE(!hs.error, INSEM_CUDA_ERR_TIMEOUT, "a tile's bulk copies did not arrive within the wait limit");
   if (hs.nonfinite) nonfinite_seen = true;
   if (opts.check_finite && !streamed)
     INSEM_REQUIRE(!hs.nonfinite, INSEM_CUDA_ERR_NONFINITE, "the solution contains NaN or Inf (unstable time step?)");
+}
+
+void Solver::enqueue_finite_check() {
+  const float* x[2] = {};
+  int64_t n[2] = {};
+  for (std::size_t i = 0; i < tdom.size() && i < 2; ++i) {
+    x[i] = tdom[i].u_cur(parity);
+    n[i] = static_cast<int64_t>(tdom[i].ncomp) * tdom[i].ng;
+  }
+  finite_check_kernel<<<grid_for(n[0] + n[1]), 256, 0, stream>>>(x[0], n[0], x[1], n[1], st);
+  CUDA_LAUNCH_CHECK();
 }
 
 }  // namespace insem_b200

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <functional>
+#include <map>
 
 #include <memory>
 #include <random>
@@ -152,20 +153,17 @@ class Solver {
   StepState* st = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  // Coupled models: the fluid's tile launches run on `side`, beside the
-  // solid's (neither reads what the other writes), forked after the step's
-  // first kernels and joined before the halo kernels.
-  cudaStream_t side = nullptr;
-  cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
 
   // ------------------------------------------------------ tiled fused path
  public:
   bool tiled = false;  // the default path: tiles + halo kernel per step
  private:
   void build_tiled(const insem_cuda_problem& p);
-  void enqueue_tiled(int parity, bool init);
-  void tiled_begin_steps();      // predictor after a complete state
-  void set_mode(int mode);
+  void enqueue_tiled(int parity, bool init, int n);
+  void tiled_initialize();
+  void tiled_begin_steps(int32_t last_step);  // predictor after a complete state
+  cudaGraphExec_t tiled_graph(int par, int n);
+  void enqueue_finite_check();
   void advance_tiled(int32_t n, const float* amp_in, double* rows_out, int32_t* n_rows);
   AllFields tiled_fields(int parity);
   std::vector<TiledDomain> tdom;
@@ -173,11 +171,9 @@ class Solver {
   DeviceBuffer<int32_t> tcpl_fluid, tcpl_solid, trec_points;
   DeviceBuffer<double> epart;
   int ep_tile[2] = {0, 0}, ep_halo[2] = {0, 0}, ep_ntile[2] = {0, 0}, ep_nhalo[2] = {0, 0};
-  cudaGraphExec_t tgraph[2] = {nullptr, nullptr};
+  std::map<std::pair<int, int>, cudaGraphExec_t> tgraph;  // (first parity, steps) -> captured sequence
   int parity = 0;
   bool complete = false;  // u, v, a hold step `step` (after an init or final step)
-  int cur_mode = -1;
-  int32_t* mode_host = nullptr;  // pinned {normal, final, init}
 
   // ------------------------------------------------------ batched stepping
  public:

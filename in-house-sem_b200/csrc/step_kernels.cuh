@@ -14,16 +14,75 @@ constexpr double kSqrtHalf = 0.70710678118654752440;
 constexpr int kReduceBlocks = 512;  // fixed grid of the deterministic reductions
 constexpr int kReduceThreads = 256;
 
-// Device-resident counters shared by the kernels of a captured step.
+// Device-resident counters of a solve.  The tiled path changes them only in
+// the last kernel of a captured sequence of steps (and before the first), so
+// every kernel of the sequence may read them at any time; a kernel's own step
+// follows from them and from its place in the sequence (StepIdx).
 struct StepState {
-  int32_t step;           // current step index (after the predictor's increment)
+  int32_t step;           // steps done (two-pass path: the current step)
   int32_t nonfinite;      // set when a NaN/Inf was found
-  int32_t mode;           // tiled path: 0 normal, 1 final (state complete), 2 initial
   int32_t error;          // a bounded device-side wait gave up
-  int32_t parity;         // batched steps: field buffer parity of the current step
-  int32_t last_step;      // batched steps: the step that runs in final mode
+  int32_t parity;         // batched steps: field buffer parity of the next step
+  int32_t last_step;      // tiled path: the step that runs in final mode
+  int32_t pad;
   double kin_c;           // dt^2 / 8 of the kinetic energy (solver.cpp:903)
 };
+
+// ------------------------------------------- overlap of successive kernels
+// The kernels of the tiled step form one chain of programmatic dependent
+// launches: a kernel may start once every CTA of the one before it has
+// started and triggered (pdl_trigger), and pdl_wait holds a thread until the
+// kernel before it has completed and its writes are visible.  Both do nothing
+// in an ordinary launch.  Every kernel of the chain waits at some point, so a
+// kernel's completion implies that of all kernels before it.
+//   kDepFirst  waits before it touches what the step before wrote, then
+//              triggers: the next kernels start after that point, so they may
+//              read all that came before this kernel without a wait of their own
+//   kDepAll    triggers at once, waits before it touches what the kernel
+//              before it wrote (constant data is read ahead of the wait)
+//   kDepLate   needs nothing of the kernel before it: triggers at once and
+//              waits only at its end
+// A small solve is bound by this chain, not by its bytes: with a full boundary
+// between kernels, the constrained gather and the receivers on the critical
+// path and a graph per step, a step of the cased borehole (3,600 order-4
+// elements, 5.6 MB) took 29.7 us and one of 32 x 32 acoustic elements 15.8;
+// chained, 20.0 and 8.5.
+enum DepMode : int32_t { kDepFirst = 0, kDepAll = 1, kDepLate = 2 };
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// At the start of a kernel, where it first needs earlier results, and at its end.
+__device__ __forceinline__ void dep_begin(int32_t dep) {
+  if (dep != kDepFirst) pdl_trigger();
+}
+__device__ __forceinline__ void dep_wait(int32_t dep) {
+  if (dep != kDepLate) pdl_wait();
+  if (dep == kDepFirst) pdl_trigger();
+}
+__device__ __forceinline__ void dep_end(int32_t dep) {
+  if (dep == kDepLate) pdl_wait();
+}
+
+// kModeIdle: a batched solve past its last step (the batch's kernels skip it).
+enum StepMode : int32_t { kModeNormal = 0, kModeFinal = 1, kModeInit = 2, kModeIdle = 3 };
+
+// Place of a launch in its sequence of steps: the sequence's k-th step (from
+// 0), or the initial step; and how it follows the kernel before it.
+struct StepIdx {
+  int32_t k = 0;
+  int32_t init = 0;
+  int32_t dep = kDepAll;
+};
+struct StepNow {
+  int32_t mode, step;
+};
+__device__ __forceinline__ StepNow step_now(const StepState* st, const StepIdx& ix) {
+  if (ix.init) return {kModeInit, 0};
+  const int32_t s = st->step + ix.k + 1, last = st->last_step;
+  return {s > last ? kModeIdle : s == last ? kModeFinal : kModeNormal, s};
+}
+__device__ __forceinline__ bool energy_step(const StepNow& now, int32_t energy_every) {
+  return energy_every > 0 && (now.mode == kModeInit || now.step % energy_every == 0);
+}
 
 // u += dt v + dt^2/2 a; v += dt/2 a   (solver.cpp:929-933)
 static __global__ void predictor_kernel(float* __restrict__ u, float* __restrict__ v, const float* __restrict__ a,
@@ -43,7 +102,11 @@ static __global__ void corrector_kernel(float* __restrict__ v, const float* __re
     v[i] = fadd(v[i], fmul(half_dt, a[i]));
 }
 
-static __global__ void advance_step_kernel(StepState* st) { st->step += 1; }
+// Last kernel of a sequence of n steps (two-pass path: first kernel of a step).
+static __global__ void advance_step_kernel(StepState* st, int32_t n) {
+  pdl_wait();
+  st->step += n;
+}
 
 // Sources (solver.cpp:679-687), merged per global point: every point's
 // contributions are applied in source order, f += coef * amp.
@@ -267,8 +330,11 @@ __device__ __forceinline__ void particle_velocity_body(const ReceiversDev& r, co
 }
 
 static __global__ void particle_velocity_kernel(ReceiversDev r, AllFields fl, const int32_t* __restrict__ acoustic_recv,
-                                         int32_t n_acoustic, double dt, int init) {
+                                         int32_t n_acoustic, double dt, int init, StepIdx ix) {
+  dep_begin(ix.dep);
+  dep_wait(ix.dep);
   particle_velocity_body(r, fl, acoustic_recv, n_acoustic, dt, init, blockIdx.x * kRecChunk + (threadIdx.x >> 5));
+  dep_end(ix.dep);
 }
 
 // One recorded column (entry t of cols) by one warp.
@@ -306,9 +372,12 @@ __device__ __forceinline__ void record_body(const ReceiversDev& r, const AllFiel
 
 static __global__ void record_kernel(ReceiversDev r, AllFields fl, const RecordColumn* __restrict__ cols, int32_t n_cols,
                               const StepState* st, int32_t record_every, double* __restrict__ traces,
-                              int32_t max_samples) {
-  record_body(r, fl, cols, n_cols, st->step, record_every, traces, max_samples,
+                              int32_t max_samples, StepIdx ix) {
+  dep_begin(ix.dep);
+  dep_wait(ix.dep);
+  record_body(r, fl, cols, n_cols, step_now(st, ix).step, record_every, traces, max_samples,
               blockIdx.x * kRecChunk + (threadIdx.x >> 5));
+  dep_end(ix.dep);
 }
 
 // ---------------------------------------------------------------- energy
@@ -499,11 +568,12 @@ static __global__ void scale_dev_kernel(const float* __restrict__ src, float* __
     x[i] = static_cast<float>(dmul(static_cast<double>(src[i]), scale));
 }
 
-// Sets st->nonfinite if any entry of x is NaN or Inf.
-static __global__ void finite_check_kernel(const float* __restrict__ x, int64_t n, StepState* st) {
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+// Sets st->nonfinite if any entry of x (n0 of them) or y (n1) is NaN or Inf.
+static __global__ void finite_check_kernel(const float* __restrict__ x, int64_t n0, const float* __restrict__ y,
+                                           int64_t n1, StepState* st) {
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n0 + n1;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    if (!isfinite(x[i])) {
+    if (!isfinite(i < n0 ? x[i] : y[i - n0])) {
       st->nonfinite = 1;
       return;
     }

@@ -93,9 +93,6 @@ __host__ __device__ constexpr int rows_elem_stride(int ng, int nc) {
   return base;
 }
 
-// kModeIdle: a batched solve past its last step (the batch's kernels skip it).
-enum StepMode : int32_t { kModeNormal = 0, kModeFinal = 1, kModeInit = 2, kModeIdle = 3 };
-
 // Slot descriptor bits.
 constexpr uint32_t kSlotPointMask = 0xffffu;      // tile point index
 constexpr int kSlotRankShift = 16;                // local assembly rank (0..254)
@@ -114,7 +111,7 @@ struct TileHdr {
   int32_t nhs;     // halo slots (entries written to the halo buffer)
   int32_t hs_off;  // offset into hs_slot
   int32_t ncs;     // constrained slots of the tile
-  int32_t cs_off;  // offset into cs_slot / cs_idx
+  int32_t cs_off;  // offset into cs_slot / cs_row
   int32_t maxrank; // highest local rank
 };
 
@@ -123,7 +120,6 @@ struct TiledDev {
   int32_t ng = 0;          // points
   int32_t n_complete = 0;  // complete points are [0, n_complete)
   int32_t n_hbuf = 0;      // halo contributions (per component): the halo points' lists, point by point
-  int32_t n_cslots = 0;    // constrained slots of the domain
   const float* inv_mass = nullptr;
   const float* mass = nullptr;
   const float* u_cur = nullptr;
@@ -139,8 +135,9 @@ struct TiledDev {
   const int32_t* mdst_off = nullptr;  // entries with several places (constrained slots feeding several points)
   const int32_t* mdst = nullptr;
   const int32_t* cs_slot = nullptr; // tile-local slot of each constrained slot
-  const int32_t* cs_idx = nullptr;  // its index into cval
-  const float* cval = nullptr;      // [ncomp][n_cslots] gathered constrained-slot values
+  const int2* cs_row = nullptr;     // its constraint row: entries [x, y) of row_dofs / row_w
+  const int32_t* row_dofs = nullptr;
+  const float* row_w = nullptr;
   float* hbuf = nullptr;            // [ncomp][n_hbuf], each halo point's contributions in its slot order
 };
 
@@ -318,34 +315,28 @@ __device__ __forceinline__ void complete_point(int mode, const StepScalars& sc, 
   }
 }
 
-// Gathers the values of constrained slots (DofMap::gather rows, dof_map.hpp:110-115).
-__device__ __forceinline__ void constrained_gather_body(int32_t n, const int32_t* __restrict__ row_of, const RowsDev& rows,
-                                                        const float* __restrict__ u, int32_t ng, int32_t ncomp,
-                                                        float* __restrict__ cval, int32_t i) {
-  if (i >= n) return;
-  const int32_t r = row_of[i];
-  for (int c = 0; c < ncomp; ++c) {
-    float s = 0.0f;
-    for (int32_t q = rows.offsets[r]; q < rows.offsets[r + 1]; ++q)
-      s = fadd(s, fmul(rows.weights[q], u[static_cast<size_t>(c) * ng + rows.dofs[q]]));
-    cval[static_cast<size_t>(c) * n + i] = s;
+// Start of a span of steps: the predictor on the whole of up to two fields in
+// place (the state is complete after a final or initial step), the step that
+// runs in final mode and, for batched solves, the buffer parity.
+struct SpanField {
+  float* u;
+  float* v;
+  const float* a;
+  int64_t n;
+};
+static __global__ void begin_span_kernel(SpanField f0, SpanField f1, float rdt, float half_dt, float half_dt2,
+                                         StepState* st, int32_t last_step, int32_t parity) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->last_step = last_step;
+    st->parity = parity;
   }
-}
-
-static __global__ void constrained_gather_kernel(int32_t n, const int32_t* __restrict__ row_of, RowsDev rows,
-                                                 const float* __restrict__ u, int32_t ng, int32_t ncomp,
-                                                 float* __restrict__ cval) {
-  constrained_gather_body(n, row_of, rows, u, ng, ncomp, cval, blockIdx.x * blockDim.x + threadIdx.x);
-}
-
-// Predictor on the whole field, in place (start of an advance() after a final step).
-static __global__ void predictor_inplace_kernel(float* __restrict__ u, float* __restrict__ v, const float* __restrict__ a,
-                                         int64_t n, float rdt, float half_dt, float half_dt2) {
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < f0.n + f1.n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const float vi = v[i], ai = a[i];
-    u[i] = fadd(u[i], fadd(fmul(rdt, vi), fmul(half_dt2, ai)));
-    v[i] = fadd(vi, fmul(half_dt, ai));
+    const SpanField& f = i < f0.n ? f0 : f1;
+    const int64_t q = i < f0.n ? i : i - f0.n;
+    const float vi = f.v[q], ai = f.a[q];
+    f.u[q] = fadd(f.u[q], fadd(fmul(rdt, vi), fmul(half_dt2, ai)));
+    f.v[q] = fadd(vi, fmul(half_dt, ai));
   }
 }
 
@@ -354,14 +345,16 @@ static __global__ void predictor_inplace_kernel(float* __restrict__ u, float* __
 // not negative, is this thread's first halo tile point (halo_tp entry
 // blockDim.x - 1 - threadIdx.x), already loaded.  `bar` is an
 // initialised mbarrier whose next phase to complete has parity `phase`.
+// The tile's constant data (element data, descriptors, coefficients) is
+// requested before dep_wait, ahead of the step before.
 // Returns false (after recording the error) if the tile's bulk copies did
 // not arrive within the wait limit.
 template <int NG, int KIND, bool EL, int M>
 __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledDev& td, const StepScalars& sc,
-                                               StepState* __restrict__ st, double* __restrict__ epartial,
-                                               int32_t tile, const TileHdr* thp, const TileLayout& L,
-                                               unsigned char* smem_raw, uint64_t* bar, uint32_t phase,
-                                               int32_t g_first = -1) {
+                                               StepState* __restrict__ st, const StepNow& now, int32_t dep,
+                                               double* __restrict__ epartial, int32_t tile, const TileHdr* thp,
+                                               const TileLayout& L, unsigned char* smem_raw, uint64_t* bar,
+                                               uint32_t phase, int32_t g_first = -1) {
   using Cfg = TileCfg<NG>;
   using CE = ElemCfg<NG, KIND, EL, M>;
   constexpr int NC = CE::NC;
@@ -390,9 +383,8 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
   // the last thread down, so thread 0 has the fewest of them
   const int issuer = 0;
   const int tg = nthreads - 1 - tid;
-  const int mode = st->mode;
-  const int32_t step = st->step;
-  const bool energy = (mode == kModeInit) ? (sc.energy_every > 0) : (sc.energy_every > 0 && step % sc.energy_every == 0);
+  const int mode = now.mode;
+  const bool energy = energy_step(now, sc.energy_every);
   const int nc4 = (th.nc + 3) & ~3;
 
   // 1. bulk copies of the tile's element data, slot descriptors and complete
@@ -408,14 +400,6 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
       bulk_load(s_wr, blk.wr + static_cast<size_t>(th.be0) * CS, eb * CS, bar);
       bulk_load(s_hoop, blk.hoop + static_cast<size_t>(th.be0) * CS, eb * CS, bar);
       bulk_load(s_r, blk.r + static_cast<size_t>(th.be0) * CS, eb * CS, bar);
-    }
-    if (nc4 > 0) {
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        bulk_load(tu + c * tp_cap, td.u_cur + static_cast<size_t>(c) * td.ng + th.cbeg, 4u * nc4, bar);
-        if (!L.late) bulk_load(s_v + c * nc_cap, td.v + static_cast<size_t>(c) * td.ng + th.cbeg, 4u * nc4, bar);
-      }
-      if (!L.late) bulk_load(s_im, td.inv_mass + th.cbeg, 4u * nc4, bar);
     }
   }
   // this column's slot descriptors, loaded while the bulk copies are in flight
@@ -433,11 +417,53 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
     if constexpr (EL) ec1 = blk.coef1[th.be0 + el];
     if constexpr (AXI) axial = blk.axial[th.be0 + el] != 0;
   }
+  if (tg < th.ntp - th.nc && g_first < 0) g_first = td.halo_tp[th.hl_off + tg];
+  dep_wait(dep);
+  if (tid == issuer && nc4 > 0) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      bulk_load(tu + c * tp_cap, td.u_cur + static_cast<size_t>(c) * td.ng + th.cbeg, 4u * nc4, bar);
+      if (!L.late) bulk_load(s_v + c * nc_cap, td.v + static_cast<size_t>(c) * td.ng + th.cbeg, 4u * nc4, bar);
+    }
+    if (!L.late) bulk_load(s_im, td.inv_mass + th.cbeg, 4u * nc4, bar);
+  }
   // halo tile points, gathered while the bulk copies are in flight
   for (int t = tg; t < th.ntp - th.nc; t += nthreads) {
-    const int32_t g = (t == tg && g_first >= 0) ? g_first : td.halo_tp[th.hl_off + t];
+    const int32_t g = t == tg ? g_first : td.halo_tp[th.hl_off + t];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) tu[c * tp_cap + nc4 + t] = td.u_cur[static_cast<size_t>(c) * td.ng + g];
+    for (int c = 0; c < NC; ++c) tu[c * tp_cap + nc4 + t] = __ldcg(td.u_cur + static_cast<size_t>(c) * td.ng + g);
+  }
+  constexpr int ES = rows_elem_stride(NG, NC);  // element stride of the rows
+  constexpr bool PAIR = NC == 2;                 // interleaved components, two-lane sums
+  // position of (component c, row j, column l) in an element's rows
+  auto ridx = [](int c, int j, int l) { return PAIR ? j * 2 * NG + 2 * l + c : (c * NG + j) * ROW + l; };
+  // constrained (hanging) slots straight into their field rows: the row's
+  // weighted sum in row order (DofMap::gather, dof_map.hpp:110-115), while
+  // the bulk copies are in flight
+  for (int q = tg; q < th.ncs; q += nthreads) {
+    const int32_t ls = td.cs_slot[th.cs_off + q];
+    const int2 row = td.cs_row[th.cs_off + q];
+    const int e = ls / NPE, k = ls - e * NPE;
+    const int jj = k / NG, ii = k - jj * NG;
+    float s[NC] = {};
+    for (int32_t m0 = row.x; m0 < row.y; m0 += 4) {
+      float w[4], x[4][NC];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const bool in = m0 + m < row.y;
+        const int32_t g = in ? td.row_dofs[m0 + m] : 0;
+        w[m] = in ? td.row_w[m0 + m] : 0.0f;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) x[m][c] = in ? __ldcg(td.u_cur + static_cast<size_t>(c) * td.ng + g) : 0.0f;
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+          if (m0 + m < row.y) s[c] = fadd(s[c], fmul(w[m], x[m][c]));
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) su[e * ES + ridx(c, jj, ii)] = s[c];
   }
   const bool arrived = mbar_wait_bounded(bar, phase, kBulkWaitLimit);
   if (__syncthreads_or(!arrived)) {
@@ -456,16 +482,12 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
   lb.hoop = s_hoop;
   lb.r = s_r;
 
-  constexpr int ES = rows_elem_stride(NG, NC);  // element stride of the rows
-  constexpr bool PAIR = NC == 2;                 // interleaved components, two-lane sums
-  // position of (component c, row j, column l) in an element's rows
-  auto ridx = [](int c, int j, int l) { return PAIR ? j * 2 * NG + 2 * l + c : (c * NG + j) * ROW + l; };
   float* urow = su + el * ES;
   float* frow = sfx + el * ES;
   constexpr int AXS = (NG + 3) & ~3;  // one axis-term array (gx0, gy0, gx1, gy1) of an element
   float* ax = sax + el * 4 * AXS;
 
-  // 2. element field rows (slots through their tile point or the constrained list)
+  // 2. element field rows (slots through their tile point)
   if (active) {
 #pragma unroll
     for (int j = 0; j < NG; ++j) {
@@ -479,15 +501,6 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
         }
       }
     }
-  }
-  for (int q = tid; q < th.ncs; q += nthreads) {
-    const int32_t ls = td.cs_slot[th.cs_off + q];
-    const int32_t ci = td.cs_idx[th.cs_off + q];
-    const int e = ls / NPE, k = ls - e * NPE;
-    const int jj = k / NG, ii = k - jj * NG;
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-      su[e * ES + ridx(c, jj, ii)] = td.cval[static_cast<size_t>(c) * td.n_cslots + ci];
   }
   __syncthreads();
 
@@ -798,10 +811,11 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
 }
 
 template <int NG, int KIND, bool EL, int M>
-__device__ __forceinline__ void tile_step_run(const BlockDev& blk, const TiledDev& td, const StepScalars& sc,
-                                              StepState* __restrict__ st, double* __restrict__ epartial,
-                                              int32_t tile0, const TileLayout& L) {
+static __global__ void __launch_bounds__(TileCfg<NG>::THREADS)
+    tile_step_kernel(BlockDev blk, TiledDev td, StepScalars sc, StepState* __restrict__ st,
+                     double* __restrict__ epartial, int32_t tile0, StepIdx ix, TileLayout L) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  dep_begin(ix.dep);
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + L.bar);
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
@@ -809,13 +823,9 @@ __device__ __forceinline__ void tile_step_run(const BlockDev& blk, const TiledDe
   }
   __syncthreads();
   const int32_t tile = tile0 + blockIdx.x;
-  tile_step_body<NG, KIND, EL, M>(blk, td, sc, st, epartial, tile, td.tiles + tile, L, smem_raw, bar, 0u);
-}
-template <int NG, int KIND, bool EL, int M>
-static __global__ void __launch_bounds__(TileCfg<NG>::THREADS)
-    tile_step_kernel(BlockDev blk, TiledDev td, StepScalars sc, StepState* __restrict__ st,
-                     double* __restrict__ epartial, int32_t tile0, TileLayout L) {
-  tile_step_run<NG, KIND, EL, M>(blk, td, sc, st, epartial, tile0, L);
+  tile_step_body<NG, KIND, EL, M>(blk, td, sc, st, step_now(st, ix), ix.dep, epartial, tile, td.tiles + tile, L,
+                                  smem_raw, bar, 0u);
+  dep_end(ix.dep);
 }
 
 // Tiles of many solves in one launch.  A segment is one block of one
@@ -850,12 +860,13 @@ static_assert(sizeof(TileItem) == 80, "TileItem is loaded as 20 words");
 // class (sized for its largest tile).
 template <int NG, int KIND, bool EL, int M>
 __device__ __forceinline__ void tile_batch_run(const TileSeg* __restrict__ segs, const TileItem* __restrict__ items,
-                                               const TileLayout& L) {
+                                               const StepIdx& ix, const TileLayout& L) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  dep_begin(ix.dep);
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ __align__(16) TileSeg s_seg;   // the item's segment, read by the body from shared memory
   __shared__ __align__(16) TileItem s_it;
-  __shared__ int32_t s_idle;
+  __shared__ StepNow s_now;
   static_assert(sizeof(TileSeg) % 4 == 0, "TileSeg is copied as 32-bit words");
   if (threadIdx.x < 20)
     reinterpret_cast<uint32_t*>(&s_it)[threadIdx.x] = reinterpret_cast<const uint32_t*>(items + blockIdx.x)[threadIdx.x];
@@ -868,7 +879,7 @@ __device__ __forceinline__ void tile_batch_run(const TileSeg* __restrict__ segs,
   const int tg = static_cast<int>(blockDim.x - 1 - threadIdx.x);
   const int32_t g_first = tg < s_it.th.ntp - s_it.th.nc ? s_it.halo_tp[tg] : -1;
   {
-    // the segment's words; on the solve's odd steps the words of u_cur and
+    // the segment's words; on steps of odd parity the words of u_cur and
     // u_nxt are exchanged (both candidates and the parity load together)
     constexpr int kUc = static_cast<int>((offsetof(TileSeg, td) + offsetof(TiledDev, u_cur)) / 4);
     constexpr int kUn = static_cast<int>((offsetof(TileSeg, td) + offsetof(TiledDev, u_nxt)) / 4);
@@ -878,22 +889,27 @@ __device__ __forceinline__ void tile_batch_run(const TileSeg* __restrict__ segs,
     for (int q = threadIdx.x; q < static_cast<int>(sizeof(TileSeg) / 4); q += blockDim.x) {
       if (q >= kUc && q < kUc + 4) {
         const uint32_t own = src[q], other = src[q < kUn ? q + 2 : q - 2];
-        dst[q] = s_it.st->parity ? other : own;
+        dst[q] = (s_it.st->parity ^ ix.k) & 1 ? other : own;
       } else {
         dst[q] = src[q];
       }
     }
   }
-  if (threadIdx.x == blockDim.x - 1) s_idle = s_it.st->mode == kModeIdle;
+  if (threadIdx.x == blockDim.x - 1) s_now = step_now(s_it.st, ix);
   __syncthreads();
-  if (s_idle) return;
-  tile_step_body<NG, KIND, EL, M>(s_seg.blk, s_seg.td, s_seg.sc, s_seg.st, s_seg.epartial, s_it.tile, &s_it.th, L,
-                                  smem_raw, bar, 0u, g_first);
+  const StepNow now = s_now;
+  if (now.mode == kModeIdle) {
+    dep_wait(ix.dep);
+  } else {
+    tile_step_body<NG, KIND, EL, M>(s_seg.blk, s_seg.td, s_seg.sc, s_seg.st, now, ix.dep, s_seg.epartial, s_it.tile,
+                                    &s_it.th, L, smem_raw, bar, 0u, g_first);
+  }
+  dep_end(ix.dep);
 }
 template <int NG, int KIND, bool EL, int M>
 static __global__ void __launch_bounds__(TileCfg<NG>::THREADS)
-    tile_batch_kernel(const TileSeg* __restrict__ segs, const TileItem* __restrict__ items, TileLayout L) {
-  tile_batch_run<NG, KIND, EL, M>(segs, items, L);
+    tile_batch_kernel(const TileSeg* __restrict__ segs, const TileItem* __restrict__ items, StepIdx ix, TileLayout L) {
+  tile_batch_run<NG, KIND, EL, M>(segs, items, ix, L);
 }
 // Register budgets for the elastic axisymmetric batch classes whose CTAs
 // per SM shared memory or the launch's thread count limit anyway: the
@@ -905,8 +921,9 @@ template <int NG, int M>
 constexpr int kBatchRegs = NG == 7 ? (M == 1 ? 128 : 96) : (M == 1 ? (NG == 6 ? 112 : NG == 5 ? 96 : 0) : 0);
 template <int NG, int KIND, bool EL, int M, int REGS>
 static __global__ void __maxnreg__(REGS)
-    tile_batch_kernel_capped(const TileSeg* __restrict__ segs, const TileItem* __restrict__ items, TileLayout L) {
-  tile_batch_run<NG, KIND, EL, M>(segs, items, L);
+    tile_batch_kernel_capped(const TileSeg* __restrict__ segs, const TileItem* __restrict__ items, StepIdx ix,
+                             TileLayout L) {
+  tile_batch_run<NG, KIND, EL, M>(segs, items, ix, L);
 }
 
 // ------------------------------------------------------------ halo kernel
@@ -944,13 +961,19 @@ template <int NC, bool ELASTIC>
 __device__ __forceinline__ void halo_step_body(const TiledDev& td, const HaloDev& hd, const CouplingDev& cp,
                                                const float* __restrict__ other, int32_t other_ng, bool pm,
                                                const float* __restrict__ amp, int32_t n_amp, const StepScalars& sc,
-                                               double h_damp, const StepState* __restrict__ st,
-                                               double* __restrict__ epartial, int32_t part, int32_t h) {
-  const int mode = st->mode;
-  const int32_t step = st->step;
-  const bool energy = (mode == kModeInit) ? (sc.energy_every > 0) : (sc.energy_every > 0 && step % sc.energy_every == 0);
+                                               double h_damp, const StepState* __restrict__ st, const StepNow& now,
+                                               int32_t dep, double* __restrict__ epartial, int32_t part, int32_t h) {
+  const int mode = now.mode;
+  const int32_t step = now.step;
+  const bool energy = energy_step(now, sc.energy_every);
+  // constant data of the point, ahead of the wait
+  const bool in = h < hd.n;
+  const float im = in ? td.inv_mass[td.n_complete + h] : 0.0f;
+  const int32_t sp = in ? hd.spec[h] : -1;
+  const int32_t b = in ? hd.off[h] : 0, e = in ? hd.off[h + 1] : 0;
+  dep_wait(dep);
   double kin = 0.0, pot = 0.0;
-  if (h < hd.n) {
+  if (in) {
     const int32_t g = td.n_complete + h;
     // the point's own values first, all loads in flight together (the
     // stores below may alias them for the compiler)
@@ -960,10 +983,7 @@ __device__ __forceinline__ void halo_step_body(const TiledDev& td, const HaloDev
       uc[c] = td.u_cur[static_cast<size_t>(c) * td.ng + g];
       vc[c] = td.v[static_cast<size_t>(c) * td.ng + g];
     }
-    const float im = td.inv_mass[g];
-    const int32_t sp = hd.spec[h];
     float f[NC], a[NC];
-    const int32_t b = hd.off[h], e = hd.off[h + 1];
     constexpr int K = 4;  // contributions gathered at once (conforming 2D points have at most 4)
     if (e - b <= K) {
       float vq[NC][K];
@@ -1094,9 +1114,11 @@ template <int NC, bool ELASTIC>
 static __global__ void __maxnreg__(kHaloRegs<NC>)
     halo_step_kernel(TiledDev td, HaloDev hd, CouplingDev cp, const float* __restrict__ other, int32_t other_ng,
                      bool pm, const float* __restrict__ amp, int32_t n_amp, StepScalars sc, double h_damp,
-                     const StepState* __restrict__ st, double* __restrict__ epartial, int32_t epart0) {
-  halo_step_body<NC, ELASTIC>(td, hd, cp, other, other_ng, pm, amp, n_amp, sc, h_damp, st, epartial,
-                              epart0 + blockIdx.x, blockIdx.x * blockDim.x + threadIdx.x);
+                     const StepState* __restrict__ st, double* __restrict__ epartial, int32_t epart0, StepIdx ix) {
+  dep_begin(ix.dep);
+  halo_step_body<NC, ELASTIC>(td, hd, cp, other, other_ng, pm, amp, n_amp, sc, h_damp, st, step_now(st, ix), ix.dep,
+                              epartial, epart0 + blockIdx.x, blockIdx.x * blockDim.x + threadIdx.x);
+  dep_end(ix.dep);
 }
 
 // energy[sample] = (time, kinetic, potential) from the per-CTA partials of
@@ -1104,13 +1126,11 @@ static __global__ void __maxnreg__(kHaloRegs<NC>)
 // u . f_int, elastic first (solver.cpp:673-678).  Partials of set d are
 // [start_d, start_d + count_d).
 __device__ __forceinline__ void tiled_energy_body(const double* __restrict__ epartial, int n_dom, int4 sets0, int4 sets1,
-                                                  const StepState* __restrict__ st, int32_t energy_every, double dt,
+                                                  const StepNow& now, int32_t energy_every, double dt,
                                                   double* __restrict__ energy, int32_t max_samples) {
   __shared__ double sh[kReduceThreads];
-  const int mode = st->mode;
-  const int32_t step = st->step;
-  const bool on = (mode == kModeInit) ? (energy_every > 0) : (energy_every > 0 && step % energy_every == 0);
-  if (!on) return;
+  const int32_t step = now.step;
+  if (!energy_step(now, energy_every)) return;
   const int starts[4] = {sets0.x, sets0.z, sets1.x, sets1.z};
   const int counts[4] = {sets0.y, sets0.w, sets1.y, sets1.w};
   double kin = 0.0, pot = 0.0;
@@ -1146,8 +1166,11 @@ __device__ __forceinline__ void tiled_energy_body(const double* __restrict__ epa
 
 static __global__ void tiled_energy_kernel(const double* __restrict__ epartial, int n_dom, int4 sets0, int4 sets1,
                                            const StepState* __restrict__ st, int32_t energy_every, double dt,
-                                           double* __restrict__ energy, int32_t max_samples) {
-  tiled_energy_body(epartial, n_dom, sets0, sets1, st, energy_every, dt, energy, max_samples);
+                                           double* __restrict__ energy, int32_t max_samples, StepIdx ix) {
+  dep_begin(ix.dep);
+  dep_wait(ix.dep);
+  tiled_energy_body(epartial, n_dom, sets0, sets1, step_now(st, ix), energy_every, dt, energy, max_samples);
+  dep_end(ix.dep);
 }
 
 // ------------------------------------------------------- batched step kernels
@@ -1155,7 +1178,6 @@ static __global__ void tiled_energy_kernel(const double* __restrict__ epartial, 
 // item (segment, chunk); the segment carries one solve's pointers and
 // scalars, the solve's StepState its step, mode and buffer parity.
 constexpr int kHaloChunk = 256;
-constexpr int kConsChunk = 128;
 
 struct HaloSeg {
   TiledDev td;          // parity-0 view
@@ -1176,40 +1198,26 @@ struct HaloSeg {
 
 template <int NC, bool ELASTIC>
 static __global__ void __maxnreg__(kHaloRegs<NC>) halo_batch_kernel(const HaloSeg* __restrict__ segs,
-                                                                         const int2* __restrict__ items) {
+                                                                         const int2* __restrict__ items, StepIdx ix) {
+  dep_begin(ix.dep);
   const int2 it = items[blockIdx.x];
   const HaloSeg& sg = segs[it.x];
-  if (sg.st->mode == kModeIdle) return;
-  const int par = sg.st->parity;
-  TiledDev td = sg.td;
-  if (par) {
-    const float* cur = td.u_cur;
-    td.u_cur = td.u_nxt;
-    td.u_nxt = const_cast<float*>(cur);
+  const StepNow now = step_now(sg.st, ix);
+  if (now.mode == kModeIdle) {
+    dep_wait(ix.dep);
+  } else {
+    const int par = (sg.st->parity ^ ix.k) & 1;
+    TiledDev td = sg.td;
+    if (par) {
+      const float* cur = td.u_cur;
+      td.u_cur = td.u_nxt;
+      td.u_nxt = const_cast<float*>(cur);
+    }
+    halo_step_body<NC, ELASTIC>(td, sg.hd, sg.cp, par ? sg.other1 : sg.other0, sg.other_ng, sg.pm != 0, sg.amp,
+                                sg.n_amp, sg.sc, sg.h_damp, sg.st, now, ix.dep, sg.epartial, sg.epart0 + it.y,
+                                it.y * kHaloChunk + static_cast<int32_t>(threadIdx.x));
   }
-  halo_step_body<NC, ELASTIC>(td, sg.hd, sg.cp, par ? sg.other1 : sg.other0, sg.other_ng, sg.pm != 0, sg.amp,
-                              sg.n_amp, sg.sc, sg.h_damp, sg.st, sg.epartial, sg.epart0 + it.y,
-                              it.y * kHaloChunk + static_cast<int32_t>(threadIdx.x));
-}
-
-struct ConsSeg {
-  int32_t n;
-  const int32_t* row_of;
-  RowsDev rows;
-  const float* u0;
-  const float* u1;
-  int32_t ng, ncomp;
-  float* cval;
-  const StepState* st;
-};
-
-static __global__ void __launch_bounds__(kConsChunk) constrained_batch_kernel(const ConsSeg* __restrict__ segs,
-                                                                               const int2* __restrict__ items) {
-  const int2 it = items[blockIdx.x];
-  const ConsSeg& sg = segs[it.x];
-  if (sg.st->mode == kModeIdle) return;
-  constrained_gather_body(sg.n, sg.row_of, sg.rows, sg.st->parity ? sg.u1 : sg.u0, sg.ng, sg.ncomp, sg.cval,
-                          it.y * kConsChunk + static_cast<int32_t>(threadIdx.x));
+  dep_end(ix.dep);
 }
 
 struct RecSeg {
@@ -1227,21 +1235,29 @@ struct RecSeg {
 };
 
 static __global__ void __launch_bounds__(kRecThreads) particle_velocity_batch_kernel(const RecSeg* __restrict__ segs,
-                                                                                   const int2* __restrict__ items) {
+                                                                                     const int2* __restrict__ items,
+                                                                                     StepIdx ix) {
+  dep_begin(ix.dep);
+  dep_wait(ix.dep);
   const int2 it = items[blockIdx.x];
   const RecSeg& sg = segs[it.x];
-  if (sg.st->mode == kModeIdle) return;
-  particle_velocity_body(sg.rv, sg.st->parity ? sg.f1 : sg.f0, sg.acoustic_recv, sg.n_acoustic, sg.dt, 0,
-                         it.y * kRecChunk + static_cast<int32_t>(threadIdx.x >> 5));
+  if (step_now(sg.st, ix).mode != kModeIdle)
+    particle_velocity_body(sg.rv, (sg.st->parity ^ ix.k) & 1 ? sg.f1 : sg.f0, sg.acoustic_recv, sg.n_acoustic, sg.dt, 0,
+                           it.y * kRecChunk + static_cast<int32_t>(threadIdx.x >> 5));
+  dep_end(ix.dep);
 }
 
 static __global__ void __launch_bounds__(kRecThreads) record_batch_kernel(const RecSeg* __restrict__ segs,
-                                                                        const int2* __restrict__ items) {
+                                                                          const int2* __restrict__ items, StepIdx ix) {
+  dep_begin(ix.dep);
+  dep_wait(ix.dep);
   const int2 it = items[blockIdx.x];
   const RecSeg& sg = segs[it.x];
-  if (sg.st->mode == kModeIdle) return;
-  record_body(sg.rv, sg.st->parity ? sg.f1 : sg.f0, sg.cols, sg.n_cols, sg.st->step, sg.record_every, sg.traces,
-              sg.max_samples, it.y * kRecChunk + static_cast<int32_t>(threadIdx.x >> 5));
+  const StepNow now = step_now(sg.st, ix);
+  if (now.mode != kModeIdle)
+    record_body(sg.rv, (sg.st->parity ^ ix.k) & 1 ? sg.f1 : sg.f0, sg.cols, sg.n_cols, now.step, sg.record_every,
+                sg.traces, sg.max_samples, it.y * kRecChunk + static_cast<int32_t>(threadIdx.x >> 5));
+  dep_end(ix.dep);
 }
 
 struct EnergySeg {
@@ -1255,25 +1271,27 @@ struct EnergySeg {
   int32_t max_samples;
 };
 
-static __global__ void __launch_bounds__(kReduceThreads) energy_batch_kernel(const EnergySeg* __restrict__ segs) {
+static __global__ void __launch_bounds__(kReduceThreads) energy_batch_kernel(const EnergySeg* __restrict__ segs,
+                                                                             StepIdx ix) {
+  dep_begin(ix.dep);
+  dep_wait(ix.dep);
   const EnergySeg& sg = segs[blockIdx.x];
-  if (sg.st->mode == kModeIdle) return;
-  tiled_energy_body(sg.epartial, sg.n_dom, sg.s0, sg.s1, sg.st, sg.energy_every, sg.dt, sg.energy, sg.max_samples);
+  const StepNow now = step_now(sg.st, ix);
+  if (now.mode != kModeIdle)
+    tiled_energy_body(sg.epartial, sg.n_dom, sg.s0, sg.s1, now, sg.energy_every, sg.dt, sg.energy, sg.max_samples);
+  dep_end(ix.dep);
 }
 
-// First kernel of a batched step: every solve's step counter, buffer parity
-// and mode (final on its last step, idle after it).
-static __global__ void batch_begin_kernel(StepState* const* __restrict__ sts, int32_t n) {
+// Last kernel of a sequence of n batched steps: every solve's step count and
+// buffer parity (a solve past its last step stays where it is).
+static __global__ void batch_end_kernel(StepState* const* __restrict__ sts, int32_t n, int32_t steps) {
+  pdl_wait();
   const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
     StepState* s = sts[i];
-    if (s->step >= s->last_step) {
-      s->mode = kModeIdle;
-    } else {
-      s->step += 1;
-      s->parity ^= 1;
-      s->mode = s->step == s->last_step ? kModeFinal : kModeNormal;
-    }
+    const int32_t d = max(0, min(steps, s->last_step - s->step));
+    s->step += d;
+    s->parity ^= d & 1;
   }
 }
 

@@ -254,7 +254,6 @@ TiledDev TiledDomain::view(int parity) const {
   t.ng = ng;
   t.n_complete = n_complete;
   t.n_hbuf = n_hbuf;
-  t.n_cslots = n_cslots;
   t.inv_mass = inv_mass.get();
   t.mass = mass.get();
   t.u_cur = parity ? u1.get() : u0.get();
@@ -270,8 +269,9 @@ TiledDev TiledDomain::view(int parity) const {
   t.mdst_off = mdst_off.get();
   t.mdst = mdst.get();
   t.cs_slot = cs_slot.get();
-  t.cs_idx = cs_idx.get();
-  t.cval = cval.get();
+  t.cs_row = cs_row.get();
+  t.row_dofs = rows_dofs.get();
+  t.row_w = rows_w.get();
   t.hbuf = const_cast<float*>(hbuf.get());
   return t;
 }
@@ -425,7 +425,7 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
   // 5. per tile: tile points, descriptors, halo and constrained slots
   std::vector<TileHdr> hdr(n_tiles);
   std::vector<uint32_t> desc(static_cast<std::size_t>(n_elements) * cs, 0u);
-  std::vector<int32_t> htp, hslot, cslot, cidx, crow;
+  std::vector<int32_t> htp, hslot, cslot, crow;
   std::vector<int32_t> hpos_of_slot(n_slots, -1);
   std::vector<int32_t> tpi(ng_dev, -1), tpi_stamp(ng, -1);
   std::vector<int32_t> block_elem_count(d.n_blocks, 0);
@@ -485,7 +485,6 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
           } else {
             dsc = kSlotConstrained | (kSlotRankNone << kSlotRankShift);
             cslot.push_back(ls);
-            cidx.push_back(static_cast<int32_t>(crow.size()));
             crow.push_back(-1 - g);
             hpos_of_slot[s] = hb + nh++;
             hslot.push_back(ls);
@@ -501,7 +500,6 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
     e_running += be;
   }
   const int32_t n_entries = hb;
-  n_cslots = static_cast<int32_t>(crow.size());
   tp_cap = 4;
   nc_cap = 4;
   rank_cap = 1;
@@ -580,9 +578,6 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
   mdst_off.upload(moff);
   mdst.upload(mlist.empty() ? std::vector<int32_t>{0} : mlist);
   cs_slot.upload(cslot.empty() ? std::vector<int32_t>{0} : cslot);
-  cs_idx.upload(cidx.empty() ? std::vector<int32_t>{0} : cidx);
-  cs_row.upload(crow.empty() ? std::vector<int32_t>{0} : crow);
-  cval.resize(static_cast<std::size_t>(ncomp) * std::max(n_cslots, 1));
   hbuf.resize(static_cast<std::size_t>(ncomp) * std::max(n_hbuf, 1));
   h_off.upload(hoff);
   if (weighted) h_w.upload(hw.empty() ? std::vector<float>{0.0f} : hw);
@@ -602,6 +597,10 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
     auto rd = host_vec(d.dofs.row_dofs, nrd);
     const auto rw = host_vec(d.dofs.row_weights, nrd);
     for (auto& g : rd) g = perm[g];
+    std::vector<int2> crange;
+    crange.reserve(crow.size());
+    for (int32_t r : crow) crange.push_back(int2{ro[r], ro[r + 1]});
+    cs_row.upload(crange.empty() ? std::vector<int2>{int2{0, 0}} : crange);
     rows_off.upload(ro.empty() ? std::vector<int32_t>{0} : ro);
     rows_dofs.upload(rd.empty() ? std::vector<int32_t>{0} : rd);
     rows_w.upload(rw.empty() ? std::vector<float>{0.0f} : std::vector<float>(rw.begin(), rw.end()));

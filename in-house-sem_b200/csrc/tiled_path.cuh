@@ -28,7 +28,7 @@ class TiledDomain {
   // tile's complete range starts on a 16-byte boundary); ng_ref: the
   // reference's point count.  Halo points are [n_complete, n_complete + n_halo).
   int medium = 0, ncomp = 1, m = 0, ng = 0, ng_ref = 0, npe = 0, n_elements = 0;
-  int n_complete = 0, n_halo = 0, n_tiles = 0, tp_cap = 0, nc_cap = 0, n_hbuf = 0, n_cslots = 0;
+  int n_complete = 0, n_halo = 0, n_tiles = 0, tp_cap = 0, nc_cap = 0, n_hbuf = 0;
   int rank_cap = 1;  // the most contributions one complete point of a tile has
   int te = 0;  // elements per tile (CTAs of tile_threads(te, ngll) threads)
   bool weighted = false;
@@ -44,8 +44,9 @@ class TiledDomain {
   DeviceBuffer<uint32_t> sdesc;
   DeviceBuffer<TileHdr> tiles;
   std::vector<TileHdr> host_tiles;  // the same headers on the host (the batched tile items copy them)
-  DeviceBuffer<int32_t> halo_tp, hs_slot, hs_dst, mdst_off, mdst, cs_slot, cs_idx, cs_row;
-  DeviceBuffer<float> cval, hbuf, mass, inv_mass;
+  DeviceBuffer<int32_t> halo_tp, hs_slot, hs_dst, mdst_off, mdst, cs_slot;
+  DeviceBuffer<int2> cs_row;
+  DeviceBuffer<float> hbuf, mass, inv_mass;
   DeviceBuffer<float> u0, u1, v, a, vn;
   DeviceBuffer<int32_t> h_off, h_spec, src_off, src_which, cpl_off, cpl_idx, abs_idx;
   DeviceBuffer<float> h_w, src_coef, abs_coef_d;
@@ -60,6 +61,24 @@ class TiledDomain {
   float* u_cur(int parity) { return parity ? u1.get() : u0.get(); }
 };
 
+// Launch of a kernel of the step chain; `overlap`: with programmatic stream
+// serialization, so it may start before the kernel ahead of it has ended.
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t stream, bool overlap,
+                           A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 // Launchers, instantiated per ngll in tiled_ng.cu.
 struct TileLaunch {
   const TiledDomain* dom = nullptr;
@@ -69,6 +88,8 @@ struct TileLaunch {
   StepState* st = nullptr;
   double* epartial = nullptr;
   bool elastic = false;
+  StepIdx ix{};
+  bool overlap = false;  // may start before the kernel ahead of it on the stream has ended (see DepMode)
   cudaStream_t stream = nullptr;
 };
 void launch_tiles_ng2(const TileLaunch&);
@@ -142,6 +163,8 @@ struct TileBatchLaunch {
   TileLayout L{};  // the class layout; its total is the dynamic shared memory
   uint32_t smem = 0;
   int grid = 0;
+  StepIdx ix{};
+  bool overlap = false;
   cudaStream_t stream = nullptr;
 };
 // launch == false: sets the class kernel's dynamic shared memory (outside
@@ -167,8 +190,9 @@ int tile_batch_cfg(const TileBatchLaunch& a, bool launch) {
       return nb;
     }
     INSEM_REQUIRE(a.te >= 1 && a.te <= TileCfg<NG>::TE, INSEM_CUDA_ERR_INVALID, "tile elements out of range");
-    kernel<<<a.grid, tile_threads(a.te, NG), a.smem, a.stream>>>(a.segs, a.items, a.L);
-    const cudaError_t err = cudaGetLastError();
+    cudaError_t err = launch_chained(kernel, a.grid, tile_threads(a.te, NG), a.smem, a.stream, a.overlap, a.segs,
+                                     a.items, a.ix, a.L);
+    if (err == cudaSuccess) err = cudaGetLastError();
     if (err != cudaSuccess)
       throw Error(INSEM_CUDA_ERR_CUDA, "batched tile kernel launch (ngll " + std::to_string(NG) + ", kind " +
                                            std::to_string(a.kind) + ", grid " + std::to_string(a.grid) + ", smem " +
@@ -216,8 +240,9 @@ void launch_tiles_cfg(const TileLaunch& a) {
     INSEM_REQUIRE(smem <= 227 * 1024, INSEM_CUDA_ERR_UNSUPPORTED, "tile needs too much shared memory");
     TiledDev td = d.view(a.parity);
     td.sdesc += static_cast<size_t>(b.e_off) * point_stride<NG * NG>();
-    kernel<<<b.ntiles, tile_threads(d.te, NG), smem, a.stream>>>(b.view(), td, a.sc, a.st, a.epartial, b.tile0, L);
-    const cudaError_t err = cudaGetLastError();
+    cudaError_t err = launch_chained(kernel, b.ntiles, tile_threads(d.te, NG), smem, a.stream, a.overlap, b.view(), td,
+                                     a.sc, a.st, a.epartial, static_cast<int32_t>(b.tile0), a.ix, L);
+    if (err == cudaSuccess) err = cudaGetLastError();
     if (err != cudaSuccess)
       throw Error(INSEM_CUDA_ERR_CUDA, "tile kernel launch (ngll " + std::to_string(NG) + ", kind " +
                                            std::to_string(b.kind) + ", tiles " + std::to_string(b.ntiles) +
