@@ -12,22 +12,34 @@ static __global__ void batch_error_kernel(StepState* const* __restrict__ sts, in
   if (i < n && sts[i]->error) atomicOr(out, 1);
 }
 
-// Streamed steps: this step's amplitudes from the staged host row into each
-// solve's amplitude table (the step about to run is st->step + 1).
-static __global__ void batch_amp_scatter_kernel(const StreamSeg* __restrict__ segs, const float* __restrict__ stage) {
+// Start of n streamed steps: every solve's step count (`from`, read by the row
+// gather) and its amplitudes of these steps from the staged host rows into its
+// amplitude table.
+static __global__ void batch_amp_scatter_kernel(const StreamSeg* __restrict__ segs, const float* __restrict__ stage,
+                                                int32_t n, int32_t amp_cols, int32_t* __restrict__ from) {
   const StreamSeg& sg = segs[blockIdx.x];
-  const int32_t s = sg.st->step + 1;
-  if (s >= sg.n_amp) return;
-  for (int32_t q = threadIdx.x; q < sg.n_sources; q += blockDim.x)
-    sg.src_amp[static_cast<size_t>(q) * sg.n_amp + s] = stage[sg.amp_off + q];
+  const int32_t s0 = sg.st->step;
+  if (threadIdx.x == 0) from[blockIdx.x] = s0;
+  if (!stage) return;
+  for (int32_t q = threadIdx.x; q < sg.n_sources * n; q += blockDim.x) {
+    const int32_t j = q / sg.n_sources, src = q - j * sg.n_sources, s = s0 + 1 + j;
+    if (s < sg.n_amp)
+      sg.src_amp[static_cast<size_t>(src) * sg.n_amp + s] = stage[static_cast<size_t>(j) * amp_cols + sg.amp_off + src];
+  }
 }
 
-// Streamed steps: each solve's latest sample row into the staged host row.
-static __global__ void batch_row_gather_kernel(const StreamSeg* __restrict__ segs, double* __restrict__ stage) {
+// End of n streamed steps: each solve's latest sample row after each of them
+// (a solve that has ended keeps its last) into the staged host rows.  CTA
+// (solve, step).
+static __global__ void batch_row_gather_kernel(const StreamSeg* __restrict__ segs, const int32_t* __restrict__ from,
+                                               int32_t row_cols, double* __restrict__ stage) {
   const StreamSeg& sg = segs[blockIdx.x];
-  const int32_t sample = sg.st->step / sg.record_every;
+  const int32_t j = blockIdx.y;
+  const int32_t step = min(from[blockIdx.x] + j + 1, sg.st->last_step);
+  const int32_t sample = step / sg.record_every;
   for (int32_t c = threadIdx.x; c < sg.n_cols; c += blockDim.x)
-    stage[sg.col_off + c] = sample < sg.max_samples ? sg.traces[static_cast<size_t>(sample) * sg.n_cols + c] : 0.0;
+    stage[static_cast<size_t>(j) * row_cols + sg.col_off + c] =
+        sample < sg.max_samples ? sg.traces[static_cast<size_t>(sample) * sg.n_cols + c] : 0.0;
 }
 
 // ------------------------------------------------------------ Solver hooks
@@ -197,7 +209,7 @@ Batch::~Batch() {
   DeviceGuard dg(opts.device);
   // members' buffers are released below: the stream must be done with them
   if (stream) cudaStreamSynchronize(stream);
-  if (graph) cudaGraphExecDestroy(graph);
+  drop_graphs();
   members.clear();
   if (herr) cudaFreeHost(herr);
   if (ev0) cudaEventDestroy(ev0);
@@ -234,10 +246,7 @@ void Batch::remove(int32_t index) {
   INSEM_REQUIRE(index >= 0 && index < size() && members[index], INSEM_CUDA_ERR_INVALID, "no such batch member");
   DeviceGuard dg(opts.device);
   CUDA_CHECK(cudaStreamSynchronize(stream));
-  if (graph) {
-    CUDA_CHECK(cudaGraphExecDestroy(graph));
-    graph = nullptr;
-  }
+  drop_graphs();
   members[index].reset();
   dirty = true;
 }
@@ -263,10 +272,7 @@ int32_t Batch::steps_to_next_completion() const {
 
 void Batch::rebuild() {
   CUDA_CHECK(cudaStreamSynchronize(stream));
-  if (graph) {
-    CUDA_CHECK(cudaGraphExecDestroy(graph));
-    graph = nullptr;
-  }
+  drop_graphs();
   BatchTables T;
   for (std::size_t i = 0; i < members.size(); ++i) {
     if (!members[i] || members[i]->s->remaining() <= 0) continue;
@@ -325,14 +331,36 @@ void Batch::rebuild() {
   n_stream = static_cast<int32_t>(T.stream_segs.size());
   amp_cols = T.amp_cols;
   row_cols = T.row_cols;
-  if (amp_stage.size() < static_cast<std::size_t>(std::max(amp_cols, 1))) amp_stage.resize(std::max(amp_cols, 1));
-  if (row_stage.size() < static_cast<std::size_t>(std::max(row_cols, 1))) row_stage.resize(std::max(row_cols, 1));
+  const std::size_t na = static_cast<std::size_t>(std::max(amp_cols, 1)) * kSequence,
+                    nr = static_cast<std::size_t>(std::max(row_cols, 1)) * kSequence;
+  if (amp_stage.size() < na) amp_stage.resize(na);
+  if (row_stage.size() < nr) row_stage.resize(nr);
+  if (stream_from.size() < static_cast<std::size_t>(std::max(n_stream, 1))) stream_from.resize(std::max(n_stream, 1));
   CUDA_CHECK(cudaStreamSynchronize(stream));
-  if (opts.use_graphs && n_states > 0) {
+  dirty = false;
+}
+
+void Batch::drop_graphs() {
+  for (cudaGraphExec_t& g : graph)
+    if (g) {
+      cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
+}
+
+// n steps: the graph of a whole sequence (kSequence steps) or of one step,
+// captured at its first use after a rebuild, or plain launches.
+void Batch::launch_steps(int32_t n) {
+  if (!opts.use_graphs || n_states == 0) {
+    enqueue(n);
+    return;
+  }
+  cudaGraphExec_t& ge = graph[n == 1 ? 0 : 1];
+  if (!ge) {
     cudaGraph_t g = nullptr;
     CUDA_CHECK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     try {
-      enqueue();
+      enqueue(n);
     } catch (...) {
       cudaStreamEndCapture(stream, &g);
       if (g) cudaGraphDestroy(g);
@@ -341,16 +369,41 @@ void Batch::rebuild() {
     CUDA_CHECK(cudaStreamEndCapture(stream, &g));
     std::size_t nn = 0;
     CUDA_CHECK(cudaGraphGetNodes(g, nullptr, &nn));
-    kernels_per_step = static_cast<int32_t>(nn);  // kernel nodes only
-    CUDA_CHECK(cudaGraphInstantiate(&graph, g, 0));
-    CUDA_CHECK(cudaGraphDestroy(g));
+    kernels_per_step = static_cast<int32_t>(nn) / n;  // kernel nodes only
+    const cudaError_t e = cudaGraphInstantiate(&ge, g, 0);
+    cudaGraphDestroy(g);
+    CUDA_CHECK(e);
   }
-  dirty = false;
+  CUDA_CHECK(cudaGraphLaunch(ge, stream));
 }
 
-// One batched step as one chain of launches (see DepMode): tile classes side by
-// side, then the halo points, receivers and energy of every solve.
-void Batch::enqueue(cudaEvent_t tiles_begin, cudaEvent_t tiles_end) {
+// n batched steps as one chain of launches (see DepMode): tile classes side by
+// side, with the receivers of the step before, then the halo points and the
+// energy of every solve.
+void Batch::enqueue(int32_t n, cudaEvent_t tiles_begin, cudaEvent_t tiles_end) {
+  auto observe = [&](int32_t k, bool beside) {
+    StepIdx ix{k, 0, beside ? kDepLate : kDepAll};
+    if (n_pv_items > 0) {
+      CUDA_CHECK(launch_chained(particle_velocity_batch_kernel, n_pv_items, kRecThreads, 0, stream, true,
+                                drec_segs.get(), dpv_items.get(), ix));
+      ix.dep = kDepAll;
+    }
+    if (n_rec_items > 0)
+      CUDA_CHECK(launch_chained(record_batch_kernel, n_rec_items, kRecThreads, 0, stream, true, drec_segs.get(),
+                                drec_items.get(), ix));
+  };
+  for (int32_t k = 0; k < n; ++k) {
+    enqueue_step(k, tiles_begin, tiles_end, [&] {
+      if (k > 0) observe(k - 1, true);
+    });
+  }
+  observe(n - 1, false);
+  CUDA_CHECK(launch_chained(batch_end_kernel, ceil_div(std::max(n_states, 1), 256), 256, 0, stream, true, dstates.get(),
+                            n_states, n));
+}
+
+template <class Fn>
+void Batch::enqueue_step(int32_t k, cudaEvent_t tiles_begin, cudaEvent_t tiles_end, Fn&& after_tiles) {
   if (tiles_begin) CUDA_CHECK(cudaEventRecord(tiles_begin, stream));
   bool first = true;
   for (const DevClass& d : dclasses) {
@@ -365,13 +418,14 @@ void Batch::enqueue(cudaEvent_t tiles_begin, cudaEvent_t tiles_end) {
     a.L = d.L;
     a.smem = d.L.total;
     a.grid = d.grid;
-    a.ix = StepIdx{0, 0, first ? kDepFirst : kDepLate};
-    a.overlap = !first;
+    a.ix = StepIdx{k, 0, first ? kDepFirst : kDepLate};
+    a.overlap = !first || k > 0;
     a.stream = stream;
     tile_batch(d.ngll, a, true);
     first = false;
   }
   if (tiles_end) CUDA_CHECK(cudaEventRecord(tiles_end, stream));
+  after_tiles();
   // solid halos first: the fluid's coupling term reads the solid's new
   // acceleration.  The two solid kernels run side by side.
   bool overlap = tiles_end == nullptr;
@@ -379,23 +433,19 @@ void Batch::enqueue(cudaEvent_t tiles_begin, cudaEvent_t tiles_end) {
   auto halo = [&](auto kernel, int cls, DepMode dep) {
     if (n_halo_items[cls] == 0) return;
     CUDA_CHECK(launch_chained(kernel, n_halo_items[cls], kHaloChunk, 0, stream, overlap, dhalo_segs[cls].get(),
-                              dhalo_items[cls].get(), StepIdx{0, 0, dep}));
+                              dhalo_items[cls].get(), StepIdx{k, 0, dep}));
     overlap = true;
   };
   halo(halo_batch_kernel<2, true>, 1, both ? kDepFirst : kDepAll);
   halo(halo_batch_kernel<3, true>, 2, both ? kDepLate : kDepAll);
   halo(halo_batch_kernel<1, false>, 0, kDepAll);
-  if (n_pv_items > 0)
-    CUDA_CHECK(launch_chained(particle_velocity_batch_kernel, n_pv_items, kRecThreads, 0, stream, true, drec_segs.get(),
-                              dpv_items.get(), StepIdx{}));
-  if (n_rec_items > 0)
-    CUDA_CHECK(launch_chained(record_batch_kernel, n_rec_items, kRecThreads, 0, stream, true, drec_segs.get(),
-                              drec_items.get(), StepIdx{}));
   if (n_energy > 0)
-    CUDA_CHECK(launch_chained(energy_batch_kernel, n_energy, kReduceThreads, 0, stream, true, denergy.get(), StepIdx{}));
-  CUDA_CHECK(launch_chained(batch_end_kernel, ceil_div(std::max(n_states, 1), 256), 256, 0, stream, true, dstates.get(),
-                            n_states, 1));
+    CUDA_CHECK(launch_chained(energy_batch_kernel, n_energy, kReduceThreads, 0, stream, true, denergy.get(),
+                              StepIdx{k, 0, kDepAll}));
 }
+
+// The length of the next sequence of steps when `left` remain.
+int32_t Batch::sequence(int32_t left) { return left >= kSequence ? kSequence : 1; }
 
 int32_t Batch::max_remaining() const {
   int32_t k = 0;
@@ -453,9 +503,10 @@ void Batch::advance(int32_t n) {
   if (dirty) rebuild();
   CUDA_CHECK(cudaMemsetAsync(derr.get(), 0, sizeof(int32_t), stream));
   CUDA_CHECK(cudaEventRecord(ev0, stream));
-  for (int32_t j = 0; j < k; ++j) {
-    if (graph) CUDA_CHECK(cudaGraphLaunch(graph, stream));
-    else enqueue();
+  for (int32_t j = 0; j < k;) {
+    const int32_t c = sequence(k - j);
+    launch_steps(c);
+    j += c;
   }
   CUDA_CHECK(cudaEventRecord(ev1, stream));
   finish_steps();
@@ -483,21 +534,28 @@ int32_t Batch::advance_streamed(int32_t n, const float* amp_in, double* rows_out
   if (dirty) rebuild();
   CUDA_CHECK(cudaMemsetAsync(derr.get(), 0, sizeof(int32_t), stream));
   CUDA_CHECK(cudaEventRecord(ev0, stream));
-  for (int32_t j = 0; j < k; ++j) {
-    if (amp_cols > 0 && amp_in) {
+  // copies, and the kernels that spread and collect them, once per sequence
+  const bool amps = amp_cols > 0 && amp_in, rows = rows_out && row_cols > 0;
+  for (int32_t j = 0; j < k;) {
+    const int32_t c = sequence(k - j);
+    if (amps)
       CUDA_CHECK(cudaMemcpyAsync(amp_stage.get(), amp_in + static_cast<std::size_t>(j) * amp_cols,
-                                 amp_cols * sizeof(float), cudaMemcpyHostToDevice, stream));
-      batch_amp_scatter_kernel<<<n_stream, 64, 0, stream>>>(dstream.get(), amp_stage.get());
+                                 static_cast<std::size_t>(c) * amp_cols * sizeof(float), cudaMemcpyHostToDevice, stream));
+    if (amps || rows) {
+      batch_amp_scatter_kernel<<<n_stream, 64, 0, stream>>>(dstream.get(), amps ? amp_stage.get() : nullptr, c, amp_cols,
+                                                            stream_from.get());
       CUDA_LAUNCH_CHECK();
     }
-    if (graph) CUDA_CHECK(cudaGraphLaunch(graph, stream));
-    else enqueue();
-    if (rows_out && row_cols > 0) {
-      batch_row_gather_kernel<<<n_stream, 64, 0, stream>>>(dstream.get(), row_stage.get());
+    launch_steps(c);
+    if (rows) {
+      batch_row_gather_kernel<<<dim3(n_stream, c), 64, 0, stream>>>(dstream.get(), stream_from.get(), row_cols,
+                                                                    row_stage.get());
       CUDA_LAUNCH_CHECK();
       CUDA_CHECK(cudaMemcpyAsync(rows_out + static_cast<std::size_t>(j) * row_cols, row_stage.get(),
-                                 row_cols * sizeof(double), cudaMemcpyDeviceToHost, stream));
+                                 static_cast<std::size_t>(c) * row_cols * sizeof(double), cudaMemcpyDeviceToHost,
+                                 stream));
     }
+    j += c;
   }
   CUDA_CHECK(cudaEventRecord(ev1, stream));
   finish_steps();
@@ -521,7 +579,7 @@ void Batch::profile(int32_t n, double* tile_ms, double* step_ms) {
     CUDA_CHECK(cudaMemsetAsync(derr.get(), 0, sizeof(int32_t), stream));
     for (int32_t j = 0; j < k; ++j) {
       CUDA_CHECK(cudaEventRecord(ev[4 * j], stream));
-      enqueue(ev[4 * j + 1], ev[4 * j + 2]);
+      enqueue(1, ev[4 * j + 1], ev[4 * j + 2]);
       CUDA_CHECK(cudaEventRecord(ev[4 * j + 3], stream));
     }
     finish_steps();

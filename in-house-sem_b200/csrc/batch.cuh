@@ -101,7 +101,15 @@ class Batch {
   void rebuild();
   void finish_steps();       // error flags of the steps just enqueued; waits for them
   void credit(int32_t k);    // host bookkeeping after k batched steps
-  void enqueue(cudaEvent_t tiles_begin = nullptr, cudaEvent_t tiles_end = nullptr);
+  void enqueue(int32_t n, cudaEvent_t tiles_begin = nullptr, cudaEvent_t tiles_end = nullptr);
+  template <class Fn>
+  void enqueue_step(int32_t k, cudaEvent_t tiles_begin, cudaEvent_t tiles_end, Fn&& after_tiles);
+  void launch_steps(int32_t n);
+  void drop_graphs();
+  // Steps per captured sequence, besides single steps: inside a sequence the
+  // receivers leave the critical path and streamed copies are shared.
+  static constexpr int32_t kSequence = 8;
+  static int32_t sequence(int32_t left);
 
   struct DevClass {
     int ngll = 0, kind = 0, m = 0, ncomp = 1;
@@ -120,7 +128,7 @@ class Batch {
   std::vector<std::unique_ptr<insem_cuda_solver>> members;  // null after remove()
   std::vector<char> prepared;
   bool dirty = true;
-  cudaGraphExec_t graph = nullptr;
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};  // one step, kSequence steps
   // device tables of the current composition
   std::vector<DevClass> dclasses;
   DeviceBuffer<HaloSeg> dhalo_segs[3];
@@ -137,6 +145,7 @@ class Batch {
   int32_t n_stream = 0, amp_cols = 0, row_cols = 0;
   DeviceBuffer<float> amp_stage;
   DeviceBuffer<double> row_stage;
+  DeviceBuffer<int32_t> stream_from;  // step counts at the start of the streamed steps in flight
   DeviceBuffer<int32_t> derr;
   int32_t* herr = nullptr;  // pinned
   std::vector<int64_t> member_points;

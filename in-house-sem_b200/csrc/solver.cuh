@@ -164,6 +164,8 @@ class Solver {
   void tiled_begin_steps(int32_t last_step);  // predictor after a complete state
   cudaGraphExec_t tiled_graph(int par, int n);
   void enqueue_finite_check();
+  void upload_amplitudes(int32_t todo, const float* amp_in, std::vector<float>& staged);
+  int32_t download_rows(int32_t todo, double* rows_out);
   void advance_tiled(int32_t n, const float* amp_in, double* rows_out, int32_t* n_rows);
   AllFields tiled_fields(int parity);
   std::vector<TiledDomain> tdom;

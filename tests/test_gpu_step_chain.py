@@ -77,3 +77,62 @@ def test_batch_spans_match_the_oracle(pkg, oracle, graphs):
         for prob, s, ref in entries:
             ref.run()
             _check(prob, s, ref)
+
+
+def _samples(prob, ref):
+    return np.concatenate([ref.trace(r, q) for r, q in prob.trace_list()], axis=1)
+
+
+@pytest.mark.parametrize("path", [0, 1])
+def test_streamed_spans_with_several_sources(pkg, oracle, path):
+    import insem_b200.cases as K
+    from insem_b200.stf import amplitudes
+
+    spans = [1, 7, 64]
+    prob = _problem(sum(spans), 0)
+    extra = K.build(K.Model(**{**_source_model(), "n_steps": 1, "dt": 1e-7}), stable_dt=1e-5).sources
+    prob.sources.extend(extra)
+    ref = oracle.OracleSolver(prob)
+    ref.run()
+    want, step = _samples(prob, ref), 0
+    with pkg.Solver(prob, path=path) as s:
+        for n in spans:
+            amp = np.ascontiguousarray(amplitudes(prob, step + 1, n))
+            rows = np.full((n, s.n_columns), np.nan)
+            got = s.advance_streamed(n, amp, rows)
+            first = step // prob.record_every + 1
+            assert np.array_equal(rows[:got], want[first:first + got]) and got == (step + n) // prob.record_every + 1 - first
+            step += n
+
+
+def _source_model():
+    import insem_b200.cases as K
+
+    b = K.borehole((0.0, 0.9), [("mud", 0.1), ("casing", 0.11)], formation_radius=0.8, dz=0.15)
+    mats = {b.regions["mud"]: K.MUD, b.regions["casing"]: K.STEEL, b.regions["formation"]: K.FAST}
+    return dict(mesh=b.mesh, order=4, regions=[(0.2, 0.2, 0.5, 0.5, 1)], materials=mats,
+                sources=[K.Source("monopole", 0.0, 0.3, stf=K.gaussian(6000.0, 1e-5))])
+
+
+def test_streamed_batch_spans(pkg, oracle):
+    from insem_b200.stf import amplitudes
+
+    lengths, n = (5, 12, 40), 21  # a whole sequence, then single steps; two members end inside
+    probs = [_problem(k, 0) for k in lengths]
+    refs = [oracle.OracleSolver(p) for p in probs]
+    for r in refs:
+        r.run()
+    with pkg.Batch() as b:
+        for p in probs:
+            b.add(p)
+        a_cols, r_cols = b.stream_layout()
+        amp = np.ascontiguousarray(np.concatenate([amplitudes(p, 1, n) for p in probs], axis=1))
+        assert amp.shape == (n, a_cols)
+        rows = np.full((n, r_cols), np.nan)
+        assert b.advance_streamed(n, amp, rows) == n
+    at = 0
+    for p, r in zip(probs, refs):
+        want = _samples(p, r)
+        for j in range(min(n, p.n_steps)):
+            assert np.array_equal(rows[j, at:at + want.shape[1]], want[(j + 1) // p.record_every])
+        at += want.shape[1]
