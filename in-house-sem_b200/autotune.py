@@ -29,7 +29,7 @@ ClassKey = Tuple[int, int, int, int, int]  # ngll, kind, medium, azimuthal order
 
 
 def te_max(ngll: int) -> int:
-    return min(64, 256 // ngll)
+    return 32
 
 
 def current(key: ClassKey) -> int:

@@ -71,7 +71,6 @@ void Solver::batch_collect(BatchTables& T) {
       TileSeg sg{};
       sg.blk = bt.view();
       sg.td = t.view(0);
-      sg.td.sdesc += static_cast<size_t>(bt.e_off) * point_stride_rt(ngll * ngll);
       sg.sc = sc;
       sg.st = st;
       sg.epartial = epart.get() + 2 * static_cast<std::size_t>(ep_tile[di]);
@@ -83,7 +82,6 @@ void Solver::batch_collect(BatchTables& T) {
       c.m = m;
       c.ncomp = t.ncomp;
       c.elastic = el;
-      c.te = std::max(c.te, t.te);
       c.tp_cap = std::max(c.tp_cap, t.tp_cap);
       c.nc_cap = std::max(c.nc_cap, t.nc_cap);
       c.rank_cap = std::max(c.rank_cap, t.rank_cap);
@@ -295,18 +293,14 @@ void Batch::rebuild() {
     d.segs.upload_async(c.segs, stream);
     d.items.upload_async(c.items, stream);
     d.n_items = static_cast<int32_t>(c.items.size());
-    d.te = c.te;
-    d.L = TileLayout::make(c.ngll, c.ncomp, c.kind, c.elastic, c.te, c.tp_cap, c.nc_cap, c.rank_cap);
+    d.L = TileLayout::make(c.ngll, c.ncomp, c.kind, c.elastic, kTileLanes, c.tp_cap, c.nc_cap, c.rank_cap);
     TileBatchLaunch a;
-    a.te = c.te;
     a.kind = c.kind;
     a.m = c.m;
     a.elastic = c.elastic;
     a.L = d.L;
     a.smem = d.L.total;
-    const int per_sm = std::max(1, tile_batch(c.ngll, a, false));
-    // one CTA per item (the call above also sets the kernel's shared memory size)
-    (void)per_sm;
+    tile_batch(c.ngll, a, false);
     d.grid = d.n_items;  // CTA b reads item b: no launch without items
     for (const TileItem& it : c.items) d.work += static_cast<double>(it.th.ne) * c.ngll * c.ngll * c.ncomp;
     dclasses.push_back(std::move(d));
@@ -414,7 +408,6 @@ void Batch::enqueue_step(int32_t k, cudaEvent_t tiles_begin, cudaEvent_t tiles_e
     a.elastic = d.elastic;
     a.segs = d.segs.get();
     a.items = d.items.get();
-    a.te = d.te;
     a.L = d.L;
     a.smem = d.L.total;
     a.grid = d.grid;

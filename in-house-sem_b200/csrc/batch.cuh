@@ -41,7 +41,7 @@ struct StreamSeg {
 struct TileClass {
   int ngll = 0, kind = 0, m = 0, ncomp = 0;
   bool elastic = false;
-  int tp_cap = 0, nc_cap = 0, te = 0, rank_cap = 1;  // largest tile of the class
+  int tp_cap = 0, nc_cap = 0, rank_cap = 1;  // largest tile of the class
   std::vector<TileSeg> segs;
   std::vector<TileItem> items;
 };
@@ -118,7 +118,6 @@ class Batch {
     DeviceBuffer<TileItem> items;
     int32_t n_items = 0;
     double work = 0.0;  // elements x points per element x components
-    int te = 0;
     TileLayout L{};
     int grid = 0;
   };

@@ -142,55 +142,63 @@ inline int metric_stride_rt(int kind, int npe) {
   return kind == INSEM_RECT ? 4 : kind == INSEM_AFFINE ? 8 : (kind == INSEM_AXISYM ? 4 : 5) * point_stride_rt(npe);
 }
 
-// Metric of block element b at point k in the device layout.
-template <int KIND, int NPE>
-__device__ __forceinline__ void load_metric(const float* metric, int b, int k, float& xi_x, float& xi_z,
-                                            float& eta_x, float& eta_z, float& jac) {
+// ------------------------------------------------------------- point math
+// Metric, axisymmetric weights and coefficients of one element point.
+struct PointData {
+  float xi_x, xi_z, eta_x, eta_z;
+  float jac;            // Cartesian kinds
+  float wr, hoop, r;    // axisymmetric
+  float c0, c1;         // lambda and mu, or 1 / rho
+};
+
+// Point k of block element b in the two-pass path's device layout.
+template <int KIND, bool ELASTIC, int NPE>
+__device__ __forceinline__ PointData load_point(const BlockDev& blk, int b, int k) {
   constexpr int CS = point_stride<NPE>();
+  PointData p{};
   if constexpr (KIND == INSEM_RECT) {
-    const float* m = metric + static_cast<size_t>(b) * 4;
-    xi_x = m[0];
-    xi_z = 0.0f;
-    eta_x = 0.0f;
-    eta_z = m[1];
-    jac = m[2];
+    const float* m = blk.metric + static_cast<size_t>(b) * 4;
+    p.xi_x = m[0];
+    p.eta_z = m[1];
+    p.jac = m[2];
   } else if constexpr (KIND == INSEM_AFFINE) {
-    const float* m = metric + static_cast<size_t>(b) * 8;
-    xi_x = m[0];
-    xi_z = m[1];
-    eta_x = m[2];
-    eta_z = m[3];
-    jac = m[4];
+    const float* m = blk.metric + static_cast<size_t>(b) * 8;
+    p.xi_x = m[0];
+    p.xi_z = m[1];
+    p.eta_x = m[2];
+    p.eta_z = m[3];
+    p.jac = m[4];
   } else {
-    const float* m = metric + static_cast<size_t>(b) * 5 * CS + k;
-    xi_x = m[0];
-    xi_z = m[CS];
-    eta_x = m[2 * CS];
-    eta_z = m[3 * CS];
-    jac = m[4 * CS];
+    const float* m = blk.metric + static_cast<size_t>(b) * (KIND == INSEM_AXISYM ? 4 : 5) * CS + k;
+    p.xi_x = m[0];
+    p.xi_z = m[CS];
+    p.eta_x = m[2 * CS];
+    p.eta_z = m[3 * CS];
+    if constexpr (KIND == INSEM_CURVED) p.jac = m[4 * CS];
   }
+  const size_t q = static_cast<size_t>(b) * CS + k;
+  p.c0 = blk.coef0[q];
+  if constexpr (ELASTIC) p.c1 = blk.coef1[q];
+  if constexpr (KIND == INSEM_AXISYM) {
+    p.wr = blk.wr[q];
+    p.hoop = blk.hoop[q];
+    p.r = blk.r[q];
+  }
+  return p;
 }
 
-// ------------------------------------------------------------- point math
 // Fluxes of one element point from its reference derivatives u_xi / u_eta
-// (per component), the point's own field values upt (hoop terms), and the
-// block data: f_xi / f_eta per component, the direct (hoop) terms, and for
+// (per component), the point's own field values upt (hoop terms), and its
+// element data: f_xi / f_eta per component, the direct (hoop) terms, and for
 // axis points of axial elements the axis terms g xi_r, g eta_r (stored at
-// row j of gx*/gy*).  The body of each reference kernel's first loop.
-// ECOEF: the element's coefficients come in as ec0 / ec1 (the material is
-// one per element, so every point of it carries the same coefficients; the
-// caller reads them once) instead of from blk.coef0 / coef1 per point.
-template <int NG, int KIND, bool ELASTIC, int M, bool ECOEF = false>
-__device__ __forceinline__ void point_flux(const BlockDev& blk, int bb, int kpt, int i, int j, bool axial,
-                                           const float* uxi, const float* ueta, const float* upt, float* fx,
-                                           float* fy, float* direct, float* gx0, float* gy0, float* gx1,
-                                           float* gy1, float w2k, float ec0 = 0.0f, float ec1 = 0.0f) {
-  constexpr int NPE = NG * NG;
-  constexpr int CS = point_stride<NPE>();
+// row j of gx*/gy*, AS floats apart).  The body of each reference kernel's
+// first loop.
+template <int NG, int KIND, bool ELASTIC, int M, int AS = 1>
+__device__ __forceinline__ void point_flux(const PointData& pd, int i, int j, bool axial, const float* uxi,
+                                           const float* ueta, const float* upt, float* fx, float* fy, float* direct,
+                                           float* gx0, float* gy0, float* gx1, float* gy1, float w2k) {
   if constexpr (KIND != INSEM_AXISYM) {
-    float xi_x, xi_z, eta_x, eta_z, jac;
-    load_metric<KIND, NPE>(blk.metric, bb, kpt, xi_x, xi_z, eta_x, eta_z, jac);
-    const size_t p = static_cast<size_t>(bb) * CS + kpt;
+    const float xi_x = pd.xi_x, xi_z = pd.xi_z, eta_x = pd.eta_x, eta_z = pd.eta_z, jac = pd.jac;
     if constexpr (ELASTIC) {
       // elastic_kernel (kernels.cpp:64-120)
       float ux_x, ux_z, uz_x, uz_z;
@@ -204,7 +212,7 @@ __device__ __forceinline__ void point_flux(const BlockDev& blk, int bb, int kpt,
         phys_grad(uxi[1], ueta[1], xi_x, xi_z, eta_x, eta_z, uz_x, uz_z);
       }
       float sxx, szz, sxz;
-      el_stress((ECOEF ? ec0 : blk.coef0[p]), (ECOEF ? ec1 : blk.coef1[p]), ux_x, ux_z, uz_x, uz_z, sxx, szz, sxz);
+      el_stress(pd.c0, pd.c1, ux_x, ux_z, uz_x, uz_z, sxx, szz, sxz);
       const float wj = fmul(w2k, jac);
       if constexpr (KIND == INSEM_RECT) {
         fx[0] = fmul(fmul(wj, sxx), xi_x);
@@ -217,7 +225,7 @@ __device__ __forceinline__ void point_flux(const BlockDev& blk, int bb, int kpt,
       }
     } else {
       // acoustic_kernel (kernels.cpp:122-158)
-      const float c = fmul(fmul(w2k, jac), (ECOEF ? ec0 : blk.coef0[p]));
+      const float c = fmul(fmul(w2k, jac), pd.c0);
       if constexpr (KIND == INSEM_RECT) {
         fx[0] = fmul(fmul(fmul(c, uxi[0]), xi_x), xi_x);
         fy[0] = fmul(fmul(fmul(c, ueta[0]), eta_z), eta_z);
@@ -228,18 +236,16 @@ __device__ __forceinline__ void point_flux(const BlockDev& blk, int bb, int kpt,
       }
     }
   } else {
-    const size_t p = static_cast<size_t>(bb) * CS + kpt;
-    const float* mt = blk.metric + static_cast<size_t>(bb) * 4 * CS + kpt;
-    const float xi_r = mt[0], xi_z = mt[CS], eta_r = mt[2 * CS], eta_z = mt[3 * CS];
+    const float xi_r = pd.xi_x, xi_z = pd.xi_z, eta_r = pd.eta_x, eta_z = pd.eta_z;
     const bool axis_pt = axial && i == 0;
     if constexpr (ELASTIC && M == 0) {
       // elastic_axisym_kernel (kernels.cpp:206-263)
       float ur_r, ur_z, uz_r, uz_z;
       phys_grad(uxi[0], ueta[0], xi_r, xi_z, eta_r, eta_z, ur_r, ur_z);
       phys_grad(uxi[1], ueta[1], xi_r, xi_z, eta_r, eta_z, uz_r, uz_z);
-      const float r = blk.r[p];
+      const float r = pd.r;
       const float e_tt = r == 0.0f ? ur_r : __fdiv_rn(upt[0], r);
-      const float lambda = (ECOEF ? ec0 : blk.coef0[p]), mu = (ECOEF ? ec1 : blk.coef1[p]);
+      const float lambda = pd.c0, mu = pd.c1;
       const float tr = fadd(fadd(ur_r, uz_z), e_tt);
       const float two_mu = fmul(2.0f, mu);
       const float ltr = fmul(lambda, tr);
@@ -247,22 +253,22 @@ __device__ __forceinline__ void point_flux(const BlockDev& blk, int bb, int kpt,
       const float szz = fadd(ltr, fmul(two_mu, uz_z));
       const float stt = fadd(ltr, fmul(two_mu, e_tt));
       const float srz = fmul(mu, fadd(ur_z, uz_r));
-      const float w = blk.wr[p];
+      const float w = pd.wr;
       ref_flux(w, srr, srz, xi_r, xi_z, eta_r, eta_z, fx[0], fy[0]);
       ref_flux(w, srz, szz, xi_r, xi_z, eta_r, eta_z, fx[1], fy[1]);
       if (axis_pt) {
         direct[0] = 0.0f;
         const float g = fmul(w, stt);
-        gx0[j] = fmul(g, xi_r);
-        gy0[j] = fmul(g, eta_r);
+        gx0[j * AS] = fmul(g, xi_r);
+        gy0[j * AS] = fmul(g, eta_r);
       } else {
-        direct[0] = fmul(blk.hoop[p], stt);
+        direct[0] = fmul(pd.hoop, stt);
       }
     } else if constexpr (!ELASTIC && M == 0) {
       // acoustic_axisym_kernel (kernels.cpp:265-294)
       float p_r, p_z;
       phys_grad(uxi[0], ueta[0], xi_r, xi_z, eta_r, eta_z, p_r, p_z);
-      ref_flux(fmul(blk.wr[p], (ECOEF ? ec0 : blk.coef0[p])), p_r, p_z, xi_r, xi_z, eta_r, eta_z, fx[0], fy[0]);
+      ref_flux(fmul(pd.wr, pd.c0), p_r, p_z, xi_r, xi_z, eta_r, eta_z, fx[0], fy[0]);
     } else if constexpr (ELASTIC && M == 1) {
       // elastic_axisym1_kernel (kernels.cpp:305-385)
       const float s2 = 1.41421356237309504880f;
@@ -271,14 +277,14 @@ __device__ __forceinline__ void point_flux(const BlockDev& blk, int bb, int kpt,
       phys_grad(uxi[0], ueta[0], xi_r, xi_z, eta_r, eta_z, up_r, up_z);
       phys_grad(uxi[1], ueta[1], xi_r, xi_z, eta_r, eta_z, um_r, um_z);
       phys_grad(uxi[2], ueta[2], xi_r, xi_z, eta_r, eta_z, uz_r, uz_z);
-      const float r = blk.r[p];
+      const float r = pd.r;
       const bool on_axis = r == 0.0f;
       const float up_over_r = on_axis ? up_r : __fdiv_rn(upt[0], r);
       const float uz_over_r = on_axis ? uz_r : __fdiv_rn(upt[2], r);
       const float ur_r = fmul(fadd(up_r, um_r), is2), ur_z = fmul(fadd(up_z, um_z), is2);
       const float ut_r = fmul(fsub(up_r, um_r), is2), ut_z = fmul(fsub(up_z, um_z), is2);
       const float e_tt = fmul(s2, up_over_r);
-      const float lambda = (ECOEF ? ec0 : blk.coef0[p]), mu = (ECOEF ? ec1 : blk.coef1[p]);
+      const float lambda = pd.c0, mu = pd.c1;
       const float tr = fadd(fadd(ur_r, uz_z), e_tt);
       const float two_mu = fmul(2.0f, mu);
       const float ltr = fmul(lambda, tr);
@@ -288,7 +294,7 @@ __device__ __forceinline__ void point_flux(const BlockDev& blk, int bb, int kpt,
       const float srz = fmul(mu, fadd(ur_z, uz_r));
       const float srt = fmul(mu, fsub(ut_r, fmul(s2, up_over_r)));
       const float stz = fmul(mu, fsub(ut_z, uz_over_r));
-      const float w = blk.wr[p];
+      const float w = pd.wr;
       ref_flux(w, fmul(fadd(srr, srt), is2), fmul(fadd(srz, stz), is2), xi_r, xi_z, eta_r, eta_z, fx[0], fy[0]);
       ref_flux(w, fmul(fsub(srr, srt), is2), fmul(fsub(srz, stz), is2), xi_r, xi_z, eta_r, eta_z, fx[1], fy[1]);
       ref_flux(w, srz, szz, xi_r, xi_z, eta_r, eta_z, fx[2], fy[2]);
@@ -298,28 +304,28 @@ __device__ __forceinline__ void point_flux(const BlockDev& blk, int bb, int kpt,
         direct[0] = 0.0f;
         direct[1] = 0.0f;
         const float gp = fmul(w, cp), gz = fmul(w, cz);
-        gx0[j] = fmul(gp, xi_r);
-        gy0[j] = fmul(gp, eta_r);
-        gx1[j] = fmul(gz, xi_r);
-        gy1[j] = fmul(gz, eta_r);
+        gx0[j * AS] = fmul(gp, xi_r);
+        gy0[j * AS] = fmul(gp, eta_r);
+        gx1[j * AS] = fmul(gz, xi_r);
+        gy1[j * AS] = fmul(gz, eta_r);
       } else {
-        direct[0] = fmul(blk.hoop[p], cp);
-        direct[1] = fmul(blk.hoop[p], cz);
+        direct[0] = fmul(pd.hoop, cp);
+        direct[1] = fmul(pd.hoop, cz);
       }
     } else {
       // acoustic_axisym1_kernel (kernels.cpp:389-431)
       float p_r, p_z;
       phys_grad(uxi[0], ueta[0], xi_r, xi_z, eta_r, eta_z, p_r, p_z);
-      const float inv_rho = (ECOEF ? ec0 : blk.coef0[p]);
-      const float wri = fmul(blk.wr[p], inv_rho);
+      const float inv_rho = pd.c0;
+      const float wri = fmul(pd.wr, inv_rho);
       ref_flux(wri, p_r, p_z, xi_r, xi_z, eta_r, eta_z, fx[0], fy[0]);
       if (axis_pt) {
         direct[0] = 0.0f;
         const float g = fmul(wri, p_r);
-        gx0[j] = fmul(g, xi_r);
-        gy0[j] = fmul(g, eta_r);
+        gx0[j * AS] = fmul(g, xi_r);
+        gy0[j * AS] = fmul(g, eta_r);
       } else {
-        direct[0] = __fdiv_rn(fmul(fmul(blk.hoop[p], inv_rho), upt[0]), blk.r[p]);
+        direct[0] = __fdiv_rn(fmul(fmul(pd.hoop, inv_rho), upt[0]), pd.r);
       }
     }
   }
@@ -330,21 +336,21 @@ __device__ __forceinline__ void point_flux(const BlockDev& blk, int bb, int kpt,
 // column update (f -= g_jq eta_r Dy[jq][ja]) reaches column 0 for every jq,
 // after that jq's row update.  dx_row0 = Dx[ia] (row 0 of Dx); dy(q) =
 // Dy[q] with q = jq * NG + ja.
-template <int NG, class DyFn>
+template <int NG, int AS, class DyFn>
 __device__ __forceinline__ float axis_spread(float f, int ia, int ja, float dx_row0, DyFn dy, const float* gx,
                                              const float* gy) {
-  if (ia != 0) return fsub(f, fmul(gx[ja], dx_row0));
+  if (ia != 0) return fsub(f, fmul(gx[ja * AS], dx_row0));
 #pragma unroll
   for (int jq = 0; jq < NG; ++jq) {
-    if (jq == ja) f = fsub(f, fmul(gx[jq], dx_row0));
-    f = fsub(f, fmul(gy[jq], dy(jq * NG + ja)));
+    if (jq == ja) f = fsub(f, fmul(gx[jq * AS], dx_row0));
+    f = fsub(f, fmul(gy[jq * AS], dy(jq * NG + ja)));
   }
   return f;
 }
 
 // Force of one element point from its weak divergence sums s[c] (the second
 // loop of each reference kernel): negation, hoop term, axis spread.
-template <int NG, int KIND, bool ELASTIC, int M, class DyFn>
+template <int NG, int KIND, bool ELASTIC, int M, int AS = 1, class DyFn>
 __device__ __forceinline__ void point_divergence(int i, int j, bool axial, const float* s, const float* direct,
                                                  float dx_row0, DyFn dy, const float* gx0, const float* gy0,
                                                  const float* gx1, const float* gy1, float* out) {
@@ -355,7 +361,7 @@ __device__ __forceinline__ void point_divergence(int i, int j, bool axial, const
   } else if constexpr (ELASTIC && M == 0) {
     out[0] = -fadd(s[0], direct[0]);
     out[1] = -s[1];
-    if (axial) out[0] = axis_spread<NG>(out[0], i, j, dx_row0, dy, gx0, gy0);
+    if (axial) out[0] = axis_spread<NG, AS>(out[0], i, j, dx_row0, dy, gx0, gy0);
   } else if constexpr (!ELASTIC && M == 0) {
     out[0] = -s[0];
   } else if constexpr (ELASTIC && M == 1) {
@@ -363,12 +369,12 @@ __device__ __forceinline__ void point_divergence(int i, int j, bool axial, const
     out[1] = -s[1];
     out[2] = -fadd(s[2], direct[1]);
     if (axial) {
-      out[0] = axis_spread<NG>(out[0], i, j, dx_row0, dy, gx0, gy0);
-      out[2] = axis_spread<NG>(out[2], i, j, dx_row0, dy, gx1, gy1);
+      out[0] = axis_spread<NG, AS>(out[0], i, j, dx_row0, dy, gx0, gy0);
+      out[2] = axis_spread<NG, AS>(out[2], i, j, dx_row0, dy, gx1, gy1);
     }
   } else {
     out[0] = -fadd(s[0], direct[0]);
-    if (axial) out[0] = axis_spread<NG>(out[0], i, j, dx_row0, dy, gx0, gy0);
+    if (axial) out[0] = axis_spread<NG, AS>(out[0], i, j, dx_row0, dy, gx0, gy0);
   }
 }
 
@@ -389,8 +395,8 @@ __device__ __forceinline__ void element_fluxes(const BlockDev& blk, int bb, int 
     ref_derivs<NG>(Dx, Dy, su[c], i, j, uxi[c], ueta[c]);
     upt[c] = su[c][kpt];
   }
-  point_flux<NG, KIND, ELASTIC, M>(blk, bb, kpt, i, j, axial, uxi, ueta, upt, fx, fy, direct, gx0, gy0, gx1, gy1,
-                                   w2[kpt]);
+  point_flux<NG, KIND, ELASTIC, M>(load_point<KIND, ELASTIC, C::NPE>(blk, bb, kpt), i, j, axial, uxi, ueta, upt, fx, fy,
+                                   direct, gx0, gy0, gx1, gy1, w2[kpt]);
 #pragma unroll
   for (int c = 0; c < C::NC; ++c) {
     f1[c][kpt] = fx[c];

@@ -910,7 +910,7 @@ void Solver::build_tiled(const insem_cuda_problem& p) {
         kind = kv.first;
       }
     const int te = choose_tile_elements(ngll, kind, d.medium == INSEM_ELASTIC, kind == INSEM_AXISYM ? d.azimuthal_order : 0,
-                                        d.ncomp, opts.tile_elements);
+                                        opts.tile_elements);
     tdom[di].build(d, ngll, te, terms,
                    host_vec(d.absorbing_coef, static_cast<std::size_t>(d.n_absorbing) * d.ncomp * d.ncomp));
   }
@@ -1283,10 +1283,10 @@ int insem_cuda_set_tile_elements(int32_t ngll, int32_t kind, int32_t medium, int
   });
 }
 
-int32_t insem_cuda_tile_elements(int32_t ngll, int32_t kind, int32_t medium, int32_t azimuthal_order, int32_t ncomp) {
+int32_t insem_cuda_tile_elements(int32_t ngll, int32_t kind, int32_t medium, int32_t azimuthal_order, int32_t) {
   int32_t out = 0;
   guarded([&] {
-    out = choose_tile_elements(ngll, kind, medium == INSEM_ELASTIC, kind == INSEM_AXISYM ? azimuthal_order : 0, ncomp, 0);
+    out = choose_tile_elements(ngll, kind, medium == INSEM_ELASTIC, kind == INSEM_AXISYM ? azimuthal_order : 0, 0);
   });
   return out;
 }

@@ -11,18 +11,22 @@
 // buffer; a halo kernel finishes those points with the full reference logic.
 //
 // Bitwise parity with the reference: each point's contributions are summed
-// in ascending slot order (DofMap::assemble, dof_map.hpp:123-141).  Inside a
-// tile, slot s of point p carries its rank (position of s in p's ascending
-// slot list); ranks are accumulated phase by phase (rank 0 stores 0 + f,
-// rank r adds), so the sum is the reference's.  Halo points sum their halo
-// buffer entries in the reference's slot order from a CSR list.
+// in ascending slot order (DofMap::assemble, dof_map.hpp:123-141).  A complete
+// point inside an element has one contribution, which its own thread adds to
+// 0; a complete point on element edges has a list of places, in that order,
+// of its contributions in shared memory; halo points sum their halo buffer
+// entries in the reference's slot order from a CSR list.
 //
-// Element math: one thread per element column i (NG threads per element).
-// A column thread holds its column of the field, its f_eta column and the
-// xi-row / xi-column of the basis derivative matrix in registers; rows of the
-// field and of f_xi come from shared memory as broadcasts within an
-// element; D entries indexed by the unrolled loop counters come from the
-// constant bank.  Every sum keeps the reference's operand order.
+// Element math: a lane holds an element and a warp a column: warp i of a CTA
+// computes column i (points i, NG + i, ...) of the tile's up to 32 elements.
+// All data of a tile lie element-minor, [...][32], so every access of a warp
+// to shared memory is free of bank conflicts and every access to global
+// memory is coalesced, and the warps of inner columns finish their inner
+// points (56 - 69 % of a tile's points at NG 5 - 7) in registers: field and
+// velocity come straight from global memory, nothing is staged or listed.
+// The elements' data arrive in one bulk copy; D entries indexed by the
+// unrolled loop counters come from the constant bank.  Every sum keeps the
+// reference's operand order.
 #pragma once
 
 #include <cstddef>
@@ -35,9 +39,6 @@ namespace insem_b200 {
 
 // GLL derivative matrix, GLJ derivative matrix and w_i w_j per ngll (2..9).
 static __constant__ float c_basis[8][3][81];
-
-// Both components of an interleaved pair in one 64-bit shared-memory load.
-__device__ __forceinline__ float2 pair_load(const float* p) { return *reinterpret_cast<const float2*>(p); }
 
 // Two-lane FP32 arithmetic on a component pair (sm_100 add/fma .f32x2).  Each
 // lane rounds exactly like the scalar instruction.  The assembler fuses a
@@ -69,50 +70,40 @@ __device__ __forceinline__ f2x mul2(f2x a, f2x b, f2x nz) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(nz));
   return d;
 }
-__device__ __forceinline__ f2x pair_load2(const float* p) { return *reinterpret_cast<const f2x*>(p); }
-
-// Element stride (floats) of the field / xi-flux rows in shared memory.
-// Two components are stored interleaved, row j of element e at
-// e * stride + j * 2 * ngll, (l, c) at + 2 l + c, so one 64-bit load gives
-// both; the stride is padded so that the elements one warp reads fall on
-// distinct 64-bit bank pairs.  Other component counts keep
-// [component][row][ROW].
-__host__ __device__ constexpr int rows_elem_stride(int ng, int nc) {
-  if (nc != 2) return nc * ng * ((ng + 1) & ~1);
-  const int base = 2 * ng * ng;
-  const int per_warp = 32 / ng + 2;
-  for (int s = base; s < base + 64; s += 2) {
-    bool ok = true;
-    for (int a = 0; a < per_warp && ok; ++a)
-      for (int b = a + 1; b < per_warp && ok; ++b) {
-        const int da = (a * s) % 32, db = (b * s) % 32;
-        if (da == db || (da + 1) % 32 == db || (db + 1) % 32 == da) ok = false;
-      }
-    if (ok) return s;
-  }
-  return base;
+// a * d rounded once per lane, for a d that the compiler takes from the
+// constant bank: two scalar products, no packing of (d, d)
+__device__ __forceinline__ f2x mulc2(f2x a, float d) {
+  const float2 v = upk2(a);
+  return pk2(fmul(v.x, d), fmul(v.y, d));
 }
 
-// Slot descriptor bits.
-constexpr uint32_t kSlotPointMask = 0xffffu;      // tile point index
-constexpr int kSlotRankShift = 16;                // local assembly rank (0..254)
-constexpr uint32_t kSlotRankNone = 0xffu;          // not assembled in the tile
-constexpr uint32_t kSlotConstrained = 1u << 24;   // value from the constrained-slot list
-constexpr uint32_t kSlotLast = 1u << 25;          // the highest rank of its (complete) point
+// Floats per element of the field / xi-flux rows: [component][point].
+__host__ __device__ constexpr int rows_elem_stride(int ng, int nc) { return nc * ng * ng; }
 
+constexpr int kTileLanes = 32;  // elements of a tile (at most)
+
+// Slot descriptors (uint16 per element slot, [tile][point][lane]): the tile
+// point that holds the slot's value.  Inner slots of direct elements have none.
+constexpr uint32_t kSlotConstrained = 0xffffu;  // the field row is filled from the constrained-slot list
+
+// Tile points: the tile's complete points on element edges first, then the
+// halo points it reads.  A direct element is one whose inner points are all
+// complete points of the tile; its lanes finish them in registers.
 struct TileHdr {
-  int32_t be0;     // first element of the tile (block-local, tile order)
+  int32_t tb;      // tile index in its block (element data, coefficients, axial flags)
   int32_t ne;      // elements
-  int32_t cbeg;    // first complete point (device numbering)
-  int32_t nc;      // complete points
-  int32_t ntp;     // tile points: nc complete + halo points the tile reads
+  int32_t nd;      // direct elements: lanes [0, nd)
+  int32_t cbeg;    // first inner point (device numbering); (i, j) of the lane's element: ((i - 1) (NG - 2) + j - 1) 32 + lane
+  int32_t ebeg;    // first edge complete point
+  int32_t nc;      // edge complete points
+  int32_t ntp;     // tile points: nc + halo points the tile reads
   int32_t hl_off;  // offset of the halo tile points in halo_tp
-  int32_t hb;      // first halo-buffer entry of the tile
   int32_t nhs;     // halo slots (entries written to the halo buffer)
-  int32_t hs_off;  // offset into hs_slot
+  int32_t hs_off;  // offset into hs_slot / hs_dst
   int32_t ncs;     // constrained slots of the tile
   int32_t cs_off;  // offset into cs_slot / cs_row
-  int32_t maxrank; // highest local rank
+  int32_t pl_off;  // offset of the edge points' place lists (points; roundup(nc, 4) of them)
+  int32_t pad;
 };
 
 // One domain of the tiled path, in device numbering.
@@ -120,6 +111,7 @@ struct TiledDev {
   int32_t ng = 0;          // points
   int32_t n_complete = 0;  // complete points are [0, n_complete)
   int32_t n_hbuf = 0;      // halo contributions (per component): the halo points' lists, point by point
+  int32_t rs = 4;          // places per list of an edge complete point
   const float* inv_mass = nullptr;
   const float* mass = nullptr;
   const float* u_cur = nullptr;
@@ -127,14 +119,15 @@ struct TiledDev {
   float* v = nullptr;
   float* a = nullptr;
   float* vn = nullptr;     // v^n at halo points (receivers)
-  const uint32_t* sdesc = nullptr;  // [n_el_tiles * npe] slot descriptors, tile order
+  const uint16_t* sdesc = nullptr;  // [tile][npe][32] slot descriptors
+  const uint16_t* plist = nullptr;  // [edge point][rs] staging places in rank order, kLastPlace on the last
   const TileHdr* tiles = nullptr;
   const int32_t* halo_tp = nullptr; // device point of each halo tile point
-  const int32_t* hs_slot = nullptr; // tile-local slot (e * npe + k) of each halo entry
+  const int32_t* hs_slot = nullptr; // staging place (point * 32 + lane) of each halo entry
   const int32_t* hs_dst = nullptr;  // its place in hbuf, or -1 - m: the places mdst[mdst_off[m] ..)
   const int32_t* mdst_off = nullptr;  // entries with several places (constrained slots feeding several points)
   const int32_t* mdst = nullptr;
-  const int32_t* cs_slot = nullptr; // tile-local slot of each constrained slot
+  const int32_t* cs_slot = nullptr; // staging place of each constrained slot
   const int2* cs_row = nullptr;     // its constraint row: entries [x, y) of row_dofs / row_w
   const int32_t* row_dofs = nullptr;
   const float* row_w = nullptr;
@@ -146,18 +139,33 @@ struct StepScalars {
   int32_t energy_every;
 };
 
-// Tile elements are chosen per domain at run time (te <= TE, one thread per
-// element column).  CTAs are whole warps: te x NG threads rounded up to a
-// multiple of 32 (the extra threads have no element and only take part in the
-// strided loops, the barriers and the warp reductions).
+constexpr uint32_t kLastPlace = 0x8000u;
+
+// A CTA has one warp per element column and one lane per element; tiles of
+// fewer elements than lanes leave lanes idle.
 template <int NG>
 struct TileCfg {
   static constexpr int NPE = NG * NG;
-  static constexpr int TE = (256 / NG) > 64 ? 64 : (256 / NG);  // elements per tile (max)
-  static constexpr int THREADS = (TE * NG + 31) / 32 * 32;       // threads per CTA (max)
-  static constexpr int ROW = (NG + 1) & ~1;                      // padded row stride (floats)
+  static constexpr int TE = kTileLanes;            // elements per tile (max)
+  static constexpr int THREADS = kTileLanes * NG;  // threads per CTA
 };
-__host__ __device__ constexpr int tile_threads(int te, int ng) { return (te * ng + 31) / 32 * 32; }
+
+// Element data of a tile.  Kinds whose metric varies in an element: pairs
+// [point][32][2] of (xi_x, xi_z), (eta_x, eta_z) and, axisymmetric, (wr, hoop),
+// then one plane [point][32] of the Jacobian (Curved) or r (axisymmetric: the
+// fluxes use the Jacobian only through wr).  Rect and Affine: [array][32] of
+// xi_x, eta_z, jac or xi_x, xi_z, eta_x, eta_z, jac.
+__host__ __device__ constexpr int tile_arrays(int kind) {
+  return kind == INSEM_RECT ? 3 : kind == INSEM_AXISYM ? 7 : 5;
+}
+__host__ __device__ constexpr bool tile_data_staged(int kind) { return kind == INSEM_CURVED || kind == INSEM_AXISYM; }
+__host__ __device__ constexpr int tile_data_floats(int kind, int npe) {
+  return tile_arrays(kind) * (tile_data_staged(kind) ? npe : 1) * kTileLanes;
+}
+// Offset (floats) of array a at point place p = point * 32 + lane (staged kinds).
+__host__ __device__ constexpr int tile_data_at(int kind, int npe, int a, int p) {
+  return a == tile_arrays(kind) - 1 ? a * npe * kTileLanes + p : (a / 2) * 2 * npe * kTileLanes + 2 * p + a % 2;
+}
 
 __device__ __forceinline__ float cbasis(int ng, int which, int idx) { return c_basis[ng - 2][which][idx]; }
 
@@ -206,88 +214,63 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 }
 constexpr uint32_t kBulkWaitLimit = 1u << 22;
 
-// Whether a class writes its f_xi rows as the fluxes are formed (into a
-// region of their own, fewer registers held across the barrier) instead of
-// after the barrier into the dead element data (less shared memory).  Only
-// three-component classes, and of the benchmarked orders only ngll 6, gain
-// from it under their register budgets (256-model batch, per class: ngll 6
-// m=1 0.147 vs 0.154 ms early vs late; ngll 5 0.106 vs 0.103; ngll 7 0.229
-// vs 0.224).
-__host__ __device__ constexpr bool early_flux_rows(int ng, int nc) { return nc == 3 && ng != 5 && ng != 7; }
+// Whether a class with staged element data keeps its f_xi rows outside it: no
+// class does.  A point's element data are read by one thread only, which
+// writes its f_xi over them: pairs of components over (xi_x, xi_z), the only or
+// third component over the last plane.
+__host__ __device__ constexpr bool early_flux_rows(int, int) { return false; }
 
 // Shared-memory layout of one tile CTA, byte offsets (16-byte aligned).
-// Per-tile data arrives by bulk copies: element data (metric, axisymmetric
-// weights), slot descriptors, and the complete points' u, v and inverse mass
-// (v and 1/M later, when `late`); halo tile points are gathered by the
-// threads into the u region after the complete points (at index
-// roundup(nc, 4) on).  The material coefficients (one pair per element) and
-// the slot descriptors (which each column thread keeps in registers) are read
-// from global memory by the threads that use them.  `pl` holds, for every
-// complete point, the staging places of its contributions in rank order
-// (`rs` entries per point, uint16).
+// `u` holds the tile points' field [component][tp_cap]; `su` the field rows
+// and later the slots' contributions, `sfx` the f_xi rows: component pairs
+// [point][32][2], then a single component [point][32].  `v`, `im` and `pl` (the
+// place lists) of the edge complete points arrive with the first copies, or
+// with a second set once the fluxes are formed (`late`): into the element data
+// between the pairs and the last plane, which hold the f_xi rows then.
 struct TileLayout {
   uint32_t bar, metric, wr, hoop, r, u, v, im, pl, su, sfx, ax, total;
-  int32_t tp_cap, nc_cap, ms, cs, row, rs;
-  int32_t late;  // 1: v and 1/M arrive by a second copy into the element-data region
+  int32_t tp_cap, nc_cap, rs;
+  int32_t late;
 
   __host__ __device__ static uint32_t up16(uint32_t x) { return (x + 15u) & ~15u; }
-  // rs: the most contributions one complete point of the class's tiles has
-  __host__ __device__ static TileLayout make(int ng, int nc, int kind, bool elastic, int te, int tp_cap, int nc_cap,
+  // rs: the most contributions one edge complete point of the class's tiles has
+  __host__ __device__ static TileLayout make(int ng, int nc, int kind, bool elastic, int /*te*/, int tp_cap, int nc_cap,
                                             int rs) {
     TileLayout L{};
     L.rs = (rs + 3) & ~3;  // a point's list is read four entries (8 bytes) at a time
-    const int npe = ng * ng;
-    L.cs = (npe + 3) & ~3;
-    L.ms = kind == INSEM_RECT ? 4 : kind == INSEM_AFFINE ? 8 : (kind == INSEM_AXISYM ? 4 : 5) * L.cs;
-    L.row = (ng + 1) & ~1;
+    const uint32_t npe = static_cast<uint32_t>(ng * ng), plane = npe * kTileLanes * 4u;
     L.tp_cap = tp_cap;
     L.nc_cap = nc_cap;
-    const bool axi = kind == INSEM_AXISYM;
+    const bool axi = kind == INSEM_AXISYM, staged = tile_data_staged(kind);
     uint32_t o = 0;
-    L.bar = o;  // two mbarriers: the tile's copies, the late v and 1/M copies
+    L.bar = o;  // two mbarriers: the first copies, the late ones
     o = up16(o + 16);
     L.metric = o;
-    o = up16(o + 4u * te * L.ms);
-    L.wr = o;
-    if (axi) o = up16(o + 4u * te * L.cs);
-    L.hoop = o;
-    if (axi) o = up16(o + 4u * te * L.cs);
-    L.r = o;
-    if (axi) o = up16(o + 4u * te * L.cs);
-    // The element data [metric, elem_end) is last read by the fluxes.  Then
-    // that region takes, when it is large enough, the f_xi rows (written
-    // after the fluxes, read by the divergence) and beside them v and 1/M
-    // (copied in after the fluxes); the point lists (written after the
-    // divergence) take the place of the f_xi rows.
+    L.wr = L.hoop = L.r = o;
+    if (axi) {
+      L.wr = L.hoop = o + 4 * plane;
+      L.r = o + 6 * plane;
+    }
+    if (staged) o += 4u * tile_data_floats(kind, static_cast<int>(npe));
     const uint32_t elem = o - L.metric;
     L.u = o;
     o = up16(o + 4u * nc * tp_cap);
     L.su = o;
-    const uint32_t rows = static_cast<uint32_t>(rows_elem_stride(ng, nc));
-    // su doubles as the halo staging area: [te][nc][npe]
-    o = up16(o + 4u * te * (rows > static_cast<uint32_t>(nc * npe) ? rows : static_cast<uint32_t>(nc * npe)));
-    const uint32_t sfx_b = up16(4u * te * rows);
-    // classes that write their f_xi rows as the fluxes are formed
-    // (early_flux_rows) cannot keep them in the element data the fluxes
-    // still read
-    if (sfx_b <= elem && !early_flux_rows(ng, nc)) {
-      L.sfx = L.metric;
-    } else {
-      L.sfx = o;
-      o += sfx_b;
-    }
-    const uint32_t pl_b = up16(2u * L.rs * nc_cap), v_b = up16(4u * nc * nc_cap), im_b = up16(4u * nc_cap);
-    const uint32_t sfx_in = L.sfx == L.metric ? sfx_b : 0u;  // f_xi rows inside the element data
-    const uint32_t head = pl_b > sfx_in ? pl_b : sfx_in;
-    L.late = head + v_b + im_b <= elem ? 1 : 0;
-    uint32_t p = L.late ? L.metric : o;
-    L.pl = p;
-    L.v = p + (L.late ? head : pl_b);
+    const uint32_t rows = plane * nc;
+    o += rows;
+    L.sfx = staged ? L.metric : o;
+    if (!staged) o += rows;
+    const uint32_t v_b = up16(4u * nc * nc_cap), im_b = up16(4u * nc_cap), pl_b = up16(2u * L.rs * nc_cap);
+    L.late = staged && rows + v_b + im_b + pl_b + plane <= elem ? 1 : 0;
+    L.v = L.late ? L.metric + rows : o;
     L.im = L.v + v_b;
-    if (!L.late) o += pl_b + v_b + im_b;
+    L.pl = L.im + im_b;
+    if (!L.late) o += v_b + im_b + pl_b;
+    // axis terms (gx, gy of up to two components) [4][ng][32], ng rounded up to 4
     L.ax = o;
-    if (axi) o = up16(o + 4u * te * 4 * ((ng + 3) & ~3));
+      if (axi) o += 4u * 4u * ((ng + 3) & ~3) * kTileLanes;
     L.total = o;
+    (void)elastic;
     return L;
   }
 };
@@ -340,6 +323,41 @@ static __global__ void begin_span_kernel(SpanField f0, SpanField f1, float rdt, 
   }
 }
 
+// Field rows in shared memory: components 0 and 1 as pairs, the only or third
+// component in a plane of its own behind them.
+// (AT: its offset, for rows kept in the element data).
+template <int NC, int NPE, int AT = -1>
+struct Rows {
+  static constexpr bool PAIR = NC >= 2, ONE = NC != 2;
+  static constexpr int ONE_AT = AT >= 0 ? AT : PAIR ? 2 * NPE * kTileLanes : 0;
+  static constexpr int ONE_C = NC == 3 ? 2 : 0;  // the component of the single plane
+  // place = point * 32 + lane
+  __device__ __forceinline__ static void store(float* rows, int place, const float* x) {
+    if constexpr (PAIR) *reinterpret_cast<float2*>(rows + 2 * place) = make_float2(x[0], x[1]);
+    if constexpr (ONE) rows[ONE_AT + place] = x[ONE_C];
+  }
+  __device__ __forceinline__ static f2x pair(const float* rows, int place) {
+    return *reinterpret_cast<const f2x*>(rows + 2 * place);
+  }
+  __device__ __forceinline__ static float one(const float* rows, int place) { return rows[ONE_AT + place]; }
+  __device__ __forceinline__ static void load(const float* rows, int place, float* x) {
+    if constexpr (PAIR) {
+      const float2 v = *reinterpret_cast<const float2*>(rows + 2 * place);
+      x[0] = v.x;
+      x[1] = v.y;
+    }
+    if constexpr (ONE) x[ONE_C] = rows[ONE_AT + place];
+  }
+};
+
+// Energy terms of one component of a point (solver.cpp:673-678, 900-915).
+__device__ __forceinline__ void add_energy(double& kin, double& pot, float u, float f, float v_n, float a, double m,
+                                           double kin_c) {
+  pot = dadd(pot, dmul(static_cast<double>(u), static_cast<double>(f)));
+  const double vv = v_n, aa = a;
+  kin = dadd(kin, dmul(m, dsub(dmul(dmul(0.5, vv), vv), dmul(dmul(kin_c, aa), aa))));
+}
+
 // One tile of the fused step (the whole CTA).  `thp` is the tile's header
 // (entry `tile` of the domain's tile table, or a copy of it).  `g_first`, if
 // not negative, is this thread's first halo tile point (halo_tp entry
@@ -355,96 +373,112 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
                                                double* __restrict__ epartial, int32_t tile, const TileHdr* thp,
                                                const TileLayout& L, unsigned char* smem_raw, uint64_t* bar,
                                                uint32_t phase, int32_t g_first = -1) {
-  using Cfg = TileCfg<NG>;
   using CE = ElemCfg<NG, KIND, EL, M>;
   constexpr int NC = CE::NC;
   constexpr int NPE = NG * NG;
-  constexpr int CS = point_stride<NPE>();
-  constexpr int ROW = Cfg::ROW;
-  constexpr bool AXI = KIND == INSEM_AXISYM;
-  constexpr int MS = KIND == INSEM_RECT ? 4 : KIND == INSEM_AFFINE ? 8 : (AXI ? 4 : 5) * CS;
-  float* s_metric = reinterpret_cast<float*>(smem_raw + L.metric);
-  float* s_wr = reinterpret_cast<float*>(smem_raw + L.wr);
-  float* s_hoop = reinterpret_cast<float*>(smem_raw + L.hoop);
-  float* s_r = reinterpret_cast<float*>(smem_raw + L.r);
-  float* tu = reinterpret_cast<float*>(smem_raw + L.u);    // [NC][tp_cap]
-  float* s_v = reinterpret_cast<float*>(smem_raw + L.v);   // [NC][nc_cap]
-  float* s_im = reinterpret_cast<float*>(smem_raw + L.im); // [nc_cap]
-  uint16_t* pl = reinterpret_cast<uint16_t*>(smem_raw + L.pl);  // [nc_cap][rs] staging places, rank order
-  float* su = reinterpret_cast<float*>(smem_raw + L.su);   // [TE][NC][NG][ROW] field rows, later staging
-  float* sfx = reinterpret_cast<float*>(smem_raw + L.sfx); // [TE][NC][NG][ROW] f_xi rows
-  float* sax = reinterpret_cast<float*>(smem_raw + L.ax);  // [TE][4][AXS] axis terms
+  constexpr int NI = NG - 2;  // inner points per direction
+  constexpr bool AXI = KIND == INSEM_AXISYM, STAGED = tile_data_staged(KIND);
+  constexpr int W = kTileLanes, NT = W * NG;
+  using R = Rows<NC, NPE>;
+  using F = Rows<NC, NPE, STAGED ? (tile_arrays(KIND) - 1) * NPE * W : -1>;  // the f_xi rows
+  const float* elem = reinterpret_cast<const float*>(smem_raw + L.metric);
+  float* tu = reinterpret_cast<float*>(smem_raw + L.u);          // [NC][tp_cap]
+  float* s_v = reinterpret_cast<float*>(smem_raw + L.v);         // [NC][nc_cap]
+  float* s_im = reinterpret_cast<float*>(smem_raw + L.im);       // [nc_cap]
+  uint16_t* pl = reinterpret_cast<uint16_t*>(smem_raw + L.pl);   // [nc_cap][rs] places, rank order
+  float* su = reinterpret_cast<float*>(smem_raw + L.su);         // field rows, later contributions
+  float* sfx = reinterpret_cast<float*>(smem_raw + L.sfx);       // f_xi rows
+  float* ax = reinterpret_cast<float*>(smem_raw + L.ax) + (threadIdx.x & (W - 1));  // axis terms [4][NG][W]
   const int tp_cap = L.tp_cap, nc_cap = L.nc_cap;
 
   const TileHdr th = *thp;
   const int tid = threadIdx.x;
-  const int nthreads = blockDim.x;  // (tile elements) x NG
+  const int lane = tid & (W - 1), i = tid / W;  // element, column
   // thread 0 issues the bulk copies; the halo tile points are gathered from
   // the last thread down, so thread 0 has the fewest of them
-  const int issuer = 0;
-  const int tg = nthreads - 1 - tid;
+  const int tg = NT - 1 - tid;
   const int mode = now.mode;
   const bool energy = energy_step(now, sc.energy_every);
   const int nc4 = (th.nc + 3) & ~3;
+  const uint32_t edge_b = 4u * nc4, list_b = 2u * td.rs * nc4;
 
-  // 1. bulk copies of the tile's element data, slot descriptors and complete
-  //    points (u; v and 1/M too unless they come late)
-  if (tid == issuer) {
-    const uint32_t eb = 4u * th.ne;
-    uint32_t total = eb * MS + eb * CS * (AXI ? 3 : 0);
-    if (nc4 > 0) total += 4u * nc4 * (L.late ? NC : 2 * NC + 1);
+  // 1. bulk copies of the element data, and of the edge complete points' u (v,
+  //    1/M and place lists too unless they come late)
+  if (tid == 0) {
+    constexpr uint32_t eb = STAGED ? 4u * tile_data_floats(KIND, NPE) : 0u;
     fence_proxy_async_smem();
-    mbar_expect_tx(bar, total);
-    bulk_load(s_metric, blk.metric + static_cast<size_t>(th.be0) * MS, eb * MS, bar);
-    if constexpr (AXI) {
-      bulk_load(s_wr, blk.wr + static_cast<size_t>(th.be0) * CS, eb * CS, bar);
-      bulk_load(s_hoop, blk.hoop + static_cast<size_t>(th.be0) * CS, eb * CS, bar);
-      bulk_load(s_r, blk.r + static_cast<size_t>(th.be0) * CS, eb * CS, bar);
+    mbar_expect_tx(bar, eb + edge_b * NC + (L.late ? 0u : edge_b * (NC + 1) + list_b));
+    if constexpr (STAGED) bulk_load(smem_raw + L.metric, blk.metric + static_cast<size_t>(th.tb) * (eb / 4u), eb, bar);
+    if (!L.late && nc4 > 0) {
+      bulk_load(s_im, td.inv_mass + th.ebeg, edge_b, bar);
+      bulk_load(pl, td.plist + static_cast<size_t>(th.pl_off) * td.rs, list_b, bar);
     }
   }
-  // this column's slot descriptors, loaded while the bulk copies are in flight
-  const int el = tid / NG;
-  const int i = tid - el * NG;
-  const bool active = el < th.ne;
+  // this lane's element and this column's descriptors, while the copies are in flight
+  const bool active = lane < th.ne, direct = lane < th.nd;
+  const bool inner_col = i > 0 && i < NG - 1;
+  const bool all_direct = th.nd == th.ne;
+  PointData pd{};
+  bool axial = false;  // axisymmetric element on the axis (GLJ basis in xi)
   uint32_t dsc[NG];
-  float ec0 = 0.0f, ec1 = 0.0f;  // the element's material coefficients
-  bool axial = false;             // axisymmetric element on the axis (GLJ basis in xi)
-  if (active) {
-    const uint32_t* gdesc = td.sdesc + static_cast<size_t>(th.be0 + el) * CS + i;
+  {
+    const size_t e = static_cast<size_t>(th.tb) * W + lane;
+    pd.c0 = blk.coef0[e];
+    if constexpr (EL) pd.c1 = blk.coef1[e];
+    if constexpr (AXI) axial = blk.axial[e] != 0;
+    if constexpr (!STAGED) {
+      const float* m = blk.metric + static_cast<size_t>(th.tb) * tile_data_floats(KIND, NPE) + lane;
+      if constexpr (KIND == INSEM_RECT) {
+        pd.xi_x = m[0];
+        pd.eta_z = m[W];
+        pd.jac = m[2 * W];
+      } else {
+        pd.xi_x = m[0];
+        pd.xi_z = m[W];
+        pd.eta_x = m[2 * W];
+        pd.eta_z = m[3 * W];
+        pd.jac = m[4 * W];
+      }
+    }
+    const uint16_t* gd = td.sdesc + (static_cast<size_t>(tile) * NPE + i) * W + lane;
 #pragma unroll
-    for (int j = 0; j < NG; ++j) dsc[j] = gdesc[j * NG];
-    ec0 = blk.coef0[th.be0 + el];
-    if constexpr (EL) ec1 = blk.coef1[th.be0 + el];
-    if constexpr (AXI) axial = blk.axial[th.be0 + el] != 0;
+    for (int j = 0; j < NG; ++j) {
+      dsc[j] = kSlotConstrained;
+      if (j == 0 || j == NG - 1 || !inner_col || !all_direct) dsc[j] = gd[j * NG * W];
+    }
   }
   if (tg < th.ntp - th.nc && g_first < 0) g_first = td.halo_tp[th.hl_off + tg];
   dep_wait(dep);
-  if (tid == issuer && nc4 > 0) {
+  if (tid == 0 && nc4 > 0) {
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      bulk_load(tu + c * tp_cap, td.u_cur + static_cast<size_t>(c) * td.ng + th.cbeg, 4u * nc4, bar);
-      if (!L.late) bulk_load(s_v + c * nc_cap, td.v + static_cast<size_t>(c) * td.ng + th.cbeg, 4u * nc4, bar);
+      bulk_load(tu + c * tp_cap, td.u_cur + static_cast<size_t>(c) * td.ng + th.ebeg, edge_b, bar);
+      if (!L.late) bulk_load(s_v + c * nc_cap, td.v + static_cast<size_t>(c) * td.ng + th.ebeg, edge_b, bar);
     }
-    if (!L.late) bulk_load(s_im, td.inv_mass + th.cbeg, 4u * nc4, bar);
   }
-  // halo tile points, gathered while the bulk copies are in flight
-  for (int t = tg; t < th.ntp - th.nc; t += nthreads) {
+  // inner points of direct elements straight into their field rows
+  const size_t g0 = static_cast<size_t>(th.cbeg + (i - 1) * NI * W + lane);  // j = 1; the rows are W points apart
+  if (inner_col) {
+    float x[NI > 0 ? NI : 1][NC];
+#pragma unroll
+    for (int j = 0; j < NI; ++j)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) x[j][c] = __ldcg(td.u_cur + static_cast<size_t>(c) * td.ng + g0 + j * W);
+#pragma unroll
+    for (int j = 0; j < NI; ++j)
+      if (direct) R::store(su, ((j + 1) * NG + i) * W + lane, x[j]);
+  }
+  // halo tile points
+  for (int t = tg; t < th.ntp - th.nc; t += NT) {
     const int32_t g = t == tg ? g_first : td.halo_tp[th.hl_off + t];
 #pragma unroll
     for (int c = 0; c < NC; ++c) tu[c * tp_cap + nc4 + t] = __ldcg(td.u_cur + static_cast<size_t>(c) * td.ng + g);
   }
-  constexpr int ES = rows_elem_stride(NG, NC);  // element stride of the rows
-  constexpr bool PAIR = NC == 2;                 // interleaved components, two-lane sums
-  // position of (component c, row j, column l) in an element's rows
-  auto ridx = [](int c, int j, int l) { return PAIR ? j * 2 * NG + 2 * l + c : (c * NG + j) * ROW + l; };
   // constrained (hanging) slots straight into their field rows: the row's
-  // weighted sum in row order (DofMap::gather, dof_map.hpp:110-115), while
-  // the bulk copies are in flight
-  for (int q = tg; q < th.ncs; q += nthreads) {
-    const int32_t ls = td.cs_slot[th.cs_off + q];
+  // weighted sum in row order (DofMap::gather, dof_map.hpp:110-115)
+  for (int q = tg; q < th.ncs; q += NT) {
+    const int32_t place = td.cs_slot[th.cs_off + q];
     const int2 row = td.cs_row[th.cs_off + q];
-    const int e = ls / NPE, k = ls - e * NPE;
-    const int jj = k / NG, ii = k - jj * NG;
     float s[NC] = {};
     for (int32_t m0 = row.x; m0 < row.y; m0 += 4) {
       float w[4], x[4][NC];
@@ -462,8 +496,7 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
         for (int c = 0; c < NC; ++c)
           if (m0 + m < row.y) s[c] = fadd(s[c], fmul(w[m], x[m][c]));
     }
-#pragma unroll
-    for (int c = 0; c < NC; ++c) su[e * ES + ridx(c, jj, ii)] = s[c];
+    R::store(su, place, s);
   }
   const bool arrived = mbar_wait_bounded(bar, phase, kBulkWaitLimit);
   if (__syncthreads_or(!arrived)) {
@@ -473,38 +506,24 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
     return false;
   }
 
-  // element data now in shared memory, indexed by the tile-local element
-  BlockDev lb = blk;
-  lb.metric = s_metric;
-  lb.coef0 = nullptr;  // one pair per element: ec0 / ec1
-  lb.coef1 = nullptr;
-  lb.wr = s_wr;
-  lb.hoop = s_hoop;
-  lb.r = s_r;
-
-  float* urow = su + el * ES;
-  float* frow = sfx + el * ES;
-  constexpr int AXS = (NG + 3) & ~3;  // one axis-term array (gx0, gy0, gx1, gy1) of an element
-  float* ax = sax + el * 4 * AXS;
-
-  // 2. element field rows (slots through their tile point)
-  if (active) {
+  // 2. the other slots' field rows from their tile points
 #pragma unroll
-    for (int j = 0; j < NG; ++j) {
-      if (!(dsc[j] & kSlotConstrained)) {
-        const int p = dsc[j] & kSlotPointMask;
-        if constexpr (PAIR) {
-          *reinterpret_cast<float2*>(urow + ridx(0, j, i)) = make_float2(tu[p], tu[tp_cap + p]);
-        } else {
+  for (int j = 0; j < NG; ++j) {
+    if (j == 0 || j == NG - 1 || !inner_col || !all_direct) {
+      const bool have = active && dsc[j] != kSlotConstrained && !(j > 0 && j < NG - 1 && inner_col && direct);
+      if (have) {
+        float x[NC];
 #pragma unroll
-          for (int c = 0; c < NC; ++c) urow[ridx(c, j, i)] = tu[c * tp_cap + p];
-        }
+        for (int c = 0; c < NC; ++c) x[c] = tu[c * tp_cap + dsc[j]];
+        R::store(su, (j * NG + i) * W + lane, x);
       }
     }
   }
   __syncthreads();
 
-  // 3. derivatives and fluxes, one column per thread
+  // 3. derivatives and fluxes, one column per thread.  Rows come from shared
+  // memory, the column's own field from registers; pairs of components are
+  // summed in two-lane instructions.
   float dxr[NG], dxc[NG], w2c[NG];  // Dx row i, Dx column i, w_i w_j
 #pragma unroll
   for (int l = 0; l < NG; ++l) {
@@ -512,205 +531,170 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
     dxc[l] = cbasis(NG, axial ? 1 : 0, l * NG + i);
     w2c[l] = cbasis(NG, 2, l * NG + i);
   }
-  float ucol[NC][NG], fe[NC][NG], fx[NC][NG], dir[2][NG];  // fx: f_xi column, stored after the barrier
-  if (active) {
-    if constexpr (PAIR) {
-      // column i of both components, one 64-bit load per row; both
-      // components' sums in two-lane instructions
-      const float nzs = c_neg_zero;
-      const f2x nz = pk2(nzs, nzs);
-      f2x uc[NG];
+  const float nzs = c_neg_zero;
+  const f2x nz = pk2(nzs, nzs);
+  float fe[NG][NC], dir[NG][2];  // f_eta column, hoop terms
+  {
+    f2x uc2[NG];
+    float uc1[NG];
 #pragma unroll
-      for (int l = 0; l < NG; ++l) {
-        uc[l] = pair_load2(urow + ridx(0, l, i));
-        const float2 v = upk2(uc[l]);
-        ucol[0][l] = v.x;
-        ucol[1][l] = v.y;
-      }
+    for (int l = 0; l < NG; ++l) {
+      if constexpr (R::PAIR) uc2[l] = R::pair(su, (l * NG + i) * W + lane);
+      if constexpr (R::ONE) uc1[l] = R::one(su, (l * NG + i) * W + lane);
+    }
 #pragma unroll
-      for (int j = 0; j < NG; ++j) {
-        const int k = j * NG + i;
-        const float* row = urow + ridx(0, j, 0);
+    for (int j = 0; j < NG; ++j) {
+      float uxi[NC], ueta[NC], upt[NC];
+      if constexpr (R::PAIR) {
         f2x a = 0ull, b = 0ull;  // (+0, +0)
 #pragma unroll
         for (int l = 0; l < NG; ++l) {
-          const float d = cbasis(NG, 0, j * NG + l);
-          a = add2(a, mul2(pk2(dxr[l], dxr[l]), pair_load2(row + 2 * l), nz));
-          b = add2(b, mul2(pk2(d, d), uc[l], nz));
+          a = add2(a, mul2(pk2(dxr[l], dxr[l]), R::pair(su, (j * NG + l) * W + lane), nz));
+          b = add2(b, mulc2(uc2[l], cbasis(NG, 0, j * NG + l)));
         }
-        const float2 av = upk2(a), bv = upk2(b);
-        float uxi[NC] = {av.x, av.y}, ueta[NC] = {bv.x, bv.y}, upt[NC] = {ucol[0][j], ucol[1][j]};
-        float fxp[NC], fy[NC], dr[2] = {0.0f, 0.0f};
-        point_flux<NG, KIND, EL, M, true>(lb, el, k, i, j, axial, uxi, ueta, upt, fxp, fy, dr, ax, ax + AXS, ax + 2 * AXS,
-                                    ax + 3 * AXS, w2c[j], ec0, ec1);
-        fx[0][j] = fxp[0];
-        fx[1][j] = fxp[1];
-        fe[0][j] = fy[0];
-        fe[1][j] = fy[1];
-        dir[0][j] = dr[0];
-        dir[1][j] = dr[1];
+        const float2 av = upk2(a), bv = upk2(b), uv = upk2(uc2[j]);
+        uxi[0] = av.x;
+        uxi[1] = av.y;
+        ueta[0] = bv.x;
+        ueta[1] = bv.y;
+        upt[0] = uv.x;
+        upt[1] = uv.y;
       }
-    } else {
+      if constexpr (R::ONE) {
+        float a = 0.0f, b = 0.0f;
 #pragma unroll
-      for (int c = 0; c < NC; ++c)
-#pragma unroll
-        for (int j = 0; j < NG; ++j) ucol[c][j] = urow[ridx(c, j, i)];
-#pragma unroll
-      for (int j = 0; j < NG; ++j) {
-        const int k = j * NG + i;
-        float uxi[NC], ueta[NC];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          // the row two entries per 8-byte load (rows are ROW = even floats
-          // long and start on 8-byte boundaries; the pad entry is never used)
-          const float* row = urow + ridx(c, j, 0);
-          float a = 0.0f, b = 0.0f;
-#pragma unroll
-          for (int l = 0; l < NG; l += 2) {
-            const float2 r2 = *reinterpret_cast<const float2*>(row + l);
-            a = fadd(a, fmul(dxr[l], r2.x));
-            b = fadd(b, fmul(cbasis(NG, 0, j * NG + l), ucol[c][l]));
-            if (l + 1 < NG) {
-              a = fadd(a, fmul(dxr[l + 1], r2.y));
-              b = fadd(b, fmul(cbasis(NG, 0, j * NG + l + 1), ucol[c][l + 1]));
-            }
-          }
-          uxi[c] = a;
-          ueta[c] = b;
+        for (int l = 0; l < NG; ++l) {
+          a = fadd(a, fmul(dxr[l], R::one(su, (j * NG + l) * W + lane)));
+          b = fadd(b, fmul(cbasis(NG, 0, j * NG + l), uc1[l]));
         }
-        float fxp[NC], fy[NC], dr[2] = {0.0f, 0.0f}, upt[NC];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) upt[c] = ucol[c][j];
-        point_flux<NG, KIND, EL, M, true>(lb, el, k, i, j, axial, uxi, ueta, upt, fxp, fy, dr, ax, ax + AXS, ax + 2 * AXS,
-                                    ax + 3 * AXS, w2c[j], ec0, ec1);
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          if constexpr (early_flux_rows(NG, NC)) frow[ridx(c, j, i)] = fxp[c];  // own region: store now
-          else fx[c][j] = fxp[c];
-          fe[c][j] = fy[c];
-        }
-        dir[0][j] = dr[0];
-        dir[1][j] = dr[1];
+        uxi[R::ONE_C] = a;
+        ueta[R::ONE_C] = b;
+        upt[R::ONE_C] = uc1[j];
       }
+      if constexpr (STAGED) {
+        const int p = (j * NG + i) * W + lane;
+        const float2 xi = *reinterpret_cast<const float2*>(elem + tile_data_at(KIND, NPE, 0, p));
+        const float2 eta = *reinterpret_cast<const float2*>(elem + tile_data_at(KIND, NPE, 2, p));
+        pd.xi_x = xi.x;
+        pd.xi_z = xi.y;
+        pd.eta_x = eta.x;
+        pd.eta_z = eta.y;
+        if constexpr (AXI) {
+          const float2 w = *reinterpret_cast<const float2*>(elem + tile_data_at(KIND, NPE, 4, p));
+          pd.wr = w.x;
+          pd.hoop = w.y;
+          pd.r = elem[tile_data_at(KIND, NPE, 6, p)];
+        } else {
+          pd.jac = elem[tile_data_at(KIND, NPE, 4, p)];
+        }
+      }
+      dir[j][0] = dir[j][1] = 0.0f;
+      float fx[NC];
+      point_flux<NG, KIND, EL, M, W>(pd, i, j, axial, uxi, ueta, upt, fx, fe[j], dir[j], ax, ax + NG * W,
+                                     ax + 2 * NG * W, ax + 3 * NG * W, w2c[j]);
+      F::store(sfx, (j * NG + i) * W + lane, fx);
     }
   }
-  __syncthreads();  // the element data is dead: the f_xi rows may overwrite it
-  // v and 1/M of the complete points, into the element-data region beside
-  // the f_xi rows, while the divergence runs
-  if (L.late && tid == issuer) {
-    fence_proxy_async_smem();
-    mbar_expect_tx(bar + 1, nc4 > 0 ? 4u * nc4 * (NC + 1) : 0u);
-    if (nc4 > 0) {
+  // velocity and 1/M of the inner points, in flight over the barrier
+  const bool mine = inner_col && direct && mode == kModeNormal && !energy;
+  float vi[NI > 0 ? NI : 1][NC], mi[NI > 0 ? NI : 1];
+  if (mine) {
 #pragma unroll
-      for (int c = 0; c < NC; ++c)
-        bulk_load(s_v + c * nc_cap, td.v + static_cast<size_t>(c) * td.ng + th.cbeg, 4u * nc4, bar + 1);
-      bulk_load(s_im, td.inv_mass + th.cbeg, 4u * nc4, bar + 1);
-    }
-  }
-  if (active && !early_flux_rows(NG, NC)) {
+    for (int j = 0; j < NI; ++j) {
+      mi[j] = td.inv_mass[g0 + j * W];
 #pragma unroll
-    for (int j = 0; j < NG; ++j) {
-      if constexpr (PAIR) {
-        *reinterpret_cast<float2*>(frow + ridx(0, j, i)) = make_float2(fx[0][j], fx[1][j]);
-      } else {
-#pragma unroll
-        for (int c = 0; c < NC; ++c) frow[ridx(c, j, i)] = fx[c][j];
-      }
+      for (int c = 0; c < NC; ++c) vi[j][c] = __ldcg(td.v + static_cast<size_t>(c) * td.ng + g0 + j * W);
     }
   }
   __syncthreads();
-
-  // 4. weak divergence (interleaved xi / eta terms), hoop and axis terms
-  float fo[NC][NG];
-  if (active) {
+  // the element data is dead but for the f_xi rows: the late copies arrive
+  // there while the divergence runs
+  if (L.late && tid == 0) {
+    fence_proxy_async_smem();
+    mbar_expect_tx(bar + 1, edge_b * (NC + 1) + list_b);
+    if (nc4 > 0) {
 #pragma unroll
-    for (int j = 0; j < NG; ++j) {
-      float s[NC];
-      if constexpr (PAIR) {
-        const float nzs = c_neg_zero;
-        const f2x nz = pk2(nzs, nzs);
-        const float* row = frow + ridx(0, j, 0);
-        f2x acc = 0ull;  // (+0, +0)
-#pragma unroll
-        for (int l = 0; l < NG; ++l) {
-          const float d = cbasis(NG, 0, l * NG + j);
-          acc = add2(acc, mul2(pk2(dxc[l], dxc[l]), pair_load2(row + 2 * l), nz));
-          acc = add2(acc, mul2(pk2(d, d), pk2(fe[0][l], fe[1][l]), nz));
-        }
-        const float2 sv = upk2(acc);
-        s[0] = sv.x;
-        s[1] = sv.y;
-      } else {
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          const float* row = frow + ridx(c, j, 0);
-          float acc = 0.0f;
-#pragma unroll
-          for (int l = 0; l < NG; l += 2) {
-            const float2 r2 = *reinterpret_cast<const float2*>(row + l);
-            acc = fadd(acc, fmul(dxc[l], r2.x));
-            acc = fadd(acc, fmul(cbasis(NG, 0, l * NG + j), fe[c][l]));
-            if (l + 1 < NG) {
-              acc = fadd(acc, fmul(dxc[l + 1], r2.y));
-              acc = fadd(acc, fmul(cbasis(NG, 0, (l + 1) * NG + j), fe[c][l + 1]));
-            }
-          }
-          s[c] = acc;
-        }
-      }
-      const float drj[2] = {dir[0][j], dir[1][j]};
-      float out[NC];
-      point_divergence<NG, KIND, EL, M>(i, j, axial, s, drj, dxc[0], [](int q) { return cbasis(NG, 0, q); }, ax,
-                                        ax + AXS, ax + 2 * AXS, ax + 3 * AXS, out);
-#pragma unroll
-      for (int c = 0; c < NC; ++c) fo[c][j] = out[c];
+      for (int c = 0; c < NC; ++c)
+        bulk_load(s_v + c * nc_cap, td.v + static_cast<size_t>(c) * td.ng + th.ebeg, edge_b, bar + 1);
+      bulk_load(s_im, td.inv_mass + th.ebeg, edge_b, bar + 1);
+      bulk_load(pl, td.plist + static_cast<size_t>(th.pl_off) * td.rs, list_b, bar + 1);
     }
   }
-  __syncthreads();  // su is reused below as halo staging; the f_xi rows are dead
 
-  // 5. every slot's contribution to the staging area; each complete point's
-  //    slots listed by rank (their sum is formed in step 7, in rank order,
-  //    which is the reference's ascending slot order).  This thread's first
-  //    halo entry (step 6) is fetched now, so that its index loads complete
-  //    meanwhile.
+  // 4. weak divergence (interleaved xi / eta terms), hoop and axis terms.  Inner
+  // points of direct elements are finished here: their force is 0 + this one
+  // contribution.  The others' contributions replace their field rows (which
+  // nobody reads any more: the inner points read back only their own).
+#pragma unroll
+  for (int j = 0; j < NG; ++j) {
+    float s[NC];
+    if constexpr (R::PAIR) {
+      f2x acc = 0ull;  // (+0, +0)
+#pragma unroll
+      for (int l = 0; l < NG; ++l) {
+        acc = add2(acc, mul2(pk2(dxc[l], dxc[l]), F::pair(sfx, (j * NG + l) * W + lane), nz));
+        acc = add2(acc, mulc2(pk2(fe[l][0], fe[l][1]), cbasis(NG, 0, l * NG + j)));
+      }
+      const float2 sv = upk2(acc);
+      s[0] = sv.x;
+      s[1] = sv.y;
+    }
+    if constexpr (R::ONE) {
+      float acc = 0.0f;
+#pragma unroll
+      for (int l = 0; l < NG; ++l) {
+        acc = fadd(acc, fmul(dxc[l], F::one(sfx, (j * NG + l) * W + lane)));
+        acc = fadd(acc, fmul(cbasis(NG, 0, l * NG + j), fe[l][R::ONE_C]));
+      }
+      s[R::ONE_C] = acc;
+    }
+    float out[NC];
+    point_divergence<NG, KIND, EL, M, W>(i, j, axial, s, dir[j], dxc[0], [](int q) { return cbasis(NG, 0, q); }, ax,
+                                         ax + NG * W, ax + 2 * NG * W, ax + 3 * NG * W, out);
+    const int place = (j * NG + i) * W + lane;
+    if (j > 0 && j < NG - 1 && mine) {
+      float u[NC];
+      R::load(su, place, u);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const size_t gi = static_cast<size_t>(c) * td.ng + g0 + (j - 1) * W;
+        const float a = fmul(fadd(0.0f, out[c]), mi[j - 1]);
+        float u_out, v_state, v_n;
+        complete_point(kModeNormal, sc, u[c], vi[j - 1][c], a, u_out, v_state, v_n);
+        td.u_nxt[gi] = u_out;
+        td.v[gi] = v_state;
+      }
+    } else {
+      R::store(su, place, out);
+    }
+  }
+
+  // 5. the late copies and every contribution have arrived.  This thread's
+  //    first halo entry is fetched ahead of the barrier.
   int32_t hs_first = 0, hd_first = 0;
   if (tid < th.nhs) {
     hs_first = td.hs_slot[th.hs_off + tid];
     hd_first = td.hs_dst[th.hs_off + tid];
   }
-  float* stage = su;  // [te][NPE][NC]: a slot's components side by side
-  const int rs = L.rs;
-  if (active) {
-#pragma unroll
-    for (int j = 0; j < NG; ++j) {
-      const int base = (el * NPE + j * NG + i) * NC;
-      if constexpr (NC == 2) {
-        *reinterpret_cast<float2*>(stage + base) = make_float2(fo[0][j], fo[1][j]);
-      } else {
-#pragma unroll
-        for (int c = 0; c < NC; ++c) stage[base + c] = fo[c][j];
-      }
-      const uint32_t rank = (dsc[j] >> kSlotRankShift) & 0xffu;
-      if (rank != kSlotRankNone)
-        pl[(dsc[j] & kSlotPointMask) * rs + rank] = static_cast<uint16_t>(base | ((dsc[j] & kSlotLast) ? 0x8000 : 0));
-    }
+  const bool late_arrived = !L.late || mbar_wait_bounded(bar + 1, phase, kBulkWaitLimit);
+  if (__syncthreads_or(!late_arrived)) {
+    if (tid == 0) atomicExch(&st->error, 1);
+    mbar_wait_bounded(bar + 1, phase, kBulkWaitLimit);
+    return false;
   }
-  __syncthreads();
 
   // 6. halo contributions out, each to its place in its halo point's list
-  for (int q = tid; q < th.nhs; q += nthreads) {
-    const int32_t ls = q == tid ? hs_first : td.hs_slot[th.hs_off + q];
+  for (int q = tid; q < th.nhs; q += NT) {
+    const int32_t place = q == tid ? hs_first : td.hs_slot[th.hs_off + q];
     const int32_t dst = q == tid ? hd_first : td.hs_dst[th.hs_off + q];
-    const int e = ls / NPE, k = ls - e * NPE;
     float val[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) val[c] = stage[(e * NPE + k) * NC + c];
+    R::load(su, place, val);
     if (dst >= 0) {
 #pragma unroll
       for (int c = 0; c < NC; ++c) td.hbuf[static_cast<size_t>(c) * td.n_hbuf + dst] = val[c];
     } else {
-      const int32_t mi = -1 - dst;
-      for (int32_t d = td.mdst_off[mi]; d < td.mdst_off[mi + 1]; ++d) {
+      const int32_t mi2 = -1 - dst;
+      for (int32_t d = td.mdst_off[mi2]; d < td.mdst_off[mi2 + 1]; ++d) {
         const int32_t p = td.mdst[d];
 #pragma unroll
         for (int c = 0; c < NC; ++c) td.hbuf[static_cast<size_t>(c) * td.n_hbuf + p] = val[c];
@@ -718,19 +702,11 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
     }
   }
 
-  if (L.late) {
-    const bool late_arrived = mbar_wait_bounded(bar + 1, phase, kBulkWaitLimit);
-    if (__syncthreads_or(!late_arrived)) {
-      if (tid == 0) atomicExch(&st->error, 1);
-      mbar_wait_bounded(bar + 1, phase, kBulkWaitLimit);
-      return false;
-    }
-  }
-
-  // 7. complete points: a = f / M, corrector, predictor; energy partials
+  // 7. edge complete points: a = f / M, corrector, predictor; energy partials
   double kin = 0.0, pot = 0.0;
-  for (int t = tid; t < th.nc; t += nthreads) {
-    const int32_t g = th.cbeg + t;
+  const int rs = td.rs;
+  for (int t = tid; t < th.nc; t += NT) {
+    const size_t g = static_cast<size_t>(th.ebeg) + t;
     const float im = s_im[t];
     // the point's force: its contributions added in rank order, 0 + f_0
     // first.  Four list entries come in one load; the values of the valid
@@ -743,43 +719,53 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
       bool valid[4];
       valid[0] = true;
 #pragma unroll
-      for (int k = 1; k < 4; ++k) valid[k] = valid[k - 1] && !(e[k - 1] & 0x8000u);
-      float x[4][NC];
+      for (int k = 1; k < 4; ++k) valid[k] = valid[k - 1] && !(e[k - 1] & kLastPlace);
+      float x[4][NC] = {};
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float* sp = stage + (e[k] & 0x7fffu);
-        if constexpr (NC == 2) {
-          const float2 q = valid[k] ? *reinterpret_cast<const float2*>(sp) : make_float2(0.0f, 0.0f);
-          x[k][0] = q.x;
-          x[k][1] = q.y;
-        } else {
-#pragma unroll
-          for (int c = 0; c < NC; ++c) x[k][c] = valid[k] ? sp[c] : 0.0f;
-        }
-      }
+      for (int k = 0; k < 4; ++k)
+        if (valid[k]) R::load(su, e[k] & (kLastPlace - 1u), x[k]);
 #pragma unroll
       for (int k = 0; k < 4; ++k)
 #pragma unroll
         for (int c = 0; c < NC; ++c)
-          if (valid[k]) fsum[c] = (r0 + k == 0) ? fadd(0.0f, x[k][c]) : fadd(fsum[c], x[k][c]);
-      more = valid[3] && !(e[3] & 0x8000u);
+          if (valid[k]) fsum[c] = fadd(fsum[c], x[k][c]);
+      more = valid[3] && !(e[3] & kLastPlace);
     }
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const size_t gi = static_cast<size_t>(c) * td.ng + g;
-      const float f = fsum[c];
-      const float a = fmul(f, im);
+      const float a = fmul(fsum[c], im);
       const float u = tu[c * tp_cap + t];
       float u_out, v_state, v_n;
       complete_point(mode, sc, u, s_v[c * nc_cap + t], a, u_out, v_state, v_n);
       td.u_nxt[gi] = u_out;
       td.v[gi] = v_state;
       if (mode != kModeNormal) td.a[gi] = a;
-      if (energy) {
-        pot = dadd(pot, dmul(static_cast<double>(u), static_cast<double>(f)));
-        const double vv = v_n, aa = a;
-        const double m = td.mass[g];
-        kin = dadd(kin, dmul(m, dsub(dmul(dmul(0.5, vv), vv), dmul(dmul(st->kin_c, aa), aa))));
+      if (energy) add_energy(kin, pot, u, fsum[c], v_n, a, td.mass[g], st->kin_c);
+    }
+  }
+  // the inner points of direct elements in the other modes and on energy steps
+  if (NI > 0 && (mode != kModeNormal || energy)) {
+    for (int t = tid; t < NI * NI * W; t += NT) {
+      const int q = t / W;
+      if (t - q * W >= th.nd) continue;
+      const int ci = q / (NI > 0 ? NI : 1) + 1, cj = q - (ci - 1) * NI + 1;
+      const size_t g = static_cast<size_t>(th.cbeg) + t;
+      const float im = td.inv_mass[g];
+      float f[NC];
+      R::load(su, (cj * NG + ci) * W + lane, f);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const size_t gi = static_cast<size_t>(c) * td.ng + g;
+        const float fc = fadd(0.0f, f[c]);
+        const float a = fmul(fc, im);
+        const float u = __ldcg(td.u_cur + gi);
+        float u_out, v_state, v_n;
+        complete_point(mode, sc, u, __ldcg(td.v + gi), a, u_out, v_state, v_n);
+        td.u_nxt[gi] = u_out;
+        td.v[gi] = v_state;
+        if (mode != kModeNormal) td.a[gi] = a;
+        if (energy) add_energy(kin, pot, u, fc, v_n, a, td.mass[g], st->kin_c);
       }
     }
   }
@@ -790,16 +776,15 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
       kin = dadd(kin, __shfl_down_sync(0xffffffffu, kin, off));
       pot = dadd(pot, __shfl_down_sync(0xffffffffu, pot, off));
     }
-    __shared__ double wk[16], wp[16];
-    const int w = tid >> 5;
-    if ((tid & 31) == 0) {
-      wk[w] = kin;
-      wp[w] = pot;
+    __shared__ double wk[NG], wp[NG];
+    if (lane == 0) {
+      wk[i] = kin;
+      wp[i] = pot;
     }
     __syncthreads();
     if (tid == 0) {
       double k2 = 0.0, p2 = 0.0;
-      for (int q = 0; q < (nthreads + 31) / 32; ++q) {
+      for (int q = 0; q < NG; ++q) {
         k2 = dadd(k2, wk[q]);
         p2 = dadd(p2, wp[q]);
       }
@@ -810,8 +795,30 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
   return true;
 }
 
+// Resident CTAs per SM the compiler makes room for in the register file, from
+// the warps each of an SM's four schedulers (16,384 registers) is to hold: 10
+// (48 registers) for one component, 8 (64) for the Cartesian elastic classes,
+// 8 to 6 (64 to 80) for the axisymmetric ones, where shared memory holds
+// about as many CTAs, and 4 or 5 (128 or 96) at NG 8 and 9.  A step of 12
+// boreholes of NG 6 and 7 took 444 us with the compiler's own choice (up to 164
+// registers, 1 - 2 CTAs of the three-component classes) and 336 with this.
 template <int NG, int KIND, bool EL, int M>
-static __global__ void __launch_bounds__(TileCfg<NG>::THREADS)
+constexpr int tile_min_ctas() {
+  const int warps = !EL ? (NG >= 8 || (KIND == INSEM_AXISYM && M == 1) ? 8 : 10)
+                    : KIND != INSEM_AXISYM ? (NG >= 8 ? 5 : 8)
+                    : NG >= 8 ? 4
+                    : NG >= 6 ? 6
+                    : M == 1 && NG == 5 ? 7
+                                        : 8;
+  return 4 * warps / NG > 1 ? 4 * warps / NG : 1;
+}
+// ONE_WAVE: the compiler's own choice of registers, for launches whose tiles
+// are all resident at once anyway: there a tile's latency counts, and more
+// registers keep more loads and sums in flight (3,600 order-4 axisymmetric
+// elements 17.5 -> 17.0 us a step, 4,087 order-8 elements 14.4 -> 11.6; but
+// 25,600 of these 33 -> 42).
+template <int NG, int KIND, bool EL, int M, bool ONE_WAVE>
+static __global__ void __launch_bounds__(TileCfg<NG>::THREADS, ONE_WAVE ? 1 : tile_min_ctas<NG, KIND, EL, M>())
     tile_step_kernel(BlockDev blk, TiledDev td, StepScalars sc, StepState* __restrict__ st,
                      double* __restrict__ epartial, int32_t tile0, StepIdx ix, TileLayout L) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -847,9 +854,8 @@ struct __align__(16) TileItem {
   TileHdr th;               // the tile's header (entry `tile` of the domain's table)
   const StepState* st;      // the segment's solve
   int32_t seg;              // segment index
-  int32_t tile;             // tile index in the domain's table (energy partials)
+  int32_t tile;             // tile index in the domain's table
   const int32_t* halo_tp;   // the tile's halo tile points (domain halo_tp + th.hl_off)
-  int64_t pad;
 };
 static_assert(sizeof(TileItem) == 80, "TileItem is loaded as 20 words");
 
@@ -907,25 +913,10 @@ __device__ __forceinline__ void tile_batch_run(const TileSeg* __restrict__ segs,
   dep_end(ix.dep);
 }
 template <int NG, int KIND, bool EL, int M>
-static __global__ void __launch_bounds__(TileCfg<NG>::THREADS)
+static __global__ void __launch_bounds__(TileCfg<NG>::THREADS, tile_min_ctas<NG, KIND, EL, M>())
     tile_batch_kernel(const TileSeg* __restrict__ segs, const TileItem* __restrict__ items, StepIdx ix, TileLayout L) {
   tile_batch_run<NG, KIND, EL, M>(segs, items, ix, L);
 }
-// Register budgets for the elastic axisymmetric batch classes whose CTAs
-// per SM shared memory or the launch's thread count limit anyway: the
-// budget is what those CTAs can use.  Uncapped, the compiler gives the ngll
-// 7 kernels 99-128 registers (2-3 CTAs per SM where 4 fit) and the ngll 5
-// and 6 m=1 kernels 80 with 44-60 bytes of spills although their shared
-// memory allows only 3 CTAs.  0: no cap (the kernel's launch bounds apply).
-template <int NG, int M>
-constexpr int kBatchRegs = NG == 7 ? (M == 1 ? 128 : 96) : (M == 1 ? (NG == 6 ? 112 : NG == 5 ? 96 : 0) : 0);
-template <int NG, int KIND, bool EL, int M, int REGS>
-static __global__ void __maxnreg__(REGS)
-    tile_batch_kernel_capped(const TileSeg* __restrict__ segs, const TileItem* __restrict__ items, StepIdx ix,
-                             TileLayout L) {
-  tile_batch_run<NG, KIND, EL, M>(segs, items, ix, L);
-}
-
 // ------------------------------------------------------------ halo kernel
 // Special-point records of a domain's halo points.
 struct HaloDev {

@@ -7,15 +7,16 @@
 //      unconstrained slot of one tile and it carries no boundary, coupling,
 //      source, receiver, Dirichlet or axis term; all other points are halo
 //      points;
-//   3. device numbering: complete points tile by tile, then halo points
-//      (both in ascending reference order inside their group);
-//   4. slot descriptors give each slot its tile point and, for complete
-//      points, its rank in the point's ascending slot list (the order of
-//      DofMap::assemble, dof_map.hpp:123-141);
+//   3. device numbering: complete points tile by tile (the inner points of
+//      its direct elements column by column across the elements, then the
+//      others in ascending reference order), then halo points in ascending
+//      reference order;
+//   4. slot descriptors give each slot its tile point; edge complete points
+//      list the places of their contributions in ascending slot order (the
+//      order of DofMap::assemble, dof_map.hpp:123-141);
 //   5. halo slots write to a halo buffer whose entries each halo point sums
 //      through a CSR in ascending slot order (weights of constrained maps kept).
 #include <algorithm>
-#include <cmath>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -33,14 +34,6 @@ void set_constant_basis_ng6(const float*, const float*, const float*);
 void set_constant_basis_ng7(const float*, const float*, const float*);
 void set_constant_basis_ng8(const float*, const float*, const float*);
 void set_constant_basis_ng9(const float*, const float*, const float*);
-int tile_elements_ng2();
-int tile_elements_ng3();
-int tile_elements_ng4();
-int tile_elements_ng5();
-int tile_elements_ng6();
-int tile_elements_ng7();
-int tile_elements_ng8();
-int tile_elements_ng9();
 
 namespace {
 // What each device's constant basis holds per ngll.  Solves of one ngll share
@@ -94,21 +87,6 @@ void set_constant_basis(int ngll, const std::vector<float>& D, const std::vector
   }
 }
 
-int tile_elements(int ngll) {
-  switch (ngll) {
-    case 2: return tile_elements_ng2();
-    case 3: return tile_elements_ng3();
-    case 4: return tile_elements_ng4();
-    case 5: return tile_elements_ng5();
-    case 6: return tile_elements_ng6();
-    case 7: return tile_elements_ng7();
-    case 8: return tile_elements_ng8();
-    case 9: return tile_elements_ng9();
-    default: check_ngll(ngll);
-  }
-  return 0;
-}
-
 void launch_tiles(int ngll, const TileLaunch& a) {
   switch (ngll) {
     case 2: launch_tiles_ng2(a); break;
@@ -131,84 +109,20 @@ int tile_key(int ngll, int kind, bool elastic, int m) { return ((ngll * 4 + kind
 
 void set_tile_elements(int ngll, int kind, bool elastic, int m, int te) {
   check_ngll(ngll);
-  INSEM_REQUIRE(te <= tile_elements(ngll), INSEM_CUDA_ERR_INVALID, "more tile elements than the kernel takes");
+  INSEM_REQUIRE(te <= 64, INSEM_CUDA_ERR_INVALID, "more tile elements than a tile may have");
   std::lock_guard<std::mutex> lk(g_tile_mutex);
   if (te <= 0) g_tile_table.erase(tile_key(ngll, kind, elastic, m));
   else g_tile_table[tile_key(ngll, kind, elastic, m)] = te;
 }
 
-int tile_step_occupancy(int ngll, int kind, bool elastic, int m, int te, uint32_t smem) {
-  switch (ngll) {
-    case 2: return tile_step_occupancy_ng2(kind, elastic, m, te, smem);
-    case 3: return tile_step_occupancy_ng3(kind, elastic, m, te, smem);
-    case 4: return tile_step_occupancy_ng4(kind, elastic, m, te, smem);
-    case 5: return tile_step_occupancy_ng5(kind, elastic, m, te, smem);
-    case 6: return tile_step_occupancy_ng6(kind, elastic, m, te, smem);
-    case 7: return tile_step_occupancy_ng7(kind, elastic, m, te, smem);
-    case 8: return tile_step_occupancy_ng8(kind, elastic, m, te, smem);
-    case 9: return tile_step_occupancy_ng9(kind, elastic, m, te, smem);
-    default: return -1;
-  }
-}
-
-int analytic_tile_elements(int ngll, int kind, bool elastic, int m, int ncomp) {
-  // one answer per class and device (the occupancy queries below ask the device)
-  static std::mutex mu;
-  static std::map<std::pair<int, int>, int> cache;
-  int dev = -1;
-  if (cudaGetDevice(&dev) != cudaSuccess) {
-    cudaGetLastError();
-    dev = -1;
-  }
-  const int key = ((((ngll * 4 + kind) * 2 + (elastic ? 1 : 0)) * 2 + m) * 4 + ncomp);
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    const auto it = cache.find({dev, key});
-    if (it != cache.end()) return it->second;
-  }
-  const int te_max = tile_elements(ngll);
-  const int q = ngll - 1;
-  double best = -1.0;
-  int best_te = te_max;
-  for (int te = te_max; te >= 1; --te) {
-    if (tile_threads(te, ngll) < 64 && te < te_max) break;
-    // tile points: interior (q^2 per element) plus the patch's perimeter
-    const int side = static_cast<int>(std::ceil(std::sqrt(static_cast<double>(te))));
-    const int nc = te * q * q;
-    const int tp = nc + 4 * side * q + 4;
-    const TileLayout L = TileLayout::make(ngll, ncomp, kind, elastic, te, (tp + 3) & ~3, (nc + 3) & ~3, 4);
-    // CTAs per SM: the device's answer for the kernel (its registers count
-    // too), else shared memory alone with 2 KB per CTA for the reserved and
-    // static parts
-    const int occ = dev >= 0 ? tile_step_occupancy(ngll, kind, elastic, m, te, L.total) : -1;
-    const int by_smem = (228 * 1024) / (static_cast<int>(L.total) + 2048);
-    const int ctas = std::min({occ >= 0 ? occ : by_smem, 2048 / tile_threads(te, ngll), 32});
-    if (ctas < 1) continue;
-    const double halo = static_cast<double>(tp - nc) / tp;                 // points shared with other tiles
-    const double overlap = ctas >= 3 ? 1.0 : ctas == 2 ? 0.9 : 0.6;       // copies of one tile under another's math
-    const double lanes = static_cast<double>(te * ngll) / tile_threads(te, ngll);  // threads with an element column
-    const double score = ctas * te * (1.0 - 0.5 * halo) * overlap * lanes;
-    if (score > best + 1e-9) {
-      best = score;
-      best_te = te;
-    }
-  }
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    cache[{dev, key}] = best_te;
-  }
-  return best_te;
-}
-
-int choose_tile_elements(int ngll, int kind, bool elastic, int m, int ncomp, int requested) {
-  const int te_max = tile_elements(ngll);
-  if (requested > 0) return std::min(requested, te_max);
-  {
+int choose_tile_elements(int ngll, int kind, bool elastic, int m, int requested) {
+  check_ngll(ngll);
+  if (requested <= 0) {
     std::lock_guard<std::mutex> lk(g_tile_mutex);
     const auto it = g_tile_table.find(tile_key(ngll, kind, elastic, m));
-    if (it != g_tile_table.end()) return std::min(it->second, te_max);
+    if (it != g_tile_table.end()) requested = it->second;
   }
-  return analytic_tile_elements(ngll, kind, elastic, m, ncomp);
+  return requested > 0 ? std::min(requested, kTileLanes) : kTileLanes;
 }
 
 int tile_batch(int ngll, const TileBatchLaunch& a, bool launch) {
@@ -239,12 +153,9 @@ BlockDev TiledDomain::BlockTiles::view() const {
   v.kind = kind;
   v.m = m;
   v.n = n;
-  v.metric = metric.get();
+  v.metric = data.get();
   v.coef0 = coef0.get();
   v.coef1 = coef1.get();
-  v.wr = wr.get();
-  v.hoop = hoop.get();
-  v.r = r.get();
   v.axial = axial.get();
   return v;
 }
@@ -261,7 +172,9 @@ TiledDev TiledDomain::view(int parity) const {
   t.v = const_cast<float*>(v.get());
   t.a = const_cast<float*>(a.get());
   t.vn = const_cast<float*>(vn.get());
+  t.rs = (rank_cap + 3) & ~3;
   t.sdesc = sdesc.get();
+  t.plist = plist.get();
   t.tiles = tiles.get();
   t.halo_tp = halo_tp.get();
   t.hs_slot = hs_slot.get();
@@ -386,22 +299,52 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
     }
     if (ok && t >= 0) owner[g] = t;
   }
-  // 3. device numbering
-  std::vector<int32_t> count(n_tiles + 1, 0);
+  // 3. device numbering.  A direct element's inner points each belong to it
+  // alone and are complete: the tile's direct elements come first (its first
+  // lanes), and their inner points are numbered column by column across them.
+  const int ni = ngll > 2 ? ngll - 2 : 0;
+  std::vector<int32_t> lane_of(n_elements, -1), n_direct(n_tiles, 0);
+  std::vector<char> inner(ng, 0);
+  auto inner_slot = [&](int q) { return (q % ni + 1) * ngll + q / ni + 1; };  // q = (i - 1) ni + j - 1
+  for (int t = 0; t < n_tiles; ++t) {
+    auto direct = [&](int32_t e) {
+      for (int q = 0; q < ni * ni; ++q) {
+        const int32_t g = l2g[static_cast<std::size_t>(e) * npe + inner_slot(q)];
+        if (g < 0 || owner[g] != t || t_off[g + 1] - t_off[g] != 1) return false;
+      }
+      return true;
+    };
+    auto& list = tile_elems[t];
+    n_direct[t] = static_cast<int32_t>(std::stable_partition(list.begin(), list.end(), direct) - list.begin());
+    for (std::size_t q = 0; q < list.size(); ++q) lane_of[list[q]] = static_cast<int32_t>(q);
+    for (int32_t l = 0; l < n_direct[t]; ++l)
+      for (int q = 0; q < ni * ni; ++q) inner[l2g[static_cast<std::size_t>(list[l]) * npe + inner_slot(q)]] = 1;
+  }
+  std::vector<int32_t> count(n_tiles + 1, 0);  // edge complete points
   for (int32_t g = 0; g < ng; ++g)
-    if (owner[g] >= 0) ++count[owner[g] + 1];
-  // every tile's complete range starts on a multiple of 4 points (16 bytes)
-  // so it can be moved by bulk copies; the gaps are unused padding points
+    if (owner[g] >= 0 && !inner[g]) ++count[owner[g] + 1];
+  // Inner points come in rows of 32 (one per lane, so that a row's accesses
+  // are whole sectors at fixed distances), edge points in ranges that start on
+  // a multiple of 4 points (16 bytes, for bulk copies); the gaps are unused
+  // padding points.
   auto up4 = [](int32_t x) { return (x + 3) & ~3; };
-  std::vector<int32_t> cbeg(n_tiles + 1, 0);
-  for (int t = 0; t < n_tiles; ++t) cbeg[t + 1] = up4(cbeg[t] + count[t + 1]);
+  std::vector<int32_t> cbeg(n_tiles + 1, 0), ebeg(n_tiles, 0);
+  for (int t = 0; t < n_tiles; ++t) {
+    ebeg[t] = cbeg[t] + kTileLanes * ni * ni;
+    cbeg[t + 1] = (ebeg[t] + count[t + 1] + kTileLanes - 1) & ~(kTileLanes - 1);
+  }
   n_complete = cbeg[n_tiles];
   perm.assign(ng, -1);
   int32_t n_halo_pts = 0;
   {
-    std::vector<int32_t> fill(cbeg.begin(), cbeg.end() - 1);
+    for (int t = 0; t < n_tiles; ++t)
+      for (int q = 0; q < ni * ni; ++q)
+        for (int32_t l = 0; l < n_direct[t]; ++l)
+          perm[l2g[static_cast<std::size_t>(tile_elems[t][l]) * npe + inner_slot(q)]] = cbeg[t] + q * kTileLanes + l;
+    std::vector<int32_t> fill(ebeg);
     int32_t h = n_complete;
     for (int32_t g = 0; g < ng; ++g) {
+      if (inner[g]) continue;
       if (owner[g] >= 0) perm[g] = fill[owner[g]]++;
       else {
         perm[g] = h++;
@@ -411,42 +354,33 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
   }
   n_halo = n_halo_pts;
   const int32_t ng_dev = std::max(up4(n_complete + n_halo), 4);
-  const int cs = point_stride_rt(npe);
+  const int W = kTileLanes;
 
-  // 4. ranks of complete points' slots
-  std::vector<uint8_t> rank_of(n_slots, 0xff);
-  for (int32_t g = 0; g < ng; ++g) {
-    if (owner[g] < 0) continue;
-    const int32_t nsl = t_off[g + 1] - t_off[g];
-    INSEM_REQUIRE(nsl < 255, INSEM_CUDA_ERR_UNSUPPORTED, "too many contributions to one point");
-    for (int32_t s = t_off[g]; s < t_off[g + 1]; ++s) rank_of[t_slots[s]] = static_cast<uint8_t>(s - t_off[g]);
-  }
-
-  // 5. per tile: tile points, descriptors, halo and constrained slots
+  // 4. per tile: tile points, descriptors, halo and constrained slots.  The
+  // place of slot k of the element in lane l is k * 32 + l.
   std::vector<TileHdr> hdr(n_tiles);
-  std::vector<uint32_t> desc(static_cast<std::size_t>(n_elements) * cs, 0u);
+  std::vector<uint16_t> desc(static_cast<std::size_t>(std::max(n_tiles, 1)) * npe * W, 0);
   std::vector<int32_t> htp, hslot, cslot, crow;
   std::vector<int32_t> hpos_of_slot(n_slots, -1);
   std::vector<int32_t> tpi(ng_dev, -1), tpi_stamp(ng, -1);
-  std::vector<int32_t> block_elem_count(d.n_blocks, 0);
-  for (int b = 0; b < d.n_blocks; ++b) blocks[b].e_off = 0;
-  int32_t e_running = 0, hb = 0;
+  int32_t hb = 0, pl_running = 0;
+  std::vector<int32_t> hp;
   for (int b = 0; b < d.n_blocks; ++b) {
-    blocks[b].e_off = e_running;
-    int32_t be = 0;
     for (int t = blocks[b].tile0; t < blocks[b].tile0 + blocks[b].ntiles; ++t) {
       TileHdr& th = hdr[t];
-      th.be0 = be;
+      th.tb = t - blocks[b].tile0;
       th.ne = static_cast<int32_t>(tile_elems[t].size());
+      th.nd = n_direct[t];
       th.cbeg = cbeg[t];
-      th.nc = count[t + 1];  // owned points; [cbeg + nc, cbeg[t + 1]) is padding
+      th.ebeg = ebeg[t];
+      th.nc = count[t + 1];  // [ebeg + nc, cbeg of the next tile) is padding
       th.hl_off = static_cast<int32_t>(htp.size());
       th.hs_off = static_cast<int32_t>(hslot.size());
       th.cs_off = static_cast<int32_t>(cslot.size());
-      th.hb = hb;
-      th.maxrank = 0;
-      // halo points read by the tile
-      std::vector<int32_t> hp;
+      th.pl_off = pl_running;
+      pl_running += up4(th.nc);
+      // halo points read by the tile; they follow the edge points' padded range
+      hp.clear();
       for (int32_t e : tile_elems[t])
         for (int k = 0; k < npe; ++k) {
           const int32_t g = l2g[static_cast<std::size_t>(e) * npe + k];
@@ -456,10 +390,8 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
           }
         }
       std::sort(hp.begin(), hp.end());
-      for (std::size_t q = 0; q < hp.size(); ++q) htp.push_back(hp[q]);
+      htp.insert(htp.end(), hp.begin(), hp.end());
       th.ntp = th.nc + static_cast<int32_t>(hp.size());
-      // tile point index of every point the tile touches
-      // halo tile points follow the complete points' padded range
       for (std::size_t q = 0; q < hp.size(); ++q) tpi[hp[q]] = up4(th.nc) + static_cast<int32_t>(q);
       int32_t nh = 0;
       for (int el = 0; el < th.ne; ++el) {
@@ -467,48 +399,61 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
         for (int k = 0; k < npe; ++k) {
           const std::size_t s = static_cast<std::size_t>(e) * npe + k;
           const int32_t g = l2g[s];
-          const int32_t ls = el * npe + k;
-          uint32_t dsc;
+          const int32_t place = k * W + el;
+          uint32_t dsc = 0;
           if (g >= 0) {
-            const int32_t pg = perm[g];
-            const int32_t p = owner[g] == t ? pg - th.cbeg : tpi[pg];
-            INSEM_REQUIRE(p >= 0 && p < 65536, INSEM_CUDA_ERR_UNSUPPORTED, "tile has too many points");
-            const uint32_t rank = owner[g] == t ? rank_of[s] : kSlotRankNone;
-            dsc = static_cast<uint32_t>(p) | (rank << kSlotRankShift);
-            if (owner[g] == t && static_cast<int32_t>(rank) == t_off[g + 1] - t_off[g] - 1) dsc |= kSlotLast;
-            if (owner[g] == t) {
-              th.maxrank = std::max<int32_t>(th.maxrank, static_cast<int32_t>(rank));
-            } else {
-              hpos_of_slot[s] = hb + nh++;
-              hslot.push_back(ls);
+            if (!inner[g]) {
+              const int32_t pg = perm[g];
+              const int32_t p = owner[g] == t ? pg - th.ebeg : tpi[pg];
+              INSEM_REQUIRE(p >= 0 && p < static_cast<int32_t>(kSlotConstrained), INSEM_CUDA_ERR_UNSUPPORTED,
+                            "tile has too many points");
+              dsc = static_cast<uint32_t>(p);
+              if (owner[g] != t) {
+                hpos_of_slot[s] = hb + nh++;
+                hslot.push_back(place);
+              }
             }
           } else {
-            dsc = kSlotConstrained | (kSlotRankNone << kSlotRankShift);
-            cslot.push_back(ls);
+            dsc = kSlotConstrained;
+            cslot.push_back(place);
             crow.push_back(-1 - g);
             hpos_of_slot[s] = hb + nh++;
-            hslot.push_back(ls);
+            hslot.push_back(place);
           }
-          desc[(static_cast<std::size_t>(e_running) + be + el) * cs + k] = dsc;
+          desc[static_cast<std::size_t>(t) * npe * W + place] = static_cast<uint16_t>(dsc);
         }
       }
       th.nhs = nh;
       th.ncs = static_cast<int32_t>(cslot.size()) - th.cs_off;
       hb += nh;
-      be += th.ne;
     }
-    e_running += be;
   }
   const int32_t n_entries = hb;
   tp_cap = 4;
   nc_cap = 4;
-  rank_cap = 1;
   for (const auto& th : hdr) {
     tp_cap = std::max(tp_cap, up4(th.nc) + th.ntp - th.nc);
     nc_cap = std::max(nc_cap, up4(th.nc));
-    rank_cap = std::max(rank_cap, th.maxrank + 1);
   }
   tp_cap = up4(tp_cap);  // keeps every component row of the staged u 16-byte aligned
+
+  // 5. place lists of the edge complete points, in ascending slot order
+  rank_cap = 1;
+  for (int32_t g = 0; g < ng; ++g)
+    if (owner[g] >= 0 && !inner[g]) rank_cap = std::max<int32_t>(rank_cap, t_off[g + 1] - t_off[g]);
+  const int rs = (rank_cap + 3) & ~3;
+  std::vector<uint16_t> lists(static_cast<std::size_t>(std::max(pl_running, 4)) * rs, static_cast<uint16_t>(kLastPlace));
+  for (int32_t g = 0; g < ng; ++g) {
+    if (owner[g] < 0 || inner[g]) continue;
+    const TileHdr& th = hdr[owner[g]];
+    const std::size_t at = static_cast<std::size_t>(th.pl_off + perm[g] - th.ebeg) * rs;
+    for (int32_t s = t_off[g]; s < t_off[g + 1]; ++s) {
+      const int32_t slot = t_slots[s], e = slot / npe;
+      uint32_t place = static_cast<uint32_t>((slot - e * npe) * W + lane_of[e]);
+      if (s + 1 == t_off[g + 1]) place |= kLastPlace;
+      lists[at + (s - t_off[g])] = static_cast<uint16_t>(place);
+    }
+  }
 
   // 6. halo CSR and special records (device order of halo points)
   std::vector<int32_t> hoff{0}, hpos, hspec(n_halo, -1), soff{0}, swhich, coff{0}, cidx2, aidx;
@@ -570,6 +515,7 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
 
   // 7. uploads
   sdesc.upload(desc);
+  plist.upload(lists);
   tiles.upload(hdr);
   host_tiles = std::move(hdr);
   halo_tp.upload(htp.empty() ? std::vector<int32_t>{0} : htp);
@@ -620,36 +566,50 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
     buf->resize(nf);
     buf->zero();
   }
-  // element data of every block in tile order, padded layout
+  // element data of every block, element-minor by tile; one material per
+  // element: the tile kernels read one coefficient pair per element
   for (int b = 0; b < d.n_blocks; ++b) {
-    std::vector<int32_t> order;  // block-local positions in tile order
-    for (int t = blocks[b].tile0; t < blocks[b].tile0 + blocks[b].ntiles; ++t)
-      for (int32_t e : tile_elems[t]) order.push_back(epos[e]);
-    PackedBlock pk = pack_block(d.blocks[b], npe, medium, order);
-    blocks[b].metric.upload(pk.metric);
-    // One material per element: the tile kernels read one coefficient pair
-    // per element instead of one per point.
-    const std::size_t cs = point_stride_rt(npe);
-    std::vector<float> c0(order.size()), c1(medium == INSEM_ELASTIC ? order.size() : 0);
-    for (std::size_t q = 0; q < order.size(); ++q) {
-      c0[q] = pk.coef0[q * cs];
-      if (!c1.empty()) c1[q] = pk.coef1[q * cs];
-      for (int k = 1; k < npe; ++k) {
-        const bool same = bits_of(pk.coef0[q * cs + k]) == bits_of(c0[q]) &&
-                          (c1.empty() || bits_of(pk.coef1[q * cs + k]) == bits_of(c1[q]));
-        INSEM_REQUIRE(same, INSEM_CUDA_ERR_UNSUPPORTED,
-                      "material coefficients vary inside an element; the tiled path takes one material per "
-                      "element (options.path = 1 takes per-point coefficients)");
+    BlockTiles& bt = blocks[b];
+    const insem_cuda_block& in = d.blocks[b];
+    const int kind = in.kind, na = tile_arrays(kind), nm = kind == INSEM_AXISYM ? 4 : na;
+    const bool el = medium == INSEM_ELASTIC, staged = tile_data_staged(kind);
+    const std::size_t per_tile = static_cast<std::size_t>(tile_data_floats(kind, npe));
+    std::vector<float> data(per_tile * bt.ntiles, 0.0f), c0(static_cast<std::size_t>(W) * bt.ntiles, 0.0f);
+    std::vector<float> c1(el ? c0.size() : 0, 0.0f);
+    std::vector<uint8_t> axial(kind == INSEM_AXISYM ? c0.size() : 0, 0);
+    for (int tb = 0; tb < bt.ntiles; ++tb) {
+      const auto& list = tile_elems[bt.tile0 + tb];
+      for (std::size_t l = 0; l < list.size(); ++l) {
+        const std::size_t o = static_cast<std::size_t>(epos[list[l]]), p0 = o * npe, at = static_cast<std::size_t>(tb) * W + l;
+        float* out = data.data() + per_tile * tb;
+        if (staged) {
+          for (int k = 0; k < npe; ++k) {
+            auto put = [&](int c, float v) { out[tile_data_at(kind, npe, c, k * W + static_cast<int>(l))] = v; };
+            for (int c = 0; c < nm; ++c) put(c, in.metric[(p0 + k) * 5 + c]);
+            if (kind == INSEM_AXISYM) {
+              put(4, in.wr[p0 + k]);
+              put(5, in.hoop[p0 + k]);
+              put(6, in.r[p0 + k]);
+            }
+          }
+        } else {
+          for (int c = 0; c < na; ++c) out[static_cast<std::size_t>(c) * W + l] = in.metric[o * na + c];
+        }
+        c0[at] = in.coef0[p0];
+        if (el) c1[at] = in.coef1[p0];
+        if (kind == INSEM_AXISYM) axial[at] = in.axial[o];
+        for (int k = 1; k < npe; ++k) {
+          const bool same = bits_of(in.coef0[p0 + k]) == bits_of(c0[at]) && (!el || bits_of(in.coef1[p0 + k]) == bits_of(c1[at]));
+          INSEM_REQUIRE(same, INSEM_CUDA_ERR_UNSUPPORTED,
+                        "material coefficients vary inside an element; the tiled path takes one material per "
+                        "element (options.path = 1 takes per-point coefficients)");
+        }
       }
     }
-    blocks[b].coef0.upload(c0);
-    if (medium == INSEM_ELASTIC) blocks[b].coef1.upload(c1);
-    if (d.blocks[b].kind == INSEM_AXISYM) {
-      blocks[b].wr.upload(pk.wr);
-      blocks[b].hoop.upload(pk.hoop);
-      blocks[b].r.upload(pk.r);
-      blocks[b].axial.upload(pk.axial);
-    }
+    bt.data.upload(data);
+    bt.coef0.upload(c0);
+    bt.coef1.upload(c1);
+    bt.axial.upload(axial);
   }
   ng = ng_dev;  // from here on the component stride of the device arrays
 }

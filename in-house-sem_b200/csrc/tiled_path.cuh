@@ -30,18 +30,18 @@ class TiledDomain {
   int medium = 0, ncomp = 1, m = 0, ng = 0, ng_ref = 0, npe = 0, n_elements = 0;
   int n_complete = 0, n_halo = 0, n_tiles = 0, tp_cap = 0, nc_cap = 0, n_hbuf = 0;
   int rank_cap = 1;  // the most contributions one complete point of a tile has
-  int te = 0;  // elements per tile (CTAs of tile_threads(te, ngll) threads)
+  int te = 0;  // elements per tile
   bool weighted = false;
   std::vector<int32_t> perm;  // reference point -> device point
   struct BlockTiles {
-    int kind = 0, m = 0, tile0 = 0, ntiles = 0, n = 0, e_off = 0;
-    DeviceBuffer<float> metric, coef0, coef1, wr, hoop, r;
+    int kind = 0, m = 0, tile0 = 0, ntiles = 0, n = 0;
+    DeviceBuffer<float> data, coef0, coef1;  // [tile][tile_data_floats], [tile][32]
     DeviceBuffer<uint8_t> axial;
     BlockDev view() const;
   };
   std::vector<BlockTiles> blocks;
   // device data
-  DeviceBuffer<uint32_t> sdesc;
+  DeviceBuffer<uint16_t> sdesc, plist;
   DeviceBuffer<TileHdr> tiles;
   std::vector<TileHdr> host_tiles;  // the same headers on the host (the batched tile items copy them)
   DeviceBuffer<int32_t> halo_tp, hs_slot, hs_dst, mdst_off, mdst, cs_slot;
@@ -79,6 +79,16 @@ cudaError_t launch_chained(void (*kernel)(P...), int grid, int threads, size_t s
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+// Opts a kernel in to all the shared memory a CTA may have beside its static
+// part: the same value for every solve, so that none lowers another's.
+template <class Kernel>
+void allow_shared_memory(Kernel kernel) {
+  cudaFuncAttributes fa;
+  CUDA_CHECK(cudaFuncGetAttributes(&fa, kernel));
+  CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  227 * 1024 - static_cast<int>(fa.sharedSizeBytes)));
+}
+
 // Launchers, instantiated per ngll in tiled_ng.cu.
 struct TileLaunch {
   const TiledDomain* dom = nullptr;
@@ -103,51 +113,11 @@ void launch_tiles_ng9(const TileLaunch&);
 void launch_tiles(int ngll, const TileLaunch& a);
 int tile_elements(int ngll);  // TileCfg<NG>::TE (the largest tile)
 // Elements per tile of a domain: `requested` if > 0, else a registered entry
-// (set_tile_elements, e.g. from the autotuner), else the analytic choice that
-// keeps the most elements resident per SM with several CTAs per SM.
-int choose_tile_elements(int ngll, int kind, bool elastic, int m, int ncomp, int requested);
+// (set_tile_elements, e.g. from the autotuner), at most the kernel's 32; by
+// default 32, which leaves no lane idle and the fewest points shared between
+// tiles.
+int choose_tile_elements(int ngll, int kind, bool elastic, int m, int requested);
 void set_tile_elements(int ngll, int kind, bool elastic, int m, int te);  // te <= 0 clears the entry
-int analytic_tile_elements(int ngll, int kind, bool elastic, int m, int ncomp);
-// CTAs per SM of the plain tile kernel of a class at te elements and smem
-// bytes of dynamic shared memory (registers, shared memory and threads as
-// the current device counts them); -1 if the device cannot be asked.
-int tile_step_occupancy(int ngll, int kind, bool elastic, int m, int te, uint32_t smem);
-int tile_step_occupancy_ng2(int kind, bool elastic, int m, int te, uint32_t smem);
-int tile_step_occupancy_ng3(int kind, bool elastic, int m, int te, uint32_t smem);
-int tile_step_occupancy_ng4(int kind, bool elastic, int m, int te, uint32_t smem);
-int tile_step_occupancy_ng5(int kind, bool elastic, int m, int te, uint32_t smem);
-int tile_step_occupancy_ng6(int kind, bool elastic, int m, int te, uint32_t smem);
-int tile_step_occupancy_ng7(int kind, bool elastic, int m, int te, uint32_t smem);
-int tile_step_occupancy_ng8(int kind, bool elastic, int m, int te, uint32_t smem);
-int tile_step_occupancy_ng9(int kind, bool elastic, int m, int te, uint32_t smem);
-
-template <int NG>
-int tile_step_occupancy_cfg(int kind, bool elastic, int m, int te, uint32_t smem) {
-  auto ask = [&](auto kernel) -> int {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess) {
-      cudaGetLastError();
-      return -1;
-    }
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, tile_threads(te, NG), smem) != cudaSuccess) {
-      cudaGetLastError();
-      return -1;
-    }
-    return nb;
-  };
-  if (kind == INSEM_AXISYM) {
-    if (m == 1) return elastic ? ask(tile_step_kernel<NG, INSEM_AXISYM, true, 1>) : ask(tile_step_kernel<NG, INSEM_AXISYM, false, 1>);
-    return elastic ? ask(tile_step_kernel<NG, INSEM_AXISYM, true, 0>) : ask(tile_step_kernel<NG, INSEM_AXISYM, false, 0>);
-  }
-  switch (kind) {
-    case INSEM_RECT:
-      return elastic ? ask(tile_step_kernel<NG, INSEM_RECT, true, 0>) : ask(tile_step_kernel<NG, INSEM_RECT, false, 0>);
-    case INSEM_AFFINE:
-      return elastic ? ask(tile_step_kernel<NG, INSEM_AFFINE, true, 0>) : ask(tile_step_kernel<NG, INSEM_AFFINE, false, 0>);
-    default:
-      return elastic ? ask(tile_step_kernel<NG, INSEM_CURVED, true, 0>) : ask(tile_step_kernel<NG, INSEM_CURVED, false, 0>);
-  }
-}
 // Uploads the GLL / GLJ basis of one ngll to constant memory (must agree with earlier uploads).
 void set_constant_basis(int ngll, const std::vector<float>& D, const std::vector<float>& Dj,
                         const std::vector<float>& w2);
@@ -159,7 +129,6 @@ struct TileBatchLaunch {
   bool elastic = false;
   const TileSeg* segs = nullptr;
   const TileItem* items = nullptr;
-  int te = 0;      // elements per tile of the class (CTA size tile_threads(te, ngll))
   TileLayout L{};  // the class layout; its total is the dynamic shared memory
   uint32_t smem = 0;
   int grid = 0;
@@ -167,8 +136,8 @@ struct TileBatchLaunch {
   bool overlap = false;
   cudaStream_t stream = nullptr;
 };
-// launch == false: sets the class kernel's dynamic shared memory (outside
-// stream capture) and returns its resident CTAs per SM; true: launches.
+// launch == false: opts the class kernel in to its dynamic shared memory
+// (outside stream capture); true: launches.
 int tile_batch_ng2(const TileBatchLaunch&, bool launch);
 int tile_batch_ng3(const TileBatchLaunch&, bool launch);
 int tile_batch_ng4(const TileBatchLaunch&, bool launch);
@@ -181,16 +150,13 @@ int tile_batch(int ngll, const TileBatchLaunch& a, bool launch);
 
 template <int NG>
 int tile_batch_cfg(const TileBatchLaunch& a, bool launch) {
-  INSEM_REQUIRE(a.smem <= 227u * 1024u, INSEM_CUDA_ERR_UNSUPPORTED, "tile needs too much shared memory");
+  INSEM_REQUIRE(a.smem <= 226u * 1024u, INSEM_CUDA_ERR_UNSUPPORTED, "tile needs too much shared memory");
   auto go = [&](auto kernel) -> int {
     if (!launch) {
-      CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(a.smem)));
-      int nb = 0;
-      CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, tile_threads(a.te, NG), a.smem));
-      return nb;
+      allow_shared_memory(kernel);
+      return 0;
     }
-    INSEM_REQUIRE(a.te >= 1 && a.te <= TileCfg<NG>::TE, INSEM_CUDA_ERR_INVALID, "tile elements out of range");
-    cudaError_t err = launch_chained(kernel, a.grid, tile_threads(a.te, NG), a.smem, a.stream, a.overlap, a.segs,
+    cudaError_t err = launch_chained(kernel, a.grid, TileCfg<NG>::THREADS, a.smem, a.stream, a.overlap, a.segs,
                                      a.items, a.ix, a.L);
     if (err == cudaSuccess) err = cudaGetLastError();
     if (err != cudaSuccess)
@@ -200,12 +166,6 @@ int tile_batch_cfg(const TileBatchLaunch& a, bool launch) {
     return 0;
   };
   if (a.kind == INSEM_AXISYM) {
-    if (a.elastic) {
-      if constexpr (kBatchRegs<NG, 1> > 0)
-        if (a.m == 1) return go(tile_batch_kernel_capped<NG, INSEM_AXISYM, true, 1, kBatchRegs<NG, 1>>);
-      if constexpr (kBatchRegs<NG, 0> > 0)
-        if (a.m == 0) return go(tile_batch_kernel_capped<NG, INSEM_AXISYM, true, 0, kBatchRegs<NG, 0>>);
-    }
     if (a.m == 1) return a.elastic ? go(tile_batch_kernel<NG, INSEM_AXISYM, true, 1>)
                                    : go(tile_batch_kernel<NG, INSEM_AXISYM, false, 1>);
     return a.elastic ? go(tile_batch_kernel<NG, INSEM_AXISYM, true, 0>) : go(tile_batch_kernel<NG, INSEM_AXISYM, false, 0>);
@@ -227,50 +187,57 @@ void launch_tiles_cfg(const TileLaunch& a) {
   const TiledDomain& d = *a.dom;
   const auto& b = d.blocks[a.block];
   if (b.ntiles == 0) return;
-  auto go = [&](auto kernel, int nc) {
-    INSEM_REQUIRE(d.te >= 1 && d.te <= TileCfg<NG>::TE, INSEM_CUDA_ERR_INVALID, "tile elements out of range");
+  auto go = [&](auto one_wave, auto many_waves, int nc) {
     const TileLayout L = TileLayout::make(NG, nc, b.kind, a.elastic, d.te, d.tp_cap, d.nc_cap, d.rank_cap);
     const size_t smem = L.total;
-    // Opt in to this launch's dynamic shared memory (outside stream capture;
-    // the first launch of every tile kernel happens in the uncaptured initial step).
+    INSEM_REQUIRE(smem <= 226 * 1024, INSEM_CUDA_ERR_UNSUPPORTED, "tile needs too much shared memory");
+    // The kernel with the compiler's own registers where it holds all tiles at
+    // once; and the opt-in to this launch's dynamic shared memory (outside
+    // stream capture; the first launch of every tile kernel happens in the
+    // uncaptured initial step).
+    auto kernel = many_waves;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CUDA_CHECK(cudaStreamIsCapturing(a.stream, &cap));
     if (cap == cudaStreamCaptureStatusNone)
-      CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    INSEM_REQUIRE(smem <= 227 * 1024, INSEM_CUDA_ERR_UNSUPPORTED, "tile needs too much shared memory");
+      for (auto k : {one_wave, many_waves})
+        allow_shared_memory(k);
+    int per_sm = 0, device = 0, sms = 0;
+    CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, one_wave, TileCfg<NG>::THREADS, smem));
+    CUDA_CHECK(cudaGetDevice(&device));
+    CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    if (b.ntiles <= per_sm * sms) kernel = one_wave;
     TiledDev td = d.view(a.parity);
-    td.sdesc += static_cast<size_t>(b.e_off) * point_stride<NG * NG>();
-    cudaError_t err = launch_chained(kernel, b.ntiles, tile_threads(d.te, NG), smem, a.stream, a.overlap, b.view(), td,
+    cudaError_t err = launch_chained(kernel, b.ntiles, TileCfg<NG>::THREADS, smem, a.stream, a.overlap, b.view(), td,
                                      a.sc, a.st, a.epartial, static_cast<int32_t>(b.tile0), a.ix, L);
     if (err == cudaSuccess) err = cudaGetLastError();
     if (err != cudaSuccess)
       throw Error(INSEM_CUDA_ERR_CUDA, "tile kernel launch (ngll " + std::to_string(NG) + ", kind " +
                                            std::to_string(b.kind) + ", tiles " + std::to_string(b.ntiles) +
-                                           ", threads " + std::to_string(tile_threads(d.te, NG)) + ", smem " +
+                                           ", threads " + std::to_string(TileCfg<NG>::THREADS) + ", smem " +
                                            std::to_string(smem) + "): " + cudaGetErrorString(err));
   };
   if (b.kind == INSEM_AXISYM) {
     if (b.m == 1) {
-      if (a.elastic) go(tile_step_kernel<NG, INSEM_AXISYM, true, 1>, 3);
-      else go(tile_step_kernel<NG, INSEM_AXISYM, false, 1>, 1);
+      if (a.elastic) go(tile_step_kernel<NG, INSEM_AXISYM, true, 1, true>, tile_step_kernel<NG, INSEM_AXISYM, true, 1, false>, 3);
+      else go(tile_step_kernel<NG, INSEM_AXISYM, false, 1, true>, tile_step_kernel<NG, INSEM_AXISYM, false, 1, false>, 1);
     } else {
-      if (a.elastic) go(tile_step_kernel<NG, INSEM_AXISYM, true, 0>, 2);
-      else go(tile_step_kernel<NG, INSEM_AXISYM, false, 0>, 1);
+      if (a.elastic) go(tile_step_kernel<NG, INSEM_AXISYM, true, 0, true>, tile_step_kernel<NG, INSEM_AXISYM, true, 0, false>, 2);
+      else go(tile_step_kernel<NG, INSEM_AXISYM, false, 0, true>, tile_step_kernel<NG, INSEM_AXISYM, false, 0, false>, 1);
     }
     return;
   }
   switch (b.kind) {
     case INSEM_RECT:
-      if (a.elastic) go(tile_step_kernel<NG, INSEM_RECT, true, 0>, 2);
-      else go(tile_step_kernel<NG, INSEM_RECT, false, 0>, 1);
+      if (a.elastic) go(tile_step_kernel<NG, INSEM_RECT, true, 0, true>, tile_step_kernel<NG, INSEM_RECT, true, 0, false>, 2);
+      else go(tile_step_kernel<NG, INSEM_RECT, false, 0, true>, tile_step_kernel<NG, INSEM_RECT, false, 0, false>, 1);
       break;
     case INSEM_AFFINE:
-      if (a.elastic) go(tile_step_kernel<NG, INSEM_AFFINE, true, 0>, 2);
-      else go(tile_step_kernel<NG, INSEM_AFFINE, false, 0>, 1);
+      if (a.elastic) go(tile_step_kernel<NG, INSEM_AFFINE, true, 0, true>, tile_step_kernel<NG, INSEM_AFFINE, true, 0, false>, 2);
+      else go(tile_step_kernel<NG, INSEM_AFFINE, false, 0, true>, tile_step_kernel<NG, INSEM_AFFINE, false, 0, false>, 1);
       break;
     default:
-      if (a.elastic) go(tile_step_kernel<NG, INSEM_CURVED, true, 0>, 2);
-      else go(tile_step_kernel<NG, INSEM_CURVED, false, 0>, 1);
+      if (a.elastic) go(tile_step_kernel<NG, INSEM_CURVED, true, 0, true>, tile_step_kernel<NG, INSEM_CURVED, true, 0, false>, 2);
+      else go(tile_step_kernel<NG, INSEM_CURVED, false, 0, true>, tile_step_kernel<NG, INSEM_CURVED, false, 0, false>, 1);
       break;
   }
 }
