@@ -98,39 +98,26 @@ void Solver::batch_collect(BatchTables& T) {
       }
     }
   }
-  CouplingDev cp{tcpl_fluid.get(), tcpl_solid.get(), cpl_cx.get(), cpl_cz.get()};
-  for (int di : {solid, fluid}) {
-    if (di < 0) continue;
-    TiledDomain& t = tdom[di];
-    if (t.n_halo == 0) continue;
-    const bool el = t.medium == INSEM_ELASTIC;
-    HaloSeg h{};
-    h.td = t.view(0);
-    h.hd = t.halo_view();
-    h.cp = cp;
-    if (n_cpl > 0) {
-      if (el) {
-        h.other0 = tdom[fluid].u0.get();
-        h.other1 = tdom[fluid].u1.get();
-        h.other_ng = tdom[fluid].ng;
-        h.pm = t.m == 1;
-      } else {
-        h.other0 = h.other1 = tdom[solid].a.get();
-        h.other_ng = tdom[solid].ng;
-        h.pm = tdom[solid].m == 1;
-      }
+  {
+    // one segment; a coupled group larger than a CTA splits it into two, the
+    // fluid's in the launch after the solid's
+    const HaloArgs A = halo_args(0, false);
+    auto add = [&](HaloArgs h, int cls) {
+      const int32_t seg = static_cast<int32_t>(T.halo_segs[cls].size());
+      T.halo_segs[cls].push_back(h);
+      for (int k = 0; k < h.nb_s + h.nb_f + h.n_chunk; ++k) T.halo_items[cls].push_back(int2{seg, k});
+    };
+    const int cls = solid < 0 ? 0 : tdom[solid].ncomp == 2 ? 1 : 2;
+    if (n_cpl > 0 && n_chunks == 0) {
+      HaloArgs one = A;
+      one.nb_f = 0;
+      add(one, cls);
+      one = A;
+      one.nb_s = 0;
+      add(one, cls + 2);
+    } else {
+      add(A, cls);
     }
-    h.amp = src_amp.get();
-    h.n_amp = n_amp;
-    h.sc = sc;
-    h.h_damp = 0.5 * dt;
-    h.st = st;
-    h.epartial = epart.get();
-    h.epart0 = ep_halo[di];
-    const int cls = !el ? 0 : (t.ncomp == 2 ? 1 : 2);
-    const int32_t seg = static_cast<int32_t>(T.halo_segs[cls].size());
-    T.halo_segs[cls].push_back(h);
-    for (int k = 0; k < ceil_div(t.n_halo, kHaloChunk); ++k) T.halo_items[cls].push_back(int2{seg, k});
   }
   if (n_acoustic_rec > 0 || n_cols > 0) {
     RecSeg r{};
@@ -158,8 +145,8 @@ void Solver::batch_collect(BatchTables& T) {
     EnergySeg e{};
     e.epartial = epart.get();
     e.n_dom = d1 >= 0 ? 2 : 1;
-    e.s0 = int4{ep_tile[d0], ep_ntile[d0], ep_halo[d0], tdom[d0].n_halo > 0 ? ep_nhalo[d0] : 0};
-    if (d1 >= 0) e.s1 = int4{ep_tile[d1], ep_ntile[d1], ep_halo[d1], tdom[d1].n_halo > 0 ? ep_nhalo[d1] : 0};
+    e.s0 = int4{ep_tile[d0], ep_ntile[d0], ep_halo[d0], ep_nhalo[d0]};
+    if (d1 >= 0) e.s1 = int4{ep_tile[d1], ep_ntile[d1], ep_halo[d1], ep_nhalo[d1]};
     e.st = st;
     e.energy_every = energy_every;
     e.dt = dt;
@@ -307,7 +294,7 @@ void Batch::rebuild() {
   }
   // largest class first: the small ones fill the chip as its last tiles run out
   std::stable_sort(dclasses.begin(), dclasses.end(), [](const DevClass& x, const DevClass& y) { return x.work > y.work; });
-  for (int c = 0; c < 3; ++c) {
+  for (int c = 0; c < kHaloClasses; ++c) {
     dhalo_segs[c].upload_async(T.halo_segs[c], stream);
     dhalo_items[c].upload_async(T.halo_items[c], stream);
     n_halo_items[c] = static_cast<int32_t>(T.halo_items[c].size());
@@ -419,19 +406,21 @@ void Batch::enqueue_step(int32_t k, cudaEvent_t tiles_begin, cudaEvent_t tiles_e
   }
   if (tiles_end) CUDA_CHECK(cudaEventRecord(tiles_end, stream));
   after_tiles();
-  // solid halos first: the fluid's coupling term reads the solid's new
-  // acceleration.  The two solid kernels run side by side.
-  bool overlap = tiles_end == nullptr;
-  const bool both = n_halo_items[1] > 0 && n_halo_items[2] > 0;
-  auto halo = [&](auto kernel, int cls, DepMode dep) {
+  // halo points: solves of a two-component solid, of a three-component one,
+  // of a fluid alone, side by side; then the fluids of split solves
+  bool first_halo = true;
+  auto halo = [&](auto kernel, int cls, bool after) {
     if (n_halo_items[cls] == 0) return;
-    CUDA_CHECK(launch_chained(kernel, n_halo_items[cls], kHaloChunk, 0, stream, overlap, dhalo_segs[cls].get(),
-                              dhalo_items[cls].get(), StepIdx{k, 0, dep}));
-    overlap = true;
+    const DepMode dep = after ? kDepAll : first_halo ? kDepFirst : kDepLate;
+    CUDA_CHECK(launch_chained(kernel, n_halo_items[cls], kHaloChunk, 0, stream, !first_halo || !tiles_end,
+                              dhalo_segs[cls].get(), dhalo_items[cls].get(), StepIdx{k, 0, dep}));
+    first_halo = false;
   };
-  halo(halo_batch_kernel<2, true>, 1, both ? kDepFirst : kDepAll);
-  halo(halo_batch_kernel<3, true>, 2, both ? kDepLate : kDepAll);
-  halo(halo_batch_kernel<1, false>, 0, kDepAll);
+  halo(halo_batch_kernel<2>, 1, false);
+  halo(halo_batch_kernel<3>, 2, false);
+  halo(halo_batch_kernel<0>, 0, false);
+  halo(halo_batch_kernel<2>, 3, true);
+  halo(halo_batch_kernel<3>, 4, true);
   if (n_energy > 0)
     CUDA_CHECK(launch_chained(energy_batch_kernel, n_energy, kReduceThreads, 0, stream, true, denergy.get(),
                               StepIdx{k, 0, kDepAll}));

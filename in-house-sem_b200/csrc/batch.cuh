@@ -6,8 +6,7 @@
 // the number of solves:
 //   one tile launch per tile class (ngll, kind, medium, order): one CTA
 //     per (segment, tile) item
-//   halo points of every solve (elastic classes, then acoustic: the fluid's
-//     coupling term reads the solid's new acceleration)
+//   halo points of every solve, by the solid's component count
 //   receivers (particle velocity, then recording) and energy of every solve
 //   step counters and buffer parities
 // The launches form one chain in which a launch may start before the one
@@ -46,11 +45,15 @@ struct TileClass {
   std::vector<TileItem> items;
 };
 
+constexpr int kHaloClasses = 5;
+
 // Host-side segment tables of one batch composition.
 struct BatchTables {
   std::map<int, TileClass> tiles;  // key: ((ngll * 4 + kind) * 2 + elastic) * 2 + m
-  std::vector<HaloSeg> halo_segs[3];  // 1 component (acoustic), 2 and 3 components (elastic)
-  std::vector<int2> halo_items[3];
+  // solves without a solid, with a solid of 2 and of 3 components; the fluids
+  // of solves whose halo points take two launches
+  std::vector<HaloArgs> halo_segs[kHaloClasses];
+  std::vector<int2> halo_items[kHaloClasses];
   std::vector<RecSeg> rec_segs;
   std::vector<int2> pv_items, rec_items;
   std::vector<EnergySeg> energy_segs;
@@ -130,9 +133,9 @@ class Batch {
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // one step, kSequence steps
   // device tables of the current composition
   std::vector<DevClass> dclasses;
-  DeviceBuffer<HaloSeg> dhalo_segs[3];
-  DeviceBuffer<int2> dhalo_items[3];
-  int32_t n_halo_items[3] = {0, 0, 0};
+  DeviceBuffer<HaloArgs> dhalo_segs[kHaloClasses];
+  DeviceBuffer<int2> dhalo_items[kHaloClasses];
+  int32_t n_halo_items[kHaloClasses] = {};
   DeviceBuffer<RecSeg> drec_segs;
   DeviceBuffer<int2> dpv_items, drec_items;
   int32_t n_pv_items = 0, n_rec_items = 0;

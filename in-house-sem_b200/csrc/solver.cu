@@ -879,6 +879,8 @@ void Solver::build_tiled(const insem_cuda_problem& p) {
                      host_vec(p.basis.w2, npe));
   const auto fp = host_vec(p.coupling.fluid_points, n_cpl), sp = host_vec(p.coupling.solid_points, n_cpl);
   tdom.resize(domains.size());
+  std::vector<int32_t> order[2];  // coupled points of the solid, of the fluid, in chunk order
+  std::vector<int4> chunks = coupled_chunks(fp, sp, order[0], order[1]);
   for (std::size_t di = 0; di < domains.size(); ++di) {
     const insem_cuda_domain& d = p.domains[di];
     SpecialTerms terms;
@@ -887,6 +889,7 @@ void Solver::build_tiled(const insem_cuda_problem& p) {
       if (static_cast<int>(di) == fluid) terms.coupling[fp[i]].push_back(i);
       if (static_cast<int>(di) == solid) terms.coupling[sp[i]].push_back(i);
     }
+    if (n_cpl > 0) terms.coupled = order[static_cast<int>(di) == solid ? 0 : 1];
     const auto ap = host_vec(d.absorbing_points, d.n_absorbing);
     for (int32_t i = 0; i < d.n_absorbing; ++i) terms.absorbing[ap[i]] = i;
     const uint8_t all = static_cast<uint8_t>((1u << d.ncomp) - 1u);
@@ -920,9 +923,23 @@ void Solver::build_tiled(const insem_cuda_problem& p) {
       f[i] = tdom[fluid].perm[fp[i]];
       s[i] = tdom[solid].perm[sp[i]];
     }
-    tcpl_fluid.upload(f);
-    tcpl_solid.upload(s);
+    const auto cx = host_vec(p.coupling.cx, n_cpl), cz = host_vec(p.coupling.cz, n_cpl);
+    tdom[solid].set_partners(f, cx, cz);
+    tdom[fluid].set_partners(s, cx, cz);
   }
+  // the chunks' ranges count from the first coupled halo point
+  n_chunks = static_cast<int32_t>(chunks.size());
+  for (int k = 0; k < 2; ++k) {
+    const int di = k == 0 ? solid : fluid;
+    n_free_halo[k] = di < 0 ? 0 : tdom[di].n_halo - static_cast<int32_t>(order[k].size());
+  }
+  for (int4& c : chunks) {
+    c.x += n_free_halo[0];
+    c.y += n_free_halo[0];
+    c.z += n_free_halo[1];
+    c.w += n_free_halo[1];
+  }
+  tchunks.upload(chunks);
   std::vector<int32_t> rp;
   for (int r = 0; r < p.n_receivers; ++r)
     for (int32_t g : host_vec(p.receivers[r].points, p.receivers[r].n_points))
@@ -934,12 +951,92 @@ void Solver::build_tiled(const insem_cuda_problem& p) {
     ep_ntile[di] = tdom[di].n_tiles;
     base += tdom[di].n_tiles;
     ep_halo[di] = base;
-    ep_nhalo[di] = ceil_div(std::max(tdom[di].n_halo, 1), 256);
+    ep_nhalo[di] = ceil_div(n_free_halo[static_cast<int>(di) == solid ? 0 : 1], kHaloChunk) + n_chunks;
     base += ep_nhalo[di];
   }
   epart.resize(2 * static_cast<std::size_t>(std::max(base, 1)));
   epart.zero();
   tiled = true;
+}
+
+// The coupled points in chunks of at most kHaloChunk per side.  A chunk holds
+// whole groups (points joined by interface entries), so that the fluid's
+// partners are finished by the same CTA.  Returns ranges into the orders;
+// nothing if a group is larger than a chunk.
+std::vector<int4> Solver::coupled_chunks(const std::vector<int32_t>& fp, const std::vector<int32_t>& sp,
+                                         std::vector<int32_t>& solid_order, std::vector<int32_t>& fluid_order) const {
+  std::vector<int4> chunks;
+  if (n_cpl == 0) return chunks;
+  std::map<int32_t, std::vector<int32_t>> of_solid, of_fluid;  // point -> entries
+  for (int32_t i = 0; i < n_cpl; ++i) {
+    of_solid[sp[i]].push_back(i);
+    of_fluid[fp[i]].push_back(i);
+  }
+  std::vector<char> seen(n_cpl, 0);
+  std::set<int32_t> s_done, f_done;
+  int4 c{0, 0, 0, 0};
+  for (int32_t i0 = 0; i0 < n_cpl; ++i0) {
+    if (seen[i0]) continue;
+    // the group of entry i0, breadth first
+    std::vector<int32_t> entries{i0}, gs, gf;
+    seen[i0] = 1;
+    for (std::size_t q = 0; q < entries.size(); ++q) {
+      const int32_t i = entries[q];
+      if (s_done.insert(sp[i]).second) gs.push_back(sp[i]);
+      if (f_done.insert(fp[i]).second) gf.push_back(fp[i]);
+      for (const auto* next : {&of_solid[sp[i]], &of_fluid[fp[i]]})
+        for (int32_t j : *next)
+          if (!seen[j]) {
+            seen[j] = 1;
+            entries.push_back(j);
+          }
+    }
+    const int32_t ns = static_cast<int32_t>(gs.size()), nf = static_cast<int32_t>(gf.size());
+    if (ns > kHaloChunk || nf > kHaloChunk) {
+      solid_order.clear();
+      fluid_order.clear();
+      return {};
+    }
+    if (c.y - c.x + ns > kHaloChunk || c.w - c.z + nf > kHaloChunk) {
+      chunks.push_back(c);
+      c = int4{c.y, c.y, c.w, c.w};
+    }
+    solid_order.insert(solid_order.end(), gs.begin(), gs.end());
+    fluid_order.insert(fluid_order.end(), gf.begin(), gf.end());
+    c.y += ns;
+    c.w += nf;
+  }
+  chunks.push_back(c);
+  return chunks;
+}
+
+// Arguments of the solve's halo kernel on the field buffers of `par`.
+HaloArgs Solver::halo_args(int par, bool init) {
+  HaloArgs A{};
+  if (solid >= 0) {
+    A.s_td = tdom[solid].view(par);
+    A.s_hd = tdom[solid].halo_view();
+    A.nb_s = ceil_div(n_free_halo[0], kHaloChunk);
+    A.ep_s = ep_halo[solid];
+    A.s_hd.n = n_free_halo[0];
+  }
+  if (fluid >= 0) {
+    A.f_td = tdom[fluid].view(par);
+    A.f_hd = tdom[fluid].halo_view();
+    A.nb_f = ceil_div(n_free_halo[1], kHaloChunk);
+    A.ep_f = ep_halo[fluid];
+    A.f_hd.n = n_free_halo[1];
+  }
+  A.n_chunk = n_chunks;
+  A.chunks = tchunks.get();
+  A.amp = src_amp.get();
+  A.n_amp = n_amp;
+  A.sc = StepScalars{static_cast<float>(dt), static_cast<float>(0.5 * dt), static_cast<float>(0.5 * dt * dt),
+                     energy_every};
+  A.h_damp = init ? 0.0 : 0.5 * dt;
+  A.st = st;
+  A.epartial = epart.get();
+  return A;
 }
 
 AllFields Solver::tiled_fields(int par) {
@@ -951,16 +1048,13 @@ AllFields Solver::tiled_fields(int par) {
 
 // n steps of the tiled path from the field buffers of `par` on (init: step 0,
 // explicit damping, no step count), as one chain of launches on the stream
-// (see DepMode).  A step's critical path is tiles -> halo points (solid, then
-// fluid).  The fluid's tiles run beside the solid's, and a step's receivers
+// (see DepMode).  A step's critical path is tiles -> halo points.  The fluid's tiles run beside the solid's, and a step's receivers
 // beside the next step's tiles: they read halo points only, which the next
 // step's halo kernels overwrite, not its tiles.   The first
 // kernel of a sequence keeps a full boundary to what is ahead of it.
 void Solver::enqueue_tiled(int par0, bool init, int n) {
   const StepScalars sc{static_cast<float>(dt), static_cast<float>(0.5 * dt), static_cast<float>(0.5 * dt * dt),
                        energy_every};
-  const double h_damp = init ? 0.0 : 0.5 * dt;
-  const CouplingDev cp{tcpl_fluid.get(), tcpl_solid.get(), cpl_cx.get(), cpl_cz.get()};
   ReceiversDev rv = receivers_view();
   rv.points = trec_points.get();
   auto observe = [&](int k, bool beside) {
@@ -1000,43 +1094,32 @@ void Solver::enqueue_tiled(int par0, bool init, int n) {
       }
     }
     if (k > 0) observe(k - 1, true);
-    for (int di : {solid, fluid}) {
-      if (di < 0) continue;
-      TiledDomain& t = tdom[di];
-      if (t.n_halo == 0) continue;
-      const bool el = t.medium == INSEM_ELASTIC;
-      const float* other = nullptr;
-      int32_t other_ng = 0;
-      bool pm = false;
-      if (n_cpl > 0) {
-        if (el) {
-          other = tdom[fluid].u_cur(par);
-          other_ng = tdom[fluid].ng;
-          pm = t.m == 1;
-        } else {
-          other = tdom[solid].a.get();
-          other_ng = tdom[solid].ng;
-          pm = tdom[solid].m == 1;
-        }
-      }
-      const StepIdx ix{k, init ? 1 : 0, kDepAll};
-      auto go = [&](auto kernel) {
-        CUDA_CHECK(launch_chained(kernel, ceil_div(t.n_halo, 256), 256, 0, stream, true, t.view(par), t.halo_view(), cp,
-                                  other, other_ng, pm, src_amp.get(), n_amp, sc, h_damp, st, epart.get(),
-                                  static_cast<int32_t>(ep_halo[di]), ix));
-      };
-      if (!el) go(halo_step_kernel<1, false>);
-      else if (t.ncomp == 2) go(halo_step_kernel<2, true>);
-      else go(halo_step_kernel<3, true>);
+    const HaloArgs A = halo_args(par, init);
+    const StepIdx ix{k, init ? 1 : 0, kDepAll};
+    auto halo = [&](const HaloArgs& h) {
+      const int grid = h.nb_s + h.nb_f + h.n_chunk;
+      if (grid == 0) return;
+      auto kernel = solid < 0 ? halo_step_kernel<0> : tdom[solid].ncomp == 2 ? halo_step_kernel<2> : halo_step_kernel<3>;
+      CUDA_CHECK(launch_chained(kernel, grid, kHaloChunk, 0, stream, true, h, ix));
+    };
+    if (n_cpl > 0 && n_chunks == 0) {  // a coupled group larger than a CTA: the solid's points, then the fluid's
+      HaloArgs one = A;
+      one.nb_f = 0;
+      halo(one);
+      one = A;
+      one.nb_s = 0;
+      halo(one);
+    } else {
+      halo(A);
     }
     if (energy_every > 0) {
       // potential order: elastic first
       const int d0 = solid >= 0 ? solid : fluid;
       const int d1 = solid >= 0 ? fluid : -1;
       const int n_dom = d1 >= 0 ? 2 : 1;
-      int4 s0{ep_tile[d0], ep_ntile[d0], ep_halo[d0], tdom[d0].n_halo > 0 ? ep_nhalo[d0] : 0};
+      int4 s0{ep_tile[d0], ep_ntile[d0], ep_halo[d0], ep_nhalo[d0]};
       int4 s1{0, 0, 0, 0};
-      if (d1 >= 0) s1 = int4{ep_tile[d1], ep_ntile[d1], ep_halo[d1], tdom[d1].n_halo > 0 ? ep_nhalo[d1] : 0};
+      if (d1 >= 0) s1 = int4{ep_tile[d1], ep_ntile[d1], ep_halo[d1], ep_nhalo[d1]};
       CUDA_CHECK(launch_chained(tiled_energy_kernel, 1, kReduceThreads, 0, stream, true, epart.get(), n_dom, s0, s1, st,
                                 energy_every, dt, energy.get(), static_cast<int32_t>(energy.size() / 3),
                                 StepIdx{k, init ? 1 : 0, kDepAll}));

@@ -170,7 +170,12 @@ class Solver {
   AllFields tiled_fields(int parity);
   std::vector<TiledDomain> tdom;
   std::vector<std::map<int32_t, std::vector<std::pair<int32_t, std::vector<float>>>>> src_per_point;
-  DeviceBuffer<int32_t> tcpl_fluid, tcpl_solid, trec_points;
+  DeviceBuffer<int32_t> trec_points;
+  std::vector<int4> coupled_chunks(const std::vector<int32_t>& fp, const std::vector<int32_t>& sp,
+                                   std::vector<int32_t>& solid_order, std::vector<int32_t>& fluid_order) const;
+  HaloArgs halo_args(int par, bool init);
+  DeviceBuffer<int4> tchunks;
+  int32_t n_chunks = 0, n_free_halo[2] = {0, 0};  // coupled chunks; halo points outside them (solid, fluid)
   DeviceBuffer<double> epart;
   int ep_tile[2] = {0, 0}, ep_halo[2] = {0, 0}, ep_ntile[2] = {0, 0}, ep_nhalo[2] = {0, 0};
   std::map<std::pair<int, int>, cudaGraphExec_t> tgraph;  // (first parity, steps) -> captured sequence

@@ -918,62 +918,92 @@ static __global__ void __launch_bounds__(TileCfg<NG>::THREADS, tile_min_ctas<NG,
   tile_batch_run<NG, KIND, EL, M>(segs, items, ix, L);
 }
 // ------------------------------------------------------------ halo kernel
-// Special-point records of a domain's halo points.
+// Special terms of a halo point: ranges of its source contributions and
+// coupling entries, Stacey index (or -1), components set to zero.
+struct HaloRec {
+  int32_t src0, src1, cpl0, cpl1, abs, zero;
+};
+// One fluid-solid interface entry of a point: the partner point in the other
+// domain's device numbering and the interface coefficients.
+struct __align__(16) CouplingEntry {
+  int32_t partner;
+  float cx, cz;
+  int32_t pad;
+};
+// A domain's halo points: device points [n_complete, n_complete + n), the
+// coupled ones last, in the order of the coupled chunks.
 struct HaloDev {
-  int32_t n = 0;                     // halo points: device points [n_complete, n_complete + n)
+  int32_t n = 0;
   const int32_t* off = nullptr;      // [n+1] each point's contributions in hbuf, ascending slot order
   const float* w = nullptr;          // its weight (constrained maps), nullptr when all are 1
   const int32_t* spec = nullptr;     // [n] special record or -1
-  const int32_t* src_off = nullptr;  // [n_spec+1] source contributions of each record
+  const HaloRec* rec = nullptr;
   const int32_t* src_which = nullptr;// source index of each contribution (row of the amplitude table)
   const float* src_coef = nullptr;   // [contributions][ncomp]
-  const int32_t* cpl_off = nullptr;  // [n_spec+1] coupling entries of each record
-  const int32_t* cpl_idx = nullptr;
-  const int32_t* abs_idx = nullptr;  // [n_spec] Stacey index or -1
+  const CouplingEntry* cpl = nullptr;
   const float* abs_coef = nullptr;   // [n_abs][ncomp*ncomp]
-  const uint8_t* zero = nullptr;     // [n_spec] components set to zero (Dirichlet, axis)
 };
 
-// Fluid-solid interface in device numbering of both domains.
-struct CouplingDev {
-  const int32_t* fluid = nullptr;
-  const int32_t* solid = nullptr;
-  const float* cx = nullptr;
-  const float* cz = nullptr;
+// What of a halo point is constant, requested ahead of the step's waits.
+struct HaloPoint {
+  float im = 0.0f;
+  int32_t b = 0, e = 0;  // contributions
+  HaloRec r{0, 0, 0, 0, -1, 0};
+  CouplingEntry c{0, 0.0f, 0.0f, 0};  // the first coupling entry
 };
+__device__ __forceinline__ HaloPoint halo_point(const TiledDev& td, const HaloDev& hd, int32_t h, bool in) {
+  HaloPoint p;
+  if (in) {
+    p.im = td.inv_mass[td.n_complete + h];
+    p.b = hd.off[h];
+    p.e = hd.off[h + 1];
+    const int32_t sp = hd.spec[h];
+    if (sp >= 0) {
+      p.r = hd.rec[sp];
+      if (p.r.cpl0 < p.r.cpl1) p.c = hd.cpl[p.r.cpl0];
+    }
+  }
+  return p;
+}
 
-// Finishes the halo points of one domain: the assembled force from the halo
-// buffer, then (solver.cpp:669-762) sources, coupling, a = f / M or the
-// implicit Stacey solve, Dirichlet / axis zeros, and the mode's update.
-// `other` is the fluid's current pressure (solid domain) or the solid's new
-// acceleration (fluid domain), in that domain's device numbering.
-// One halo point per thread; CTAs of 256 threads, `part` = the CTA's energy partial.
+// Finishes halo point h of one domain (every thread of the CTA calls; `in`: it
+// has a point): the assembled force from the halo buffer, then
+// (solver.cpp:669-762) sources, coupling, a = f / M or the implicit Stacey
+// solve, Dirichlet / axis zeros, and the mode's update.  `other` is the
+// fluid's current pressure (solid domain) or the solid's new acceleration
+// (fluid domain), in that domain's device numbering.  CTAs of 256 threads,
+// `part` = the CTA's energy partial.
 template <int NC, bool ELASTIC>
-__device__ __forceinline__ void halo_step_body(const TiledDev& td, const HaloDev& hd, const CouplingDev& cp,
-                                               const float* __restrict__ other, int32_t other_ng, bool pm,
-                                               const float* __restrict__ amp, int32_t n_amp, const StepScalars& sc,
-                                               double h_damp, const StepState* __restrict__ st, const StepNow& now,
-                                               int32_t dep, double* __restrict__ epartial, int32_t part, int32_t h) {
+__device__ __forceinline__ void halo_finish(const TiledDev& td, const float* u_cur, float* u_nxt, const HaloDev& hd,
+                                            const HaloPoint& hp, const float* other, int32_t other_ng, bool pm,
+                                            const float* __restrict__ amp, int32_t n_amp, const StepScalars& sc,
+                                            double h_damp, const StepState* __restrict__ st, const StepNow& now,
+                                            double* __restrict__ epartial, int32_t part, int32_t h, bool in) {
   const int mode = now.mode;
   const int32_t step = now.step;
   const bool energy = energy_step(now, sc.energy_every);
-  // constant data of the point, ahead of the wait
-  const bool in = h < hd.n;
-  const float im = in ? td.inv_mass[td.n_complete + h] : 0.0f;
-  const int32_t sp = in ? hd.spec[h] : -1;
-  const int32_t b = in ? hd.off[h] : 0, e = in ? hd.off[h + 1] : 0;
-  dep_wait(dep);
   double kin = 0.0, pot = 0.0;
   if (in) {
     const int32_t g = td.n_complete + h;
-    // the point's own values first, all loads in flight together (the
-    // stores below may alias them for the compiler)
+    const int32_t b = hp.b, e = hp.e;
+    // the point's own values and its partner's first, all loads in flight
+    // together (the stores below may alias them for the compiler)
     float uc[NC], vc[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      uc[c] = td.u_cur[static_cast<size_t>(c) * td.ng + g];
+      uc[c] = u_cur[static_cast<size_t>(c) * td.ng + g];
       vc[c] = td.v[static_cast<size_t>(c) * td.ng + g];
     }
+    const bool coupled = hp.r.cpl0 < hp.r.cpl1;
+    float o[3] = {0.0f, 0.0f, 0.0f};
+    auto partner = [&](int32_t gp) {
+      o[0] = other[gp];
+      if constexpr (!ELASTIC) {
+        o[1] = other[static_cast<size_t>(other_ng) + gp];
+        if (pm) o[2] = other[static_cast<size_t>(2) * other_ng + gp];
+      }
+    };
+    if (coupled) partner(hp.c.partner);
     float f[NC], a[NC];
     constexpr int K = 4;  // contributions gathered at once (conforming 2D points have at most 4)
     if (e - b <= K) {
@@ -1005,41 +1035,39 @@ __device__ __forceinline__ void halo_step_body(const TiledDev& td, const HaloDev
 #pragma unroll
       for (int c = 0; c < NC; ++c) pot = dadd(pot, dmul(static_cast<double>(uc[c]), static_cast<double>(f[c])));
     }
-    int32_t ai = -1;
-    uint8_t zmask = 0;
-    if (sp >= 0) {
-      for (int32_t q = hd.src_off[sp]; q < hd.src_off[sp + 1]; ++q) {
-        const float am = amp[static_cast<size_t>(hd.src_which[q]) * n_amp + step];
+    for (int32_t q = hp.r.src0; q < hp.r.src1; ++q) {
+      const float am = amp[static_cast<size_t>(hd.src_which[q]) * n_amp + step];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) f[c] = fadd(f[c], fmul(hd.src_coef[static_cast<size_t>(q) * NC + c], am));
-      }
+      for (int c = 0; c < NC; ++c) f[c] = fadd(f[c], fmul(hd.src_coef[static_cast<size_t>(q) * NC + c], am));
+    }
+    if (coupled) {
       const float hs = static_cast<float>(kSqrtHalf);
-      for (int32_t q = hd.cpl_off[sp]; q < hd.cpl_off[sp + 1]; ++q) {
-        const int32_t ci = hd.cpl_idx[q];
+      CouplingEntry ce = hp.c;
+      for (int32_t q = hp.r.cpl0;;) {
         if constexpr (ELASTIC) {
-          const float p = other[cp.fluid[ci]];
+          const float p = o[0];
           if (pm) {
-            const float t = fmul(fmul(hs, cp.cx[ci]), p);
+            const float t = fmul(fmul(hs, ce.cx), p);
             f[0] = fadd(f[0], t);
             f[1] = fadd(f[1], t);
           } else {
-            f[0] = fadd(f[0], fmul(cp.cx[ci], p));
+            f[0] = fadd(f[0], fmul(ce.cx, p));
           }
-          f[NC - 1] = fadd(f[NC - 1], fmul(cp.cz[ci], p));
+          f[NC - 1] = fadd(f[NC - 1], fmul(ce.cz, p));
         } else {
-          const int32_t gs = cp.solid[ci];
-          const float ar = pm ? fmul(hs, fadd(other[gs], other[static_cast<size_t>(other_ng) + gs])) : other[gs];
-          const float az = other[static_cast<size_t>(pm ? 2 : 1) * other_ng + gs];
-          f[0] = fsub(f[0], fadd(fmul(cp.cx[ci], ar), fmul(cp.cz[ci], az)));
+          const float ar = pm ? fmul(hs, fadd(o[0], o[1])) : o[0];
+          const float az = pm ? o[2] : o[1];
+          f[0] = fsub(f[0], fadd(fmul(ce.cx, ar), fmul(ce.cz, az)));
         }
+        if (++q >= hp.r.cpl1) break;
+        ce = hd.cpl[q];
+        partner(ce.partner);
       }
-      ai = hd.abs_idx[sp];
-      zmask = hd.zero[sp];
     }
 #pragma unroll
-    for (int c = 0; c < NC; ++c) a[c] = fmul(f[c], im);
-    if (ai >= 0) {
-      const float* cc = hd.abs_coef + static_cast<size_t>(ai) * NC * NC;
+    for (int c = 0; c < NC; ++c) a[c] = fmul(f[c], hp.im);
+    if (hp.r.abs >= 0) {
+      const float* cc = hd.abs_coef + static_cast<size_t>(hp.r.abs) * NC * NC;
       double A[NC * NC], rhs[NC];
       const double mass = td.mass[g];
 #pragma unroll
@@ -1057,11 +1085,11 @@ __device__ __forceinline__ void halo_step_body(const TiledDev& td, const HaloDev
     }
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      if (zmask & (1u << c)) a[c] = 0.0f;
+      if (hp.r.zero & (1 << c)) a[c] = 0.0f;
       const size_t gi = static_cast<size_t>(c) * td.ng + g;
       float u_out, v_state, v_n;
       complete_point(mode, sc, uc[c], vc[c], a[c], u_out, v_state, v_n);
-      td.u_nxt[gi] = u_out;
+      u_nxt[gi] = u_out;
       td.v[gi] = v_state;
       td.a[gi] = a[c];
       td.vn[gi] = v_n;
@@ -1095,20 +1123,83 @@ __device__ __forceinline__ void halo_step_body(const TiledDev& td, const HaloDev
   }
 }
 
-// Register budgets of the halo kernels (256 threads per CTA): two-component
-// points fit in 48 registers without spills (5 CTAs per SM instead of 4);
-// three-component ones in 64 with 40 bytes of spills in the rarely taken
-// Stacey solve (4 CTAs instead of 3).
+// The halo points of one solve: CTAs [0, n_chunk) finish a coupled chunk each,
+// the next nb_s the solid's points that are not coupled, the last nb_f the
+// fluid's.  The fluid's coupling term reads its partners' new acceleration, so
+// a chunk holds whole groups of coupled points, and its CTA finishes the
+// solid's before the fluid's (and starts first: it takes twice as long).  One
+// launch and one wait where two dependent launches took two, with the point's
+// constant data requested ahead of it: a step of the cased borehole went from
+// 17.0 to 12.8 us, one of 40,000 coupled order-5 elements from 25.6 to 22.4.  (A
+// group larger than a CTA keeps two launches: n_chunk is 0 then, and the
+// fluid's CTAs come after the solid's.)
+constexpr int kHaloChunk = 256;
+struct HaloArgs {
+  TiledDev s_td, f_td;
+  HaloDev s_hd, f_hd;
+  int32_t nb_s, nb_f, n_chunk;
+  int32_t n_amp;
+  const int4* chunks;  // halo points [x, y) of the solid, [z, w) of the fluid
+  const float* amp;
+  StepScalars sc;
+  int32_t ep_s, ep_f;  // first energy partials
+  double h_damp;
+  const StepState* st;
+  double* epartial;
+};
+// NC: the solid's components (0: no solid); odd: the views' field buffers are
+// exchanged (steps of odd parity).
 template <int NC>
-constexpr int kHaloRegs = NC == 2 ? 48 : 64;
-template <int NC, bool ELASTIC>
-static __global__ void __maxnreg__(kHaloRegs<NC>)
-    halo_step_kernel(TiledDev td, HaloDev hd, CouplingDev cp, const float* __restrict__ other, int32_t other_ng,
-                     bool pm, const float* __restrict__ amp, int32_t n_amp, StepScalars sc, double h_damp,
-                     const StepState* __restrict__ st, double* __restrict__ epartial, int32_t epart0, StepIdx ix) {
+__device__ __forceinline__ void halo_block(const HaloArgs& A, bool odd, const StepNow& now, int32_t dep, int32_t block) {
+  constexpr bool PM = NC == 3;
+  constexpr int SC = NC == 0 ? 1 : NC;
+  const float* s_cur = odd ? A.s_td.u_nxt : A.s_td.u_cur;
+  const float* f_cur = odd ? A.f_td.u_nxt : A.f_td.u_cur;
+  float* s_nxt = odd ? const_cast<float*>(A.s_td.u_cur) : A.s_td.u_nxt;
+  float* f_nxt = odd ? const_cast<float*>(A.f_td.u_cur) : A.f_td.u_nxt;
+  auto solid = [&](const HaloPoint& p, int32_t part, int32_t h, bool in) {
+    halo_finish<SC, true>(A.s_td, s_cur, s_nxt, A.s_hd, p, f_cur, A.f_td.ng, PM, A.amp, A.n_amp, A.sc, A.h_damp, A.st, now,
+                          A.epartial, A.ep_s + part, h, in);
+  };
+  auto fluid = [&](const HaloPoint& p, int32_t part, int32_t h, bool in) {
+    halo_finish<1, false>(A.f_td, f_cur, f_nxt, A.f_hd, p, A.s_td.a, A.s_td.ng, PM, A.amp, A.n_amp, A.sc, A.h_damp, A.st,
+                          now, A.epartial, A.ep_f + part, h, in);
+  };
+  const int32_t t = threadIdx.x;
+  if (NC > 0 && block < A.n_chunk) {
+    const int4 ch = A.chunks[block];
+    const int32_t hs = ch.x + t, hf = ch.z + t;
+    const HaloPoint ps = halo_point(A.s_td, A.s_hd, hs, hs < ch.y);
+    const HaloPoint pf = halo_point(A.f_td, A.f_hd, hf, hf < ch.w);
+    dep_wait(dep);
+    solid(ps, block, hs, hs < ch.y);
+    __syncthreads();
+    fluid(pf, block, hf, hf < ch.w);
+    return;
+  }
+  const int32_t b = block - A.n_chunk;
+  if (NC > 0 && b < A.nb_s) {
+    const int32_t h = b * kHaloChunk + t;
+    const HaloPoint p = halo_point(A.s_td, A.s_hd, h, h < A.s_hd.n);
+    dep_wait(dep);
+    solid(p, block, h, h < A.s_hd.n);
+  } else {
+    const int32_t h = (b - A.nb_s) * kHaloChunk + t;
+    const HaloPoint p = halo_point(A.f_td, A.f_hd, h, h < A.f_hd.n);
+    dep_wait(dep);
+    fluid(p, block - A.nb_s, h, h < A.f_hd.n);
+  }
+}
+
+// Register budgets of the halo kernels (256 threads per CTA): 3 to 5 CTAs per
+// SM.  With 16 more or fewer per thread the dipole borehole (30k elements) took
+// 49 and 47 us a step for 46, the ocean bottom (147k) 67 and 64 for 66.
+template <int NC>
+constexpr int kHaloRegs = NC == 3 ? 80 : NC == 2 ? 64 : 48;
+template <int NC>
+static __global__ void __maxnreg__(kHaloRegs<NC>) halo_step_kernel(const __grid_constant__ HaloArgs A, StepIdx ix) {
   dep_begin(ix.dep);
-  halo_step_body<NC, ELASTIC>(td, hd, cp, other, other_ng, pm, amp, n_amp, sc, h_damp, st, step_now(st, ix), ix.dep,
-                              epartial, epart0 + blockIdx.x, blockIdx.x * blockDim.x + threadIdx.x);
+  halo_block<NC>(A, false, step_now(A.st, ix), ix.dep, blockIdx.x);
   dep_end(ix.dep);
 }
 
@@ -1168,45 +1259,24 @@ static __global__ void tiled_energy_kernel(const double* __restrict__ epartial, 
 // The point-wise kernels of many solves in one launch each: one CTA per work
 // item (segment, chunk); the segment carries one solve's pointers and
 // scalars, the solve's StepState its step, mode and buffer parity.
-constexpr int kHaloChunk = 256;
 
-struct HaloSeg {
-  TiledDev td;          // parity-0 view
-  HaloDev hd;
-  CouplingDev cp;
-  const float* other0;  // coupling input at parity 0 / 1 (fluid u, or the solid's a at both)
-  const float* other1;
-  int32_t other_ng;
-  int32_t pm;
-  const float* amp;
-  int32_t n_amp;
-  StepScalars sc;
-  double h_damp;
-  const StepState* st;
-  double* epartial;
-  int32_t epart0;
-};
-
-template <int NC, bool ELASTIC>
-static __global__ void __maxnreg__(kHaloRegs<NC>) halo_batch_kernel(const HaloSeg* __restrict__ segs,
-                                                                         const int2* __restrict__ items, StepIdx ix) {
+// A segment is one solve (its views at parity 0).
+template <int NC>
+static __global__ void __maxnreg__(kHaloRegs<NC>) halo_batch_kernel(const HaloArgs* __restrict__ segs,
+                                                                    const int2* __restrict__ items, StepIdx ix) {
   dep_begin(ix.dep);
+  __shared__ __align__(16) uint32_t s_words[sizeof(HaloArgs) / 4];  // the segment
+  static_assert(sizeof(HaloArgs) % 4 == 0, "HaloArgs is copied as 32-bit words");
   const int2 it = items[blockIdx.x];
-  const HaloSeg& sg = segs[it.x];
-  const StepNow now = step_now(sg.st, ix);
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(segs + it.x);
+  for (int q = threadIdx.x; q < static_cast<int>(sizeof(HaloArgs) / 4); q += kHaloChunk) s_words[q] = src[q];
+  __syncthreads();
+  const HaloArgs& A = *reinterpret_cast<const HaloArgs*>(s_words);
+  const StepNow now = step_now(A.st, ix);
   if (now.mode == kModeIdle) {
     dep_wait(ix.dep);
   } else {
-    const int par = (sg.st->parity ^ ix.k) & 1;
-    TiledDev td = sg.td;
-    if (par) {
-      const float* cur = td.u_cur;
-      td.u_cur = td.u_nxt;
-      td.u_nxt = const_cast<float*>(cur);
-    }
-    halo_step_body<NC, ELASTIC>(td, sg.hd, sg.cp, par ? sg.other1 : sg.other0, sg.other_ng, sg.pm != 0, sg.amp,
-                                sg.n_amp, sg.sc, sg.h_damp, sg.st, now, ix.dep, sg.epartial, sg.epart0 + it.y,
-                                it.y * kHaloChunk + static_cast<int32_t>(threadIdx.x));
+    halo_block<NC>(A, (A.st->parity ^ ix.k) & 1, now, ix.dep, it.y);
   }
   dep_end(ix.dep);
 }

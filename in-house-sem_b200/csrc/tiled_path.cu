@@ -195,15 +195,22 @@ HaloDev TiledDomain::halo_view() const {
   h.off = h_off.get();
   h.w = weighted ? h_w.get() : nullptr;
   h.spec = h_spec.get();
-  h.src_off = src_off.get();
+  h.rec = h_rec.get();
   h.src_which = src_which.get();
   h.src_coef = src_coef.get();
-  h.cpl_off = cpl_off.get();
-  h.cpl_idx = cpl_idx.get();
-  h.abs_idx = abs_idx.get();
+  h.cpl = h_cpl.get();
   h.abs_coef = abs_coef_d.get();
-  h.zero = zero.get();
   return h;
+}
+
+// The coupling entries' partner points (device numbering of the other domain)
+// and coefficients, by entry of the interface.
+void TiledDomain::set_partners(const std::vector<int32_t>& partner, const std::vector<float>& cx,
+                               const std::vector<float>& cz) {
+  std::vector<CouplingEntry> e(std::max<std::size_t>(cpl_entry.size(), 1), CouplingEntry{0, 0.0f, 0.0f, 0});
+  for (std::size_t q = 0; q < cpl_entry.size(); ++q)
+    e[q] = CouplingEntry{partner[cpl_entry[q]], cx[cpl_entry[q]], cz[cpl_entry[q]], 0};
+  h_cpl.upload(e);
 }
 
 void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const SpecialTerms& sp,
@@ -342,15 +349,15 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
         for (int32_t l = 0; l < n_direct[t]; ++l)
           perm[l2g[static_cast<std::size_t>(tile_elems[t][l]) * npe + inner_slot(q)]] = cbeg[t] + q * kTileLanes + l;
     std::vector<int32_t> fill(ebeg);
+    std::vector<char> last(ng, 0);
+    for (int32_t g : sp.coupled) last[g] = 1;
     int32_t h = n_complete;
     for (int32_t g = 0; g < ng; ++g) {
-      if (inner[g]) continue;
-      if (owner[g] >= 0) perm[g] = fill[owner[g]]++;
-      else {
-        perm[g] = h++;
-        ++n_halo_pts;
-      }
+      if (inner[g] || last[g]) continue;
+      perm[g] = owner[g] >= 0 ? fill[owner[g]]++ : h++;
     }
+    for (int32_t g : sp.coupled) perm[g] = h++;
+    n_halo_pts = h - n_complete;
   }
   n_halo = n_halo_pts;
   const int32_t ng_dev = std::max(up4(n_complete + n_halo), 4);
@@ -456,9 +463,10 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
   }
 
   // 6. halo CSR and special records (device order of halo points)
-  std::vector<int32_t> hoff{0}, hpos, hspec(n_halo, -1), soff{0}, swhich, coff{0}, cidx2, aidx;
+  std::vector<int32_t> hoff{0}, hpos, hspec(n_halo, -1), swhich;
+  std::vector<HaloRec> recs;
   std::vector<float> hw, scoef;
-  std::vector<uint8_t> zm;
+  cpl_entry.clear();
   std::vector<int32_t> halo_orig(n_halo);
   for (int32_t g = 0; g < ng; ++g)
     if (owner[g] < 0) halo_orig[perm[g] - n_complete] = g;
@@ -472,21 +480,20 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
     }
     hoff.push_back(static_cast<int32_t>(hpos.size()));
     if (!special[g]) continue;
-    const int32_t rec = static_cast<int32_t>(aidx.size());
-    hspec[h] = rec;
+    hspec[h] = static_cast<int32_t>(recs.size());
+    HaloRec r{static_cast<int32_t>(swhich.size()), 0, static_cast<int32_t>(cpl_entry.size()), 0, -1, 0};
     if (auto it = sp.sources.find(g); it != sp.sources.end())
       for (const auto& [s, cs] : it->second) {
         swhich.push_back(s);
         scoef.insert(scoef.end(), cs.begin(), cs.end());
       }
-    soff.push_back(static_cast<int32_t>(swhich.size()));
+    r.src1 = static_cast<int32_t>(swhich.size());
     if (auto it = sp.coupling.find(g); it != sp.coupling.end())
-      for (int32_t ci : it->second) cidx2.push_back(ci);
-    coff.push_back(static_cast<int32_t>(cidx2.size()));
-    auto ia = sp.absorbing.find(g);
-    aidx.push_back(ia == sp.absorbing.end() ? -1 : ia->second);
-    auto iz = sp.zero.find(g);
-    zm.push_back(iz == sp.zero.end() ? 0 : iz->second);
+      cpl_entry.insert(cpl_entry.end(), it->second.begin(), it->second.end());
+    r.cpl1 = static_cast<int32_t>(cpl_entry.size());
+    if (auto ia = sp.absorbing.find(g); ia != sp.absorbing.end()) r.abs = ia->second;
+    if (auto iz = sp.zero.find(g); iz != sp.zero.end()) r.zero = iz->second;
+    recs.push_back(r);
   }
 
   // Places of the halo-buffer entries in hbuf: hbuf holds each halo point's
@@ -528,13 +535,9 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
   h_off.upload(hoff);
   if (weighted) h_w.upload(hw.empty() ? std::vector<float>{0.0f} : hw);
   h_spec.upload(hspec.empty() ? std::vector<int32_t>{0} : hspec);
-  src_off.upload(soff);
   src_which.upload(swhich.empty() ? std::vector<int32_t>{0} : swhich);
   src_coef.upload(scoef.empty() ? std::vector<float>{0.0f} : scoef);
-  cpl_off.upload(coff);
-  cpl_idx.upload(cidx2.empty() ? std::vector<int32_t>{0} : cidx2);
-  abs_idx.upload(aidx.empty() ? std::vector<int32_t>{0} : aidx);
-  zero.upload(zm.empty() ? std::vector<uint8_t>{0} : zm);
+  h_rec.upload(recs.empty() ? std::vector<HaloRec>(1, HaloRec{0, 0, 0, 0, -1, 0}) : recs);
   abs_coef_d.upload(abs_coef_host.empty() ? std::vector<float>{0.0f} : abs_coef_host);
   // constraint rows with device-numbered dofs (weights rounded as the gather does)
   {

@@ -16,6 +16,7 @@ struct SpecialTerms {
   std::map<int32_t, int32_t> absorbing;                                           // point -> Stacey index
   std::map<int32_t, uint8_t> zero;                                                // point -> zeroed components
   std::vector<int32_t> receivers;                                                 // points read by receivers
+  std::vector<int32_t> coupled;  // coupled points in chunk order: numbered last, in this order
 };
 
 // One domain of the tiled path.
@@ -48,9 +49,12 @@ class TiledDomain {
   DeviceBuffer<int2> cs_row;
   DeviceBuffer<float> hbuf, mass, inv_mass;
   DeviceBuffer<float> u0, u1, v, a, vn;
-  DeviceBuffer<int32_t> h_off, h_spec, src_off, src_which, cpl_off, cpl_idx, abs_idx;
+  DeviceBuffer<int32_t> h_off, h_spec, src_which;
+  DeviceBuffer<HaloRec> h_rec;
+  DeviceBuffer<CouplingEntry> h_cpl;
   DeviceBuffer<float> h_w, src_coef, abs_coef_d;
-  DeviceBuffer<uint8_t> zero;
+  std::vector<int32_t> cpl_entry;  // coupling entry of each h_cpl element (its partner is filled in by set_partners)
+  void set_partners(const std::vector<int32_t>& partner, const std::vector<float>& cx, const std::vector<float>& cz);
   DeviceBuffer<int32_t> rows_off, rows_dofs;  // constraint rows in device numbering
   DeviceBuffer<float> rows_w;
   RowsDev rows() const { return {rows_off.get(), rows_dofs.get(), rows_w.get()}; }
