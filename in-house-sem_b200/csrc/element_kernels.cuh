@@ -18,21 +18,33 @@ namespace insem_b200 {
 // Value of slot k of element e, component c, of a global field
 // (DofMap::gather, dof_map.hpp:95-120): direct, or the constraint row's
 // weighted sum in row order starting from zero.
-__device__ __forceinline__ float gather_slot(const float* __restrict__ g, int32_t m, const RowsDev& rows) {
-  if (m >= 0) return __ldg(g + m);
+template <class Value>
+__device__ __forceinline__ float gather_slot(int32_t m, const RowsDev& rows, Value&& value) {
+  if (m >= 0) return value(m);
   const int32_t r = -1 - m;
   float s = 0.0f;
-  for (int32_t q = rows.offsets[r]; q < rows.offsets[r + 1]; ++q) s = fadd(s, fmul(rows.weights[q], __ldg(g + rows.dofs[q])));
+  for (int32_t q = rows.offsets[r]; q < rows.offsets[r + 1]; ++q) s = fadd(s, fmul(rows.weights[q], value(rows.dofs[q])));
   return s;
 }
+__device__ __forceinline__ float gather_slot(const float* g, int32_t m, const RowsDev& rows) {
+  return gather_slot(m, rows, [g](int32_t p) { return g[p]; });
+}
+// A float field times a double factor, rounded to float (the power
+// iteration's fields, whose factor is applied where they are read).
+__device__ __forceinline__ float scaled(float x, double scale) {
+  return static_cast<float>(dmul(static_cast<double>(x), scale));
+}
 
-template <int NG, int KIND, bool ELASTIC, int M, bool GATHER>
+// Where an element kernel takes its field from.
+enum FieldSource : int { kFieldLocal = 0, kFieldGlobal = 1, kFieldScaled = 2 };
+
+template <int NG, int KIND, bool ELASTIC, int M, int SOURCE>
 __global__ void __launch_bounds__(ElemCfg<NG, KIND, ELASTIC, M>::THREADS)
-    element_forces_kernel(BasisDev basis, BlockDev blk, const float* __restrict__ u_in,
-                          const int32_t* __restrict__ l2g, RowsDev rows, int32_t n_global,
-                          float* __restrict__ f_local) {
+    element_forces_kernel(BasisDev basis, BlockDev blk, const float* u_in, const int32_t* __restrict__ l2g, RowsDev rows,
+                          int32_t n_global, const double* scale, int32_t dep, float* __restrict__ f_local) {
   using C = ElemCfg<NG, KIND, ELASTIC, M>;
   __shared__ ElemSmem<C> sm;
+  dep_begin(dep);
   const int tid = threadIdx.x;
   for (int t = tid; t < C::NPE; t += C::THREADS) {
     sm.D[t] = basis.D[t];
@@ -45,13 +57,25 @@ __global__ void __launch_bounds__(ElemCfg<NG, KIND, ELASTIC, M>::THREADS)
   const bool active = bb < blk.n;
   int e = 0;
   bool axial = false;
+  int32_t slot = 0;
   if (active) {
     e = blk.elements[bb];
     if constexpr (C::AXI) axial = blk.axial[bb] != 0;
-    if constexpr (GATHER) {
-      const int32_t m = l2g[static_cast<size_t>(e) * C::NPE + kpt];
+    if constexpr (SOURCE != kFieldLocal) slot = l2g[static_cast<size_t>(e) * C::NPE + kpt];
+  }
+  dep_wait(dep);
+  if (active) {
+    if constexpr (SOURCE != kFieldLocal) {
+      double f = 1.0;
+      if constexpr (SOURCE == kFieldScaled) f = *scale;
 #pragma unroll
-      for (int c = 0; c < C::NC; ++c) sm.u[el][c][kpt] = gather_slot(u_in + static_cast<size_t>(c) * n_global, m, rows);
+      for (int c = 0; c < C::NC; ++c) {
+        const float* g = u_in + static_cast<size_t>(c) * n_global;
+        if constexpr (SOURCE == kFieldScaled)
+          sm.u[el][c][kpt] = gather_slot(slot, rows, [g, f](int32_t p) { return scaled(g[p], f); });
+        else
+          sm.u[el][c][kpt] = gather_slot(g, slot, rows);
+      }
     } else {
 #pragma unroll
       for (int c = 0; c < C::NC; ++c) sm.u[el][c][kpt] = u_in[(static_cast<size_t>(e) * C::NC + c) * C::NPE + kpt];
@@ -74,6 +98,7 @@ __global__ void __launch_bounds__(ElemCfg<NG, KIND, ELASTIC, M>::THREADS)
 #pragma unroll
     for (int c = 0; c < C::NC; ++c) f_local[(static_cast<size_t>(e) * C::NC + c) * C::NPE + kpt] = out[c];
   }
+  dep_end(dep);
 }
 
 // Arguments of one element-forces launch.
@@ -86,7 +111,10 @@ struct ElementLaunch {
   int32_t n_global = 0;            // gathering only
   float* f_local = nullptr;
   bool gather = false;
+  const double* scale = nullptr;   // gathering only: factor of the field
   bool elastic = false;
+  int32_t dep = kDepAll;           // how the launch follows the one ahead of it
+  bool overlap = false;
   // load the kernel this launch would run (its module, under lazy loading)
   // without launching it
   bool preload = false;
@@ -97,21 +125,19 @@ template <int NG, int KIND, bool ELASTIC, int M>
 void launch_element_cfg(const ElementLaunch& a) {
   using C = ElemCfg<NG, KIND, ELASTIC, M>;
   if (a.blk.n <= 0) return;
-  if (a.preload) {
-    cudaFuncAttributes fa;
-    if (a.gather) CUDA_CHECK(cudaFuncGetAttributes(&fa, element_forces_kernel<NG, KIND, ELASTIC, M, true>));
-    else CUDA_CHECK(cudaFuncGetAttributes(&fa, element_forces_kernel<NG, KIND, ELASTIC, M, false>));
-    return;
-  }
-  const int grid = ceil_div(a.blk.n, C::EPB);
-  if (a.gather) {
-    element_forces_kernel<NG, KIND, ELASTIC, M, true>
-        <<<grid, C::THREADS, 0, a.stream>>>(a.basis, a.blk, a.u_in, a.l2g, a.rows, a.n_global, a.f_local);
-  } else {
-    element_forces_kernel<NG, KIND, ELASTIC, M, false>
-        <<<grid, C::THREADS, 0, a.stream>>>(a.basis, a.blk, a.u_in, a.l2g, a.rows, a.n_global, a.f_local);
-  }
-  CUDA_LAUNCH_CHECK();
+  auto go = [&](auto kernel) {
+    if (a.preload) {
+      cudaFuncAttributes fa;
+      CUDA_CHECK(cudaFuncGetAttributes(&fa, kernel));
+      return;
+    }
+    CUDA_CHECK(launch_chained(kernel, ceil_div(a.blk.n, C::EPB), C::THREADS, 0, a.stream, a.overlap, a.basis, a.blk, a.u_in,
+                              a.l2g, a.rows, a.n_global, a.scale, a.dep, a.f_local));
+    CUDA_LAUNCH_CHECK();
+  };
+  if (!a.gather) go(element_forces_kernel<NG, KIND, ELASTIC, M, kFieldLocal>);
+  else if (!a.scale) go(element_forces_kernel<NG, KIND, ELASTIC, M, kFieldGlobal>);
+  else go(element_forces_kernel<NG, KIND, ELASTIC, M, kFieldScaled>);
 }
 
 template <int NG>
@@ -149,6 +175,19 @@ void launch_element_ng6(const ElementLaunch&);
 void launch_element_ng7(const ElementLaunch&);
 void launch_element_ng8(const ElementLaunch&);
 void launch_element_ng9(const ElementLaunch&);
+
+struct PowerLaunch;
+#define INSEM_POWER(N) void launch_power_ng##N(const PowerLaunch&);
+INSEM_POWER(2)
+INSEM_POWER(3)
+INSEM_POWER(4)
+INSEM_POWER(5)
+INSEM_POWER(6)
+INSEM_POWER(7)
+INSEM_POWER(8)
+INSEM_POWER(9)
+#undef INSEM_POWER
+void launch_power(int ngll, const PowerLaunch& a);
 
 // Dispatch on the number of GLL points; unsupported values fail like
 // physics::select (kernels.cpp:451-468).

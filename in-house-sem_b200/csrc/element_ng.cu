@@ -1,6 +1,6 @@
-// Element-forces launchers for one number of GLL points, selected at compile
+// Element-forces and power-iteration launchers for one number of GLL points, selected at compile
 // time with -DINSEM_NG=<2..9>; the build compiles this file once per value.
-#include "element_kernels.cuh"
+#include "power.cuh"
 
 #ifndef INSEM_NG
 #error "compile with -DINSEM_NG=<number of GLL points>"
@@ -12,5 +12,7 @@
 namespace insem_b200 {
 
 void INSEM_CAT(launch_element_ng, INSEM_NG)(const ElementLaunch& a) { launch_element_ng<INSEM_NG>(a); }
+
+void INSEM_CAT(launch_power_ng, INSEM_NG)(const PowerLaunch& a) { launch_power_cfg<INSEM_NG>(a); }
 
 }  // namespace insem_b200

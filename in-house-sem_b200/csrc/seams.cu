@@ -28,6 +28,20 @@ void launch_element_forces(int ngll, const ElementLaunch& a) {
   }
 }
 
+void launch_power(int ngll, const PowerLaunch& a) {
+  switch (ngll) {
+    case 2: launch_power_ng2(a); break;
+    case 3: launch_power_ng3(a); break;
+    case 4: launch_power_ng4(a); break;
+    case 5: launch_power_ng5(a); break;
+    case 6: launch_power_ng6(a); break;
+    case 7: launch_power_ng7(a); break;
+    case 8: launch_power_ng8(a); break;
+    case 9: launch_power_ng9(a); break;
+    default: check_ngll(ngll);
+  }
+}
+
 // ------------------------------------------------------- gather / assemble
 // DofMap::gather (dof_map.hpp:95-120): one thread per element slot.
 __global__ void gather_kernel(const int32_t* __restrict__ l2g, RowsDev rows, int32_t n_slots, int32_t npe,

@@ -15,6 +15,7 @@
 #include <set>
 
 #include "device_data.cuh"
+#include "power.cuh"
 #include "solver.cuh"
 #include "stf.hpp"
 
@@ -86,15 +87,6 @@ void DeviceDomainData::alloc_fields(cudaStream_t s) {
   fields_ready = true;
 }
 
-void DeviceDomainData::free_fields() {
-  u.resize(0);
-  v.resize(0);
-  a.resize(0);
-  f.resize(0);
-  f_local.resize(0);
-  fields_ready = false;
-}
-
 Solver::Solver(const insem_cuda_problem& p, const insem_cuda_options* opt, bool setup_only,
                const insem_cuda_time* time) {
   if (opt) opts = *opt;
@@ -152,8 +144,6 @@ Solver::Solver(const insem_cuda_problem& p, const insem_cuda_options* opt, bool 
     if (time->n_steps > 0) n_steps = time->n_steps;
     else if (time->duration > 0.0) n_steps = static_cast<int32_t>(std::ceil(time->duration / dt - 1e-9));
     else n_steps = 0;
-    // the power iteration's two-pass fields; the path chosen below allocates what it uses
-    for (auto& d : domains) d.free_fields();
   }
   build_sources(p);
   build_receivers(p);
@@ -423,17 +413,10 @@ void Solver::coupling_forces(int di) {
   CUDA_LAUNCH_CHECK();
 }
 
-// Sum of the kReduceBlocks partials of set 0, in a fixed order on the host.
-double Solver::reduce_partials() {
-  std::vector<double> h(kReduceBlocks);
-  CUDA_CHECK(cudaMemcpyAsync(h.data(), partial.get(), kReduceBlocks * sizeof(double), cudaMemcpyDeviceToHost, stream));
-  CUDA_CHECK(cudaStreamSynchronize(stream));
-  double s = 0.0;
-  for (double v : h) s += v;
-  return s;
-}
-
-void Solver::replay(int n, const std::function<void()>& body) {
+// Runs `body` (launches on `stream` only) n times: captured once as a CUDA
+// graph, which the stream replays.  The graph is kept until the caller has
+// waited for the stream.
+void Solver::replay(int n, const std::function<void()>& body, std::vector<cudaGraphExec_t>& graphs) {
   if (n <= 0) return;
   cudaGraph_t g = nullptr;
   CUDA_CHECK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
@@ -450,59 +433,205 @@ void Solver::replay(int n, const std::function<void()>& body) {
   const cudaError_t e = cudaGraphInstantiate(&ge, g, 0);
   cudaGraphDestroy(g);
   CUDA_CHECK(e);
-  cudaError_t le = cudaSuccess;
-  for (int i = 0; i < n && le == cudaSuccess; ++i) le = cudaGraphLaunch(ge, stream);
-  const cudaError_t se = cudaStreamSynchronize(stream);
-  cudaGraphExecDestroy(ge);
-  CUDA_CHECK(le);
-  CUDA_CHECK(se);
+  graphs.push_back(ge);
+  for (int i = 0; i < n; ++i) CUDA_CHECK(cudaGraphLaunch(ge, stream));
 }
 
+namespace {
+// The start vectors' numbers: std::uniform_real_distribution<double>(-1, 1)
+// over std::mt19937(12345), rounded to float.  The Mersenne twister (Matsumoto
+// and Nishimura 1998) refilled a state at a time, in loops the compiler
+// vectorises; two outputs a, b make (a + b 2^32) / 2^64, as the standard's
+// generate_canonical takes 53 bits from a 32-bit engine.
+class StartVector {
+ public:
+  StartVector() {
+    mt_[0] = 12345u;
+    for (uint32_t k = 1; k < kN; ++k) mt_[k] = 1812433253u * (mt_[k - 1] ^ (mt_[k - 1] >> 30)) + k;
+  }
+  void fill(float* out, std::size_t n) {
+    for (std::size_t i = 0; i < n; ++i) {
+      if (at_ >= kN) refill();
+      const double r = (static_cast<double>(out_[at_]) + static_cast<double>(out_[at_ + 1]) * 4294967296.0) / 18446744073709551616.0;
+      out[i] = static_cast<float>((r < 1.0 ? r : std::nextafter(1.0, 0.0)) * 2.0 + -1.0);
+      at_ += 2;  // 624 is even: a pair never straddles two states
+    }
+  }
+
+ private:
+  static constexpr uint32_t kN = 624, kM = 397;
+  static uint32_t mix(uint32_t hi, uint32_t lo) {
+    const uint32_t y = (hi & 0x80000000u) | (lo & 0x7fffffffu);
+    return (y >> 1) ^ ((0u - (lo & 1u)) & 0x9908b0dfu);
+  }
+  void refill() {
+    for (uint32_t k = 0; k < kN - kM; ++k) mt_[k] = mt_[k + kM] ^ mix(mt_[k], mt_[k + 1]);
+    for (uint32_t k = kN - kM; k < kN - 1; ++k) mt_[k] = mt_[k + kM - kN] ^ mix(mt_[k], mt_[k + 1]);
+    mt_[kN - 1] = mt_[kM - 1] ^ mix(mt_[kN - 1], mt_[0]);
+    for (uint32_t k = 0; k < kN; ++k) {
+      uint32_t y = mt_[k];
+      y ^= y >> 11;
+      y ^= (y << 7) & 0x9d2c5680u;
+      y ^= (y << 15) & 0xefc60000u;
+      out_[k] = y ^ (y >> 18);
+    }
+    at_ = 0;
+  }
+  uint32_t mt_[kN], out_[kN];
+  uint32_t at_ = kN;
+};
+}  // namespace
+
 // estimate_stable_dt (solver.cpp:583-619): 100 power iterations per domain
-// with x ~ U(-1, 1) from mt19937(12345), Rayleigh quotients in double.
+// with x ~ U(-1, 1), Rayleigh quotients in double; then coupled_lambda_max
+// (solver.cpp:621-667): growth of the mass norm under the coupled operator, 120
+// iterations, sqrt(ny / nx) from iteration 60 on.
 double Solver::stable_dt() {
   DeviceGuard dg(device);
-  for (auto& d : domains) d.alloc_fields(stream);
-  std::mt19937 rng(12345);
-  std::uniform_real_distribution<double> dist(-1.0, 1.0);
-  DeviceBuffer<double> pw(kPwCount);
-  pw.zero(stream);
-  auto reduce_into = [&](int slot, double sign) {
-    sum_partials_kernel<<<1, kReduceBlocks, 0, stream>>>(partial.get(), kReduceBlocks, sign, pw.get(), slot);
-    CUDA_LAUNCH_CHECK();
+  struct Work {
+    DeviceBuffer<float> x, f_local;
+    DeviceBuffer<uint8_t> zero;
+    DeviceBuffer<int32_t> cpl_off;
+    DeviceBuffer<PowerEntry> cpl;
+    DeviceBuffer<double> partial;
+    std::vector<float> start;
   };
-  for (auto& d : domains) {
-    const int64_t n = static_cast<int64_t>(d.ncomp) * d.ng;
-    std::vector<float> x(n);
-    for (auto& v : x) v = static_cast<float>(dist(rng));
-    DeviceBuffer<float> dx(n);
-    CUDA_CHECK(cudaMemcpyAsync(dx.get(), x.data(), n * sizeof(float), cudaMemcpyHostToDevice, stream));
+  std::vector<Work> work(domains.size());
+  std::vector<float> start2[2];
+  std::vector<cudaGraphExec_t> graphs;
+  DeviceBuffer<double> pw(kPwCount);
+  DeviceBuffer<uint32_t> counter(1);
+  const double one = 1.0;
+  struct Release {  // the work buffers and host vectors outlive the stream's use of them
+    cudaStream_t s;
+    std::vector<cudaGraphExec_t>& g;
+    ~Release() {
+      cudaStreamSynchronize(s);
+      for (cudaGraphExec_t e : g) cudaGraphExecDestroy(e);
+    }
+  } release{stream, graphs};
+  StartVector rng;
+  pw.zero(stream);
+  counter.zero(stream);
+  // element forces of a domain's scaled field
+  auto forces = [&](int di, int32_t dep_forces) {
+    DeviceDomainData& d = domains[di];
+    Work& w = work[di];
+    bool first = true;
+    for (const DeviceBlock& b : d.blocks) {
+      ElementLaunch a;
+      a.basis = basis.view();
+      a.blk = b.view();
+      a.u_in = w.x.get();
+      a.l2g = d.dofs.l2g.get();
+      a.rows = d.dofs.rows();
+      a.n_global = d.ng;
+      a.f_local = w.f_local.get();
+      a.gather = true;
+      a.scale = pw.get() + kPwScale;
+      a.elastic = d.medium == INSEM_ELASTIC;
+      a.dep = first ? dep_forces : kDepLate;
+      a.overlap = true;
+      a.stream = stream;
+      launch_element_forces(ngll, a);
+      first = false;
+    }
+  };
+  auto point = [&](int di, int mode, bool late) {
+    DeviceDomainData& d = domains[di];
+    Work& w = work[di];
+    PowerLaunch a;
+    a.mode = mode;
+    a.ncomp = d.ncomp;
+    a.stream = stream;
+    a.d.ng = d.ng;
+    a.d.t_offsets = d.dofs.t_offsets.get();
+    a.d.t_slots = d.dofs.t_slots.get();
+    a.d.t_weights = d.dofs.weighted ? d.dofs.t_weights.get() : nullptr;
+    a.d.f_local = w.f_local.get();
+    a.d.x = w.x.get();
+    a.d.mass = d.mass.get();
+    a.d.inv_mass = d.inv_mass.get();
+    a.d.zero = w.zero.get();
+    a.d.cpl_off = w.cpl_off.get();
+    a.d.cpl = w.cpl.get();
+    a.d.partial = w.partial.get();
+    a.d.counter = counter.get();
+    a.d.pw = pw.get();
+    a.d.late = late;
+    if (mode != kPowerAlone) {
+      const int oi = di == solid ? fluid : solid;
+      a.d.other = work[oi].x.get();
+      a.d.other_ng = domains[oi].ng;
+      a.d.pm = domains[solid].m == 1;
+      a.d.partial_s = work[solid].partial.get();
+      a.d.blocks_s = power_blocks(domains[solid].ng);
+    }
+    launch_power(ngll, a);
+  };
+  auto begin = [&](int di, const std::vector<float>& x) {
+    CUDA_CHECK(cudaMemcpyAsync(work[di].x.get(), x.data(), x.size() * sizeof(float), cudaMemcpyHostToDevice, stream));
+    zero_constrained(domains[di], work[di].x.get());
+  };
+  auto reset = [&] {
     CUDA_CHECK(cudaMemsetAsync(pw.get() + kPwDone, 0, sizeof(double), stream));
-    replay(100, [&] {
-      zero_constrained(d, dx.get());
-      internal_forces(d, dx.get(), d.f.get());
-      dot_partial_kernel<<<kReduceBlocks, kReduceThreads, 0, stream>>>(dx.get(), d.f.get(), n, st, 0, 1,
-                                                                       partial.get());
-      CUDA_LAUNCH_CHECK();
-      reduce_into(kPwA, -1.0);  // x.Kx = -(x . f_int)
-      mass_norm_partial_kernel<<<kReduceBlocks, kReduceThreads, 0, stream>>>(dx.get(), d.mass.get(), d.ng,
-                                                                             d.ncomp, partial.get());
-      CUDA_LAUNCH_CHECK();
-      reduce_into(kPwB, 1.0);
-      power_update_kernel<<<kReduceBlocks, kReduceThreads, 0, stream>>>(d.f.get(), d.inv_mass.get(), dx.get(),
-                                                                        d.ng, d.ncomp, partial.get());
-      CUDA_LAUNCH_CHECK();
-      reduce_into(kPwNorm, 1.0);
-      power_step_kernel<<<1, 1, 0, stream>>>(pw.get());
-      CUDA_LAUNCH_CHECK();
-      scale_dev_kernel<<<grid_for(n), 256, 0, stream>>>(dx.get(), dx.get(), n, pw.get());
-      CUDA_LAUNCH_CHECK();
-    });
-    d.f.zero(stream);
-    // dx is released below: its last kernels must have run
-    CUDA_CHECK(cudaStreamSynchronize(stream));
+    CUDA_CHECK(cudaMemcpyAsync(pw.get() + kPwScale, &one, sizeof(double), cudaMemcpyHostToDevice, stream));
+  };
+  constexpr int kPerGraph = 10;
+  for (std::size_t di = 0; di < domains.size(); ++di) {
+    DeviceDomainData& d = domains[di];
+    Work& w = work[di];
+    const std::size_t n = static_cast<std::size_t>(d.ncomp) * d.ng;
+    w.x.resize(n);
+    w.f_local.resize(static_cast<std::size_t>(d.ncomp) * d.n_elements * d.npe);
+    w.f_local.zero(stream);  // elements of no block contribute nothing
+    w.partial.resize(3 * static_cast<std::size_t>(power_blocks(d.ng)));
+    std::vector<uint8_t> zero(std::max(d.ng, 1), 0);
+    for (int64_t z : d.host_zero) zero[z % d.ng] |= static_cast<uint8_t>(1u << (z / d.ng));
+    w.zero.upload(zero);
+    w.start.resize(n);
+    rng.fill(w.start.data(), n);
+    begin(static_cast<int>(di), w.start);
+    reset();
+    replay(100 / kPerGraph, [&] {
+      for (int k = 0; k < kPerGraph; ++k) {
+        forces(static_cast<int>(di), kDepFirst);
+        point(static_cast<int>(di), kPowerAlone, false);
+      }
+    }, graphs);
   }
-  if (n_cpl > 0) coupled_lambda_max(rng, pw.get());
+  if (n_cpl > 0) {
+    int q = 0;
+    for (int di : {solid, fluid}) {
+      DeviceDomainData& d = domains[di];
+      Work& w = work[di];
+      // interface entries by point, in the interface's order
+      const auto own = (di == solid ? cpl_solid : cpl_fluid).download(), other = (di == solid ? cpl_fluid : cpl_solid).download();
+      const auto cx = cpl_cx.download(), cz = cpl_cz.download();
+      std::vector<int32_t> off(static_cast<std::size_t>(d.ng) + 1, 0);
+      for (int32_t g : own) ++off[g + 1];
+      for (int g = 0; g < d.ng; ++g) off[g + 1] += off[g];
+      std::vector<PowerEntry> e(n_cpl);
+      std::vector<int32_t> fill(off.begin(), off.end() - 1);
+      for (int i = 0; i < n_cpl; ++i) e[fill[own[i]]++] = PowerEntry{other[i], cx[i], cz[i]};
+      w.cpl_off.upload(off);
+      w.cpl.upload(e);
+      auto& x = start2[q++];
+      x.resize(static_cast<std::size_t>(d.ncomp) * d.ng);
+      rng.fill(x.data(), x.size());
+      begin(di, x);
+    }
+    reset();
+    for (bool late : {false, true})
+      replay(60 / kPerGraph, [&] {
+        for (int k = 0; k < kPerGraph; ++k) {
+          forces(solid, kDepFirst);
+          forces(fluid, kDepLate);
+          point(solid, kPowerSolid, late);
+          point(fluid, kPowerFluid, late);
+        }
+      }, graphs);
+  }
   double h[kPwCount];
   CUDA_CHECK(cudaMemcpyAsync(h, pw.get(), sizeof(h), cudaMemcpyDeviceToHost, stream));
   CUDA_CHECK(cudaStreamSynchronize(stream));
@@ -510,69 +639,6 @@ double Solver::stable_dt() {
   if (n_cpl > 0) lambda = std::max(lambda, h[kPwCoupled]);
   INSEM_REQUIRE(lambda > 0.0, INSEM_CUDA_ERR_INVALID, "could not estimate the stable time step (empty or rigid model?)");
   return 2.0 / std::sqrt(lambda);
-}
-
-// coupled_lambda_max (solver.cpp:621-667): growth of the mass norm under the
-// coupled operator, 120 iterations, sqrt(ny / nx) from iteration 60 on; the
-// result lands in pw[kPwCoupled].
-void Solver::coupled_lambda_max(std::mt19937& rng, double* pw) {
-  DeviceDomainData& sd = domains[solid];
-  DeviceDomainData& fd = domains[fluid];
-  std::uniform_real_distribution<double> dist(-1.0, 1.0);
-  std::vector<std::vector<float>> x0(2);
-  int q = 0;
-  for (DeviceDomainData* d : {&sd, &fd}) {
-    auto& x = x0[q++];
-    x.resize(static_cast<std::size_t>(d->ncomp) * d->ng);
-    for (auto& v : x) v = static_cast<float>(dist(rng));
-    CUDA_CHECK(cudaMemcpyAsync(d->u.get(), x.data(), x.size() * sizeof(float), cudaMemcpyHostToDevice, stream));
-  }
-  CUDA_CHECK(cudaMemsetAsync(pw + kPwDone, 0, sizeof(double), stream));
-  CUDA_CHECK(cudaMemsetAsync(pw + kPwCoupled, 0, sizeof(double), stream));
-  auto mass_norm = [&](DeviceDomainData& d, const float* x, int slot) {
-    mass_norm_partial_kernel<<<kReduceBlocks, kReduceThreads, 0, stream>>>(x, d.mass.get(), d.ng, d.ncomp,
-                                                                           partial.get());
-    CUDA_LAUNCH_CHECK();
-    sum_partials_kernel<<<1, kReduceBlocks, 0, stream>>>(partial.get(), kReduceBlocks, 1.0, pw, slot);
-    CUDA_LAUNCH_CHECK();
-  };
-  // iterations 0..59 and 60..119 differ only in coupled_step_kernel's test it >= 60
-  auto iteration = [&](int it) {
-    zero_constrained(sd, sd.u.get());
-    zero_constrained(fd, fd.u.get());
-    mass_norm(sd, sd.u.get(), kPwA);
-    mass_norm(fd, fd.u.get(), kPwB);
-    sum_ab_kernel<<<1, 1, 0, stream>>>(pw, kPwNx);
-    CUDA_LAUNCH_CHECK();
-    for (int di : {solid, fluid}) {
-      DeviceDomainData& d = domains[di];
-      internal_forces(d, d.u.get(), d.f.get());
-      coupling_forces(di);
-      inv_mass_kernel<<<grid_for(static_cast<int64_t>(d.ng) * d.ncomp), 256, 0, stream>>>(
-          d.f.get(), d.inv_mass.get(), d.a.get(), d.ng, d.ncomp);
-      CUDA_LAUNCH_CHECK();
-      zero_constrained(d, d.a.get());
-    }
-    mass_norm(sd, sd.a.get(), kPwA);
-    mass_norm(fd, fd.a.get(), kPwB);
-    sum_ab_kernel<<<1, 1, 0, stream>>>(pw, kPwNy);
-    CUDA_LAUNCH_CHECK();
-    coupled_step_kernel<<<1, 1, 0, stream>>>(pw, it);
-    CUDA_LAUNCH_CHECK();
-    for (DeviceDomainData* d : {&sd, &fd}) {
-      const int64_t n = static_cast<int64_t>(d->ncomp) * d->ng;
-      scale_dev_kernel<<<grid_for(n), 256, 0, stream>>>(d->a.get(), d->u.get(), n, pw);
-      CUDA_LAUNCH_CHECK();
-    }
-  };
-  replay(60, [&] { iteration(0); });
-  replay(60, [&] { iteration(60); });
-  for (DeviceDomainData* d : {&sd, &fd}) {
-    d->u.zero(stream);
-    d->a.zero(stream);
-    d->f.zero(stream);
-  }
-  CUDA_CHECK(cudaStreamSynchronize(stream));  // the host start vectors are read until here
 }
 
 // Kernels of the whole acceleration solve, elastic first (solver.cpp:674).

@@ -5,7 +5,6 @@
 #include <map>
 
 #include <memory>
-#include <random>
 #include <vector>
 
 #include "device_data.cuh"
@@ -30,7 +29,6 @@ struct DeviceDomainData {
   DeviceBuffer<float> u, v, a, f, f_local;  // two-pass path only (alloc_fields)
   bool fields_ready = false;
   void alloc_fields(cudaStream_t s = nullptr);
-  void free_fields();
 
   void upload(const insem_cuda_domain& d, const insem_cuda_basis& basis);
 };
@@ -121,13 +119,9 @@ class Solver {
   void observers(int force_energy, int init);
   void enqueue_step();
   void initialize();
-  double reduce_partials();
   void zero_constrained(DeviceDomainData& d, float* x);
   void coupling_forces(int di);
-  void coupled_lambda_max(std::mt19937& rng, double* pw);
-  // Runs `body` (launches on `stream` only) n times: captured once as a CUDA
-  // graph and replayed; returns after the stream has drained.
-  void replay(int n, const std::function<void()>& body);
+  void replay(int n, const std::function<void()>& body, std::vector<cudaGraphExec_t>& graphs);
 
   DeviceBasis basis;
   int solid = -1, fluid = -1;

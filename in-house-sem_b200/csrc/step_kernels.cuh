@@ -28,40 +28,6 @@ struct StepState {
   double kin_c;           // dt^2 / 8 of the kinetic energy (solver.cpp:903)
 };
 
-// ------------------------------------------- overlap of successive kernels
-// The kernels of the tiled step form one chain of programmatic dependent
-// launches: a kernel may start once every CTA of the one before it has
-// started and triggered (pdl_trigger), and pdl_wait holds a thread until the
-// kernel before it has completed and its writes are visible.  Both do nothing
-// in an ordinary launch.  Every kernel of the chain waits at some point, so a
-// kernel's completion implies that of all kernels before it.
-//   kDepFirst  waits before it touches what the step before wrote, then
-//              triggers: the next kernels start after that point, so they may
-//              read all that came before this kernel without a wait of their own
-//   kDepAll    triggers at once, waits before it touches what the kernel
-//              before it wrote (constant data is read ahead of the wait)
-//   kDepLate   needs nothing of the kernel before it: triggers at once and
-//              waits only at its end
-// A small solve is bound by this chain, not by its bytes: with a full boundary
-// between kernels, the constrained gather and the receivers on the critical
-// path and a graph per step, a step of the cased borehole (3,600 order-4
-// elements, 5.6 MB) took 29.7 us and one of 32 x 32 acoustic elements 15.8;
-// chained, 20.0 and 8.5.
-enum DepMode : int32_t { kDepFirst = 0, kDepAll = 1, kDepLate = 2 };
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// At the start of a kernel, where it first needs earlier results, and at its end.
-__device__ __forceinline__ void dep_begin(int32_t dep) {
-  if (dep != kDepFirst) pdl_trigger();
-}
-__device__ __forceinline__ void dep_wait(int32_t dep) {
-  if (dep != kDepLate) pdl_wait();
-  if (dep == kDepFirst) pdl_trigger();
-}
-__device__ __forceinline__ void dep_end(int32_t dep) {
-  if (dep == kDepLate) pdl_wait();
-}
-
 // kModeIdle: a batched solve past its last step (the batch's kernels skip it).
 enum StepMode : int32_t { kModeNormal = 0, kModeFinal = 1, kModeInit = 2, kModeIdle = 3 };
 
@@ -448,124 +414,6 @@ static __global__ void energy_finalize_kernel(const double* partial, int n_kin, 
     energy[sample * 3 + 1] = kin;
     energy[sample * 3 + 2] = pot;
   }
-}
-
-// ------------------------------------------------------- power iteration
-// partial[blockIdx] = sum mass[g] x x over [ncomp][ng]   (solver.cpp:597-601, 631-638)
-static __global__ void mass_norm_partial_kernel(const float* __restrict__ x, const float* __restrict__ mass, int32_t ng,
-                                         int32_t ncomp, double* partial) {
-  __shared__ double sh[kReduceThreads];
-  const int64_t n = static_cast<int64_t>(ng) * ncomp;
-  double s = 0.0;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const double xi = x[i];
-    s = dadd(s, dmul(dmul(static_cast<double>(mass[i % ng]), xi), xi));
-  }
-  const double b = block_reduce(s, sh);
-  if (threadIdx.x == 0) partial[blockIdx.x] = b;
-}
-
-// x = (float)(-f * inv_mass); partial = sum y^2   (solver.cpp:603-609)
-static __global__ void power_update_kernel(const float* __restrict__ f, const float* __restrict__ inv_mass,
-                                    float* __restrict__ x, int32_t ng, int32_t ncomp, double* partial) {
-  __shared__ double sh[kReduceThreads];
-  const int64_t n = static_cast<int64_t>(ng) * ncomp;
-  double s = 0.0;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const double y = dmul(-static_cast<double>(f[i]), static_cast<double>(inv_mass[i % ng]));
-    x[i] = static_cast<float>(y);
-    s = dadd(s, dmul(y, y));
-  }
-  const double b = block_reduce(s, sh);
-  if (threadIdx.x == 0) partial[blockIdx.x] = b;
-}
-
-// x = (float)(src * scale)
-static __global__ void scale_kernel(const float* __restrict__ src, float* __restrict__ x, int64_t n, double scale) {
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    x[i] = static_cast<float>(dmul(static_cast<double>(src[i]), scale));
-}
-
-// Power-iteration scalars kept on the device, so an iteration needs no host
-// round trip: the partial sums, their reductions and the scalar logic of
-// estimate_stable_dt / coupled_lambda_max (solver.cpp:583-667) all run in
-// stream order; the host reads the result once.
-enum PowerSlot : int {
-  kPwLambda = 0,   // running max of the Rayleigh quotients (uncoupled domains)
-  kPwA = 1,        // reduction results
-  kPwB = 2,
-  kPwNorm = 3,
-  kPwDone = 4,     // the loop has stopped (the reference's break)
-  kPwScale = 5,    // factor of the next scaling
-  kPwNx = 6,
-  kPwNy = 7,
-  kPwCoupled = 8,  // running max of sqrt(ny / nx) (coupled operator)
-  kPwCount = 9
-};
-
-// pw[slot] = sign x (sum of partial[0..n) in index order, as the host loop
-// adds them).  One CTA of kReduceBlocks threads stages the partials in shared
-// memory with parallel loads; thread 0 then adds them in order.
-static __global__ void __launch_bounds__(kReduceBlocks) sum_partials_kernel(const double* __restrict__ partial, int n,
-                                                                          double sign, double* pw, int slot) {
-  __shared__ double sh[kReduceBlocks];
-  for (int i = threadIdx.x; i < n && i < kReduceBlocks; i += blockDim.x) sh[i] = partial[i];
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  double s = 0.0;
-  for (int i = 0; i < n && i < kReduceBlocks; ++i) s = dadd(s, sh[i]);
-  pw[slot] = sign < 0.0 ? -s : s;
-}
-
-// pw[dst] = pw[kPwA] + pw[kPwB]
-static __global__ void sum_ab_kernel(double* pw, int dst) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) pw[dst] = dadd(pw[kPwA], pw[kPwB]);
-}
-
-// One uncoupled power iteration's scalars (solver.cpp:597-612): lambda from
-// x.Kx / x.Mx, then stop on a zero norm or set the scale 1 / sqrt(norm).
-static __global__ void power_step_kernel(double* pw) {
-  if (blockIdx.x != 0 || threadIdx.x != 0 || pw[kPwDone] != 0.0) return;
-  const double xmx = pw[kPwB];
-  if (xmx > 0.0) {
-    const double q = pw[kPwA] / xmx;
-    if (pw[kPwLambda] < q) pw[kPwLambda] = q;
-  }
-  const double norm = pw[kPwNorm];
-  if (norm == 0.0) {
-    pw[kPwDone] = 1.0;
-    return;
-  }
-  pw[kPwScale] = 1.0 / sqrt(norm);
-}
-
-// One coupled iteration's scalars (solver.cpp:641-662): stop on a zero norm,
-// sqrt(ny / nx) from iteration 60 on, scale -1 / sqrt(ny).
-static __global__ void coupled_step_kernel(double* pw, int it) {
-  if (blockIdx.x != 0 || threadIdx.x != 0 || pw[kPwDone] != 0.0) return;
-  const double nx = pw[kPwNx], ny = pw[kPwNy];
-  if (nx <= 0.0 || ny <= 0.0) {
-    pw[kPwDone] = 1.0;
-    return;
-  }
-  if (it >= 60) {
-    const double q = sqrt(ny / nx);
-    if (pw[kPwCoupled] < q) pw[kPwCoupled] = q;
-  }
-  pw[kPwScale] = -1.0 / sqrt(ny);
-}
-
-// x = (float)(src * pw[kPwScale]) unless the loop has stopped.
-static __global__ void scale_dev_kernel(const float* __restrict__ src, float* __restrict__ x, int64_t n,
-                                        const double* __restrict__ pw) {
-  if (pw[kPwDone] != 0.0) return;
-  const double scale = pw[kPwScale];
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    x[i] = static_cast<float>(dmul(static_cast<double>(src[i]), scale));
 }
 
 // Sets st->nonfinite if any entry of x (n0 of them) or y (n1) is NaN or Inf.

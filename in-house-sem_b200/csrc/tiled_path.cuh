@@ -65,24 +65,6 @@ class TiledDomain {
   float* u_cur(int parity) { return parity ? u1.get() : u0.get(); }
 };
 
-// Launch of a kernel of the step chain; `overlap`: with programmatic stream
-// serialization, so it may start before the kernel ahead of it has ended.
-template <class... P, class... A>
-cudaError_t launch_chained(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t stream, bool overlap,
-                           A&&... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = overlap ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
-}
-
 // Opts a kernel in to all the shared memory a CTA may have beside its static
 // part: the same value for every solve, so that none lowers another's.
 template <class Kernel>
