@@ -74,11 +74,12 @@ void Solver::batch_collect(BatchTables& T) {
       sg.sc = sc;
       sg.st = st;
       sg.epartial = epart.get() + 2 * static_cast<std::size_t>(ep_tile[di]);
-      const int m = bt.kind == INSEM_AXISYM ? bt.m : 0;
-      const int key = ((ngll * 4 + bt.kind) * 2 + (el ? 1 : 0)) * 2 + m;
+      const int m = is_axisym(bt.kind) ? bt.m : 0;
+      const int key = ((ngll * 8 + bt.kind) * 2 + (el ? 1 : 0)) * 2 + m;
       TileClass& c = T.tiles[key];
       c.ngll = ngll;
       c.kind = bt.kind;
+      c.any_axial |= bt.any_axial;
       c.m = m;
       c.ncomp = t.ncomp;
       c.elastic = el;
@@ -286,7 +287,8 @@ void Batch::rebuild() {
     a.m = c.m;
     a.elastic = c.elastic;
     a.L = d.L;
-    a.smem = d.L.total;
+    d.smem = c.any_axial || !is_axisym(c.kind) ? d.L.total : d.L.ax;
+    a.smem = d.smem;
     tile_batch(c.ngll, a, false);
     d.grid = d.n_items;  // CTA b reads item b: no launch without items
     for (const TileItem& it : c.items) d.work += static_cast<double>(it.th.ne) * c.ngll * c.ngll * c.ncomp;
@@ -396,7 +398,7 @@ void Batch::enqueue_step(int32_t k, cudaEvent_t tiles_begin, cudaEvent_t tiles_e
     a.segs = d.segs.get();
     a.items = d.items.get();
     a.L = d.L;
-    a.smem = d.L.total;
+    a.smem = d.smem;
     a.grid = d.grid;
     a.ix = StepIdx{k, 0, first ? kDepFirst : kDepLate};
     a.overlap = !first || k > 0;

@@ -39,7 +39,7 @@ struct StreamSeg {
 
 struct TileClass {
   int ngll = 0, kind = 0, m = 0, ncomp = 0;
-  bool elastic = false;
+  bool elastic = false, any_axial = false;
   int tp_cap = 0, nc_cap = 0, rank_cap = 1;  // largest tile of the class
   std::vector<TileSeg> segs;
   std::vector<TileItem> items;
@@ -49,7 +49,7 @@ constexpr int kHaloClasses = 5;
 
 // Host-side segment tables of one batch composition.
 struct BatchTables {
-  std::map<int, TileClass> tiles;  // key: ((ngll * 4 + kind) * 2 + elastic) * 2 + m
+  std::map<int, TileClass> tiles;  // key: ((ngll * 8 + kind) * 2 + elastic) * 2 + m
   // solves without a solid, with a solid of 2 and of 3 components; the fluids
   // of solves whose halo points take two launches
   std::vector<HaloArgs> halo_segs[kHaloClasses];
@@ -122,6 +122,7 @@ class Batch {
     int32_t n_items = 0;
     double work = 0.0;  // elements x points per element x components
     TileLayout L{};
+    uint32_t smem = 0;
     int grid = 0;
   };
 

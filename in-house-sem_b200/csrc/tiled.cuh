@@ -150,17 +150,38 @@ struct TileCfg {
   static constexpr int THREADS = kTileLanes * NG;  // threads per CTA
 };
 
-// Element data of a tile.  Kinds whose metric varies in an element: pairs
-// [point][32][2] of (xi_x, xi_z), (eta_x, eta_z) and, axisymmetric, (wr, hoop),
-// then one plane [point][32] of the Jacobian (Curved) or r (axisymmetric: the
-// fluxes use the Jacobian only through wr).  Rect and Affine: [array][32] of
-// xi_x, eta_z, jac or xi_x, xi_z, eta_x, eta_z, jac.
+// Kinds of the tile kernels: insem_cuda_kind, and axisymmetric blocks whose
+// elements are rectangles as far as their data tell (every borehole's): xi_r,
+// eta_r and eta_z carry one value per element and r one per column, bit for
+// bit (xi_z does not: it holds rounding noise).  These are kept once, which
+// leaves three values per point of seven: less to fetch, and room for one or
+// two more CTAs per SM.  A step of the 30k-element dipole borehole went from
+// 45.6 to 39.5 us, of 12 boreholes from 316 to 284, of 10 mixed requests from
+// 110.5 to 103.3 (with 7, 9 and 8 warps per scheduler: one more or less of the
+// NG 6 and 7 classes 282 - 297 and 104 - 109).
+constexpr int kAxisymSeparable = 4;
+__host__ __device__ constexpr bool is_axisym(int kind) { return kind == INSEM_AXISYM || kind == kAxisymSeparable; }
+__host__ __device__ constexpr int element_kind(int kind) { return kind == kAxisymSeparable ? INSEM_AXISYM : kind; }
+
+// Element data of a tile.  Kinds whose metric varies in an element (staged in
+// shared memory): pairs [point][32][2] of (xi_x, xi_z), (eta_x, eta_z) and,
+// axisymmetric, (wr, hoop), then one plane [point][32] of the Jacobian (Curved)
+// or r (axisymmetric: the fluxes use the Jacobian only through wr); separable:
+// the pairs (wr, hoop) and the plane xi_z.  Read by the lanes themselves: Rect
+// and Affine [array][32] of xi_x, eta_z, jac or xi_x, xi_z, eta_x, eta_z, jac;
+// separable, behind the staged part, xi_r, eta_r, eta_z and r of the ng columns.
 __host__ __device__ constexpr int tile_arrays(int kind) {
-  return kind == INSEM_RECT ? 3 : kind == INSEM_AXISYM ? 7 : 5;
+  return kind == INSEM_RECT || kind == kAxisymSeparable ? 3 : kind == INSEM_AXISYM ? 7 : 5;
 }
-__host__ __device__ constexpr bool tile_data_staged(int kind) { return kind == INSEM_CURVED || kind == INSEM_AXISYM; }
-__host__ __device__ constexpr int tile_data_floats(int kind, int npe) {
-  return tile_arrays(kind) * (tile_data_staged(kind) ? npe : 1) * kTileLanes;
+__host__ __device__ constexpr bool tile_data_staged(int kind) { return kind == INSEM_CURVED || is_axisym(kind); }
+__host__ __device__ constexpr int tile_staged_floats(int kind, int ng) {
+  return tile_data_staged(kind) ? tile_arrays(kind) * ng * ng * kTileLanes : 0;
+}
+__host__ __device__ constexpr int tile_lane_floats(int kind, int ng) {
+  return kTileLanes * (kind == kAxisymSeparable ? 3 + ng : tile_data_staged(kind) ? 0 : tile_arrays(kind));
+}
+__host__ __device__ constexpr int tile_data_floats(int kind, int ng) {
+  return tile_staged_floats(kind, ng) + tile_lane_floats(kind, ng);
 }
 // Offset (floats) of array a at point place p = point * 32 + lane (staged kinds).
 __host__ __device__ constexpr int tile_data_at(int kind, int npe, int a, int p) {
@@ -241,17 +262,17 @@ struct TileLayout {
     const uint32_t npe = static_cast<uint32_t>(ng * ng), plane = npe * kTileLanes * 4u;
     L.tp_cap = tp_cap;
     L.nc_cap = nc_cap;
-    const bool axi = kind == INSEM_AXISYM, staged = tile_data_staged(kind);
+    const bool axi = is_axisym(kind), staged = tile_data_staged(kind);
     uint32_t o = 0;
     L.bar = o;  // two mbarriers: the first copies, the late ones
     o = up16(o + 16);
     L.metric = o;
     L.wr = L.hoop = L.r = o;
-    if (axi) {
+    if (kind == INSEM_AXISYM) {
       L.wr = L.hoop = o + 4 * plane;
       L.r = o + 6 * plane;
     }
-    if (staged) o += 4u * tile_data_floats(kind, static_cast<int>(npe));
+    o += 4u * tile_staged_floats(kind, ng);
     const uint32_t elem = o - L.metric;
     L.u = o;
     o = up16(o + 4u * nc * tp_cap);
@@ -266,7 +287,8 @@ struct TileLayout {
     L.im = L.v + v_b;
     L.pl = L.im + im_b;
     if (!L.late) o += v_b + im_b + pl_b;
-    // axis terms (gx, gy of up to two components) [4][ng][32], ng rounded up to 4
+    // axis terms (gx, gy of up to two components) [4][ng][32], ng rounded up to
+    // 4; last, for launches without axial elements leave them out
     L.ax = o;
       if (axi) o += 4u * 4u * ((ng + 3) & ~3) * kTileLanes;
     L.total = o;
@@ -373,11 +395,13 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
                                                double* __restrict__ epartial, int32_t tile, const TileHdr* thp,
                                                const TileLayout& L, unsigned char* smem_raw, uint64_t* bar,
                                                uint32_t phase, int32_t g_first = -1) {
-  using CE = ElemCfg<NG, KIND, EL, M>;
+  constexpr int EK = element_kind(KIND);
+  constexpr bool SEP = KIND == kAxisymSeparable;
+  using CE = ElemCfg<NG, EK, EL, M>;
   constexpr int NC = CE::NC;
   constexpr int NPE = NG * NG;
   constexpr int NI = NG - 2;  // inner points per direction
-  constexpr bool AXI = KIND == INSEM_AXISYM, STAGED = tile_data_staged(KIND);
+  constexpr bool AXI = is_axisym(KIND), STAGED = tile_data_staged(KIND);
   constexpr int W = kTileLanes, NT = W * NG;
   using R = Rows<NC, NPE>;
   using F = Rows<NC, NPE, STAGED ? (tile_arrays(KIND) - 1) * NPE * W : -1>;  // the f_xi rows
@@ -405,10 +429,11 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
   // 1. bulk copies of the element data, and of the edge complete points' u (v,
   //    1/M and place lists too unless they come late)
   if (tid == 0) {
-    constexpr uint32_t eb = STAGED ? 4u * tile_data_floats(KIND, NPE) : 0u;
+    constexpr uint32_t eb = 4u * tile_staged_floats(KIND, NG);
     fence_proxy_async_smem();
     mbar_expect_tx(bar, eb + edge_b * NC + (L.late ? 0u : edge_b * (NC + 1) + list_b));
-    if constexpr (STAGED) bulk_load(smem_raw + L.metric, blk.metric + static_cast<size_t>(th.tb) * (eb / 4u), eb, bar);
+    if constexpr (STAGED)
+      bulk_load(smem_raw + L.metric, blk.metric + static_cast<size_t>(th.tb) * tile_data_floats(KIND, NG), eb, bar);
     if (!L.late && nc4 > 0) {
       bulk_load(s_im, td.inv_mass + th.ebeg, edge_b, bar);
       bulk_load(pl, td.plist + static_cast<size_t>(th.pl_off) * td.rs, list_b, bar);
@@ -426,8 +451,15 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
     pd.c0 = blk.coef0[e];
     if constexpr (EL) pd.c1 = blk.coef1[e];
     if constexpr (AXI) axial = blk.axial[e] != 0;
-    if constexpr (!STAGED) {
-      const float* m = blk.metric + static_cast<size_t>(th.tb) * tile_data_floats(KIND, NPE) + lane;
+    if constexpr (SEP) {
+      const float* m = blk.metric + static_cast<size_t>(th.tb) * tile_data_floats(KIND, NG) +
+                       tile_staged_floats(KIND, NG) + lane;
+      pd.xi_x = m[0];
+      pd.eta_x = m[W];
+      pd.eta_z = m[2 * W];
+      pd.r = m[(3 + i) * W];
+    } else if constexpr (!STAGED) {
+      const float* m = blk.metric + static_cast<size_t>(th.tb) * tile_data_floats(KIND, NG) + lane;
       if constexpr (KIND == INSEM_RECT) {
         pd.xi_x = m[0];
         pd.eta_z = m[W];
@@ -571,7 +603,13 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
         ueta[R::ONE_C] = b;
         upt[R::ONE_C] = uc1[j];
       }
-      if constexpr (STAGED) {
+      if constexpr (SEP) {
+        const int p = (j * NG + i) * W + lane;
+        const float2 w = *reinterpret_cast<const float2*>(elem + tile_data_at(KIND, NPE, 0, p));
+        pd.wr = w.x;
+        pd.hoop = w.y;
+        pd.xi_z = elem[tile_data_at(KIND, NPE, 2, p)];
+      } else if constexpr (STAGED) {
         const int p = (j * NG + i) * W + lane;
         const float2 xi = *reinterpret_cast<const float2*>(elem + tile_data_at(KIND, NPE, 0, p));
         const float2 eta = *reinterpret_cast<const float2*>(elem + tile_data_at(KIND, NPE, 2, p));
@@ -590,7 +628,7 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
       }
       dir[j][0] = dir[j][1] = 0.0f;
       float fx[NC];
-      point_flux<NG, KIND, EL, M, W>(pd, i, j, axial, uxi, ueta, upt, fx, fe[j], dir[j], ax, ax + NG * W,
+      point_flux<NG, EK, EL, M, W>(pd, i, j, axial, uxi, ueta, upt, fx, fe[j], dir[j], ax, ax + NG * W,
                                      ax + 2 * NG * W, ax + 3 * NG * W, w2c[j]);
       F::store(sfx, (j * NG + i) * W + lane, fx);
     }
@@ -649,7 +687,7 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
       s[R::ONE_C] = acc;
     }
     float out[NC];
-    point_divergence<NG, KIND, EL, M, W>(i, j, axial, s, dir[j], dxc[0], [](int q) { return cbasis(NG, 0, q); }, ax,
+    point_divergence<NG, EK, EL, M, W>(i, j, axial, s, dir[j], dxc[0], [](int q) { return cbasis(NG, 0, q); }, ax,
                                          ax + NG * W, ax + 2 * NG * W, ax + 3 * NG * W, out);
     const int place = (j * NG + i) * W + lane;
     if (j > 0 && j < NG - 1 && mine) {
@@ -798,13 +836,15 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
 // Resident CTAs per SM the compiler makes room for in the register file, from
 // the warps each of an SM's four schedulers (16,384 registers) is to hold: 10
 // (48 registers) for one component, 8 (64) for the Cartesian elastic classes,
-// 8 to 6 (64 to 80) for the axisymmetric ones, where shared memory holds
+// 9 to 6 (56 to 80) for the axisymmetric ones, where shared memory holds
 // about as many CTAs, and 4 or 5 (128 or 96) at NG 8 and 9.  A step of 12
 // boreholes of NG 6 and 7 took 444 us with the compiler's own choice (up to 164
 // registers, 1 - 2 CTAs of the three-component classes) and 336 with this.
 template <int NG, int KIND, bool EL, int M>
 constexpr int tile_min_ctas() {
-  const int warps = !EL ? (NG >= 8 || (KIND == INSEM_AXISYM && M == 1) ? 8 : 10)
+  const int sep = NG >= 8 ? 5 : M == 1 ? 7 : NG == 7 ? 9 : 8;
+  const int warps = !EL ? (NG >= 8 || (is_axisym(KIND) && M == 1) ? 8 : 10)
+                    : KIND == kAxisymSeparable ? sep
                     : KIND != INSEM_AXISYM ? (NG >= 8 ? 5 : 8)
                     : NG >= 8 ? 4
                     : NG >= 6 ? 6

@@ -571,25 +571,49 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
   }
   // element data of every block, element-minor by tile; one material per
   // element: the tile kernels read one coefficient pair per element
+  auto separable = [&](const insem_cuda_block& in) {
+    if (in.kind != INSEM_AXISYM) return false;
+    for (std::size_t e = 0; e < static_cast<std::size_t>(in.n_elements); ++e) {
+      const float *m = in.metric + e * npe * 5, *r = in.r + e * npe;
+      for (int k = 1; k < npe; ++k) {
+        for (int c : {0, 2, 3})
+          if (bits_of(m[k * 5 + c]) != bits_of(m[c])) return false;
+        if (bits_of(r[k]) != bits_of(r[k % ngll])) return false;
+      }
+    }
+    return true;
+  };
   for (int b = 0; b < d.n_blocks; ++b) {
     BlockTiles& bt = blocks[b];
     const insem_cuda_block& in = d.blocks[b];
-    const int kind = in.kind, na = tile_arrays(kind), nm = kind == INSEM_AXISYM ? 4 : na;
+    const bool sep = separable(in), axi = in.kind == INSEM_AXISYM;
+    const int kind = sep ? kAxisymSeparable : in.kind, na = tile_arrays(kind);
+    bt.kind = kind;
     const bool el = medium == INSEM_ELASTIC, staged = tile_data_staged(kind);
-    const std::size_t per_tile = static_cast<std::size_t>(tile_data_floats(kind, npe));
+    const std::size_t per_tile = static_cast<std::size_t>(tile_data_floats(kind, ngll));
     std::vector<float> data(per_tile * bt.ntiles, 0.0f), c0(static_cast<std::size_t>(W) * bt.ntiles, 0.0f);
     std::vector<float> c1(el ? c0.size() : 0, 0.0f);
-    std::vector<uint8_t> axial(kind == INSEM_AXISYM ? c0.size() : 0, 0);
+    std::vector<uint8_t> axial(axi ? c0.size() : 0, 0);
     for (int tb = 0; tb < bt.ntiles; ++tb) {
       const auto& list = tile_elems[bt.tile0 + tb];
       for (std::size_t l = 0; l < list.size(); ++l) {
         const std::size_t o = static_cast<std::size_t>(epos[list[l]]), p0 = o * npe, at = static_cast<std::size_t>(tb) * W + l;
         float* out = data.data() + per_tile * tb;
-        if (staged) {
+        if (sep) {
+          for (int k = 0; k < npe; ++k) {
+            const int p = k * W + static_cast<int>(l);
+            out[tile_data_at(kind, npe, 0, p)] = in.wr[p0 + k];
+            out[tile_data_at(kind, npe, 1, p)] = in.hoop[p0 + k];
+            out[tile_data_at(kind, npe, 2, p)] = in.metric[(p0 + k) * 5 + 1];
+          }
+          float* lane = out + tile_staged_floats(kind, ngll) + l;
+          for (int c = 0; c < 3; ++c) lane[static_cast<std::size_t>(c) * W] = in.metric[p0 * 5 + (c == 0 ? 0 : c + 1)];
+          for (int i = 0; i < ngll; ++i) lane[static_cast<std::size_t>(3 + i) * W] = in.r[p0 + i];
+        } else if (staged) {
           for (int k = 0; k < npe; ++k) {
             auto put = [&](int c, float v) { out[tile_data_at(kind, npe, c, k * W + static_cast<int>(l))] = v; };
-            for (int c = 0; c < nm; ++c) put(c, in.metric[(p0 + k) * 5 + c]);
-            if (kind == INSEM_AXISYM) {
+            for (int c = 0; c < (axi ? 4 : 5); ++c) put(c, in.metric[(p0 + k) * 5 + c]);
+            if (axi) {
               put(4, in.wr[p0 + k]);
               put(5, in.hoop[p0 + k]);
               put(6, in.r[p0 + k]);
@@ -600,7 +624,10 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
         }
         c0[at] = in.coef0[p0];
         if (el) c1[at] = in.coef1[p0];
-        if (kind == INSEM_AXISYM) axial[at] = in.axial[o];
+        if (axi) {
+          axial[at] = in.axial[o];
+          bt.any_axial |= in.axial[o] != 0;
+        }
         for (int k = 1; k < npe; ++k) {
           const bool same = bits_of(in.coef0[p0 + k]) == bits_of(c0[at]) && (!el || bits_of(in.coef1[p0 + k]) == bits_of(c1[at]));
           INSEM_REQUIRE(same, INSEM_CUDA_ERR_UNSUPPORTED,

@@ -35,7 +35,8 @@ class TiledDomain {
   bool weighted = false;
   std::vector<int32_t> perm;  // reference point -> device point
   struct BlockTiles {
-    int kind = 0, m = 0, tile0 = 0, ntiles = 0, n = 0;
+    int kind = 0, m = 0, tile0 = 0, ntiles = 0, n = 0;  // kind of the tile kernels
+    bool any_axial = false;
     DeviceBuffer<float> data, coef0, coef1;  // [tile][tile_data_floats], [tile][32]
     DeviceBuffer<uint8_t> axial;
     BlockDev view() const;
@@ -115,7 +116,7 @@ struct TileBatchLaunch {
   bool elastic = false;
   const TileSeg* segs = nullptr;
   const TileItem* items = nullptr;
-  TileLayout L{};  // the class layout; its total is the dynamic shared memory
+  TileLayout L{};  // the class layout
   uint32_t smem = 0;
   int grid = 0;
   StepIdx ix{};
@@ -151,6 +152,11 @@ int tile_batch_cfg(const TileBatchLaunch& a, bool launch) {
                                            std::to_string(a.smem) + "): " + cudaGetErrorString(err));
     return 0;
   };
+  if (a.kind == kAxisymSeparable) {
+    if (a.m == 1)
+      return a.elastic ? go(tile_batch_kernel<NG, kAxisymSeparable, true, 1>) : go(tile_batch_kernel<NG, kAxisymSeparable, false, 1>);
+    return a.elastic ? go(tile_batch_kernel<NG, kAxisymSeparable, true, 0>) : go(tile_batch_kernel<NG, kAxisymSeparable, false, 0>);
+  }
   if (a.kind == INSEM_AXISYM) {
     if (a.m == 1) return a.elastic ? go(tile_batch_kernel<NG, INSEM_AXISYM, true, 1>)
                                    : go(tile_batch_kernel<NG, INSEM_AXISYM, false, 1>);
@@ -175,7 +181,7 @@ void launch_tiles_cfg(const TileLaunch& a) {
   if (b.ntiles == 0) return;
   auto go = [&](auto one_wave, auto many_waves, int nc) {
     const TileLayout L = TileLayout::make(NG, nc, b.kind, a.elastic, d.te, d.tp_cap, d.nc_cap, d.rank_cap);
-    const size_t smem = L.total;
+    const size_t smem = b.any_axial || !is_axisym(b.kind) ? L.total : L.ax;
     INSEM_REQUIRE(smem <= 226 * 1024, INSEM_CUDA_ERR_UNSUPPORTED, "tile needs too much shared memory");
     // The kernel with the compiler's own registers where it holds all tiles at
     // once; and the opt-in to this launch's dynamic shared memory (outside
@@ -202,6 +208,17 @@ void launch_tiles_cfg(const TileLaunch& a) {
                                            ", threads " + std::to_string(TileCfg<NG>::THREADS) + ", smem " +
                                            std::to_string(smem) + "): " + cudaGetErrorString(err));
   };
+  if (b.kind == kAxisymSeparable) {
+    constexpr int K = kAxisymSeparable;
+    if (b.m == 1) {
+      if (a.elastic) go(tile_step_kernel<NG, K, true, 1, true>, tile_step_kernel<NG, K, true, 1, false>, 3);
+      else go(tile_step_kernel<NG, K, false, 1, true>, tile_step_kernel<NG, K, false, 1, false>, 1);
+    } else {
+      if (a.elastic) go(tile_step_kernel<NG, K, true, 0, true>, tile_step_kernel<NG, K, true, 0, false>, 2);
+      else go(tile_step_kernel<NG, K, false, 0, true>, tile_step_kernel<NG, K, false, 0, false>, 1);
+    }
+    return;
+  }
   if (b.kind == INSEM_AXISYM) {
     if (b.m == 1) {
       if (a.elastic) go(tile_step_kernel<NG, INSEM_AXISYM, true, 1, true>, tile_step_kernel<NG, INSEM_AXISYM, true, 1, false>, 3);

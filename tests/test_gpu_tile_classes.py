@@ -10,7 +10,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-KINDS = ["rect", "affine", "curved", "monopole", "dipole"]
+KINDS = ["rect", "affine", "curved", "monopole", "dipole", "bent monopole", "bent dipole"]
 
 
 def _model(order, kind, nx, nz):
@@ -23,6 +23,15 @@ def _model(order, kind, nx, nz):
                     boundaries={b.boundaries["outer"]: "absorbing", b.boundaries["top"]: "rigid"},
                     sources=[K.Source(kind, 0.0, 0.05 * nz, (1.0, 0.0, 0.0), K.ricker(8000.0))], dt=1e-7)
         where = [("acoustic", 0.04, 0.043 * nz), ("elastic", 0.06 * nx + 0.05, 0.07 * nz)]
+    elif kind.startswith("bent"):  # axisymmetric, with a metric that varies inside the elements
+        h = nz // 2
+        top = lambda x: 0.1 * (h + 0.5 * np.sin(20.0 * x))  # noqa: E731
+        mesh = K.layered((0.0, 0.1 * nx), [0.0, top, 0.1 * nz], [h, nz - h], [1, 0], nx=nx, quadratic=True,
+                         coords="axisymmetric")
+        m = K.Model(mesh, order=order, azimuthal_order=int(kind.endswith("dipole")),
+                    materials={0: K.MUD, 1: K.FAST}, boundaries={K.RIGHT: "absorbing", K.TOP: "rigid"},
+                    sources=[K.Source(kind.split()[1], 0.0, 0.083 * nz, (1.0, 0.0, 0.0), K.ricker(8000.0))], dt=1e-7)
+        where = [("acoustic", 0.04 * nx, 0.08 * nz), ("elastic", 0.06 * nx, 0.02 * nz)]
     else:
         slope = {"rect": lambda x: 0.0 * x, "affine": lambda x: 0.2 * x, "curved": lambda x: 0.3 * np.sin(x)}[kind]
         h = nz // 2
@@ -68,6 +77,6 @@ def test_small_domains(pkg, oracle, order, kind):
 
 
 @pytest.mark.parametrize("order,kind,nx,nz", [(3, "rect", 300, 320), (5, "curved", 210, 220), (4, "monopole", 220, 230),
-                                              (6, "dipole", 130, 140), (8, "affine", 120, 130)])
+                                              (6, "dipole", 130, 140), (8, "affine", 120, 130), (5, "bent monopole", 200, 210)])
 def test_domains_of_many_tiles(pkg, oracle, order, kind, nx, nz):
     _check(pkg, oracle, _model(order, kind, nx, nz))
