@@ -34,6 +34,7 @@ class TiledDomain {
   int te = 0;  // elements per tile
   bool weighted = false;
   std::vector<int32_t> perm;  // reference point -> device point
+  DeviceBuffer<int32_t> device_perm;  // the same on the device, from the first state() on
   struct BlockTiles {
     int kind = 0, m = 0, tile0 = 0, ntiles = 0, n = 0;  // kind of the tile kernels
     bool any_axial = false;
