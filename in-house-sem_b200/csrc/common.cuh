@@ -213,12 +213,16 @@ class DeviceGuard {
  public:
   explicit DeviceGuard(int device) {
     CUDA_CHECK(cudaGetDevice(&old_));
-    if (device != old_) CUDA_CHECK(cudaSetDevice(device));
+    changed_ = device != old_;
+    if (changed_) CUDA_CHECK(cudaSetDevice(device));
   }
-  ~DeviceGuard() { cudaSetDevice(old_); }
+  ~DeviceGuard() {
+    if (changed_) cudaSetDevice(old_);
+  }
 
  private:
   int old_ = 0;
+  bool changed_ = false;
 };
 
 // ------------------------------------------------- IEEE-ordered arithmetic

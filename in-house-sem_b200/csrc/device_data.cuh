@@ -2,6 +2,7 @@
 // element blocks, DofMap), converted to the device layouts the kernels read.
 #pragma once
 
+#include <algorithm>
 #include <memory>
 
 #include "element_kernels.cuh"
@@ -93,6 +94,7 @@ struct DeviceBlock {
   DeviceBuffer<float> metric, coef0, coef1, wr, hoop, r;
   DeviceBuffer<uint8_t> axial;
   std::vector<int32_t> host_elements;
+  int32_t min_element = 0, max_element = -1;
   bool any_axial = false;
 
   void upload(const insem_cuda_block& b, int ngll, int medium) {
@@ -106,6 +108,11 @@ struct DeviceBlock {
     INSEM_REQUIRE(n >= 0, INSEM_CUDA_ERR_INVALID, "negative block size");
     const int npe = ngll * ngll;
     host_elements = host_vec(b.elements, n);
+    if (n > 0) {
+      const auto mm = std::minmax_element(host_elements.begin(), host_elements.end());
+      min_element = *mm.first;
+      max_element = *mm.second;
+    }
     elements.upload(host_elements);
     std::vector<int32_t> order(n);
     for (int q = 0; q < n; ++q) order[q] = q;
@@ -180,10 +187,10 @@ struct DeviceDofMap {
   RowsDev rows() const { return {row_offsets.get(), row_dofs.get(), row_weights.get()}; }
 };
 
-// Element-local gather and CSR assemble (DofMap seam), in dofmap_kernels.cu.
+// Element-local gather and CSR assemble (DofMap seam).  `preload` loads the
+// kernel (its module, under lazy loading) without launching it.
 void launch_gather(const DeviceDofMap& d, int ncomp, const float* global, float* local, cudaStream_t s);
-void launch_assemble(const DeviceDofMap& d, int ncomp, const float* local, float* global, cudaStream_t s);
-// Loads assemble_kernel<weighted> (its module, under lazy loading) without launching it.
-void preload_assemble(bool weighted);
+void launch_assemble(const DeviceDofMap& d, int ncomp, const float* local, float* global, cudaStream_t s,
+                     bool preload = false);
 
 }  // namespace insem_b200

@@ -35,6 +35,114 @@ __device__ __forceinline__ float scaled(float x, double scale) {
   return static_cast<float>(dmul(static_cast<double>(x), scale));
 }
 
+// DofMap::assemble of one global point (dof_map.hpp:123-141): its contributions
+// in ascending slot order from zero, every component at once.  The slots of
+// four contributions load together, then their values: two dependent loads
+// for most points, where a loop over components and contributions took two
+// per contribution (and divided by a run-time ngll^2).  Gather, element forces
+// and assembly of 16,384 coupled order-5 elements take 27 us with their
+// launches chained, 45-52 before; internal forces of the cased borehole's two
+// domains 18, 31 before.
+template <int NG, int NC, bool WEIGHTED>
+__device__ __forceinline__ void assemble_point(const int32_t* __restrict__ t_slots, const float* __restrict__ t_weights,
+                                               const float* local, int32_t b, int32_t e, float (&f)[NC]) {
+  constexpr int NPE = NG * NG;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) f[c] = 0.0f;
+  for (int32_t q0 = b; q0 < e; q0 += 4) {
+    int32_t slot[4];
+    float w[4], v[4][NC];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      slot[k] = q0 + k < e ? t_slots[q0 + k] : -1;
+      if constexpr (WEIGHTED) w[k] = q0 + k < e ? t_weights[q0 + k] : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int32_t el = slot[k] / NPE;
+      const float* p = local + static_cast<size_t>(el) * NC * NPE + (slot[k] - el * NPE);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) v[k][c] = slot[k] >= 0 ? p[c * NPE] : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+        if (slot[k] >= 0) f[c] = fadd(f[c], WEIGHTED ? fmul(w[k], v[k][c]) : v[k][c]);
+  }
+}
+
+template <int NG, int NC, bool WEIGHTED>
+static __global__ void __launch_bounds__(256) assemble_kernel(const int32_t* __restrict__ t_offsets,
+                                                              const int32_t* __restrict__ t_slots,
+                                                              const float* __restrict__ t_weights, int32_t n_global,
+                                                              const float* local, float* __restrict__ global) {
+  dep_begin(kDepAll);
+  const int32_t g = blockIdx.x * 256 + threadIdx.x;
+  const bool in = g < n_global;
+  const int32_t b = in ? t_offsets[g] : 0, e = in ? t_offsets[g + 1] : 0;
+  dep_wait(kDepAll);
+  if (!in) return;
+  float f[NC];
+  assemble_point<NG, NC, WEIGHTED>(t_slots, t_weights, local, b, e, f);
+#pragma unroll
+  for (int c = 0; c < NC; ++c) global[static_cast<size_t>(c) * n_global + g] = f[c];
+}
+
+// DofMap::gather (dof_map.hpp:95-120): one thread per element slot.
+template <int NG, int NC>
+static __global__ void __launch_bounds__(256) gather_kernel(const int32_t* __restrict__ l2g, RowsDev rows, int32_t n_slots,
+                                                            int32_t n_global, const float* global,
+                                                            float* __restrict__ local) {
+  constexpr int NPE = NG * NG;
+  dep_begin(kDepAll);
+  const int32_t s = blockIdx.x * 256 + threadIdx.x;
+  const bool in = s < n_slots;
+  const int32_t m = in ? l2g[s] : 0;
+  dep_wait(kDepAll);
+  if (!in) return;
+  const int32_t e = s / NPE;
+  float* out = local + static_cast<size_t>(e) * NC * NPE + (s - e * NPE);
+  float v[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) v[c] = gather_slot(global + static_cast<size_t>(c) * n_global, m, rows);
+#pragma unroll
+  for (int c = 0; c < NC; ++c) out[c * NPE] = v[c];
+}
+
+// Arguments of a gather or assembly launch.
+struct DofMapLaunch {
+  int32_t n = 0;  // slots (gather) or global points (assembly)
+  int32_t n_global = 0;
+  int ncomp = 1;
+  const int32_t* l2g = nullptr;
+  RowsDev rows;
+  const int32_t* t_offsets = nullptr;
+  const int32_t* t_slots = nullptr;
+  const float* t_weights = nullptr;  // null: all weights 1
+  const float* in = nullptr;
+  float* out = nullptr;
+  bool gather = false;
+  bool preload = false;  // load the kernel without launching it
+  cudaStream_t stream = nullptr;
+};
+
+template <int NG, int NC>
+void launch_dofmap_cfg(const DofMapLaunch& a) {
+  auto go = [&](auto kernel, auto... args) {
+    if (a.preload) {
+      cudaFuncAttributes fa;
+      CUDA_CHECK(cudaFuncGetAttributes(&fa, kernel));
+      return;
+    }
+    CUDA_CHECK(launch_chained(kernel, ceil_div(a.n, 256), 256, 0, a.stream, true, args...));
+    CUDA_LAUNCH_CHECK();
+  };
+  if (a.gather) go(gather_kernel<NG, NC>, a.l2g, a.rows, a.n, a.n_global, a.in, a.out);
+  else if (a.t_weights) go(assemble_kernel<NG, NC, true>, a.t_offsets, a.t_slots, a.t_weights, a.n, a.in, a.out);
+  else go(assemble_kernel<NG, NC, false>, a.t_offsets, a.t_slots, a.t_weights, a.n, a.in, a.out);
+}
+
 // Where an element kernel takes its field from.
 enum FieldSource : int { kFieldLocal = 0, kFieldGlobal = 1, kFieldScaled = 2 };
 
@@ -177,7 +285,9 @@ void launch_element_ng8(const ElementLaunch&);
 void launch_element_ng9(const ElementLaunch&);
 
 struct PowerLaunch;
-#define INSEM_POWER(N) void launch_power_ng##N(const PowerLaunch&);
+#define INSEM_POWER(N)                         \
+  void launch_power_ng##N(const PowerLaunch&); \
+  void launch_dofmap_ng##N(const DofMapLaunch&);
 INSEM_POWER(2)
 INSEM_POWER(3)
 INSEM_POWER(4)
@@ -188,6 +298,7 @@ INSEM_POWER(8)
 INSEM_POWER(9)
 #undef INSEM_POWER
 void launch_power(int ngll, const PowerLaunch& a);
+void launch_dofmap(int ngll, const DofMapLaunch& a);
 
 // Dispatch on the number of GLL points; unsupported values fail like
 // physics::select (kernels.cpp:451-468).

@@ -56,7 +56,7 @@ void Solver::prepare_noalloc() {
       a.preload = true;
       launch_element_forces(ngll, a);
     }
-    preload_assemble(d.dofs.weighted);
+    launch_assemble(d.dofs, d.ncomp, nullptr, nullptr, nullptr, true);
   }
 }
 
@@ -69,8 +69,10 @@ void Solver::internal_forces_noalloc(int32_t di, const float* u_global, float* f
                     " floats; the allocation-free entry point holds at most " +
                     std::to_string(kNoAllocScratchFloats) + " (use insem_cuda_solver_internal_forces)");
   float* scratch = scratch_on_current_device();
-  // the array keeps the previous call's values: start from zeros
-  CUDA_CHECK(cudaMemsetAsync(scratch, 0, need * sizeof(float), s));
+  // The array keeps the previous call's values; the blocks' kernels write every
+  // element they hold, so only elements of no block need zeros.
+  if (!d.blocks_cover) CUDA_CHECK(cudaMemsetAsync(scratch, 0, need * sizeof(float), s));
+  bool first = true;
   for (const DeviceBlock& b : d.blocks) {
     ElementLaunch a;
     a.basis = basis.view();
@@ -82,8 +84,11 @@ void Solver::internal_forces_noalloc(int32_t di, const float* u_global, float* f
     a.f_local = scratch;
     a.gather = true;
     a.elastic = d.medium == INSEM_ELASTIC;
+    a.dep = first ? kDepFirst : kDepLate;
+    a.overlap = true;
     a.stream = s;
     launch_element_forces(ngll, a);
+    first = false;
   }
   launch_assemble(d.dofs, d.ncomp, scratch, f_global, s);
 }

@@ -93,15 +93,8 @@ static __global__ void __launch_bounds__(kPowerThreads) power_kernel(PowerDev d)
   const double scale = d.pw[kPwScale];
   double acc[3] = {0.0, 0.0, 0.0};
   for (int32_t g = blockIdx.x * kPowerThreads + threadIdx.x; g < d.ng; g += gridDim.x * kPowerThreads) {
-    // DofMap::assemble (dof_map.hpp:123-141), every component of the point
-    float f[NC] = {};
-    const int32_t b = d.t_offsets[g], e = d.t_offsets[g + 1];
-    for (int32_t q = b; q < e; ++q) {
-      const int32_t slot = d.t_slots[q], el = slot / (NG * NG), k = slot - el * (NG * NG);
-      const float* v = d.f_local + static_cast<size_t>(el) * NC * (NG * NG) + k;
-#pragma unroll
-      for (int c = 0; c < NC; ++c) f[c] = fadd(f[c], WEIGHTED ? fmul(d.t_weights[q], v[c * NG * NG]) : v[c * NG * NG]);
-    }
+    float f[NC];
+    assemble_point<NG, NC, WEIGHTED>(d.t_slots, d.t_weights, d.f_local, d.t_offsets[g], d.t_offsets[g + 1], f);
     const double m = d.mass[g];
     const float im = d.inv_mass[g];
     const uint32_t zero = d.zero[g];

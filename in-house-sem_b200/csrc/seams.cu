@@ -43,64 +43,48 @@ void launch_power(int ngll, const PowerLaunch& a) {
 }
 
 // ------------------------------------------------------- gather / assemble
-// DofMap::gather (dof_map.hpp:95-120): one thread per element slot.
-__global__ void gather_kernel(const int32_t* __restrict__ l2g, RowsDev rows, int32_t n_slots, int32_t npe,
-                              int32_t ncomp, int32_t n_global, const float* __restrict__ global,
-                              float* __restrict__ local) {
-  const int32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n_slots) return;
-  const int32_t e = s / npe, k = s - e * npe;
-  const int32_t m = l2g[s];
-  for (int c = 0; c < ncomp; ++c)
-    local[(static_cast<size_t>(e) * ncomp + c) * npe + k] =
-        gather_slot(global + static_cast<size_t>(c) * n_global, m, rows);
-}
-
-// DofMap::assemble (dof_map.hpp:123-141): one thread per global point, its
-// contributions summed in ascending slot order from zero.
-template <bool WEIGHTED>
-__global__ void assemble_kernel(const int32_t* __restrict__ t_offsets, const int32_t* __restrict__ t_slots,
-                                const float* __restrict__ t_weights, int32_t n_global, int32_t npe,
-                                int32_t ncomp, const float* __restrict__ local, float* __restrict__ global) {
-  const int32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= n_global) return;
-  const int32_t b = t_offsets[g], en = t_offsets[g + 1];
-  for (int c = 0; c < ncomp; ++c) {
-    float sum = 0.0f;
-    for (int32_t q = b; q < en; ++q) {
-      const int32_t slot = t_slots[q];
-      const int32_t e = slot / npe, k = slot - e * npe;
-      const float v = local[(static_cast<size_t>(e) * ncomp + c) * npe + k];
-      sum = fadd(sum, WEIGHTED ? fmul(t_weights[q], v) : v);
-    }
-    global[static_cast<size_t>(c) * n_global + g] = sum;
+void launch_dofmap(int ngll, const DofMapLaunch& a) {
+  switch (ngll) {
+    case 2: launch_dofmap_ng2(a); break;
+    case 3: launch_dofmap_ng3(a); break;
+    case 4: launch_dofmap_ng4(a); break;
+    case 5: launch_dofmap_ng5(a); break;
+    case 6: launch_dofmap_ng6(a); break;
+    case 7: launch_dofmap_ng7(a); break;
+    case 8: launch_dofmap_ng8(a); break;
+    case 9: launch_dofmap_ng9(a); break;
+    default: check_ngll(ngll);
   }
 }
 
 void launch_gather(const DeviceDofMap& d, int ncomp, const float* global, float* local, cudaStream_t s) {
-  const int32_t n_slots = d.n_elements * d.npe;
-  if (n_slots == 0) return;
-  gather_kernel<<<ceil_div(n_slots, 256), 256, 0, s>>>(d.l2g.get(), d.rows(), n_slots, d.npe, ncomp, d.n_global,
-                                                         global, local);
-  CUDA_LAUNCH_CHECK();
+  DofMapLaunch a;
+  a.gather = true;
+  a.n = d.n_elements * d.npe;
+  if (a.n == 0) return;
+  a.n_global = d.n_global;
+  a.ncomp = ncomp;
+  a.l2g = d.l2g.get();
+  a.rows = d.rows();
+  a.in = global;
+  a.out = local;
+  a.stream = s;
+  launch_dofmap(d.ngll, a);
 }
 
-void preload_assemble(bool weighted) {
-  cudaFuncAttributes fa;
-  if (weighted) CUDA_CHECK(cudaFuncGetAttributes(&fa, assemble_kernel<true>));
-  else CUDA_CHECK(cudaFuncGetAttributes(&fa, assemble_kernel<false>));
-}
-
-void launch_assemble(const DeviceDofMap& d, int ncomp, const float* local, float* global, cudaStream_t s) {
-  if (d.n_global == 0) return;
-  if (d.weighted) {
-    assemble_kernel<true><<<ceil_div(d.n_global, 256), 256, 0, s>>>(
-        d.t_offsets.get(), d.t_slots.get(), d.t_weights.get(), d.n_global, d.npe, ncomp, local, global);
-  } else {
-    assemble_kernel<false><<<ceil_div(d.n_global, 256), 256, 0, s>>>(
-        d.t_offsets.get(), d.t_slots.get(), nullptr, d.n_global, d.npe, ncomp, local, global);
-  }
-  CUDA_LAUNCH_CHECK();
+void launch_assemble(const DeviceDofMap& d, int ncomp, const float* local, float* global, cudaStream_t s, bool preload) {
+  DofMapLaunch a;
+  a.n = a.n_global = d.n_global;
+  if (a.n == 0) return;
+  a.ncomp = ncomp;
+  a.t_offsets = d.t_offsets.get();
+  a.t_slots = d.t_slots.get();
+  a.t_weights = d.weighted ? d.t_weights.get() : nullptr;
+  a.in = local;
+  a.out = global;
+  a.preload = preload;
+  a.stream = s;
+  launch_dofmap(d.ngll, a);
 }
 
 }  // namespace insem_b200
@@ -162,8 +146,8 @@ int insem_cuda_block_forces(insem_cuda_block_h* h, int32_t n_local_elements, con
                             float* f_local, void* stream) {
   return guarded([&] {
     INSEM_REQUIRE(h && u_local && f_local, INSEM_CUDA_ERR_INVALID, "null argument");
-    for (int32_t e : h->block.host_elements)
-      INSEM_REQUIRE(e >= 0 && e < n_local_elements, INSEM_CUDA_ERR_INVALID, "block element outside the local array");
+    INSEM_REQUIRE(h->block.n == 0 || (h->block.min_element >= 0 && h->block.max_element < n_local_elements),
+                  INSEM_CUDA_ERR_INVALID, "block element outside the local array");
     DeviceGuard dg(h->device);
     ElementLaunch a;
     a.basis = h->basis.view();
@@ -171,6 +155,7 @@ int insem_cuda_block_forces(insem_cuda_block_h* h, int32_t n_local_elements, con
     a.u_in = u_local;
     a.f_local = f_local;
     a.elastic = h->medium == INSEM_ELASTIC;
+    a.overlap = true;
     a.stream = static_cast<cudaStream_t>(stream);
     launch_element_forces(h->basis.ngll, a);
   });

@@ -41,6 +41,10 @@ void DeviceDomainData::upload(const insem_cuda_domain& d, const insem_cuda_basis
       INSEM_REQUIRE(e >= 0 && e < n_elements, INSEM_CUDA_ERR_INVALID, "block element out of range");
     any_axial |= blocks[b].any_axial;
   }
+  std::vector<char> covered(n_elements, 0);
+  for (const DeviceBlock& b : blocks)
+    for (int32_t e : b.host_elements) covered[e] = 1;
+  blocks_cover = std::count(covered.begin(), covered.end(), 1) == n_elements;
   host_mass = host_vec(d.mass, ng);
   mass.upload(host_mass);
   inv_mass.upload(host_vec(d.inv_mass, ng));

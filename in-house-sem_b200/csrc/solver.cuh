@@ -19,6 +19,7 @@ struct DeviceDomainData {
   DeviceDofMap dofs;
   std::vector<DeviceBlock> blocks;
   bool any_axial = false;
+  bool blocks_cover = false;  // every element is in a block
   std::vector<float> host_mass;
   DeviceBuffer<float> mass, inv_mass;
   int32_t n_abs = 0;
