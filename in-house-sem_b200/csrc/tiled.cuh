@@ -297,6 +297,16 @@ struct TileLayout {
   }
 };
 
+// A pointer into global memory, which the compiler cannot see where it was
+// read from a structure in shared memory: without this the batched kernels
+// access everything by generic loads and stores, which also stay in order with
+// those to shared memory.
+template <class T>
+__device__ __forceinline__ T* glob(T* p) {
+  __builtin_assume(__isGlobal(p));
+  return p;
+}
+
 // Mode-dependent completion of a point (solver.cpp:924-944 fused):
 //   normal: v = v_half + dt/2 a; u' = u + dt v + dt^2/2 a; v' = v + dt/2 a
 //   final:  v = v_half + dt/2 a; u' = u                      (state complete)
@@ -433,10 +443,10 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
     fence_proxy_async_smem();
     mbar_expect_tx(bar, eb + edge_b * NC + (L.late ? 0u : edge_b * (NC + 1) + list_b));
     if constexpr (STAGED)
-      bulk_load(smem_raw + L.metric, blk.metric + static_cast<size_t>(th.tb) * tile_data_floats(KIND, NG), eb, bar);
+      bulk_load(smem_raw + L.metric, glob(blk.metric) + static_cast<size_t>(th.tb) * tile_data_floats(KIND, NG), eb, bar);
     if (!L.late && nc4 > 0) {
-      bulk_load(s_im, td.inv_mass + th.ebeg, edge_b, bar);
-      bulk_load(pl, td.plist + static_cast<size_t>(th.pl_off) * td.rs, list_b, bar);
+      bulk_load(s_im, glob(td.inv_mass) + th.ebeg, edge_b, bar);
+      bulk_load(pl, glob(td.plist) + static_cast<size_t>(th.pl_off) * td.rs, list_b, bar);
     }
   }
   // this lane's element and this column's descriptors, while the copies are in flight
@@ -448,18 +458,18 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
   uint32_t dsc[NG];
   {
     const size_t e = static_cast<size_t>(th.tb) * W + lane;
-    pd.c0 = blk.coef0[e];
-    if constexpr (EL) pd.c1 = blk.coef1[e];
-    if constexpr (AXI) axial = blk.axial[e] != 0;
+    pd.c0 = glob(blk.coef0)[e];
+    if constexpr (EL) pd.c1 = glob(blk.coef1)[e];
+    if constexpr (AXI) axial = glob(blk.axial)[e] != 0;
     if constexpr (SEP) {
-      const float* m = blk.metric + static_cast<size_t>(th.tb) * tile_data_floats(KIND, NG) +
+      const float* m = glob(blk.metric) + static_cast<size_t>(th.tb) * tile_data_floats(KIND, NG) +
                        tile_staged_floats(KIND, NG) + lane;
       pd.xi_x = m[0];
       pd.eta_x = m[W];
       pd.eta_z = m[2 * W];
       pd.r = m[(3 + i) * W];
     } else if constexpr (!STAGED) {
-      const float* m = blk.metric + static_cast<size_t>(th.tb) * tile_data_floats(KIND, NG) + lane;
+      const float* m = glob(blk.metric) + static_cast<size_t>(th.tb) * tile_data_floats(KIND, NG) + lane;
       if constexpr (KIND == INSEM_RECT) {
         pd.xi_x = m[0];
         pd.eta_z = m[W];
@@ -472,20 +482,20 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
         pd.jac = m[4 * W];
       }
     }
-    const uint16_t* gd = td.sdesc + (static_cast<size_t>(tile) * NPE + i) * W + lane;
+    const uint16_t* gd = glob(td.sdesc) + (static_cast<size_t>(tile) * NPE + i) * W + lane;
 #pragma unroll
     for (int j = 0; j < NG; ++j) {
       dsc[j] = kSlotConstrained;
       if (j == 0 || j == NG - 1 || !inner_col || !all_direct) dsc[j] = gd[j * NG * W];
     }
   }
-  if (tg < th.ntp - th.nc && g_first < 0) g_first = td.halo_tp[th.hl_off + tg];
+  if (tg < th.ntp - th.nc && g_first < 0) g_first = glob(td.halo_tp)[th.hl_off + tg];
   dep_wait(dep);
   if (tid == 0 && nc4 > 0) {
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      bulk_load(tu + c * tp_cap, td.u_cur + static_cast<size_t>(c) * td.ng + th.ebeg, edge_b, bar);
-      if (!L.late) bulk_load(s_v + c * nc_cap, td.v + static_cast<size_t>(c) * td.ng + th.ebeg, edge_b, bar);
+      bulk_load(tu + c * tp_cap, glob(td.u_cur) + static_cast<size_t>(c) * td.ng + th.ebeg, edge_b, bar);
+      if (!L.late) bulk_load(s_v + c * nc_cap, glob(td.v) + static_cast<size_t>(c) * td.ng + th.ebeg, edge_b, bar);
     }
   }
   // inner points of direct elements straight into their field rows
@@ -495,32 +505,32 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
 #pragma unroll
     for (int j = 0; j < NI; ++j)
 #pragma unroll
-      for (int c = 0; c < NC; ++c) x[j][c] = __ldcg(td.u_cur + static_cast<size_t>(c) * td.ng + g0 + j * W);
+      for (int c = 0; c < NC; ++c) x[j][c] = __ldcg(glob(td.u_cur) + static_cast<size_t>(c) * td.ng + g0 + j * W);
 #pragma unroll
     for (int j = 0; j < NI; ++j)
       if (direct) R::store(su, ((j + 1) * NG + i) * W + lane, x[j]);
   }
   // halo tile points
   for (int t = tg; t < th.ntp - th.nc; t += NT) {
-    const int32_t g = t == tg ? g_first : td.halo_tp[th.hl_off + t];
+    const int32_t g = t == tg ? g_first : glob(td.halo_tp)[th.hl_off + t];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) tu[c * tp_cap + nc4 + t] = __ldcg(td.u_cur + static_cast<size_t>(c) * td.ng + g);
+    for (int c = 0; c < NC; ++c) tu[c * tp_cap + nc4 + t] = __ldcg(glob(td.u_cur) + static_cast<size_t>(c) * td.ng + g);
   }
   // constrained (hanging) slots straight into their field rows: the row's
   // weighted sum in row order (DofMap::gather, dof_map.hpp:110-115)
   for (int q = tg; q < th.ncs; q += NT) {
-    const int32_t place = td.cs_slot[th.cs_off + q];
-    const int2 row = td.cs_row[th.cs_off + q];
+    const int32_t place = glob(td.cs_slot)[th.cs_off + q];
+    const int2 row = glob(td.cs_row)[th.cs_off + q];
     float s[NC] = {};
     for (int32_t m0 = row.x; m0 < row.y; m0 += 4) {
       float w[4], x[4][NC];
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
         const bool in = m0 + m < row.y;
-        const int32_t g = in ? td.row_dofs[m0 + m] : 0;
-        w[m] = in ? td.row_w[m0 + m] : 0.0f;
+        const int32_t g = in ? glob(td.row_dofs)[m0 + m] : 0;
+        w[m] = in ? glob(td.row_w)[m0 + m] : 0.0f;
 #pragma unroll
-        for (int c = 0; c < NC; ++c) x[m][c] = in ? __ldcg(td.u_cur + static_cast<size_t>(c) * td.ng + g) : 0.0f;
+        for (int c = 0; c < NC; ++c) x[m][c] = in ? __ldcg(glob(td.u_cur) + static_cast<size_t>(c) * td.ng + g) : 0.0f;
       }
 #pragma unroll
       for (int m = 0; m < 4; ++m)
@@ -639,9 +649,9 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
   if (mine) {
 #pragma unroll
     for (int j = 0; j < NI; ++j) {
-      mi[j] = td.inv_mass[g0 + j * W];
+      mi[j] = glob(td.inv_mass)[g0 + j * W];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) vi[j][c] = __ldcg(td.v + static_cast<size_t>(c) * td.ng + g0 + j * W);
+      for (int c = 0; c < NC; ++c) vi[j][c] = __ldcg(glob(td.v) + static_cast<size_t>(c) * td.ng + g0 + j * W);
     }
   }
   __syncthreads();
@@ -653,9 +663,9 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
     if (nc4 > 0) {
 #pragma unroll
       for (int c = 0; c < NC; ++c)
-        bulk_load(s_v + c * nc_cap, td.v + static_cast<size_t>(c) * td.ng + th.ebeg, edge_b, bar + 1);
-      bulk_load(s_im, td.inv_mass + th.ebeg, edge_b, bar + 1);
-      bulk_load(pl, td.plist + static_cast<size_t>(th.pl_off) * td.rs, list_b, bar + 1);
+        bulk_load(s_v + c * nc_cap, glob(td.v) + static_cast<size_t>(c) * td.ng + th.ebeg, edge_b, bar + 1);
+      bulk_load(s_im, glob(td.inv_mass) + th.ebeg, edge_b, bar + 1);
+      bulk_load(pl, glob(td.plist) + static_cast<size_t>(th.pl_off) * td.rs, list_b, bar + 1);
     }
   }
 
@@ -699,8 +709,8 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
         const float a = fmul(fadd(0.0f, out[c]), mi[j - 1]);
         float u_out, v_state, v_n;
         complete_point(kModeNormal, sc, u[c], vi[j - 1][c], a, u_out, v_state, v_n);
-        td.u_nxt[gi] = u_out;
-        td.v[gi] = v_state;
+        glob(td.u_nxt)[gi] = u_out;
+        glob(td.v)[gi] = v_state;
       }
     } else {
       R::store(su, place, out);
@@ -711,8 +721,8 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
   //    first halo entry is fetched ahead of the barrier.
   int32_t hs_first = 0, hd_first = 0;
   if (tid < th.nhs) {
-    hs_first = td.hs_slot[th.hs_off + tid];
-    hd_first = td.hs_dst[th.hs_off + tid];
+    hs_first = glob(td.hs_slot)[th.hs_off + tid];
+    hd_first = glob(td.hs_dst)[th.hs_off + tid];
   }
   const bool late_arrived = !L.late || mbar_wait_bounded(bar + 1, phase, kBulkWaitLimit);
   if (__syncthreads_or(!late_arrived)) {
@@ -723,19 +733,19 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
 
   // 6. halo contributions out, each to its place in its halo point's list
   for (int q = tid; q < th.nhs; q += NT) {
-    const int32_t place = q == tid ? hs_first : td.hs_slot[th.hs_off + q];
-    const int32_t dst = q == tid ? hd_first : td.hs_dst[th.hs_off + q];
+    const int32_t place = q == tid ? hs_first : glob(td.hs_slot)[th.hs_off + q];
+    const int32_t dst = q == tid ? hd_first : glob(td.hs_dst)[th.hs_off + q];
     float val[NC];
     R::load(su, place, val);
     if (dst >= 0) {
 #pragma unroll
-      for (int c = 0; c < NC; ++c) td.hbuf[static_cast<size_t>(c) * td.n_hbuf + dst] = val[c];
+      for (int c = 0; c < NC; ++c) glob(td.hbuf)[static_cast<size_t>(c) * td.n_hbuf + dst] = val[c];
     } else {
       const int32_t mi2 = -1 - dst;
-      for (int32_t d = td.mdst_off[mi2]; d < td.mdst_off[mi2 + 1]; ++d) {
-        const int32_t p = td.mdst[d];
+      for (int32_t d = glob(td.mdst_off)[mi2]; d < glob(td.mdst_off)[mi2 + 1]; ++d) {
+        const int32_t p = glob(td.mdst)[d];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) td.hbuf[static_cast<size_t>(c) * td.n_hbuf + p] = val[c];
+        for (int c = 0; c < NC; ++c) glob(td.hbuf)[static_cast<size_t>(c) * td.n_hbuf + p] = val[c];
       }
     }
   }
@@ -776,10 +786,10 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
       const float u = tu[c * tp_cap + t];
       float u_out, v_state, v_n;
       complete_point(mode, sc, u, s_v[c * nc_cap + t], a, u_out, v_state, v_n);
-      td.u_nxt[gi] = u_out;
-      td.v[gi] = v_state;
-      if (mode != kModeNormal) td.a[gi] = a;
-      if (energy) add_energy(kin, pot, u, fsum[c], v_n, a, td.mass[g], st->kin_c);
+      glob(td.u_nxt)[gi] = u_out;
+      glob(td.v)[gi] = v_state;
+      if (mode != kModeNormal) glob(td.a)[gi] = a;
+      if (energy) add_energy(kin, pot, u, fsum[c], v_n, a, glob(td.mass)[g], st->kin_c);
     }
   }
   // the inner points of direct elements in the other modes and on energy steps
@@ -789,7 +799,7 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
       if (t - q * W >= th.nd) continue;
       const int ci = q / (NI > 0 ? NI : 1) + 1, cj = q - (ci - 1) * NI + 1;
       const size_t g = static_cast<size_t>(th.cbeg) + t;
-      const float im = td.inv_mass[g];
+      const float im = glob(td.inv_mass)[g];
       float f[NC];
       R::load(su, (cj * NG + ci) * W + lane, f);
 #pragma unroll
@@ -797,13 +807,13 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
         const size_t gi = static_cast<size_t>(c) * td.ng + g;
         const float fc = fadd(0.0f, f[c]);
         const float a = fmul(fc, im);
-        const float u = __ldcg(td.u_cur + gi);
+        const float u = __ldcg(glob(td.u_cur) + gi);
         float u_out, v_state, v_n;
-        complete_point(mode, sc, u, __ldcg(td.v + gi), a, u_out, v_state, v_n);
-        td.u_nxt[gi] = u_out;
-        td.v[gi] = v_state;
-        if (mode != kModeNormal) td.a[gi] = a;
-        if (energy) add_energy(kin, pot, u, fc, v_n, a, td.mass[g], st->kin_c);
+        complete_point(mode, sc, u, __ldcg(glob(td.v) + gi), a, u_out, v_state, v_n);
+        glob(td.u_nxt)[gi] = u_out;
+        glob(td.v)[gi] = v_state;
+        if (mode != kModeNormal) glob(td.a)[gi] = a;
+        if (energy) add_energy(kin, pot, u, fc, v_n, a, glob(td.mass)[g], st->kin_c);
       }
     }
   }
@@ -994,13 +1004,13 @@ struct HaloPoint {
 __device__ __forceinline__ HaloPoint halo_point(const TiledDev& td, const HaloDev& hd, int32_t h, bool in) {
   HaloPoint p;
   if (in) {
-    p.im = td.inv_mass[td.n_complete + h];
-    p.b = hd.off[h];
-    p.e = hd.off[h + 1];
-    const int32_t sp = hd.spec[h];
+    p.im = glob(td.inv_mass)[td.n_complete + h];
+    p.b = glob(hd.off)[h];
+    p.e = glob(hd.off)[h + 1];
+    const int32_t sp = glob(hd.spec)[h];
     if (sp >= 0) {
-      p.r = hd.rec[sp];
-      if (p.r.cpl0 < p.r.cpl1) p.c = hd.cpl[p.r.cpl0];
+      p.r = glob(hd.rec)[sp];
+      if (p.r.cpl0 < p.r.cpl1) p.c = glob(hd.cpl)[p.r.cpl0];
     }
   }
   return p;
@@ -1032,7 +1042,7 @@ __device__ __forceinline__ void halo_finish(const TiledDev& td, const float* u_c
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       uc[c] = u_cur[static_cast<size_t>(c) * td.ng + g];
-      vc[c] = td.v[static_cast<size_t>(c) * td.ng + g];
+      vc[c] = glob(td.v)[static_cast<size_t>(c) * td.ng + g];
     }
     const bool coupled = hp.r.cpl0 < hp.r.cpl1;
     float o[3] = {0.0f, 0.0f, 0.0f};
@@ -1051,13 +1061,13 @@ __device__ __forceinline__ void halo_finish(const TiledDev& td, const float* u_c
 #pragma unroll
       for (int q = 0; q < K; ++q)
 #pragma unroll
-        for (int c = 0; c < NC; ++c) vq[c][q] = b + q < e ? td.hbuf[static_cast<size_t>(c) * td.n_hbuf + b + q] : 0.0f;
+        for (int c = 0; c < NC; ++c) vq[c][q] = b + q < e ? glob(td.hbuf)[static_cast<size_t>(c) * td.n_hbuf + b + q] : 0.0f;
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         float s = 0.0f;
 #pragma unroll
         for (int q = 0; q < K; ++q)
-          if (b + q < e) s = fadd(s, hd.w ? fmul(hd.w[b + q], vq[c][q]) : vq[c][q]);
+          if (b + q < e) s = fadd(s, hd.w ? fmul(glob(hd.w)[b + q], vq[c][q]) : vq[c][q]);
         f[c] = s;
       }
     } else {
@@ -1065,8 +1075,8 @@ __device__ __forceinline__ void halo_finish(const TiledDev& td, const float* u_c
       for (int c = 0; c < NC; ++c) {
         float s = 0.0f;
         for (int32_t q = b; q < e; ++q) {
-          const float v = td.hbuf[static_cast<size_t>(c) * td.n_hbuf + q];
-          s = fadd(s, hd.w ? fmul(hd.w[q], v) : v);
+          const float v = glob(td.hbuf)[static_cast<size_t>(c) * td.n_hbuf + q];
+          s = fadd(s, hd.w ? fmul(glob(hd.w)[q], v) : v);
         }
         f[c] = s;
       }
@@ -1076,9 +1086,9 @@ __device__ __forceinline__ void halo_finish(const TiledDev& td, const float* u_c
       for (int c = 0; c < NC; ++c) pot = dadd(pot, dmul(static_cast<double>(uc[c]), static_cast<double>(f[c])));
     }
     for (int32_t q = hp.r.src0; q < hp.r.src1; ++q) {
-      const float am = amp[static_cast<size_t>(hd.src_which[q]) * n_amp + step];
+      const float am = amp[static_cast<size_t>(glob(hd.src_which)[q]) * n_amp + step];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) f[c] = fadd(f[c], fmul(hd.src_coef[static_cast<size_t>(q) * NC + c], am));
+      for (int c = 0; c < NC; ++c) f[c] = fadd(f[c], fmul(glob(hd.src_coef)[static_cast<size_t>(q) * NC + c], am));
     }
     if (coupled) {
       const float hs = static_cast<float>(kSqrtHalf);
@@ -1100,16 +1110,16 @@ __device__ __forceinline__ void halo_finish(const TiledDev& td, const float* u_c
           f[0] = fsub(f[0], fadd(fmul(ce.cx, ar), fmul(ce.cz, az)));
         }
         if (++q >= hp.r.cpl1) break;
-        ce = hd.cpl[q];
+        ce = glob(hd.cpl)[q];
         partner(ce.partner);
       }
     }
 #pragma unroll
     for (int c = 0; c < NC; ++c) a[c] = fmul(f[c], hp.im);
     if (hp.r.abs >= 0) {
-      const float* cc = hd.abs_coef + static_cast<size_t>(hp.r.abs) * NC * NC;
+      const float* cc = glob(hd.abs_coef) + static_cast<size_t>(hp.r.abs) * NC * NC;
       double A[NC * NC], rhs[NC];
-      const double mass = td.mass[g];
+      const double mass = glob(td.mass)[g];
 #pragma unroll
       for (int r = 0; r < NC; ++r) {
         rhs[r] = static_cast<double>(f[r]);
@@ -1130,12 +1140,12 @@ __device__ __forceinline__ void halo_finish(const TiledDev& td, const float* u_c
       float u_out, v_state, v_n;
       complete_point(mode, sc, uc[c], vc[c], a[c], u_out, v_state, v_n);
       u_nxt[gi] = u_out;
-      td.v[gi] = v_state;
-      td.a[gi] = a[c];
-      td.vn[gi] = v_n;
+      glob(td.v)[gi] = v_state;
+      glob(td.a)[gi] = a[c];
+      glob(td.vn)[gi] = v_n;
       if (energy) {
         const double vv = v_n, aa = a[c];
-        kin = dadd(kin, dmul(static_cast<double>(td.mass[g]), dsub(dmul(dmul(0.5, vv), vv), dmul(dmul(st->kin_c, aa), aa))));
+        kin = dadd(kin, dmul(static_cast<double>(glob(td.mass)[g]), dsub(dmul(dmul(0.5, vv), vv), dmul(dmul(st->kin_c, aa), aa))));
       }
     }
   }
@@ -1193,21 +1203,21 @@ template <int NC>
 __device__ __forceinline__ void halo_block(const HaloArgs& A, bool odd, const StepNow& now, int32_t dep, int32_t block) {
   constexpr bool PM = NC == 3;
   constexpr int SC = NC == 0 ? 1 : NC;
-  const float* s_cur = odd ? A.s_td.u_nxt : A.s_td.u_cur;
-  const float* f_cur = odd ? A.f_td.u_nxt : A.f_td.u_cur;
-  float* s_nxt = odd ? const_cast<float*>(A.s_td.u_cur) : A.s_td.u_nxt;
-  float* f_nxt = odd ? const_cast<float*>(A.f_td.u_cur) : A.f_td.u_nxt;
+  const float* s_cur = glob(odd ? A.s_td.u_nxt : A.s_td.u_cur);
+  const float* f_cur = glob(odd ? A.f_td.u_nxt : A.f_td.u_cur);
+  float* s_nxt = glob(odd ? const_cast<float*>(A.s_td.u_cur) : A.s_td.u_nxt);
+  float* f_nxt = glob(odd ? const_cast<float*>(A.f_td.u_cur) : A.f_td.u_nxt);
   auto solid = [&](const HaloPoint& p, int32_t part, int32_t h, bool in) {
-    halo_finish<SC, true>(A.s_td, s_cur, s_nxt, A.s_hd, p, f_cur, A.f_td.ng, PM, A.amp, A.n_amp, A.sc, A.h_damp, A.st, now,
+    halo_finish<SC, true>(A.s_td, s_cur, s_nxt, A.s_hd, p, f_cur, A.f_td.ng, PM, glob(A.amp), A.n_amp, A.sc, A.h_damp, A.st, now,
                           A.epartial, A.ep_s + part, h, in);
   };
   auto fluid = [&](const HaloPoint& p, int32_t part, int32_t h, bool in) {
-    halo_finish<1, false>(A.f_td, f_cur, f_nxt, A.f_hd, p, A.s_td.a, A.s_td.ng, PM, A.amp, A.n_amp, A.sc, A.h_damp, A.st,
+    halo_finish<1, false>(A.f_td, f_cur, f_nxt, A.f_hd, p, glob(A.s_td.a), A.s_td.ng, PM, glob(A.amp), A.n_amp, A.sc, A.h_damp, A.st,
                           now, A.epartial, A.ep_f + part, h, in);
   };
   const int32_t t = threadIdx.x;
   if (NC > 0 && block < A.n_chunk) {
-    const int4 ch = A.chunks[block];
+    const int4 ch = glob(A.chunks)[block];
     const int32_t hs = ch.x + t, hf = ch.z + t;
     const HaloPoint ps = halo_point(A.s_td, A.s_hd, hs, hs < ch.y);
     const HaloPoint pf = halo_point(A.f_td, A.f_hd, hf, hf < ch.w);
