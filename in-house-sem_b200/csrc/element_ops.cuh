@@ -191,9 +191,9 @@ __device__ __forceinline__ PointData load_point(const BlockDev& blk, int b, int 
 // (per component), the point's own field values upt (hoop terms), and its
 // element data: f_xi / f_eta per component, the direct (hoop) terms, and for
 // axis points of axial elements the axis terms g xi_r, g eta_r (stored at
-// row j of gx*/gy*, AS floats apart).  The body of each reference kernel's
-// first loop.
-template <int NG, int KIND, bool ELASTIC, int M, int AS = 1>
+// row j of gx*/gy*, AS floats apart).  OFF_AXIS: no point of the block has
+// r = 0.  The body of each reference kernel's first loop.
+template <int NG, int KIND, bool ELASTIC, int M, int AS = 1, bool OFF_AXIS = false>
 __device__ __forceinline__ void point_flux(const PointData& pd, int i, int j, bool axial, const float* uxi,
                                            const float* ueta, const float* upt, float* fx, float* fy, float* direct,
                                            float* gx0, float* gy0, float* gx1, float* gy1, float w2k) {
@@ -244,7 +244,7 @@ __device__ __forceinline__ void point_flux(const PointData& pd, int i, int j, bo
       phys_grad(uxi[0], ueta[0], xi_r, xi_z, eta_r, eta_z, ur_r, ur_z);
       phys_grad(uxi[1], ueta[1], xi_r, xi_z, eta_r, eta_z, uz_r, uz_z);
       const float r = pd.r;
-      const float e_tt = r == 0.0f ? ur_r : __fdiv_rn(upt[0], r);
+      const float e_tt = !OFF_AXIS && r == 0.0f ? ur_r : __fdiv_rn(upt[0], r);
       const float lambda = pd.c0, mu = pd.c1;
       const float tr = fadd(fadd(ur_r, uz_z), e_tt);
       const float two_mu = fmul(2.0f, mu);
@@ -278,7 +278,7 @@ __device__ __forceinline__ void point_flux(const PointData& pd, int i, int j, bo
       phys_grad(uxi[1], ueta[1], xi_r, xi_z, eta_r, eta_z, um_r, um_z);
       phys_grad(uxi[2], ueta[2], xi_r, xi_z, eta_r, eta_z, uz_r, uz_z);
       const float r = pd.r;
-      const bool on_axis = r == 0.0f;
+      const bool on_axis = !OFF_AXIS && r == 0.0f;
       const float up_over_r = on_axis ? up_r : __fdiv_rn(upt[0], r);
       const float uz_over_r = on_axis ? uz_r : __fdiv_rn(upt[2], r);
       const float ur_r = fmul(fadd(up_r, um_r), is2), ur_z = fmul(fadd(up_z, um_z), is2);

@@ -587,7 +587,10 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
     BlockTiles& bt = blocks[b];
     const insem_cuda_block& in = d.blocks[b];
     const bool sep = separable(in), axi = in.kind == INSEM_AXISYM;
-    const int kind = sep ? kAxisymSeparable : in.kind, na = tile_arrays(kind);
+    bool off_axis = sep && medium == INSEM_ELASTIC;
+    for (std::size_t q = 0; off_axis && q < static_cast<std::size_t>(in.n_elements) * npe; ++q)
+      off_axis = in.r[q] != 0.0f && !in.axial[q / npe];
+    const int kind = off_axis ? kAxisymOffAxis : sep ? kAxisymSeparable : in.kind, na = tile_arrays(kind);
     bt.kind = kind;
     const bool el = medium == INSEM_ELASTIC, staged = tile_data_staged(kind);
     const std::size_t per_tile = static_cast<std::size_t>(tile_data_floats(kind, ngll));

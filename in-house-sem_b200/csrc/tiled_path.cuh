@@ -153,6 +153,8 @@ int tile_batch_cfg(const TileBatchLaunch& a, bool launch) {
                                            std::to_string(a.smem) + "): " + cudaGetErrorString(err));
     return 0;
   };
+  if (a.kind == kAxisymOffAxis)
+    return a.m == 1 ? go(tile_batch_kernel<NG, kAxisymOffAxis, true, 1>) : go(tile_batch_kernel<NG, kAxisymOffAxis, true, 0>);
   if (a.kind == kAxisymSeparable) {
     if (a.m == 1)
       return a.elastic ? go(tile_batch_kernel<NG, kAxisymSeparable, true, 1>) : go(tile_batch_kernel<NG, kAxisymSeparable, false, 1>);
@@ -209,6 +211,12 @@ void launch_tiles_cfg(const TileLaunch& a) {
                                            ", threads " + std::to_string(TileCfg<NG>::THREADS) + ", smem " +
                                            std::to_string(smem) + "): " + cudaGetErrorString(err));
   };
+  if (b.kind == kAxisymOffAxis) {
+    constexpr int K = kAxisymOffAxis;
+    if (b.m == 1) go(tile_step_kernel<NG, K, true, 1, true>, tile_step_kernel<NG, K, true, 1, false>, 3);
+    else go(tile_step_kernel<NG, K, true, 0, true>, tile_step_kernel<NG, K, true, 0, false>, 2);
+    return;
+  }
   if (b.kind == kAxisymSeparable) {
     constexpr int K = kAxisymSeparable;
     if (b.m == 1) {

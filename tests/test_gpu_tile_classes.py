@@ -10,7 +10,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-KINDS = ["rect", "affine", "curved", "monopole", "dipole", "bent monopole", "bent dipole"]
+KINDS = ["rect", "affine", "curved", "monopole", "dipole", "bent monopole", "bent dipole", "flat monopole", "flat dipole"]
 
 
 def _model(order, kind, nx, nz):
@@ -23,10 +23,10 @@ def _model(order, kind, nx, nz):
                     boundaries={b.boundaries["outer"]: "absorbing", b.boundaries["top"]: "rigid"},
                     sources=[K.Source(kind, 0.0, 0.05 * nz, (1.0, 0.0, 0.0), K.ricker(8000.0))], dt=1e-7)
         where = [("acoustic", 0.04, 0.043 * nz), ("elastic", 0.06 * nx + 0.05, 0.07 * nz)]
-    elif kind.startswith("bent"):  # axisymmetric, with a metric that varies inside the elements
+    elif kind.startswith(("bent", "flat")):  # axisymmetric, with a metric that varies inside the elements; a solid on the axis
         h = nz // 2
-        top = lambda x: 0.1 * (h + 0.5 * np.sin(20.0 * x))  # noqa: E731
-        mesh = K.layered((0.0, 0.1 * nx), [0.0, top, 0.1 * nz], [h, nz - h], [1, 0], nx=nx, quadratic=True,
+        top = lambda x: 0.1 * (h + 0.5 * np.sin(20.0 * x) * kind.startswith("bent"))  # noqa: E731
+        mesh = K.layered((0.0, 0.1 * nx), [0.0, top, 0.1 * nz], [h, nz - h], [1, 0], nx=nx, quadratic=kind.startswith("bent"),
                          coords="axisymmetric")
         m = K.Model(mesh, order=order, azimuthal_order=int(kind.endswith("dipole")),
                     materials={0: K.MUD, 1: K.FAST}, boundaries={K.RIGHT: "absorbing", K.TOP: "rigid"},
