@@ -1,14 +1,11 @@
 """Tile-size autotuner of the tiled step.
 
-A tile is one CTA of ``te`` elements, with one thread per element column.
-Its best size depends on the class:
-- ngll, geometry kind, medium and azimuthal order set the shared memory per
-  element and the registers per thread;
-- the element count per tile sets how many CTAs stay resident per SM, and
-  how many points each tile shares with its neighbours (halo work).
+A tile is one CTA of ``te`` elements, at most 32: one warp per element
+column, one lane per element.  The full 32, the library's default, leave no
+lane idle and share the fewest points with other tiles (halo work); smaller
+tiles only help where a problem has too few elements to fill the GPU.
 
-The library starts from an occupancy-based choice. This module times
-candidate sizes around that choice on real problems, one class at a time,
+This module times candidate sizes below that default on real problems, one class at a time,
 with the other classes held: ``tune`` on solo solves, ``tune_batched`` on the
 tile launches of a batch of the class's largest problems (the setting of the
 batched workload). It keeps the fastest and registers it

@@ -1,9 +1,9 @@
 """Batched solves: many independent problems advanced by shared launches.
 
-Every batched step is one CUDA graph with a fixed number of launches,
-whatever the number of problems:
-- one tile kernel per tile class, one CTA per tile; the classes spread over
-  ``tile_streams`` streams (default 2) and run side by side;
+A batched step has a fixed number of launches, whatever the number of
+problems, and is replayed from CUDA graphs of eight steps or one:
+- one tile kernel per tile class, one CTA per tile; the classes overlap in one
+  chain of launches (``tile_streams`` is accepted and has no effect);
 - then the point-wise kernels of all problems run.
 
 Each problem keeps its own time step and step count. A problem's results in

@@ -1,6 +1,6 @@
 // Device-resident twin of solver::Solver (cpp/include/insem/solver/solver.hpp:91-228)
 // and its C ABI.  Fields, boundary data, sources and receivers live in HBM;
-// the host only launches the step (a CUDA graph per step) and copies traces,
+// the host only launches the steps (CUDA graphs of several) and copies traces,
 // energy and state back on request.
 //
 // Step order per solver.cpp:917-963:

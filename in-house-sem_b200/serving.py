@@ -304,7 +304,7 @@ class _Pipeline:
 # Tile sizes that autotune.tune_batched measured on a B200 for the borehole
 # tile classes (axisymmetric elastic, ngll 5-7, m = 0 and 1: the classes of
 # every borehole request), in autotune.save's format.  Other classes keep the
-# occupancy-based default.  Tile sizes change speed only, never results.
+# default of full tiles.  Tile sizes change speed only, never results.
 DEFAULT_TILE_TABLE = Path(__file__).resolve().parent / "data" / "tile_table_b200.json"
 
 
