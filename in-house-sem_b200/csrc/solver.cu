@@ -914,15 +914,20 @@ int32_t Solver::n_energy() const {
 }
 
 namespace {
-// u, v and a of a domain as the caller has them: [field][component][point] in
-// the reference numbering, as doubles.  `perm` is null where the device keeps
-// that numbering.  Block y: field and component.
+// Fields of a domain as the caller has them: [field][component][point] in the
+// reference numbering, as doubles.  `perm` is null where the device keeps that
+// numbering.  Block y: field and component.
 struct StateFields {
   const float* f[3];
 };
 // Up to here one copy to the host, from where the three arrays are filled:
 // a pageable copy costs some 7 us however small (65 KB: 62 -> 48 us; 400 KB: 93 -> 152).
 constexpr std::size_t kStateOneCopy = std::size_t{1} << 17;
+// Values renumbered at a time, and points whose numbering stays on the device
+// between calls: 8 and 4 MB, so that a solve that fills the device can still
+// be read.
+constexpr std::size_t kStateValues = std::size_t{1} << 20;
+constexpr int32_t kStatePoints = 1 << 20;
 __global__ void state_out_kernel(StateFields in, const int32_t* __restrict__ perm, int32_t ng, int32_t stride,
                                  int32_t ncomp, double* __restrict__ out) {
   const int32_t field = blockIdx.y / ncomp, c = blockIdx.y - field * ncomp;
@@ -937,32 +942,70 @@ void Solver::copy_state(int32_t di, double* u_out, double* v_out, double* a_out)
   INSEM_REQUIRE(di >= 0 && di < static_cast<int32_t>(domains.size()), INSEM_CUDA_ERR_INVALID, "domain out of range");
   DeviceDomainData& d = domains[di];
   StateFields in{{d.u.get(), d.v.get(), d.a.get()}};
+  const int32_t* host_perm = nullptr;
   const int32_t* perm = nullptr;
   int32_t stride = d.ng;
   if (tiled) {  // before the first step: the set state, a = 0
     TiledDomain& t = tdom[di];
-    if (t.device_perm.size() == 0) t.device_perm.upload(t.perm);
-    perm = t.device_perm.get();
+    host_perm = t.perm.data();
+    if (d.ng <= kStatePoints) {
+      if (t.device_perm.size() == 0) t.device_perm.upload(t.perm);
+      perm = t.device_perm.get();
+    }
     stride = t.ng;
     in = StateFields{{t.u_cur(parity), t.v.get(), t.a.get()}};
   }
   const std::size_t n = static_cast<std::size_t>(d.ncomp) * d.ng;
   if (n == 0) return;
   // renumbered and widened on the device (the host took 1.6 ns per value and
-  // two more copies); the buffer is given back in the stream's order
+  // two more copies); the buffers are given back in the stream's order
+  const std::size_t cap = std::min(3 * n, kStateValues);
+  const bool send_perm = host_perm && !perm;
   double* buf = nullptr;
-  CUDA_CHECK(cudaMallocAsync(reinterpret_cast<void**>(&buf), 3 * n * sizeof(double), stream));
-  state_out_kernel<<<dim3(grid_for(d.ng), 3 * d.ncomp), 256, 0, stream>>>(in, perm, d.ng, stride, d.ncomp, buf);
-  cudaError_t err = cudaGetLastError();
+  int32_t* part = nullptr;
+  CUDA_CHECK(cudaMallocAsync(reinterpret_cast<void**>(&buf), cap * sizeof(double), stream));
+  cudaError_t err = cudaSuccess;
+  auto ok = [&](cudaError_t e) {
+    if (err == cudaSuccess) err = e;
+    return err == cudaSuccess;
+  };
+  if (send_perm) ok(cudaMallocAsync(reinterpret_cast<void**>(&part), kStatePoints * sizeof(int32_t), stream));
   double* out[3] = {u_out, v_out, a_out};
   std::vector<double> small(3 * n * sizeof(double) <= kStateOneCopy ? 3 * n : 0);
-  if (!small.empty()) {
-    if (err == cudaSuccess)
-      err = cudaMemcpyAsync(small.data(), buf, small.size() * sizeof(double), cudaMemcpyDeviceToHost, stream);
-  } else {
-    for (int k = 0; k < 3 && err == cudaSuccess; ++k)
-      if (out[k]) err = cudaMemcpyAsync(out[k], buf + k * n, n * sizeof(double), cudaMemcpyDeviceToHost, stream);
+  auto renumber = [&](const StateFields& f, const int32_t* pm, int32_t points, int32_t rows, int32_t ncomp) {
+    if (err != cudaSuccess) return;
+    state_out_kernel<<<dim3(grid_for(points), rows), 256, 0, stream>>>(f, pm, points, stride, ncomp, buf);
+    ok(cudaGetLastError());
+  };
+  auto fetch = [&](double* to, std::size_t from, std::size_t count) {
+    if (err == cudaSuccess && to)
+      ok(cudaMemcpyAsync(to, buf + from, count * sizeof(double), cudaMemcpyDeviceToHost, stream));
+  };
+  if (3 * n <= kStateValues) {  // all at once
+    renumber(in, perm, d.ng, 3 * d.ncomp, d.ncomp);
+    if (!small.empty()) fetch(small.data(), 0, 3 * n);
+    else
+      for (int k = 0; k < 3; ++k) fetch(out[k], k * n, n);
+  } else if (n <= kStateValues && !send_perm) {  // field by field
+    for (int k = 0; k < 3; ++k) {
+      if (!out[k]) continue;
+      renumber(StateFields{{in.f[k]}}, perm, d.ng, d.ncomp, d.ncomp);
+      fetch(out[k], 0, n);
+    }
+  } else {  // by ranges of points
+    const int32_t most = std::min<int32_t>(kStatePoints, static_cast<int32_t>(kStateValues));
+    for (int32_t g = 0; g < d.ng && err == cudaSuccess; g += most) {
+      const int32_t m = std::min(most, d.ng - g);
+      if (send_perm) ok(cudaMemcpyAsync(part, host_perm + g, m * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
+      for (int k = 0; k < 3; ++k)
+        for (int32_t c = 0; c < d.ncomp && out[k]; ++c) {
+          const float* x = in.f[k] + static_cast<std::size_t>(c) * stride;
+          renumber(StateFields{{host_perm ? x : x + g}}, send_perm ? part : perm ? perm + g : nullptr, m, 1, 1);
+          fetch(out[k] + static_cast<std::size_t>(c) * d.ng + g, 0, m);
+        }
+    }
   }
+  if (part) cudaFreeAsync(part, stream);
   cudaFreeAsync(buf, stream);
   const cudaError_t sync = cudaStreamSynchronize(stream);
   CUDA_CHECK(err);
