@@ -1016,6 +1016,8 @@ void Solver::copy_state(int32_t di, double* u_out, double* v_out, double* a_out)
 }
 
 // ------------------------------------------------------------ tiled path
+constexpr int32_t kPaddedPoints = 1 << 22;  // most points of a domain in tiles of fewer than 32 elements
+
 void Solver::build_tiled(const insem_cuda_problem& p) {
   const std::size_t npe = static_cast<std::size_t>(ngll) * ngll;
   set_constant_basis(ngll, host_vec(p.basis.D, npe), p.basis.Dj ? host_vec(p.basis.Dj, npe) : std::vector<float>{},
@@ -1055,8 +1057,13 @@ void Solver::build_tiled(const insem_cuda_problem& p) {
         most = kv.second;
         kind = kv.first;
       }
-    const int te = choose_tile_elements(ngll, kind, d.medium == INSEM_ELASTIC, kind == INSEM_AXISYM ? d.azimuthal_order : 0,
-                                        opts.tile_elements);
+    // A tile's data is laid out for 32 elements whatever it holds, so smaller
+    // tiles, which only pay where elements are few, are not taken where their
+    // padding would cost gigabytes.
+    const int te = domains[di].ng > kPaddedPoints
+                       ? kTileLanes
+                       : choose_tile_elements(ngll, kind, d.medium == INSEM_ELASTIC,
+                                              kind == INSEM_AXISYM ? d.azimuthal_order : 0, opts.tile_elements);
     tdom[di].build(d, ngll, te, terms,
                    host_vec(d.absorbing_coef, static_cast<std::size_t>(d.n_absorbing) * d.ncomp * d.ncomp));
   }

@@ -344,8 +344,9 @@ int32_t insem_cuda_solver_n_columns(const insem_cuda_solver* h);
 int32_t insem_cuda_solver_kernels_per_step(insem_cuda_solver* h);
 /* Elements per tile (one CTA) of the tiled path.  A solver takes
  * options.tile_elements when > 0, else the entry set here for its domain's
- * class (ngll, dominant geometry kind, medium, azimuthal order), else an
- * occupancy-based default.  The autotuner (insem_b200.autotune) times
+ * class (ngll, dominant geometry kind, medium, azimuthal order), else 32, a
+ * full tile; at most 32, and 32 in a domain of more than 2^22 points (smaller
+ * tiles are padded to 32 elements).  The autotuner (insem_b200.autotune) times
  * candidates and sets the entries; tile_elements <= 0 clears one.  Applies to
  * solvers created afterwards; process-wide. */
 int insem_cuda_set_tile_elements(int32_t ngll, int32_t kind, int32_t medium, int32_t azimuthal_order,

@@ -80,3 +80,15 @@ def test_small_domains(pkg, oracle, order, kind):
                                               (6, "dipole", 130, 140), (8, "affine", 120, 130), (5, "bent monopole", 200, 210)])
 def test_domains_of_many_tiles(pkg, oracle, order, kind, nx, nz):
     _check(pkg, oracle, _model(order, kind, nx, nz))
+
+
+@pytest.mark.parametrize("n,want", [(255, 8), (257, 32)])  # 4.16M and 4.23M points, about 2^22
+def test_large_domains_take_full_tiles(pkg, n, want):
+    import insem_b200.cases as K
+
+    m = K.Model(K.layered((0.0, 1.0), [0.0, 1.0], [n], [0], nx=n), order=8,
+                materials={0: K.Material.acoustic(1500.0, 1000.0)}, dt=1e-9)
+    m.n_steps = 1
+    prob = K.build(m, stable_dt=1e-6)
+    with pkg.Solver(prob, tile_elements=8) as s:
+        assert pkg.native.lib().insem_cuda_solver_tile_elements(s._h, 0) == want
