@@ -72,8 +72,11 @@ void Solver::internal_forces_noalloc(int32_t di, const float* u_global, float* f
   // The array keeps the previous call's values; the blocks' kernels write every
   // element they hold, so only elements of no block need zeros.
   if (!d.blocks_cover) CUDA_CHECK(cudaMemsetAsync(scratch, 0, need * sizeof(float), s));
+  // the first block that launches waits for what is ahead on the stream (the
+  // caller's field, the last reader of the scratch); the others follow it
   bool first = true;
   for (const DeviceBlock& b : d.blocks) {
+    if (b.n == 0) continue;
     ElementLaunch a;
     a.basis = basis.view();
     a.blk = b.view();

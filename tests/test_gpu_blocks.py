@@ -1,0 +1,99 @@
+"""Domains of several element blocks against the oracle: a block without
+elements ahead of the others, in their middle or at the end, and one block
+split in two.  The blocks of a domain follow one another in a chain of
+launches of which only the first waits for what is ahead of it, so that first
+one has to be a block that launches."""
+
+from __future__ import annotations
+
+import copy
+import ctypes as C
+from dataclasses import fields, replace
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+FORMS = ["empty first", "empty middle", "empty last", "split"]
+
+
+def _take(b, npe, lo, hi):
+    """Elements [lo, hi) of a block."""
+    n, out = b.n_elements, {}
+    for f in fields(b):
+        x = getattr(b, f.name)
+        if isinstance(x, np.ndarray):
+            out[f.name] = np.ascontiguousarray(x.reshape(n, -1)[lo:hi].ravel()) if x.size else x
+    return replace(b, **out)
+
+
+def _with_blocks(prob, form):
+    """The problem with every domain's one block in the given form."""
+    prob, npe = copy.deepcopy(prob), prob.ngll ** 2
+    for d in prob.domains:
+        (b,) = d.blocks
+        n = b.n_elements
+        first, second, none = _take(b, npe, 0, n // 2), _take(b, npe, n // 2, n), _take(b, npe, 0, 0)
+        d.blocks = {"empty first": [none, first, second], "empty middle": [first, none, second],
+                    "empty last": [first, second, none], "split": [first, second]}[form]
+    return prob
+
+
+def _problem(kind, n=24, n_steps=1, order=4):
+    import insem_b200.cases as K
+
+    if kind == "dipole":
+        b = K.borehole((0.0, 0.1 * n), [("mud", 0.1)], formation_radius=0.08 * n, dz=0.1)
+        mats = {b.regions["mud"]: K.MUD, b.regions["formation"]: K.FAST}
+        m = K.Model(b.mesh, order=order, azimuthal_order=1, materials=mats, boundaries={b.boundaries["outer"]: "absorbing"},
+                    sources=[K.Source("dipole", 0.0, 0.05 * n, (1.0, 0.0, 0.0), K.ricker(3000.0))], dt=1e-8,
+                    receivers=[K.Receiver("p", 0.04, 0.043 * n, ["pressure"], "acoustic")])
+    else:
+        mesh = K.rectangle((0.0, float(n)), (0.0, float(n)), nx=n, nz=n, material=lambda x, z: int(z < 0.4 * n))
+        m = K.Model(mesh, order=order, materials={0: K.Material.acoustic(1500.0, 1000.0), 1: K.FAST}, dt=1e-8,
+                    boundaries={K.BOTTOM: "absorbing", K.LEFT: "rigid"}, energy_every=3,
+                    sources=[K.Source("monopole", 0.41 * n, 0.83 * n, stf=K.ricker(300.0))],
+                    receivers=[K.Receiver("p", 0.32 * n, 0.71 * n, ["pressure"], "acoustic")])
+    m.n_steps = n_steps
+    return K.build(m, stable_dt=1.0)
+
+
+@pytest.mark.parametrize("form", FORMS + ["uncovered"])
+@pytest.mark.parametrize("kind", ["plain", "dipole"])
+def test_forces_without_allocation(pkg, oracle, kind, form):
+    """Both domains one after the other, many times, over one scratch array and
+    with the field rewritten ahead of each call."""
+    import torch
+
+    from insem_b200 import native as N
+
+    prob = _problem(kind, n=48)
+    if form == "uncovered":  # elements of no block contribute nothing (two-pass path only)
+        prob = _with_blocks(prob, "empty first")
+        for d in prob.domains:
+            d.blocks.pop()
+    else:
+        prob = _with_blocks(prob, form)
+    ref = oracle.OracleSolver(prob)
+    rng = np.random.default_rng(5)
+    with pkg.Solver(prob, path=1) as s:
+        host = [rng.uniform(-1, 1, d.ncomp * d.n_global).astype(np.float32) for d in prob.domains]
+        want = [ref.internal_forces(i, u) for i, u in enumerate(host)]
+        src = [torch.from_numpy(u).cuda() for u in host]
+        u = [torch.empty_like(x) for x in src]
+        reps = 20
+        f = [[torch.full_like(x, float("nan")) for x in src] for _ in range(reps)]
+        side = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            for k in range(reps):
+                for i in range(len(src)):
+                    u[i].zero_()
+                    torch.add(u[i], src[i], out=u[i])
+                    N.check(N.lib().insem_cuda_solver_internal_forces_noalloc(
+                        s._h, i, C.c_void_p(u[i].data_ptr()), C.c_void_p(f[k][i].data_ptr()), C.c_void_p(side.cuda_stream)))
+        torch.cuda.synchronize()
+        for k in range(reps):
+            for i in range(len(src)):
+                assert np.array_equal(f[k][i].cpu().numpy(), want[i]), (k, i)
