@@ -517,12 +517,14 @@ double Solver::stable_dt() {
   StartVector rng;
   pw.zero(stream);
   counter.zero(stream);
-  // element forces of a domain's scaled field
-  auto forces = [&](int di, int32_t dep_forces) {
+  // element forces of a domain's scaled field: the first block that launches
+  // waits for what is ahead, unless a launch of this iteration did (`first`,
+  // returned for the launches that follow)
+  auto forces = [&](int di, bool first) {
     DeviceDomainData& d = domains[di];
     Work& w = work[di];
-    bool first = true;
     for (const DeviceBlock& b : d.blocks) {
+      if (b.n == 0) continue;
       ElementLaunch a;
       a.basis = basis.view();
       a.blk = b.view();
@@ -534,12 +536,13 @@ double Solver::stable_dt() {
       a.gather = true;
       a.scale = pw.get() + kPwScale;
       a.elastic = d.medium == INSEM_ELASTIC;
-      a.dep = first ? dep_forces : kDepLate;
+      a.dep = first ? kDepFirst : kDepLate;
       a.overlap = true;
       a.stream = stream;
       launch_element_forces(ngll, a);
       first = false;
     }
+    return first;
   };
   auto point = [&](int di, int mode, bool late) {
     DeviceDomainData& d = domains[di];
@@ -599,7 +602,7 @@ double Solver::stable_dt() {
     reset();
     replay(100 / kPerGraph, [&] {
       for (int k = 0; k < kPerGraph; ++k) {
-        forces(static_cast<int>(di), kDepFirst);
+        forces(static_cast<int>(di), true);
         point(static_cast<int>(di), kPowerAlone, false);
       }
     }, graphs);
@@ -629,8 +632,7 @@ double Solver::stable_dt() {
     for (bool late : {false, true})
       replay(60 / kPerGraph, [&] {
         for (int k = 0; k < kPerGraph; ++k) {
-          forces(solid, kDepFirst);
-          forces(fluid, kDepLate);
+          forces(fluid, forces(solid, true));
           point(solid, kPowerSolid, late);
           point(fluid, kPowerFluid, late);
         }

@@ -97,3 +97,34 @@ def test_forces_without_allocation(pkg, oracle, kind, form):
         for k in range(reps):
             for i in range(len(src)):
                 assert np.array_equal(f[k][i].cpu().numpy(), want[i]), (k, i)
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("kind", ["plain", "dipole"])
+def test_stable_dt(pkg, kind, form):
+    """The estimate of the problem as built, bit for bit: blocks only share out
+    the elements."""
+    from insem_b200.solver import estimate_stable_dt
+
+    prob = _problem(kind)
+    want, other = estimate_stable_dt(prob), _with_blocks(prob, form)
+    for _ in range(3):
+        assert estimate_stable_dt(other) == want
+
+
+@pytest.mark.parametrize("kind", ["coupled", "dipole"])
+@pytest.mark.parametrize("blocks", ["none", "empty"])
+def test_stable_dt_with_a_solid_that_launches_nothing(pkg, oracle, kind, blocks):
+    """The solid then has no stiffness; its mass still takes part in the coupled
+    iteration, in which the fluid's forces come first."""
+    from insem_b200.solver import estimate_stable_dt
+    from test_gpu_stable_dt import _expected, _problem as small
+
+    prob = small(4, kind)
+    d = prob.domains[prob.domain_index("elastic")]
+    d.blocks = [] if blocks == "none" else [_take(d.blocks[0], prob.ngll ** 2, 0, 0)]
+    with np.errstate(invalid="ignore"):  # the solid alone: 0 / 0 after its first iteration, which no maximum takes
+        want = _expected(prob, oracle)
+    got = estimate_stable_dt(prob)
+    assert abs(got - want) <= 2e-6 * want, (got, want)
+    assert got == estimate_stable_dt(prob)
