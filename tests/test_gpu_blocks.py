@@ -128,3 +128,95 @@ def test_stable_dt_with_a_solid_that_launches_nothing(pkg, oracle, kind, blocks)
     got = estimate_stable_dt(prob)
     assert abs(got - want) <= 2e-6 * want, (got, want)
     assert got == estimate_stable_dt(prob)
+
+
+def _check(prob, s, ref):
+    for name, quantity in prob.trace_list():
+        assert np.array_equal(s.trace(name, quantity), ref.trace(name, quantity)), (name, quantity)
+    for i, medium in enumerate(prob.media):
+        for x, y in zip(s.state(medium), ref.state(i)):
+            assert np.array_equal(x, y), medium
+
+
+def _mixed(n, n_steps=1):
+    """Rect, Affine and Curved elements: three blocks of one domain."""
+    import insem_b200.cases as K
+
+    a, b = 0.35 * n, 0.7 * n
+    rise = lambda x: np.where(x < a, 0.0, np.where(x < b, 0.2 * (x - a), 0.2 * (b - a) + 0.3 * np.sin(x - b)))  # noqa: E731
+    mesh = K.layered((0.0, float(n)), [rise, lambda x: n + rise(x)], [n], [1], nx=n, quadratic=True)
+    m = K.Model(mesh, order=4, materials={1: K.FAST}, boundaries={K.LEFT: "absorbing", K.TOP: "free"}, dt=1e-6,
+                sources=[K.Source("force", 0.36 * n, 0.49 * n, (0.0, 1.0, 0.0), K.ricker(300.0))],
+                receivers=[K.Receiver("v", 0.68 * n, 0.46 * n, ["velocity"], "elastic")], energy_every=3)
+    m.n_steps = n_steps
+    prob = K.build(m, stable_dt=1.0)
+    assert [x.kind for x in prob.domains[0].blocks] == [0, 1, 2]
+    return prob
+
+
+def _set(prob, *solvers):
+    rng = np.random.default_rng(2)
+    for d, medium in zip(prob.domains, prob.media):
+        u, v = (1e3 if d.medium == 0 else 1e-6) * rng.standard_normal((2, d.ncomp, d.n_global))
+        for s in solvers:
+            s.set_state(medium, u, v)
+
+
+def _steps_problem(kind, form, n_steps):
+    return _mixed(20, n_steps) if kind == "mixed" else _with_blocks(_problem(kind, n_steps=n_steps), form)
+
+
+CASES = [(kind, form) for kind in ("plain", "dipole") for form in FORMS] + [("mixed", "built")]
+
+
+@pytest.mark.parametrize("kind,form", CASES)
+@pytest.mark.parametrize("path", [0, 1])
+def test_steps(pkg, oracle, kind, form, path):
+    prob = _steps_problem(kind, form, 23)
+    ref = oracle.OracleSolver(prob)
+    with pkg.Solver(prob, path=path) as s:
+        _set(prob, s, ref)
+        for n in (1, 21, 1):
+            s.advance(n)
+        ref.run()
+        _check(prob, s, ref)
+
+
+def test_batched_steps(pkg, oracle):
+    with pkg.Batch() as b:
+        entries = []
+        for kind, form in CASES:
+            prob = _steps_problem(kind, form, 11)
+            s, ref = b.add(prob), oracle.OracleSolver(prob)
+            _set(prob, s, ref)
+            entries.append((prob, s, ref))
+        b.run()
+        for prob, s, ref in entries:
+            ref.run()
+            _check(prob, s, ref)
+
+
+def test_mixed_kinds_forces_and_stable_dt(pkg, oracle):
+    import torch
+
+    from insem_b200 import native as N
+    from insem_b200.solver import estimate_stable_dt
+    from test_gpu_stable_dt import _expected
+
+    prob = _mixed(6)
+    want, got = _expected(prob, oracle), estimate_stable_dt(prob)
+    assert abs(got - want) <= 2e-6 * want, (got, want)
+    assert got == estimate_stable_dt(prob)
+    prob = _mixed(20)
+    d = prob.domains[0]
+    u = np.random.default_rng(4).uniform(-1, 1, d.ncomp * d.n_global).astype(np.float32)
+    u_dev = torch.from_numpy(u).cuda()
+    f = [torch.empty_like(u_dev) for _ in range(10)]
+    torch.cuda.synchronize()
+    with pkg.Solver(prob) as s:
+        for x in f:
+            N.check(N.lib().insem_cuda_solver_internal_forces_noalloc(s._h, 0, C.c_void_p(u_dev.data_ptr()),
+                                                                      C.c_void_p(x.data_ptr()), None))
+        torch.cuda.synchronize()
+    want = oracle.OracleSolver(prob).internal_forces(0, u)
+    assert all(np.array_equal(x.cpu().numpy(), want) for x in f)
