@@ -743,6 +743,9 @@ void Solver::set_state(int32_t medium, const double* u_in, const double* v_in) {
     CUDA_CHECK(cudaMemcpy(t.u_cur(parity), pu.data(), nd * sizeof(float), cudaMemcpyHostToDevice));
     CUDA_CHECK(cudaMemcpy(t.v.get(), pv.data(), nd * sizeof(float), cudaMemcpyHostToDevice));
   }
+  // a copy from pageable memory may return before its DMA has landed; the
+  // readers run on the solver's non-blocking stream
+  CUDA_CHECK(cudaStreamSynchronize(nullptr));
 }
 
 void Solver::advance(int32_t n) {

@@ -1,0 +1,52 @@
+"""set_state() again and again on one solver, each time followed at once by a
+read of the state or by the first step: the values just set are the ones read."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(n, order=4):
+    import insem_b200.cases as K
+
+    mesh = K.layered((0.0, 1.0), [0.0, 1.0], [n], [0], nx=n)
+    m = K.Model(mesh, order=order, materials={0: K.Material.acoustic(1500.0, 1000.0)}, dt=1e-9)
+    m.n_steps = 2
+    return K.build(m, stable_dt=1e-6)
+
+
+# points: 81 and 10k (copied through the driver's buffer at once), 160k, 1.05M
+# (read by ranges, without a numbering uploaded on the first read)
+@pytest.mark.parametrize("path", [1, 2])
+@pytest.mark.parametrize("n", [2, 25, 100, 256])
+def test_values_set_are_the_values_read(pkg, n, path):
+    prob = _problem(n)
+    d = prob.domains[0]
+    rng = np.random.default_rng(n)
+    with pkg.Solver(prob, path=path) as s:
+        for _ in range(8):
+            u, v = rng.standard_normal((2, d.ncomp, d.n_global)).astype(np.float32).astype(np.float64)
+            s.set_state("acoustic", u, v)
+            got = s.state("acoustic")
+            assert np.array_equal(got[0], u) and np.array_equal(got[1], v) and not got[2].any()
+
+
+@pytest.mark.parametrize("path", [1, 2])
+@pytest.mark.parametrize("n", [2, 25, 100])
+def test_the_first_step_starts_from_the_values_set(pkg, oracle, n, path):
+    prob = _problem(n)
+    d = prob.domains[0]
+    rng = np.random.default_rng(n)
+    ref = oracle.OracleSolver(prob)
+    with pkg.Solver(prob, path=path) as s:
+        for _ in range(3):
+            u, v = rng.standard_normal((2, d.ncomp, d.n_global))
+            s.set_state("acoustic", u, v)
+        ref.set_state("acoustic", u, v)
+        s.run()
+        ref.run()
+        for x, y in zip(s.state("acoustic"), ref.state(0)):
+            assert np.array_equal(x, y)
