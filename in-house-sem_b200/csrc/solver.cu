@@ -954,6 +954,7 @@ void Solver::copy_state(int32_t di, double* u_out, double* v_out, double* a_out)
     TiledDomain& t = tdom[di];
     host_perm = t.perm.data();
     if (d.ng <= kStatePoints) {
+      std::lock_guard<std::mutex> lk(perm_mutex);  // several threads may read one solve
       if (t.device_perm.size() == 0) t.device_perm.upload(t.perm);
       perm = t.device_perm.get();
     }

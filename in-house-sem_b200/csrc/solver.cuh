@@ -5,6 +5,7 @@
 #include <map>
 
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "device_data.cuh"
@@ -164,6 +165,7 @@ class Solver {
   void advance_tiled(int32_t n, const float* amp_in, double* rows_out, int32_t* n_rows);
   AllFields tiled_fields(int parity);
   std::vector<TiledDomain> tdom;
+  std::mutex perm_mutex;  // the domains' device_perm, made by the first state()
   std::vector<std::map<int32_t, std::vector<std::pair<int32_t, std::vector<float>>>>> src_per_point;
   DeviceBuffer<int32_t> trec_points;
   std::vector<int4> coupled_chunks(const std::vector<int32_t>& fp, const std::vector<int32_t>& sp,

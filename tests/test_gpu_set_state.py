@@ -3,6 +3,9 @@ read of the state or by the first step: the values just set are the ones read.""
 
 from __future__ import annotations
 
+from concurrent.futures import ThreadPoolExecutor
+from threading import Barrier
+
 import numpy as np
 import pytest
 
@@ -50,3 +53,23 @@ def test_the_first_step_starts_from_the_values_set(pkg, oracle, n, path):
         ref.run()
         for x, y in zip(s.state("acoustic"), ref.state(0)):
             assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("path", [1, 2])
+def test_several_threads_read_one_solver(pkg, path):
+    """The first reads of a solver's state come from several threads at once."""
+    prob, threads = _problem(100), 6
+    d = prob.domains[0]
+    u, v = np.random.default_rng(1).standard_normal((2, d.ncomp, d.n_global)).astype(np.float32).astype(np.float64)
+    with ThreadPoolExecutor(threads) as pool:
+        for _ in range(10):
+            with pkg.Solver(prob, path=path) as s:
+                s.set_state("acoustic", u, v)
+                start = Barrier(threads)
+
+                def read():
+                    start.wait(30)
+                    return s.state("acoustic")
+
+                for got in [f.result() for f in [pool.submit(read) for _ in range(threads)]]:
+                    assert np.array_equal(got[0], u) and np.array_equal(got[1], v) and not got[2].any()
