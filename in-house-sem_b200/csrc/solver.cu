@@ -929,8 +929,8 @@ struct StateFields {
 // a pageable copy costs some 7 us however small (65 KB: 62 -> 48 us; 400 KB: 93 -> 152).
 constexpr std::size_t kStateOneCopy = std::size_t{1} << 17;
 // Values renumbered at a time, and points whose numbering stays on the device
-// between calls: 8 and 4 MB, so that a solve that fills the device can still
-// be read.
+// between calls: 8 and 4 MB (a device without that much to spare is read by
+// plain copies).
 constexpr std::size_t kStateValues = std::size_t{1} << 20;
 constexpr int32_t kStatePoints = 1 << 20;
 __global__ void state_out_kernel(StateFields in, const int32_t* __restrict__ perm, int32_t ng, int32_t stride,
@@ -943,40 +943,65 @@ __global__ void state_out_kernel(StateFields in, const int32_t* __restrict__ per
 }
 }  // namespace
 
+// The point numbering of a domain of at most kStatePoints points on the device,
+// uploaded by the first state(); null without the memory for it.
+const int32_t* Solver::state_numbering(int32_t di) {
+  std::lock_guard<std::mutex> lk(perm_mutex);  // several threads may read one solve
+  TiledDomain& t = tdom[di];
+  if (t.device_perm.size() == 0) {
+    try {
+      t.device_perm.upload(t.perm);
+    } catch (const Error& e) {
+      if (e.code != INSEM_CUDA_ERR_NOMEM) throw;
+    }
+  }
+  return t.device_perm.get();
+}
+
 void Solver::copy_state(int32_t di, double* u_out, double* v_out, double* a_out) {
   INSEM_REQUIRE(di >= 0 && di < static_cast<int32_t>(domains.size()), INSEM_CUDA_ERR_INVALID, "domain out of range");
   DeviceDomainData& d = domains[di];
   StateFields in{{d.u.get(), d.v.get(), d.a.get()}};
   const int32_t* host_perm = nullptr;
-  const int32_t* perm = nullptr;
   int32_t stride = d.ng;
   if (tiled) {  // before the first step: the set state, a = 0
     TiledDomain& t = tdom[di];
     host_perm = t.perm.data();
-    if (d.ng <= kStatePoints) {
-      std::lock_guard<std::mutex> lk(perm_mutex);  // several threads may read one solve
-      if (t.device_perm.size() == 0) t.device_perm.upload(t.perm);
-      perm = t.device_perm.get();
-    }
     stride = t.ng;
     in = StateFields{{t.u_cur(parity), t.v.get(), t.a.get()}};
   }
   const std::size_t n = static_cast<std::size_t>(d.ncomp) * d.ng;
   if (n == 0) return;
+  double* out[3] = {u_out, v_out, a_out};
   // renumbered and widened on the device (the host took 1.6 ns per value and
   // two more copies); the buffers are given back in the stream's order
   const std::size_t cap = std::min(3 * n, kStateValues);
-  const bool send_perm = host_perm && !perm;
+  const bool send_perm = host_perm && d.ng > kStatePoints;
   double* buf = nullptr;
   int32_t* part = nullptr;
-  CUDA_CHECK(cudaMallocAsync(reinterpret_cast<void**>(&buf), cap * sizeof(double), stream));
-  cudaError_t err = cudaSuccess;
+  cudaError_t err = cudaMallocAsync(reinterpret_cast<void**>(&buf), cap * sizeof(double), stream);
+  if (err == cudaSuccess && send_perm)
+    err = cudaMallocAsync(reinterpret_cast<void**>(&part), kStatePoints * sizeof(int32_t), stream);
+  const int32_t* perm = err == cudaSuccess && host_perm && !send_perm ? state_numbering(di) : nullptr;
+  if (err != cudaSuccess || (host_perm && !send_perm && !perm)) {
+    // no device memory to spare: the fields as they are, renumbered on the host
+    cudaGetLastError();
+    if (buf) cudaFreeAsync(buf, stream);
+    std::vector<float> h(static_cast<std::size_t>(d.ncomp) * stride);
+    for (int k = 0; k < 3; ++k) {
+      if (!out[k]) continue;
+      CUDA_CHECK(cudaMemcpyAsync(h.data(), in.f[k], h.size() * sizeof(float), cudaMemcpyDeviceToHost, stream));
+      CUDA_CHECK(cudaStreamSynchronize(stream));
+      for (int c = 0; c < d.ncomp; ++c)
+        for (int32_t g = 0; g < d.ng; ++g)
+          out[k][static_cast<std::size_t>(c) * d.ng + g] = h[static_cast<std::size_t>(c) * stride + (host_perm ? host_perm[g] : g)];
+    }
+    return;
+  }
   auto ok = [&](cudaError_t e) {
     if (err == cudaSuccess) err = e;
     return err == cudaSuccess;
   };
-  if (send_perm) ok(cudaMallocAsync(reinterpret_cast<void**>(&part), kStatePoints * sizeof(int32_t), stream));
-  double* out[3] = {u_out, v_out, a_out};
   std::vector<double> small(3 * n * sizeof(double) <= kStateOneCopy ? 3 * n : 0);
   auto renumber = [&](const StateFields& f, const int32_t* pm, int32_t points, int32_t rows, int32_t ncomp) {
     if (err != cudaSuccess) return;

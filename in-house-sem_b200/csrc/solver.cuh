@@ -165,6 +165,7 @@ class Solver {
   void advance_tiled(int32_t n, const float* amp_in, double* rows_out, int32_t* n_rows);
   AllFields tiled_fields(int parity);
   std::vector<TiledDomain> tdom;
+  const int32_t* state_numbering(int32_t di);
   std::mutex perm_mutex;  // the domains' device_perm, made by the first state()
   std::vector<std::map<int32_t, std::vector<std::pair<int32_t, std::vector<float>>>>> src_per_point;
   DeviceBuffer<int32_t> trec_points;
