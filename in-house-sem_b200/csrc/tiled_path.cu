@@ -327,22 +327,17 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
     for (int32_t l = 0; l < n_direct[t]; ++l)
       for (int q = 0; q < ni * ni; ++q) inner[l2g[static_cast<std::size_t>(list[l]) * npe + inner_slot(q)]] = 1;
   }
-  std::vector<int32_t> count(n_tiles + 1, 0);  // edge complete points
-  for (int32_t g = 0; g < ng; ++g)
-    if (owner[g] >= 0 && !inner[g]) ++count[owner[g] + 1];
-  // Inner points come in rows of 32 (one per lane, so that a row's accesses
-  // are whole sectors at fixed distances), edge points in ranges that start on
-  // a multiple of 4 points (16 bytes, for bulk copies); the gaps are unused
-  // padding points.
-  auto up4 = [](int32_t x) { return (x + 3) & ~3; };
-  std::vector<int32_t> cbeg(n_tiles + 1, 0), ebeg(n_tiles, 0);
-  for (int t = 0; t < n_tiles; ++t) {
-    ebeg[t] = cbeg[t] + kTileLanes * ni * ni;
-    cbeg[t + 1] = (ebeg[t] + count[t + 1] + kTileLanes - 1) & ~(kTileLanes - 1);
+  std::vector<int32_t> count(n_tiles, 0);  // edge complete points
+  n_halo = 0;
+  for (int32_t g = 0; g < ng; ++g) {
+    if (owner[g] < 0) ++n_halo;
+    else if (!inner[g]) ++count[owner[g]];
   }
-  n_complete = cbeg[n_tiles];
+  auto up4 = [](int32_t x) { return (x + 3) & ~3; };
+  const TileNumbers numbers = number_tiles(count, ni, n_halo);
+  const auto &cbeg = numbers.cbeg, &ebeg = numbers.ebeg;
+  n_complete = numbers.n_complete;
   perm.assign(ng, -1);
-  int32_t n_halo_pts = 0;
   {
     for (int t = 0; t < n_tiles; ++t)
       for (int q = 0; q < ni * ni; ++q)
@@ -357,10 +352,8 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
       perm[g] = owner[g] >= 0 ? fill[owner[g]]++ : h++;
     }
     for (int32_t g : sp.coupled) perm[g] = h++;
-    n_halo_pts = h - n_complete;
   }
-  n_halo = n_halo_pts;
-  const int32_t ng_dev = std::max(up4(n_complete + n_halo), 4);
+  const int32_t ng_dev = numbers.stride;
   const int W = kTileLanes;
 
   // 4. per tile: tile points, descriptors, halo and constrained slots.  The
@@ -380,7 +373,7 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
       th.nd = n_direct[t];
       th.cbeg = cbeg[t];
       th.ebeg = ebeg[t];
-      th.nc = count[t + 1];  // [ebeg + nc, cbeg of the next tile) is padding
+      th.nc = count[t];  // [ebeg + nc, cbeg of the next tile) is padding
       th.hl_off = static_cast<int32_t>(htp.size());
       th.hs_off = static_cast<int32_t>(hslot.size());
       th.cs_off = static_cast<int32_t>(cslot.size());

@@ -1,6 +1,8 @@
 // Host side of the tiled fused step: tiling, device numbering and launches.
 #pragma once
 
+#include <algorithm>
+#include <cstdint>
 #include <map>
 #include <vector>
 
@@ -18,6 +20,39 @@ struct SpecialTerms {
   std::vector<int32_t> receivers;                                                 // points read by receivers
   std::vector<int32_t> coupled;  // coupled points in chunk order: numbered last, in this order
 };
+
+// First device points of every tile: inner points in `ni` x `ni` rows of 32,
+// one per lane, whatever the tile holds (so that rows lie at fixed distances),
+// then its edge points, each range starting on a multiple of 32 points; then
+// the halo points.  The gaps are unused padding points.
+struct TileNumbers {
+  std::vector<int32_t> cbeg, ebeg;  // [tiles + 1] inner points, [tiles] edge points
+  int32_t n_complete = 0;
+  int32_t stride = 0;               // points of a component: all of them, rounded up to 4 (16 bytes), at least 4
+};
+// edge_points[t]: edge complete points of tile t.  Device points are 32-bit:
+// the padding of many part-filled tiles may need more, which is refused here
+// before anything is sized by it.
+inline TileNumbers number_tiles(const std::vector<int32_t>& edge_points, int ni, int32_t n_halo) {
+  TileNumbers t;
+  t.cbeg.reserve(edge_points.size() + 1);
+  t.ebeg.reserve(edge_points.size());
+  int64_t at = 0;
+  auto point = [&](int64_t p) {
+    INSEM_REQUIRE(p <= INT32_MAX, INSEM_CUDA_ERR_UNSUPPORTED,
+                  "the domain's tiles need more than 2^31 - 1 points with their padding (options.path = 1 takes none)");
+    return static_cast<int32_t>(p);
+  };
+  for (int32_t edge : edge_points) {
+    t.cbeg.push_back(point(at));
+    t.ebeg.push_back(point(at + kTileLanes * ni * ni));
+    at = (at + kTileLanes * ni * ni + edge + kTileLanes - 1) / kTileLanes * kTileLanes;
+  }
+  t.cbeg.push_back(point(at));
+  t.n_complete = point(at);
+  t.stride = point(std::max<int64_t>((at + n_halo + 3) / 4 * 4, 4));
+  return t;
+}
 
 // One domain of the tiled path.
 class TiledDomain {
