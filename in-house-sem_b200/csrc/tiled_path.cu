@@ -328,11 +328,10 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
       for (int q = 0; q < ni * ni; ++q) inner[l2g[static_cast<std::size_t>(list[l]) * npe + inner_slot(q)]] = 1;
   }
   std::vector<int32_t> count(n_tiles, 0);  // edge complete points
-  n_halo = 0;
-  for (int32_t g = 0; g < ng; ++g) {
-    if (owner[g] < 0) ++n_halo;
-    else if (!inner[g]) ++count[owner[g]];
-  }
+  for (int32_t g = 0; g < ng; ++g)
+    if (owner[g] >= 0 && !inner[g]) ++count[owner[g]];
+  n_halo = ng;
+  for (int t = 0; t < n_tiles; ++t) n_halo -= n_direct[t] * ni * ni + count[t];
   auto up4 = [](int32_t x) { return (x + 3) & ~3; };
   const TileNumbers numbers = number_tiles(count, ni, n_halo);
   const auto &cbeg = numbers.cbeg, &ebeg = numbers.ebeg;
