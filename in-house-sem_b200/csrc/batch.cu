@@ -411,18 +411,18 @@ void Batch::enqueue_step(int32_t k, cudaEvent_t tiles_begin, cudaEvent_t tiles_e
   // halo points: solves of a two-component solid, of a three-component one,
   // of a fluid alone, side by side; then the fluids of split solves
   bool first_halo = true;
-  auto halo = [&](auto kernel, int cls, bool after) {
+  auto halo = [&](auto kernel, auto late_kernel, int cls, bool after) {
     if (n_halo_items[cls] == 0) return;
     const DepMode dep = after ? kDepAll : first_halo ? kDepFirst : kDepLate;
-    CUDA_CHECK(launch_chained(kernel, n_halo_items[cls], kHaloChunk, 0, stream, !first_halo || !tiles_end,
+    CUDA_CHECK(launch_chained(dep == kDepLate ? late_kernel : kernel, n_halo_items[cls], kHaloChunk, 0, stream, !first_halo || !tiles_end,
                               dhalo_segs[cls].get(), dhalo_items[cls].get(), StepIdx{k, 0, dep}));
     first_halo = false;
   };
-  halo(halo_batch_kernel<2>, 1, false);
-  halo(halo_batch_kernel<3>, 2, false);
-  halo(halo_batch_kernel<0>, 0, false);
-  halo(halo_batch_kernel<2>, 3, true);
-  halo(halo_batch_kernel<3>, 4, true);
+  halo(halo_batch_kernel<2, false>, halo_batch_kernel<2, true>, 1, false);
+  halo(halo_batch_kernel<3, false>, halo_batch_kernel<3, true>, 2, false);
+  halo(halo_batch_kernel<0, false>, halo_batch_kernel<0, true>, 0, false);
+  halo(halo_batch_kernel<2, false>, halo_batch_kernel<2, true>, 3, true);
+  halo(halo_batch_kernel<3, false>, halo_batch_kernel<3, true>, 4, true);
   if (n_energy > 0)
     CUDA_CHECK(launch_chained(energy_batch_kernel, n_energy, kReduceThreads, 0, stream, true, denergy.get(),
                               StepIdx{k, 0, kDepAll}));

@@ -250,12 +250,18 @@ inline int grid_for(int64_t n, int threads = 256) {
 // in an ordinary launch.  Every kernel of the chain waits at some point, so a
 // kernel's completion implies that of all kernels before it.
 //   kDepFirst  waits before it touches what the step before wrote, then
-//              triggers: the next kernels start after that point, so they may
-//              read all that came before this kernel without a wait of their own
+//              triggers: the next kernels start after that point, when all that
+//              came before this kernel has completed
 //   kDepAll    triggers at once, waits before it touches what the kernel
 //              before it wrote (constant data is read ahead of the wait)
 //   kDepLate   needs nothing of the kernel before it: triggers at once and
-//              waits only at its end
+//              waits only at its end.  It starts after the completion that the
+//              kDepFirst kernel waited for, but that is an order in time: only a
+//              wait of its own would make earlier writes visible in its SM's
+//              first-level cache.  What the launches of a sequence change it
+//              therefore reads from the second level (__ldcg), or by bulk copies;
+//              what was complete before the sequence's first launch (tables,
+//              amplitudes, step counters) it reads as constant
 // A small solve is bound by this chain, not by its bytes: with a full boundary
 // between kernels, the constrained gather and the receivers on the critical
 // path and a graph per step, a step of the cased borehole (3,600 order-4
@@ -274,6 +280,12 @@ __device__ __forceinline__ void dep_wait(int32_t dep) {
 }
 __device__ __forceinline__ void dep_end(int32_t dep) {
   if (dep == kDepLate) pdl_wait();
+}
+// What an earlier launch of the sequence wrote, as a kernel reads it that is (LATE) launched as kDepLate.
+template <bool LATE, class T>
+__device__ __forceinline__ T load_step(const T* p) {
+  if constexpr (LATE) return __ldcg(p);
+  else return *p;
 }
 
 // Launch of a kernel of a chain; `overlap`: with programmatic stream

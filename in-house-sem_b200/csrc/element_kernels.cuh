@@ -174,15 +174,17 @@ __global__ void __launch_bounds__(ElemCfg<NG, KIND, ELASTIC, M>::THREADS)
   dep_wait(dep);
   if (active) {
     if constexpr (SOURCE != kFieldLocal) {
+      const bool late = dep == kDepLate;
+      auto value = [late](const float* p) { return late ? __ldcg(p) : *p; };
       double f = 1.0;
-      if constexpr (SOURCE == kFieldScaled) f = *scale;
+      if constexpr (SOURCE == kFieldScaled) f = late ? __ldcg(scale) : *scale;
 #pragma unroll
       for (int c = 0; c < C::NC; ++c) {
         const float* g = u_in + static_cast<size_t>(c) * n_global;
         if constexpr (SOURCE == kFieldScaled)
-          sm.u[el][c][kpt] = gather_slot(slot, rows, [g, f](int32_t p) { return scaled(g[p], f); });
+          sm.u[el][c][kpt] = gather_slot(slot, rows, [g, f, value](int32_t p) { return scaled(value(g + p), f); });
         else
-          sm.u[el][c][kpt] = gather_slot(g, slot, rows);
+          sm.u[el][c][kpt] = gather_slot(slot, rows, [g, value](int32_t p) { return value(g + p); });
       }
     } else {
 #pragma unroll

@@ -259,7 +259,7 @@ __device__ __forceinline__ void warp_ordered_dots(const float* const (&coef)[N],
       const int32_t p = pts[q0 + lane];
 #pragma unroll
       for (int k = 0; k < N; ++k)
-        term[k] = dmul(static_cast<double>(coef[k][q0 + lane]), static_cast<double>(field[k][p]));
+        term[k] = dmul(static_cast<double>(coef[k][q0 + lane]), static_cast<double>(__ldcg(field[k] + p)));
     }
     for (int32_t q = 0; q < m; q += 8) {
 #pragma unroll
@@ -288,8 +288,8 @@ __device__ __forceinline__ void particle_velocity_body(const ReceiversDev& r, co
   double* pv = r.pv + static_cast<size_t>(rec) * 4;
   if (!init) {
     const double hdt = dmul(0.5, dt);
-    pv[2] = dadd(pv[2], dmul(hdt, dadd(pv[0], ax)));
-    pv[3] = dadd(pv[3], dmul(hdt, dadd(pv[1], az)));
+    pv[2] = dadd(__ldcg(pv + 2), dmul(hdt, dadd(__ldcg(pv), ax)));
+    pv[3] = dadd(__ldcg(pv + 3), dmul(hdt, dadd(__ldcg(pv + 1), az)));
   }
   pv[0] = ax;
   pv[1] = az;
@@ -314,7 +314,7 @@ __device__ __forceinline__ void record_body(const ReceiversDev& r, const AllFiel
   const RecordColumn col = cols[t];
   double out;
   if (col.field == 3) {
-    out = r.pv[static_cast<size_t>(col.receiver) * 4 + (col.mode == 3 ? 2 : 3)];
+    out = __ldcg(r.pv + static_cast<size_t>(col.receiver) * 4 + (col.mode == 3 ? 2 : 3));
   } else {
     const DomainFields& d = fl.d[r.domain[col.receiver]];
     const float* field = col.field == 0 ? d.u : col.field == 1 ? d.v : d.a;

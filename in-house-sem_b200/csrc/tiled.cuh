@@ -1029,7 +1029,7 @@ __device__ __forceinline__ HaloPoint halo_point(const TiledDev& td, const HaloDe
 // fluid's current pressure (solid domain) or the solid's new acceleration
 // (fluid domain), in that domain's device numbering.  CTAs of 256 threads,
 // `part` = the CTA's energy partial.
-template <int NC, bool ELASTIC>
+template <int NC, bool ELASTIC, bool LATE>
 __device__ __forceinline__ void halo_finish(const TiledDev& td, const float* u_cur, float* u_nxt, const HaloDev& hd,
                                             const HaloPoint& hp, const float* other, int32_t other_ng, bool pm,
                                             const float* __restrict__ amp, int32_t n_amp, const StepScalars& sc,
@@ -1047,14 +1047,16 @@ __device__ __forceinline__ void halo_finish(const TiledDev& td, const float* u_c
     float uc[NC], vc[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      uc[c] = u_cur[static_cast<size_t>(c) * td.ng + g];
-      vc[c] = glob(td.v)[static_cast<size_t>(c) * td.ng + g];
+      uc[c] = load_step<LATE>(u_cur + static_cast<size_t>(c) * td.ng + g);
+      vc[c] = load_step<LATE>(glob(td.v) + static_cast<size_t>(c) * td.ng + g);
     }
     const bool coupled = hp.r.cpl0 < hp.r.cpl1;
     float o[3] = {0.0f, 0.0f, 0.0f};
     auto partner = [&](int32_t gp) {
-      o[0] = other[gp];
-      if constexpr (!ELASTIC) {
+      if constexpr (ELASTIC) {
+        o[0] = load_step<LATE>(other + gp);
+      } else {  // written by this CTA, or by a launch this one has waited for
+        o[0] = other[gp];
         o[1] = other[static_cast<size_t>(other_ng) + gp];
         if (pm) o[2] = other[static_cast<size_t>(2) * other_ng + gp];
       }
@@ -1067,7 +1069,7 @@ __device__ __forceinline__ void halo_finish(const TiledDev& td, const float* u_c
 #pragma unroll
       for (int q = 0; q < K; ++q)
 #pragma unroll
-        for (int c = 0; c < NC; ++c) vq[c][q] = b + q < e ? glob(td.hbuf)[static_cast<size_t>(c) * td.n_hbuf + b + q] : 0.0f;
+        for (int c = 0; c < NC; ++c) vq[c][q] = b + q < e ? load_step<LATE>(glob(td.hbuf) + static_cast<size_t>(c) * td.n_hbuf + b + q) : 0.0f;
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         float s = 0.0f;
@@ -1081,7 +1083,7 @@ __device__ __forceinline__ void halo_finish(const TiledDev& td, const float* u_c
       for (int c = 0; c < NC; ++c) {
         float s = 0.0f;
         for (int32_t q = b; q < e; ++q) {
-          const float v = glob(td.hbuf)[static_cast<size_t>(c) * td.n_hbuf + q];
+          const float v = load_step<LATE>(glob(td.hbuf) + static_cast<size_t>(c) * td.n_hbuf + q);
           s = fadd(s, hd.w ? fmul(glob(hd.w)[q], v) : v);
         }
         f[c] = s;
@@ -1205,7 +1207,7 @@ struct HaloArgs {
 };
 // NC: the solid's components (0: no solid); odd: the views' field buffers are
 // exchanged (steps of odd parity).
-template <int NC>
+template <int NC, bool LATE>
 __device__ __forceinline__ void halo_block(const HaloArgs& A, bool odd, const StepNow& now, int32_t dep, int32_t block) {
   constexpr bool PM = NC == 3;
   constexpr int SC = NC == 0 ? 1 : NC;
@@ -1214,11 +1216,11 @@ __device__ __forceinline__ void halo_block(const HaloArgs& A, bool odd, const St
   float* s_nxt = glob(odd ? const_cast<float*>(A.s_td.u_cur) : A.s_td.u_nxt);
   float* f_nxt = glob(odd ? const_cast<float*>(A.f_td.u_cur) : A.f_td.u_nxt);
   auto solid = [&](const HaloPoint& p, int32_t part, int32_t h, bool in) {
-    halo_finish<SC, true>(A.s_td, s_cur, s_nxt, A.s_hd, p, f_cur, A.f_td.ng, PM, glob(A.amp), A.n_amp, A.sc, A.h_damp, A.st, now,
+    halo_finish<SC, true, LATE>(A.s_td, s_cur, s_nxt, A.s_hd, p, f_cur, A.f_td.ng, PM, glob(A.amp), A.n_amp, A.sc, A.h_damp, A.st, now,
                           A.epartial, A.ep_s + part, h, in);
   };
   auto fluid = [&](const HaloPoint& p, int32_t part, int32_t h, bool in) {
-    halo_finish<1, false>(A.f_td, f_cur, f_nxt, A.f_hd, p, glob(A.s_td.a), A.s_td.ng, PM, glob(A.amp), A.n_amp, A.sc, A.h_damp, A.st,
+    halo_finish<1, false, LATE>(A.f_td, f_cur, f_nxt, A.f_hd, p, glob(A.s_td.a), A.s_td.ng, PM, glob(A.amp), A.n_amp, A.sc, A.h_damp, A.st,
                           now, A.epartial, A.ep_f + part, h, in);
   };
   const int32_t t = threadIdx.x;
@@ -1255,7 +1257,7 @@ constexpr int kHaloRegs = NC == 3 ? 80 : NC == 2 ? 64 : 48;
 template <int NC>
 static __global__ void __maxnreg__(kHaloRegs<NC>) halo_step_kernel(const __grid_constant__ HaloArgs A, StepIdx ix) {
   dep_begin(ix.dep);
-  halo_block<NC>(A, false, step_now(A.st, ix), ix.dep, blockIdx.x);
+  halo_block<NC, false>(A, false, step_now(A.st, ix), ix.dep, blockIdx.x);
   dep_end(ix.dep);
 }
 
@@ -1316,8 +1318,8 @@ static __global__ void tiled_energy_kernel(const double* __restrict__ epartial, 
 // item (segment, chunk); the segment carries one solve's pointers and
 // scalars, the solve's StepState its step, mode and buffer parity.
 
-// A segment is one solve (its views at parity 0).
-template <int NC>
+// A segment is one solve (its views at parity 0).  LATE: launched as kDepLate.
+template <int NC, bool LATE>
 static __global__ void __maxnreg__(kHaloRegs<NC>) halo_batch_kernel(const HaloArgs* __restrict__ segs,
                                                                     const int2* __restrict__ items, StepIdx ix) {
   dep_begin(ix.dep);
@@ -1332,7 +1334,7 @@ static __global__ void __maxnreg__(kHaloRegs<NC>) halo_batch_kernel(const HaloAr
   if (now.mode == kModeIdle) {
     dep_wait(ix.dep);
   } else {
-    halo_block<NC>(A, (A.st->parity ^ ix.k) & 1, now, ix.dep, it.y);
+    halo_block<NC, LATE>(A, (A.st->parity ^ ix.k) & 1, now, ix.dep, it.y);
   }
   dep_end(ix.dep);
 }
