@@ -352,7 +352,7 @@ void Batch::launch_steps(int32_t n) {
     CUDA_CHECK(cudaStreamEndCapture(stream, &g));
     std::size_t nn = 0;
     CUDA_CHECK(cudaGraphGetNodes(g, nullptr, &nn));
-    kernels_per_step = static_cast<int32_t>(nn) / n;  // kernel nodes only
+    kernels_per_step = static_cast<int32_t>(nn - 1) / n;  // kernel nodes only; the last closes the sequence
     const cudaError_t e = cudaGraphInstantiate(&ge, g, 0);
     cudaGraphDestroy(g);
     CUDA_CHECK(e);

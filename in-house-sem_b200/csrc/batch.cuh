@@ -97,7 +97,7 @@ class Batch {
 
   insem_cuda_options opts{};
   double last_ms = 0.0;           // device time of the last advance()
-  int32_t kernels_per_step = 0;   // kernel nodes of the step graph
+  int32_t kernels_per_step = 0;   // launches of a step
   int64_t point_updates = 0;      // sum of points x steps of the last advance()
 
  private:

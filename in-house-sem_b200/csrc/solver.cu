@@ -1342,7 +1342,7 @@ cudaGraphExec_t Solver::tiled_graph(int par, int n) {
   if (kernels_per_step == 0) {
     std::size_t nn = 0;
     CUDA_CHECK(cudaGraphGetNodes(g, nullptr, &nn));
-    kernels_per_step = static_cast<int32_t>(nn) / n;  // kernel nodes only
+    kernels_per_step = static_cast<int32_t>(nn - 1) / n;  // kernel nodes only; the last closes the sequence
   }
   cudaGraphExec_t ge = nullptr;
   const cudaError_t e = cudaGraphInstantiate(&ge, g, 0);

@@ -340,7 +340,8 @@ int insem_cuda_solver_advance_streamed(insem_cuda_solver* h, int32_t n, const fl
                                        int32_t* n_rows);
 /* Columns of a recorded sample row (all traces side by side, in trace order). */
 int32_t insem_cuda_solver_n_columns(const insem_cuda_solver* h);
-/* Kernel launches of one captured step (the step graph's kernel nodes). */
+/* Kernel launches of one step, 0 before the first captured one (tiled path: the
+ * launch that closes a sequence of steps is not counted). */
 int32_t insem_cuda_solver_kernels_per_step(insem_cuda_solver* h);
 /* Elements per tile (one CTA) of the tiled path.  A solver takes
  * options.tile_elements when > 0, else the entry set here for its domain's
@@ -447,7 +448,8 @@ int32_t insem_cuda_batch_steps_to_completion(const insem_cuda_batch* h);
 /* Device time of the last advance / run segment, ms; points x steps it did. */
 double insem_cuda_batch_last_advance_ms(const insem_cuda_batch* h);
 int64_t insem_cuda_batch_point_updates(const insem_cuda_batch* h);
-/* Kernel nodes of the current batched-step graph. */
+/* Kernel launches of one batched step of the current composition (the launch
+ * that closes a sequence of steps is not counted). */
 int32_t insem_cuda_batch_kernels_per_step(const insem_cuda_batch* h);
 
 #ifdef __cplusplus
