@@ -29,8 +29,6 @@ void INSEM_CAT(set_constant_basis_ng, INSEM_NG)(const float* D, const float* Dj,
   CUDA_CHECK(cudaMemcpyToSymbol(c_neg_zero, &neg_zero, sizeof(float)));
 }
 
-int INSEM_CAT(tile_batch_ng, INSEM_NG)(const TileBatchLaunch& a, bool launch) {
-  return tile_batch_cfg<INSEM_NG>(a, launch);
-}
+void INSEM_CAT(tile_batch_ng, INSEM_NG)(const TileBatchLaunch& a, bool launch) { tile_batch_cfg<INSEM_NG>(a, launch); }
 
 }  // namespace insem_b200

@@ -125,19 +125,18 @@ int choose_tile_elements(int ngll, int kind, bool elastic, int m, int requested)
   return requested > 0 ? std::min(requested, kTileLanes) : kTileLanes;
 }
 
-int tile_batch(int ngll, const TileBatchLaunch& a, bool launch) {
+void tile_batch(int ngll, const TileBatchLaunch& a, bool launch) {
   switch (ngll) {
-    case 2: return tile_batch_ng2(a, launch);
-    case 3: return tile_batch_ng3(a, launch);
-    case 4: return tile_batch_ng4(a, launch);
-    case 5: return tile_batch_ng5(a, launch);
-    case 6: return tile_batch_ng6(a, launch);
-    case 7: return tile_batch_ng7(a, launch);
-    case 8: return tile_batch_ng8(a, launch);
-    case 9: return tile_batch_ng9(a, launch);
+    case 2: tile_batch_ng2(a, launch); break;
+    case 3: tile_batch_ng3(a, launch); break;
+    case 4: tile_batch_ng4(a, launch); break;
+    case 5: tile_batch_ng5(a, launch); break;
+    case 6: tile_batch_ng6(a, launch); break;
+    case 7: tile_batch_ng7(a, launch); break;
+    case 8: tile_batch_ng8(a, launch); break;
+    case 9: tile_batch_ng9(a, launch); break;
     default: check_ngll(ngll);
   }
-  return 0;
 }
 
 namespace {

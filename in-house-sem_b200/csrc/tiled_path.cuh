@@ -134,7 +134,6 @@ void launch_tiles_ng7(const TileLaunch&);
 void launch_tiles_ng8(const TileLaunch&);
 void launch_tiles_ng9(const TileLaunch&);
 void launch_tiles(int ngll, const TileLaunch& a);
-int tile_elements(int ngll);  // TileCfg<NG>::TE (the largest tile)
 // Elements per tile of a domain: `requested` if > 0, else a registered entry
 // (set_tile_elements, e.g. from the autotuner), at most the kernel's 32; by
 // default 32, which leaves no lane idle and the fewest points shared between
@@ -161,23 +160,23 @@ struct TileBatchLaunch {
 };
 // launch == false: opts the class kernel in to its dynamic shared memory
 // (outside stream capture); true: launches.
-int tile_batch_ng2(const TileBatchLaunch&, bool launch);
-int tile_batch_ng3(const TileBatchLaunch&, bool launch);
-int tile_batch_ng4(const TileBatchLaunch&, bool launch);
-int tile_batch_ng5(const TileBatchLaunch&, bool launch);
-int tile_batch_ng6(const TileBatchLaunch&, bool launch);
-int tile_batch_ng7(const TileBatchLaunch&, bool launch);
-int tile_batch_ng8(const TileBatchLaunch&, bool launch);
-int tile_batch_ng9(const TileBatchLaunch&, bool launch);
-int tile_batch(int ngll, const TileBatchLaunch& a, bool launch);
+void tile_batch_ng2(const TileBatchLaunch&, bool launch);
+void tile_batch_ng3(const TileBatchLaunch&, bool launch);
+void tile_batch_ng4(const TileBatchLaunch&, bool launch);
+void tile_batch_ng5(const TileBatchLaunch&, bool launch);
+void tile_batch_ng6(const TileBatchLaunch&, bool launch);
+void tile_batch_ng7(const TileBatchLaunch&, bool launch);
+void tile_batch_ng8(const TileBatchLaunch&, bool launch);
+void tile_batch_ng9(const TileBatchLaunch&, bool launch);
+void tile_batch(int ngll, const TileBatchLaunch& a, bool launch);
 
 template <int NG>
-int tile_batch_cfg(const TileBatchLaunch& a, bool launch) {
+void tile_batch_cfg(const TileBatchLaunch& a, bool launch) {
   INSEM_REQUIRE(a.smem <= 226u * 1024u, INSEM_CUDA_ERR_UNSUPPORTED, "tile needs too much shared memory");
-  auto go = [&](auto kernel) -> int {
+  auto go = [&](auto kernel) {
     if (!launch) {
       allow_shared_memory(kernel);
-      return 0;
+      return;
     }
     cudaError_t err = launch_chained(kernel, a.grid, TileCfg<NG>::THREADS, a.smem, a.stream, a.overlap, a.segs,
                                      a.items, a.ix, a.L);
@@ -186,7 +185,6 @@ int tile_batch_cfg(const TileBatchLaunch& a, bool launch) {
       throw Error(INSEM_CUDA_ERR_CUDA, "batched tile kernel launch (ngll " + std::to_string(NG) + ", kind " +
                                            std::to_string(a.kind) + ", grid " + std::to_string(a.grid) + ", smem " +
                                            std::to_string(a.smem) + "): " + cudaGetErrorString(err));
-    return 0;
   };
   if (a.kind == kAxisymOffAxis)
     return a.m == 1 ? go(tile_batch_kernel<NG, kAxisymOffAxis, true, 1>) : go(tile_batch_kernel<NG, kAxisymOffAxis, true, 0>);
