@@ -8,7 +8,7 @@
 //   3. the weak divergence per point (element_divergence), written to the
 //      element-local force array.
 // The launchers are compiled once per ngll (element_ng.cu with
-// INSEM_NG = 2..9) so the 160 instantiations build in parallel.
+// INSEM_NG = 2..9) so that the instantiations build in parallel.
 #pragma once
 
 #include "element_ops.cuh"
@@ -143,8 +143,11 @@ void launch_dofmap_cfg(const DofMapLaunch& a) {
   else go(assemble_kernel<NG, NC, false>, a.t_offsets, a.t_slots, a.t_weights, a.n, a.in, a.out);
 }
 
-// Where an element kernel takes its field from.
-enum FieldSource : int { kFieldLocal = 0, kFieldGlobal = 1, kFieldScaled = 2 };
+// Where an element kernel takes its field from.  The late sources are those of
+// launches without a wait of their own (kDepLate).  Chosen at run time, the loads
+// took the estimate of 9,216 order-4 elements from 4.32 to 4.38 ms; with kernels
+// of their own it stays at 4.21 (both sides of a later call).
+enum FieldSource : int { kFieldLocal = 0, kFieldGlobal = 1, kFieldScaled = 2, kFieldGlobalLate = 3, kFieldScaledLate = 4 };
 
 template <int NG, int KIND, bool ELASTIC, int M, int SOURCE>
 __global__ void __launch_bounds__(ElemCfg<NG, KIND, ELASTIC, M>::THREADS)
@@ -174,17 +177,16 @@ __global__ void __launch_bounds__(ElemCfg<NG, KIND, ELASTIC, M>::THREADS)
   dep_wait(dep);
   if (active) {
     if constexpr (SOURCE != kFieldLocal) {
-      const bool late = dep == kDepLate;
-      auto value = [late](const float* p) { return late ? __ldcg(p) : *p; };
+      constexpr bool LATE = SOURCE >= kFieldGlobalLate, SCALED = SOURCE == kFieldScaled || SOURCE == kFieldScaledLate;
       double f = 1.0;
-      if constexpr (SOURCE == kFieldScaled) f = late ? __ldcg(scale) : *scale;
+      if constexpr (SCALED) f = load_step<LATE>(scale);
 #pragma unroll
       for (int c = 0; c < C::NC; ++c) {
         const float* g = u_in + static_cast<size_t>(c) * n_global;
-        if constexpr (SOURCE == kFieldScaled)
-          sm.u[el][c][kpt] = gather_slot(slot, rows, [g, f, value](int32_t p) { return scaled(value(g + p), f); });
+        if constexpr (SCALED)
+          sm.u[el][c][kpt] = gather_slot(slot, rows, [g, f](int32_t p) { return scaled(load_step<LATE>(g + p), f); });
         else
-          sm.u[el][c][kpt] = gather_slot(slot, rows, [g, value](int32_t p) { return value(g + p); });
+          sm.u[el][c][kpt] = gather_slot(slot, rows, [g](int32_t p) { return load_step<LATE>(g + p); });
       }
     } else {
 #pragma unroll
@@ -246,6 +248,8 @@ void launch_element_cfg(const ElementLaunch& a) {
     CUDA_LAUNCH_CHECK();
   };
   if (!a.gather) go(element_forces_kernel<NG, KIND, ELASTIC, M, kFieldLocal>);
+  else if (a.dep == kDepLate && !a.scale) go(element_forces_kernel<NG, KIND, ELASTIC, M, kFieldGlobalLate>);
+  else if (a.dep == kDepLate) go(element_forces_kernel<NG, KIND, ELASTIC, M, kFieldScaledLate>);
   else if (!a.scale) go(element_forces_kernel<NG, KIND, ELASTIC, M, kFieldGlobal>);
   else go(element_forces_kernel<NG, KIND, ELASTIC, M, kFieldScaled>);
 }

@@ -48,13 +48,17 @@ float* scratch_on_current_device() {
 void Solver::prepare_noalloc() {
   scratch_on_current_device();
   for (const DeviceDomainData& d : domains) {
+    bool first = true;  // the kernel follows from the place among the blocks, as below
     for (const DeviceBlock& b : d.blocks) {
+      if (b.n == 0) continue;
       ElementLaunch a;
       a.blk = b.view();
       a.gather = true;
       a.elastic = d.medium == INSEM_ELASTIC;
+      a.dep = first ? kDepFirst : kDepLate;
       a.preload = true;
       launch_element_forces(ngll, a);
+      first = false;
     }
     launch_assemble(d.dofs, d.ncomp, nullptr, nullptr, nullptr, true);
   }
