@@ -16,9 +16,10 @@ value      device time (CUDA events) of K batched steps, every input resident
            in HBM; a batched step touches ~16 GB, far more than L2.
 plain      the same models with the plain one-solve-per-launch path (each
            solve's own step graph, solves one after another), device time.
-e2e        the same metric through the C ABI's streamed batched steps: every
-           step copies all models' source amplitudes in from pinned host
-           memory and all models' sample rows back, wall clock.
+e2e        the same metric through the C ABI's streamed batched steps: all
+           models' source amplitudes of every step are copied in from pinned
+           host memory and all models' sample rows back (by the library, once
+           per eight steps), wall clock.
 roofline   HBM roofline of the tile kernels (the dominant launches): their
            algorithmic bytes per batched step (element terms + points finished
            in tiles, the fixed B_step formula split by point class) over their

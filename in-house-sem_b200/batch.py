@@ -112,9 +112,9 @@ class Batch:
 
     def advance_streamed(self, n_steps: int, amplitudes, rows_out=None) -> int:
         """n_steps batched steps (fewer if every member ends sooner) with
-        per-step host I/O: ``amplitudes`` [n_steps, amp_cols] float32 in (None:
-        the members' own source time functions), ``rows_out`` [n_steps,
-        row_cols] float64 out (numpy arrays or pinned torch tensors).  A member
+        ``amplitudes`` [n_steps, amp_cols] float32 in (None: the members' own
+        source time functions) and ``rows_out`` [n_steps, row_cols] float64 out
+        (numpy arrays or pinned torch tensors), copied once per eight steps.  A member
         with r steps left has valid rows for its first r steps.  Returns the
         steps done."""
         def ptr(x, ctype):

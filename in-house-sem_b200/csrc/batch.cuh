@@ -2,21 +2,21 @@
 // geometry kind, medium and azimuthal order advance together, one step of
 // every unfinished solve per batched step.
 //
-// A batched step is one CUDA graph of a fixed number of launches whatever
-// the number of solves:
+// A batched step is a fixed number of launches whatever the number of solves,
+// replayed from CUDA graphs of kSequence steps or of one:
 //   one tile launch per tile class (ngll, kind, medium, order): one CTA
 //     per (segment, tile) item
 //   halo points of every solve, by the solid's component count
 //   receivers (particle velocity, then recording) and energy of every solve
-//   step counters and buffer parities
+//   step counters and buffer parities (once per sequence)
 // The launches form one chain in which a launch may start before the one
-// ahead of it has ended (DepMode in step_kernels.cuh): the tile classes fill
+// ahead of it has ended (DepMode in common.cuh): the tile classes fill
 // the chip one behind the other without waiting for each other's last tiles.
 // Each solve keeps its own device data, time step, parity and step count,
 // so its results are the ones it gets alone, bit for bit.  Solves that
 // reach their last step run it in final mode and idle (every batched kernel
 // skips them) until the tables are rebuilt without them: membership changes
-// re-capture the graph at the next advance.
+// re-capture the graphs at the next advance.
 #pragma once
 
 #include <map>
@@ -28,7 +28,7 @@
 namespace insem_b200 {
 
 // Streamed batched steps: where each solve's amplitudes and sample columns sit
-// in the per-step host rows.
+// in a step's host row.
 struct StreamSeg {
   float* src_amp;        // [n_sources][n_amp] amplitude table of the solve
   int32_t n_amp, n_sources, amp_off;
@@ -77,7 +77,8 @@ class Batch {
   void advance(int32_t n);
   // Steps until every solve is complete.
   void run();
-  // n steps (fewer if every solve ends sooner) with per-step host I/O:
+  // n steps (fewer if every solve ends sooner) with amplitudes in and sample
+  // rows out, one copy each way per sequence of steps (kSequence, else 1):
   // amp_in[step][amp_cols] are the active solves' source amplitudes (in index
   // order, each solve's sources in order), rows_out[step][row_cols] their
   // latest sample rows.  Returns the steps done.

@@ -1229,10 +1229,11 @@ AllFields Solver::tiled_fields(int par) {
 
 // n steps of the tiled path from the field buffers of `par` on (init: step 0,
 // explicit damping, no step count), as one chain of launches on the stream
-// (see DepMode).  A step's critical path is tiles -> halo points.  The fluid's tiles run beside the solid's, and a step's receivers
-// beside the next step's tiles: they read halo points only, which the next
-// step's halo kernels overwrite, not its tiles.   The first
-// kernel of a sequence keeps a full boundary to what is ahead of it.
+// (see DepMode).  A step's critical path is tiles -> halo points.  The fluid's
+// tiles run beside the solid's, and a step's receivers beside the next step's
+// tiles: they read halo points only, which the next step's halo kernels
+// overwrite, not its tiles.  The first kernel of a sequence keeps a full
+// boundary to what is ahead of it.
 void Solver::enqueue_tiled(int par0, bool init, int n) {
   const StepScalars sc{static_cast<float>(dt), static_cast<float>(0.5 * dt), static_cast<float>(0.5 * dt * dt),
                        energy_every};
@@ -1361,8 +1362,9 @@ void Solver::tiled_initialize() {
   initialized = true;
 }
 
-// advance(n) on the tiled path; with rows_out, the streamed variant (amplitudes
-// in, recorded rows out, per step).
+// advance(n) on the tiled path; with amp_in or rows_out, the streamed variant:
+// the steps' amplitudes copied in ahead of the first, their recorded rows out
+// after the last.
 void Solver::advance_tiled(int32_t n, const float* amp_in, double* rows_out, int32_t* n_rows) {
   const bool streamed = rows_out != nullptr || amp_in != nullptr;
   CUDA_CHECK(cudaEventRecord(ev0, stream));

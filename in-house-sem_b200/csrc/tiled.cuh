@@ -21,9 +21,12 @@
 // computes column i (points i, NG + i, ...) of the tile's up to 32 elements.
 // All data of a tile lie element-minor, [...][32], so every access of a warp
 // to shared memory is free of bank conflicts and every access to global
-// memory is coalesced, and the warps of inner columns finish their inner
-// points (56 - 69 % of a tile's points at NG 5 - 7) in registers: field and
-// velocity come straight from global memory, nothing is staged or listed.
+// memory is 32 adjacent values, and the warps of inner columns finish their
+// inner points (56 - 69 % of a tile's points at NG 5 - 7) in registers: field
+// and velocity come straight from global memory, nothing is staged or listed.
+// (A row of the first component is one 128-byte line; components follow at a
+// stride of a multiple of 4 points, so a row of the others starts on any
+// 16-byte boundary and may touch two lines.)
 // The elements' data arrive in one bulk copy; D entries indexed by the
 // unrolled loop counters come from the constant bank.  Every sum keeps the
 // reference's operand order.
@@ -242,9 +245,9 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 constexpr uint32_t kBulkWaitLimit = 1u << 22;
 
 // Whether a class with staged element data keeps its f_xi rows outside it: no
-// class does.  A point's element data are read by one thread only, which
-// writes its f_xi over them: pairs of components over (xi_x, xi_z), the only or
-// third component over the last plane.
+// class does (the host check of the layout asks).  A point's element data are
+// read by one thread only, which writes its f_xi over them: pairs of components
+// over the first pairs, the only or third component over the last plane.
 __host__ __device__ constexpr bool early_flux_rows(int, int) { return false; }
 
 // Shared-memory layout of one tile CTA, byte offsets (16-byte aligned).
@@ -296,7 +299,7 @@ struct TileLayout {
     // axis terms (gx, gy of up to two components) [4][ng][32], ng rounded up to
     // 4; last, for launches without axial elements leave them out
     L.ax = o;
-      if (axi) o += 4u * 4u * ((ng + 3) & ~3) * kTileLanes;
+    if (axi) o += 4u * 4u * ((ng + 3) & ~3) * kTileLanes;
     L.total = o;
     (void)elastic;
     return L;
@@ -856,6 +859,10 @@ __device__ __forceinline__ bool tile_step_body(const BlockDev& blk, const TiledD
 // about as many CTAs, and 4 or 5 (128 or 96) at NG 8 and 9.  A step of 12
 // boreholes of NG 6 and 7 took 444 us with the compiler's own choice (up to 164
 // registers, 1 - 2 CTAs of the three-component classes) and 336 with this.
+// Compared with one warp more or fewer are the separable elastic classes of NG
+// 6 and 7 (kAxisymSeparable above) and, with 9 and 10 for 8, the curved elastic
+// ones of NG 6 (147k elements 70.4 us a step for 65.4); the other entries follow
+// the same rule without a comparison of their own.
 template <int NG, int KIND, bool EL, int M>
 constexpr int tile_min_ctas() {
   const int sep = NG >= 8 ? 5 : M == 1 ? 7 : NG == 7 ? 9 : 8;

@@ -153,7 +153,9 @@ class ProblemData:
         sum_domains n_g (16 ncomp + 4) + sum_elements [4 npe + metric(kind) + coef],
         metric Rect 12, Affine 20, Curved 20 npe, Axisym 28 npe (xi_r, xi_z,
         eta_r, eta_z, wr, hoop, r: the axisymmetric fluxes use the Jacobian only
-        through wr); coef elastic 8 npe, acoustic 4 npe."""
+        through wr); coef elastic 8 npe, acoustic 4 npe.  A fixed formula: the
+        tiled path reads one material per element, and of axisymmetric elements
+        that are rectangles about 12 npe."""
         npe = self.ngll * self.ngll
         total = 0
         for d in self.domains:

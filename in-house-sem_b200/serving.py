@@ -7,8 +7,9 @@ Requests arrive as a Poisson stream. Each one goes through these stages:
    request.
 3. Batched stepping: the batch advances in short chunks of batched steps.
    Between chunks, newly set-up requests join and completed ones leave.
-4. Streaming: every step streams all active requests' sample rows back to
-   the host, so a request's traces are on the host when its last step ends.
+4. Streaming: all active requests' sample rows of every step stream back to
+   the host, one copy per eight steps (per step at the end of a chunk), so a
+   request's traces are on the host when the chunk of its last step ends.
    Each request's fields, sources (their time-function tables) and receivers
    stay resident on the device.
 

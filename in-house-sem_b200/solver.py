@@ -102,8 +102,9 @@ class Solver:
         N.check(N.lib().insem_cuda_solver_prepare_for_batch(self._h))
 
     def advance_streamed(self, n_steps: int, amplitudes: np.ndarray, rows_out: np.ndarray) -> int:
-        """n steps with per-step source amplitudes in ([n][n_sources] float32, host) and
-        the recorded rows out ([>= n / record_every][n_columns] float64, host)."""
+        """n steps with their source amplitudes in ([n][n_sources] float32, host) and
+        the recorded rows out ([>= n / record_every][n_columns] float64, host),
+        one copy each per call."""
         assert amplitudes.dtype == np.float32 and amplitudes.flags.c_contiguous
         assert rows_out.dtype == np.float64 and rows_out.flags.c_contiguous
         n = C.c_int32()

@@ -330,12 +330,15 @@ int insem_cuda_solver_state(insem_cuda_solver* h, int32_t domain, double* u, dou
 double insem_cuda_solver_last_advance_ms(const insem_cuda_solver* h);
 /* Internal forces f = -K u of a domain for a host field (Solver::internal_forces). */
 int insem_cuda_solver_internal_forces(insem_cuda_solver* h, int32_t domain, const float* u, float* f);
-/* Streamed advance: n steps where every step first copies that step's source
- * amplitudes amp_in[s * n_sources + k] (host, pinned for best speed) to the
- * device and, on record steps, copies the recorded sample row back to
- * rows_out[r * n_columns ...] (host); *n_rows receives the rows written.
- * Amplitudes given here replace the ones computed from the source time
- * functions for those steps.  One synchronisation at the end. */
+/* Streamed advance: n steps with their source amplitudes
+ * amp_in[s * n_sources + k] (host, pinned for best speed) in and the sample
+ * rows recorded by them out, to rows_out[r * n_columns ...] (host); *n_rows
+ * receives the rows written.  The amplitudes of all n steps are copied to the
+ * device before the first of them, and the rows back after the last, so amp_in
+ * must be complete at the call and rows_out is written at its end: a caller
+ * that wants rows sooner calls with fewer steps.  Amplitudes given here replace
+ * the ones computed from the source time functions for those steps.  One
+ * synchronisation at the end. */
 int insem_cuda_solver_advance_streamed(insem_cuda_solver* h, int32_t n, const float* amp_in, double* rows_out,
                                        int32_t* n_rows);
 /* Columns of a recorded sample row (all traces side by side, in trace order). */
@@ -347,9 +350,11 @@ int32_t insem_cuda_solver_kernels_per_step(insem_cuda_solver* h);
  * options.tile_elements when > 0, else the entry set here for its domain's
  * class (ngll, dominant geometry kind, medium, azimuthal order), else 32, a
  * full tile; at most 32, and 32 in a domain of more than 2^22 points (smaller
- * tiles are padded to 32 elements).  The autotuner (insem_b200.autotune) times
- * candidates and sets the entries; tile_elements <= 0 clears one.  Applies to
- * solvers created afterwards; process-wide. */
+ * tiles are padded to 32 elements).  A domain whose points with that padding
+ * exceed 2^31 - 1 is refused with INSEM_CUDA_ERR_UNSUPPORTED (path 1 takes it).
+ * The autotuner (insem_b200.autotune) times candidates and sets the entries;
+ * tile_elements <= 0 clears one.  Applies to solvers created afterwards;
+ * process-wide. */
 int insem_cuda_set_tile_elements(int32_t ngll, int32_t kind, int32_t medium, int32_t azimuthal_order,
                                  int32_t tile_elements);
 /* The choice a new solver would make for that class (ncomp: field components). */
@@ -376,8 +381,8 @@ int32_t insem_cuda_solver_tile_elements(const insem_cuda_solver* h, int32_t doma
  *   - Each call looks up the array's device address on the current device
  *     (a host-side lookup, nothing cached).
  *   - All calls share the array: calls whose work overlaps on the GPU (other
- *     streams, other threads, other handles) race on it.  Each call clears
- *     the part it uses before use. */
+ *     streams, other threads, other handles) race on it.  Each call writes the
+ *     part it uses before use. */
 int insem_cuda_solver_internal_forces_noalloc(insem_cuda_solver* h, int32_t domain, const float* u, float* f,
                                               void* stream);
 /* Points of a domain finished inside their tile's kernel and by the halo
@@ -392,10 +397,10 @@ int insem_cuda_stable_dt(const insem_cuda_problem* problem, int32_t device, doub
 
 /* ---------------------------------------------------------- batched solves */
 /* Many independent solves (models, shots) of any ngll, geometry kind, medium
- * and azimuthal order, advanced together: every batched step is one CUDA
- * graph of a fixed number of launches (one tile launch per tile class, its
- * CTAs fed by a device work queue, then the point-wise kernels of all
- * solves).  Each solve keeps its own time step and step count and gets the
+ * and azimuthal order, advanced together: a batched step is a fixed number of
+ * launches (one tile launch per tile class, one CTA per work item, then the
+ * point-wise kernels of all solves), replayed from CUDA graphs of eight steps
+ * or one.  Each solve keeps its own time step and step count and gets the
  * results it gets alone, bit for bit.  The reference has no batch API; its
  * nearest form is one Simulation per thread (bindings.cpp:336-337).
  * Members are insem_cuda_solver handles owned by the batch: read them with
@@ -429,8 +434,10 @@ insem_cuda_solver* insem_cuda_batch_member(insem_cuda_batch* h, int32_t index);
  * the call
  * (index order, each member's sources in order, FP32 as the reference casts
  * them), and writes rows_out[step][row_cols], each active member's latest
- * sample row (its columns as insem_cuda_solver_n_columns lays them out); one
- * host-to-device and one device-to-host copy per step.  amp_in NULL: the
+ * sample row (its columns as insem_cuda_solver_n_columns lays them out).  One
+ * host-to-device and one device-to-host copy per eight steps (per step for
+ * what is left of n), ahead of and behind them: amp_in must be complete at the
+ * call.  amp_in NULL: the
  * solves' own source time functions (resident tables); rows_out may be NULL. */
 int insem_cuda_batch_advance_streamed(insem_cuda_batch* h, int32_t n, const float* amp_in, double* rows_out,
                                       int32_t* n_done);
