@@ -223,11 +223,10 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
   npe = ngll * ngll;
   n_elements = d.dofs.n_elements;
   const std::size_t n_slots = static_cast<std::size_t>(n_elements) * npe;
-  const auto l2g = host_vec(d.dofs.l2g, n_slots);
-  const auto t_off = host_vec(d.dofs.t_offsets, static_cast<std::size_t>(ng) + 1);
-  const auto t_slots = host_vec(d.dofs.t_slots, static_cast<std::size_t>(t_off.back()));
+  // the maps are read where they are: the domain's upload has checked them
+  const int32_t *l2g = d.dofs.l2g, *t_off = d.dofs.t_offsets, *t_slots = d.dofs.t_slots;
   weighted = d.dofs.n_rows > 0 && d.dofs.t_weights != nullptr;
-  const auto t_w = weighted ? host_vec(d.dofs.t_weights, static_cast<std::size_t>(t_off.back())) : std::vector<double>{};
+  const double* t_w = d.dofs.t_weights;
 
   // special points
   std::vector<char> special(ng, 0);
@@ -264,6 +263,7 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
       tile_elems.emplace_back();
       tile_block.push_back(b);
       auto& te_list = tile_elems.back();
+      te_list.reserve(te);
       queue.clear();
       queue.push_back(seed);
       stamp[seed] = t;
@@ -458,6 +458,8 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
   std::vector<HaloRec> recs;
   std::vector<float> hw, scoef;
   cpl_entry.clear();
+  hoff.reserve(static_cast<std::size_t>(n_halo) + 1);
+  hpos.reserve(n_entries);
   std::vector<int32_t> halo_orig(n_halo);
   for (int32_t g = 0; g < ng; ++g)
     if (owner[g] < 0) halo_orig[perm[g] - n_complete] = g;
@@ -497,17 +499,17 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
   for (int32_t e : hpos) ++ecount[e];
   std::vector<int32_t> hdst(n_entries, 0), moff{0}, mlist;
   {
-    std::vector<std::vector<int32_t>> multi(n_entries);
-    for (int32_t q = 0; q < n_hbuf; ++q) {
-      const int32_t e = hpos[q];
-      if (ecount[e] == 1) hdst[e] = q;
-      else multi[e].push_back(q);
-    }
     for (int32_t e = 0; e < n_entries; ++e) {
       if (ecount[e] == 1) continue;
       hdst[e] = -1 - (static_cast<int32_t>(moff.size()) - 1);
-      mlist.insert(mlist.end(), multi[e].begin(), multi[e].end());
-      moff.push_back(static_cast<int32_t>(mlist.size()));
+      moff.push_back(moff.back() + ecount[e]);
+    }
+    mlist.resize(moff.back());
+    std::vector<int32_t> fill(moff.begin(), moff.end() - 1);
+    for (int32_t q = 0; q < n_hbuf; ++q) {
+      const int32_t e = hpos[q];
+      if (ecount[e] == 1) hdst[e] = q;
+      else mlist[fill[-1 - hdst[e]]++] = q;
     }
   }
 
@@ -546,12 +548,11 @@ void TiledDomain::build(const insem_cuda_domain& d, int ngll, int te, const Spec
     rows_w.upload(rw.empty() ? std::vector<float>{0.0f} : std::vector<float>(rw.begin(), rw.end()));
   }
   // mass in device numbering
-  const auto mh = host_vec(d.mass, ng), imh = host_vec(d.inv_mass, ng);
   host_mass.assign(ng_dev, 0.0f);
   std::vector<float> im(ng_dev, 0.0f);
   for (int32_t g = 0; g < ng; ++g) {
-    host_mass[perm[g]] = mh[g];
-    im[perm[g]] = imh[g];
+    host_mass[perm[g]] = d.mass[g];
+    im[perm[g]] = d.inv_mass[g];
   }
   mass.upload(host_mass);
   inv_mass.upload(im);
