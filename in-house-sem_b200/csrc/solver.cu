@@ -720,29 +720,26 @@ void Solver::set_state(int32_t medium, const double* u_in, const double* v_in) {
     if (domains[i].medium == medium) di = static_cast<int>(i);
   INSEM_REQUIRE(di >= 0, INSEM_CUDA_ERR_INVALID, "the model has no such medium");
   auto& d = domains[di];
-  const std::size_t n = static_cast<std::size_t>(d.ncomp) * d.ng;
   INSEM_REQUIRE(u_in && v_in, INSEM_CUDA_ERR_INVALID, "null state array");
-  std::vector<float> fu(n), fv(n);
-  for (std::size_t i = 0; i < n; ++i) {
-    fu[i] = static_cast<float>(u_in[i]);
-    fv[i] = static_cast<float>(v_in[i]);
-  }
-  for (int64_t z : d.host_zero) fu[z] = fv[z] = 0.0f;
-  if (!tiled) {
-    CUDA_CHECK(cudaMemcpy(d.u.get(), fu.data(), n * sizeof(float), cudaMemcpyHostToDevice));
-    CUDA_CHECK(cudaMemcpy(d.v.get(), fv.data(), n * sizeof(float), cudaMemcpyHostToDevice));
-  } else {
-    TiledDomain& t = tdom[di];
-    const std::size_t nd = static_cast<std::size_t>(d.ncomp) * t.ng;
-    std::vector<float> pu(nd, 0.0f), pv(nd, 0.0f);
-    for (int c = 0; c < d.ncomp; ++c)
-      for (int32_t g = 0; g < d.ng; ++g) {
-        pu[static_cast<std::size_t>(c) * t.ng + t.perm[g]] = fu[static_cast<std::size_t>(c) * d.ng + g];
-        pv[static_cast<std::size_t>(c) * t.ng + t.perm[g]] = fv[static_cast<std::size_t>(c) * d.ng + g];
-      }
-    CUDA_CHECK(cudaMemcpy(t.u_cur(parity), pu.data(), nd * sizeof(float), cudaMemcpyHostToDevice));
-    CUDA_CHECK(cudaMemcpy(t.v.get(), pv.data(), nd * sizeof(float), cudaMemcpyHostToDevice));
-  }
+  // rounded to float at the points' places on the device, zero where held
+  const int32_t* perm = tiled ? tdom[di].perm.data() : nullptr;
+  const int32_t stride = tiled ? tdom[di].ng : d.ng;
+  const std::size_t nd = static_cast<std::size_t>(d.ncomp) * stride;
+  auto copy = [&](const double* in, float* out) {
+    std::vector<float> h(nd, 0.0f);
+    for (int c = 0; c < d.ncomp; ++c) {
+      const double* x = in + static_cast<std::size_t>(c) * d.ng;
+      float* o = h.data() + static_cast<std::size_t>(c) * stride;
+      for (int32_t g = 0; g < d.ng; ++g) o[perm ? perm[g] : g] = static_cast<float>(x[g]);
+    }
+    for (int64_t z : d.host_zero) {
+      const int32_t g = static_cast<int32_t>(z % d.ng);
+      h[static_cast<std::size_t>(z / d.ng) * stride + (perm ? perm[g] : g)] = 0.0f;
+    }
+    CUDA_CHECK(cudaMemcpy(out, h.data(), nd * sizeof(float), cudaMemcpyHostToDevice));
+  };
+  copy(u_in, tiled ? tdom[di].u_cur(parity) : d.u.get());
+  copy(v_in, tiled ? tdom[di].v.get() : d.v.get());
   // a copy from pageable memory may return before its DMA has landed; the
   // readers run on the solver's non-blocking stream
   CUDA_CHECK(cudaStreamSynchronize(nullptr));
